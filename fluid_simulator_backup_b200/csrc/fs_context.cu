@@ -92,6 +92,12 @@ struct fs_ctx {
   double* rb_x = nullptr;          // black FP64 iterate
   float *rb_r = nullptr, *rb_p = nullptr, *rb_q = nullptr, *rb_tau = nullptr;
   unsigned short* rb_dinv = nullptr;  // black bf16 1/diag
+  // multigrid-preconditioned FP32 pressure solve (fs_multigrid.cu); level 0
+  // shares the couplings above and the red-black vectors
+  Multigrid mg;
+  MgState *mgst = nullptr, *mgst_host = nullptr;  // device, pinned
+  cudaGraphExec_t mg_graph = nullptr;
+  int mg_launches[3] = {0, 0, 0};  // kernels of its start, of one iteration, of its end
   PipeGeom pipe{};  // the oil/water pipe's geometry (pipe.on = 0: the box)
   void* pgen[3] = {nullptr, nullptr, nullptr};  // pipe: masked periodic velocity copies
   void* pgx[3] = {nullptr, nullptr, nullptr};   // pipe: their ENO3-guarded copies along x
@@ -138,6 +144,7 @@ struct fs_ctx {
   int flux32 = 2;               // params.flux_arithmetic (Op7::flux32)
   int lean = 1;                 // FP32 pressure solve preconditioned by the bf16 inverse diagonal (Op7::dinv16)
   bool red_black = false;       // FP32 pressure solve on the red-black Schur complement
+  bool multigrid = false;       // FP32 pressure solve preconditioned by the multigrid cycle
   bool rb_ic0 = true;           // its preconditioner: 1/diag(S) (IC(0) in red-black order), else the black 1/diag
   int adj_unconverged = 0;      // adjoint solves of the current call that stopped before their tolerance
   double adj_worst_rel = 0.0;   // and the worst relative residual they reached
@@ -178,15 +185,71 @@ fs_status dalloc(fs_ctx* c, void** out, size_t bytes) {
   return FS_OK;
 }
 
-void release(fs_ctx* c) {
-  if (!c) return;
+// The multigrid hierarchy of an FP32 box context.
+fs_status mg_alloc(fs_ctx* c) {
+  Multigrid& M = c->mg;
+  int ext[kMgMaxLevels][3];
+  M.levels = mg_plan(c->grid.nx, c->grid.ny, c->grid.nz, ext, &M.top);
+  for (int l = 0; l < M.levels; ++l) {
+    MgLevel& m = M.level[l];
+    m.L = make_lay(ext[l][0], ext[l][1], ext[l][2]);
+    m.H = make_half_lay(m.L);
+    if (l == 0) {
+      m.ax = (float*)c->pax;
+      m.ay = (float*)c->pay;
+      m.az = (float*)c->paz;
+      m.b[0] = c->rb_p;
+      m.b[1] = c->rb_r;
+      m.x[0] = c->rb_tau;
+      m.x[1] = c->rb_q;
+    }
+  }
+  // everything else in one allocation, each array 256-byte aligned: first
+  // its size, then the pointers
+  char* base = nullptr;
+  for (int pass = 0; pass < 2; ++pass) {
+    size_t off = 0;
+    auto take = [&](void** p, size_t bytes) {
+      if (pass) *p = base + off;
+      off += (bytes + 255) / 256 * 256;
+    };
+    for (int l = 0; l < M.levels; ++l) {
+      MgLevel& m = M.level[l];
+      if (l > 0) {
+        for (float** p : {&m.ax, &m.ay, &m.az}) take((void**)p, m.L.total * sizeof(float));
+        if (l <= M.top)
+          for (float** p : {&m.x[0], &m.x[1], &m.b[0], &m.b[1]}) take((void**)p, m.H.total * sizeof(float));
+      }
+      if (l < M.top)
+        for (unsigned char** p : {&m.cls[0], &m.cls[1]}) take((void**)p, m.H.total);
+    }
+    if (!pass) CKS(dalloc(c, (void**)&base, off));
+  }
+  CKS(dalloc(c, (void**)&c->mgst, sizeof(MgState)));
+  if (cudaMallocHost((void**)&c->mgst_host, sizeof(MgState)) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("pinned host allocation failed");
+    return FS_OOM;
+  }
+  return FS_OK;
+}
+
+void drop_graphs(fs_ctx* c) {
   for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
   c->graphs.clear();
+  if (c->mg_graph) cudaGraphExecDestroy(c->mg_graph);
+  c->mg_graph = nullptr;
+}
+
+void release(fs_ctx* c) {
+  if (!c) return;
+  drop_graphs(c);
   for (auto& b : c->owned) cudaFree(b.p);
   c->owned.clear();
   c->mesh.release();
   if (c->st_host) cudaFreeHost(c->st_host);
   if (c->sc_host) cudaFreeHost(c->sc_host);
+  if (c->mgst_host) cudaFreeHost(c->mgst_host);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->evp0) cudaEventDestroy(c->evp0);
   if (c->evp1) cudaEventDestroy(c->evp1);
@@ -271,14 +334,26 @@ void apply_params(fs_ctx* c) {
   c->reliable_delta = p.reliable_delta > 0.0 ? p.reliable_delta : 0.1;
   c->flux32 = p.flux_arithmetic;
   c->lean = p.pressure_preconditioner != FS_PRECOND_JACOBI;
-  // FP32_REFINE: the default is red-black IC(0), which halves the
-  // iterations of the Jacobi-PCG (FP64 keeps the reference's Jacobi); the
-  // pipe mode's default is the bf16 Jacobi (its red cells would need the
-  // pipe's Neumann cells in the FP64 elimination)
+  // FP32_REFINE: red-black IC(0) halves the iterations of the Jacobi-PCG
+  // (FP64 keeps the reference's Jacobi); the pipe mode's default is the bf16
+  // Jacobi (its red cells would need the pipe's Neumann cells in the FP64
+  // elimination)
   c->red_black = c->fp32 && !p.pipe && (p.pressure_preconditioner == FS_PRECOND_DEFAULT ||
                               p.pressure_preconditioner == FS_PRECOND_RED_BLACK ||
                               p.pressure_preconditioner == FS_PRECOND_RED_BLACK_JACOBI);
   c->rb_ic0 = p.pressure_preconditioner != FS_PRECOND_RED_BLACK_JACOBI;
+  // The default of the corrected box projection: CG preconditioned by one
+  // multigrid cycle, on the singular system.  The faithful projection keeps
+  // the red-black solve (its deflated matrix is not singular, which the cycle
+  // assumes), as does a solve the cycle gives up on.
+  c->multigrid = c->red_black && p.pressure_preconditioner == FS_PRECOND_DEFAULT &&
+                 !(p.flags & FS_FLAG_FAITHFUL_PROJECTION);
+  const double inv2 = 1.0 / (c->grid.dx * c->grid.dx);
+  for (int l = 0; l < c->mg.levels; ++l) {
+    // each level's uniform coupling is twice the finer one's
+    c->mg.level[l].a[0] = (float)(1.0 / p.rho_neg * inv2) * (float)(1 << l);
+    c->mg.level[l].a[1] = (float)(1.0 / p.rho_pos * inv2) * (float)(1 << l);
+  }
 }
 
 // The pressure system keeps the reference's deflation of the first cell only
@@ -726,20 +801,157 @@ fs_status viscosity_t(fs_ctx* c, double dt, int* iters_out) {
   return FS_OK;
 }
 
+// The multigrid-preconditioned solve of A(phi) x = b in the same precisions
+// as mixed_solve below, as ONE graph launch: the operator's set-up, the first
+// cycle, a conditional while node whose body is one iteration, and the shift
+// of the result's constant.  The operands that change between calls are in
+// the device state, so one graph serves them all.  *st is PCG_STAGNATED when
+// the cycle gave up (x is then the best usable iterate).
+template <class S>
+fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int* outer_out, double* rel_out,
+                   int* st_out) {
+  const fs_params& P = c->prm;
+  const double dx = c->grid.dx;
+  cudaStream_t s = c->stream;
+  MgState init{};
+  init.phi = phi;
+  init.x = x;
+  init.b = b;
+  init.bak = c->p64bak;
+  init.bb_src = c->scalars + 1;
+  init.tol = P.tolerance;
+  init.delta = c->reliable_delta;
+  init.max_iter = P.max_iteration;
+  *c->mgst_host = init;
+  float *p = (float*)c->pp, *q = (float*)c->pq;
+  const RbOp R{(float*)c->pax, (float*)c->pay, (float*)c->paz, c->Lc, c->Lh, c->scalars + 12};
+  auto start = [&]() {
+    int n = mg_build<S>(c->mg, c->mgst, dx, P.rho_neg, P.rho_pos, c->scalars + 12, s);
+    rb_schur_dinv(R, c->rb_dinv, s);
+    mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, false, s);
+    return n + 2 + mg_start<S>(c->mg, p, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, s);
+  };
+  auto finish = [&]() {
+    mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, s);
+    return 2;
+  };
+  CK(cudaMemcpyAsync(c->mgst, c->mgst_host, sizeof(MgState), cudaMemcpyHostToDevice, s));
+  CK(cudaEventRecord(c->evp0, s));
+  if (c->prm.host_loop) {
+    int n = start();
+    CK(cudaMemcpyAsync(c->mgst_host, c->mgst, sizeof(MgState), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    int done = 0;
+    while (!c->mgst_host->done && done <= P.max_iteration) {
+      n += mg_iteration<S>(c->mg, p, q, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, false,
+                           cudaGraphConditionalHandle{}, s);
+      CK(cudaGetLastError());
+      ++done;
+      CK(cudaMemcpyAsync(c->mgst_host, c->mgst, sizeof(MgState), cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+    }
+    n += finish();
+    c->launches += n;
+    c->pcg_launched_iterations += done;
+  } else {
+    if (!c->mg_graph) {
+      cudaGraph_t g = nullptr;
+      CK(cudaGraphCreate(&g, 0));
+      cudaGraphConditionalHandle h;
+      CK(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+      CK(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+      c->mg_launches[0] = start() + 1;
+      mg_loop_start(h, c->mgst, s);
+      cudaStreamCaptureStatus cs;
+      const cudaGraphNode_t* deps = nullptr;
+      size_t ndeps = 0;
+      CK(cudaStreamGetCaptureInfo_v2(s, &cs, nullptr, nullptr, &deps, &ndeps));
+      if (ndeps != 1) { set_error("unexpected capture state"); return FS_CUDA_ERROR; }
+      cudaGraphNode_t last = deps[0];
+      CK(cudaStreamEndCapture(s, &g));
+      cudaGraphNodeParams cp = {};
+      cp.type = cudaGraphNodeTypeConditional;
+      cp.conditional.handle = h;
+      cp.conditional.type = cudaGraphCondTypeWhile;
+      cp.conditional.size = 1;
+      cudaGraphNode_t loop = nullptr;
+      CK(cudaGraphAddNode(&loop, g, &last, 1, &cp));
+      cudaGraph_t body = cp.conditional.phGraph_out[0];
+      CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+      c->mg_launches[1] = mg_iteration<S>(c->mg, p, q, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, true, h, s);
+      CK(cudaStreamEndCapture(s, &body));
+      CK(cudaStreamBeginCaptureToGraph(s, g, &loop, nullptr, 1, cudaStreamCaptureModeThreadLocal));
+      c->mg_launches[2] = finish();
+      CK(cudaStreamEndCapture(s, &g));
+      CK(cudaGraphInstantiate(&c->mg_graph, g, 0));
+      cudaGraphDestroy(g);
+    }
+    CK(cudaGraphLaunch(c->mg_graph, s));
+  }
+  CK(cudaEventRecord(c->evp1, s));
+  CK(cudaMemcpyAsync(c->mgst_host, c->mgst, sizeof(MgState), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  float ms = 0.0f;
+  CK(cudaEventElapsedTime(&ms, c->evp0, c->evp1));
+  c->pcg_ms += ms;
+  const MgState& m = *c->mgst_host;
+  if (!c->prm.host_loop) {
+    c->launches += c->mg_launches[0] + (int64_t)m.batches * c->mg_launches[1] + c->mg_launches[2];
+    c->pcg_launched_iterations += (int)m.batches;
+  }
+  *iters_out = m.iter;
+  *outer_out = m.outer;
+  *rel_out = m.bb > 0 ? std::sqrt(m.rr_true / m.bb) : 0.0;
+  *st_out = m.status;
+  c->st_host->rz = m.rz;
+  if (c->debug)
+    std::fprintf(stderr, "[fs] multigrid solve: %d iterations, %d true residuals, status %d, rel %.3e\n", m.iter,
+                 m.outer, m.status, *rel_out);
+  if (m.status == PCG_NONFINITE) {
+    set_error("non-finite defect residual");
+    return FS_NONFINITE;
+  }
+  if (m.status == PCG_MAXITER && m.rr_true > m.rr0) {
+    // the cap came before any progress: leave the better pressure
+    CK(cudaMemcpyAsync(x, c->p64bak, c->Lc.total * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    *rel_out = m.bb > 0 ? std::sqrt(m.rr0 / m.bb) : 0.0;
+  }
+  if (m.status == PCG_STAGNATED && !(m.rr_true <= m.rr0))
+    CK(cudaMemcpyAsync(x, c->p64bak, c->Lc.total * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  return FS_OK;
+}
+
 // The FP32 + FP64 defect-correction solve of A(phi) x = b (A the pressure
 // operator evaluated from phi, b and x FP64 cell fields): the projection's
 // solve and, in FP32 contexts, the adjoint's transposed solve with the same
 // symmetric operator.  *iters, *outer, *rel and *st report the Krylov
 // iterations, the defect corrections, the final relative FP64 residual and
 // the PCG status.
+// transposed: the adjoint's solve.  It keeps the red-black iteration: the
+// density bars amplify what a solve leaves over by about 1e7 (96^3 dam break:
+// 1.1e-4 relative at tolerance 1e-11, where the multigrid solve is 5e-7 off),
+// so another iteration's remainder would move them.
 template <class S>
 fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int* outer_out, double* rel_out,
-                      int* st_out) {
+                      int* st_out, bool transposed = false) {
   const fs_params& P = c->prm;
   const double dx = c->grid.dx;
   cudaStream_t s = c->stream;
   int iters = 0, outer = 0, st = 0;
   double rel = 0.0;
+  bool handed_over = false;  // from the multigrid solve
+  int mg_iters = 0, mg_outer = 0;
+  if constexpr (sizeof(S) == sizeof(float)) {
+    if (c->multigrid && !transposed) {
+      CKS(mg_solve<S>(c, phi, b, x, &mg_iters, &mg_outer, rel_out, st_out));
+      if (*st_out != PCG_STAGNATED) {
+        *iters_out = mg_iters;
+        *outer_out = mg_outer;
+        return FS_OK;
+      }
+      handed_over = true;
+    }
+  }
   const bool rb = c->red_black;
   build_pressure_operator<S, float>(phi, c->Lc, dx, P.rho_neg, P.rho_pos, (float*)c->pax, (float*)c->pay,
                                     (float*)c->paz, (float*)c->pdiag, c->scalars + 12, deflate(c), s,
@@ -891,8 +1103,16 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     CK(cudaEventElapsedTime(&ms, c->evp0, c->evp1));
     c->pcg_ms += ms;
   }
-  *iters_out = iters;
-  *outer_out = outer;
+  if (handed_over) {
+    // the constant of the whole solve: the sum kept before the cycles
+    c->mgst_host->status = PCG_CONVERGED;
+    CK(cudaMemcpyAsync(c->mgst, c->mgst_host, sizeof(MgState), cudaMemcpyHostToDevice, s));
+    mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, s);
+    c->launches += 2;
+    CK(cudaGetLastError());
+  }
+  *iters_out = mg_iters + iters;
+  *outer_out = mg_outer + outer;
   *rel_out = rel;
   *st_out = st;
   return FS_OK;
@@ -1329,7 +1549,7 @@ fs_status adj_projection(fs_ctx* c, void* phi, void* const ustar[3], const doubl
   double rel = 0.0;
   if constexpr (sizeof(S) == sizeof(float)) {
     int outer = 0;
-    CKS(mixed_solve<S>(c, F<S>(phi), pbar, lam, &it, &outer, &rel, &st));
+    CKS(mixed_solve<S>(c, F<S>(phi), pbar, lam, &it, &outer, &rel, &st, true));
   } else {
     build_pressure_operator<S, double>(F<S>(phi), c->Lc, dx, P.rho_neg, P.rho_pos, c->a_ax, c->a_ay, c->a_az,
                                        c->a_diag, c->scalars + 12, deflate(c), s);
@@ -1652,6 +1872,14 @@ fs_status fs_create(const fs_grid_desc* grid, const fs_params* params, fs_ctx** 
     float** hv[] = {&c->rb_r, &c->rb_p, &c->rb_q, &c->rb_tau};
     for (float** p : hv) if ((s = dalloc(c, (void**)p, hb * sizeof(float))) != FS_OK) return fail(s);
     if ((s = dalloc(c, (void**)&c->rb_dinv, hb * sizeof(unsigned short))) != FS_OK) return fail(s);
+    if (!prm.pipe) {
+      if ((s = mg_alloc(c)) != FS_OK) return fail(s);
+      apply_params(c);  // the levels' uniform couplings
+      if (mg_prepare() != cudaSuccess) {
+        set_error("shared memory of the multigrid cycle: %s", cudaGetErrorString(cudaGetLastError()));
+        return fail(FS_CUDA_ERROR);
+      }
+    }
   }
   if (prm.pipe) {
     const size_t fb[3] = {ub, vb, wb};
@@ -1671,7 +1899,7 @@ fs_status fs_create(const fs_grid_desc* grid, const fs_params* params, fs_ctx** 
   cg_prepare<float, float>();
   int nblk = std::max(pcg_blocks(c->Lu), std::max(pcg_blocks(c->Lv), pcg_blocks(c->Lw))) * 2 + 64;
   for (const Lay* L : {&c->Lc, &c->Lu, &c->Lv, &c->Lw}) nblk = std::max(nblk, cg_max_blocks(*L));
-  if (c->fp32) nblk = std::max(nblk, rb_blocks(c->Lh));
+  if (c->fp32) nblk = std::max(nblk, std::max(rb_blocks(c->Lh), mg_max_blocks(c->Lh)));
   if ((s = dalloc(c, (void**)&c->partials, (size_t)nblk * 3 * sizeof(double))) != FS_OK) return fail(s);
   if ((s = dalloc(c, (void**)&c->tickets, 8 * sizeof(unsigned int))) != FS_OK) return fail(s);
   if ((s = dalloc(c, (void**)&c->scalars, 16 * sizeof(double))) != FS_OK) return fail(s);
@@ -1718,8 +1946,7 @@ fs_status fs_set_params(fs_ctx* c, const fs_params* p) {
   apply_params(c);
   // captured solver graphs hold the operator's arithmetic and preconditioner
   // as kernel arguments: capture them again under the new settings
-  for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return FS_OK;
 }
 

@@ -222,6 +222,58 @@ template <class V, class R = V>
 void pcg_resume(const Op7<V>& A, const R* r, V* p, PcgState* st, double* partials, int restart, cudaStream_t s);
 int pcg_blocks(const Lay& L);
 
+// ---- multigrid-preconditioned pressure solve (fs_multigrid.cu)
+constexpr int kMgMaxLevels = 14;
+struct MgLevel {
+  Lay L, H;                            // cell layout of the couplings, packed layout of each colour
+  float *ax = nullptr, *ay = nullptr, *az = nullptr;
+  unsigned char* cls[2] = {};          // per colour: 1 or 2, the phase whose uniform coupling all faces carry; 0: mixed
+  float* x[2] = {};                    // by colour (0 red, 1 black): the cycle's solution (level 0: z)
+  float* b[2] = {};                    // and right-hand side (level 0: the residual r)
+  float a[2] = {};                     // the uniform couplings of the two phases
+};
+// levels 0 .. top-1 run as grid kernels, top .. levels-1 in one thread block
+struct Multigrid {
+  int levels = 0, top = 0;
+  MgLevel level[kMgMaxLevels];
+};
+// Device state of one solve.  The host sets the first group.
+struct MgState {
+  const void* phi;       // level set
+  double* x;             // FP64 iterate, in and out
+  const double* b;       // FP64 right-hand side
+  double* bak;           // receives the initial guess
+  const double* bb_src;  // ||b||^2
+  double tol;            // relative to ||b||
+  double delta;          // reliable_delta
+  int max_iter;
+  double tol2, bb, rr, rr_true, rr0, best, max_rr;  // squared norms
+  double rz, alpha, beta, anchor, shift;
+  int iter, done, status, pause, restart, outer, stall;
+  unsigned int ticket, batches;
+};
+int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top);
+cudaError_t mg_prepare();
+int mg_max_blocks(const Lay& H);
+// Each returns the number of kernels launched.  mg_build: the operator of
+// every level from st->phi.  mg_start: true residual, first cycle and
+// direction.  mg_iteration: one CG iteration; with `loop` its last kernel
+// continues the graph's while node `handle`.
+template <class T>
+int mg_build(const Multigrid& M, const MgState* st, double dx, double rho_neg, double rho_pos, double* extra0,
+             cudaStream_t s);
+template <class T>
+int mg_start(const Multigrid& M, float* p, MgState* st, double* partials, double dx, double rho_neg, double rho_pos,
+             cudaStream_t s);
+template <class T>
+int mg_iteration(const Multigrid& M, float* p, float* q, MgState* st, double* partials, double dx, double rho_neg,
+                 double rho_pos, bool loop, cudaGraphConditionalHandle handle, cudaStream_t s);
+// before the solve: keep the sum that fixes the pressure's constant; after
+// it: shift st->x to that sum (not after a solve that stagnated)
+void mg_anchor(const Multigrid& M, const unsigned short* dinv, MgState* st, double* partials, bool after,
+               cudaStream_t s);
+void mg_loop_start(cudaGraphConditionalHandle handle, const MgState* st, cudaStream_t s);
+
 // ---- projection family (fs_projection.cu)
 struct ProjParams {
   double dx, dt, rho_neg, rho_pos;
