@@ -608,10 +608,12 @@ fs_status advect_levelset_t(fs_ctx* c, double dt, Tape* tp = nullptr) {
     if (tp && stage < 3)
       cudaMemcpyAsync(tp->ls[stage], src, c->Lc.total * c->S(), cudaMemcpyDeviceToDevice, s);
     ++stage;
-    if (pg) fill_periodic_y<S>(src, c->Lc, s);
-    else fill_extrap<S>(src, c->Lc, s);
+    if (pg) {
+      fill_periodic_y<S>(src, c->Lc, s);
+      c->launches += 1;
+    }
     weno5_levelset<S>(src, base, out, u, v, w, c->Lc, c->Lu, c->Lv, c->Lw, dx, eps, dt, c0, c1, s, pg);
-    c->launches += 2;
+    c->launches += 1;
   };
   if (P.order == 3 && !(P.flags & FS_FLAG_LEVELSET_FORWARD_EULER)) {
     fe(phi, phi, t1, 0.0, 1.0);                        // phi1 = phi0 + dt L(phi0)
@@ -720,17 +722,16 @@ fs_status reinit_block_t(fs_ctx* c, void* in, void* out, void* base, double c0, 
     else if (out != in) CK(cudaMemcpyAsync(out, in, c->Lc.total * c->S(), cudaMemcpyDeviceToDevice, s));
     return FS_OK;
   }
-  sign_function<S>(F<S>(in), F<S>(c->sgn), c->Lc, dx, s);
-  c->launches += 1 + 2 * n;
+  c->launches += (c->pipe.on ? 2 : 1) * n;
   void* cur = in;
   for (int it = 0; it < n; ++it) {
     const bool last = it == n - 1;
     void* dst = last ? out : (cur == scrA ? scrB : scrA);
     if (tape) CK(cudaMemcpyAsync((*tape)[it], cur, c->Lc.total * c->S(), cudaMemcpyDeviceToDevice, s));
     if (c->pipe.on) fill_periodic_y<S>(F<S>(cur), c->Lc, s);  // ADVECTION_3D.h:360-378
-    else fill_extrap<S>(F<S>(cur), c->Lc, s);
     sussman_step<S>(F<S>(cur), F<S>(c->sgn), F<S>(base), F<S>(dst), c->Lc, dx, P.weno_epsilon, dtau,
-                    last ? c0 : 0.0, last ? c1 : 1.0, (P.flags & FS_FLAG_REINIT_TYPO) ? 1 : 0, s);
+                    last ? c0 : 0.0, last ? c1 : 1.0, (P.flags & FS_FLAG_REINIT_TYPO) ? 1 : 0, it == 0 ? 1 : 0,
+                    c->pipe.on ? 0 : 1, s);
     cur = dst;
   }
   CK(cudaGetLastError());

@@ -69,6 +69,8 @@ template <class T>
 void pipe_velocity_correct(T* u, T* v, T* w, const double* p, const T* phi, const double* kappa, const Lay& Lc,
                            const Lay& Lu, const Lay& Lv, const Lay& Lw, const PipeGeom& G, double dx, double dt,
                            double rho_neg, double rho_pos, double sigma, cudaStream_t s);
+// one WENO5 level-set update; in the box the ghosts of src are extrapolated
+// by the kernel itself, in the pipe (pipe != nullptr) they are read
 template <class T>
 void weno5_levelset(const T* src, const T* base, T* out, const T* u, const T* v, const T* w, const Lay& L,
                     const Lay& Lu, const Lay& Lv, const Lay& Lw, double dx, double eps, double dt, double c0, double c1,
@@ -99,9 +101,11 @@ cudaError_t polygonize(const T* phi, const Lay& L, double dx, SurfaceMesh* mesh,
 template <class T>
 int fast_sweeping(const T* in, T* out, unsigned char* fixed, const Lay& L, double dx, int direction, int pairs,
                   int typo, int* stale_read, cudaStream_t s);
+// one Sussman pseudo-step; first: sgn is formed from src and written;
+// extrapolate: level-set ghosts are extrapolated by the kernel itself (0: read)
 template <class T>
-void sussman_step(const T* src, const T* sgn, const T* base, T* out, const Lay& L, double dx, double eps, double dtau,
-                  double c0, double c1, int typo, cudaStream_t s);
+void sussman_step(const T* src, T* sgn, const T* base, T* out, const Lay& L, double dx, double eps, double dtau,
+                  double c0, double c1, int typo, int first, int extrapolate, cudaStream_t s);
 template <class T> void axpby(T* out, const T* x, const T* y, double a, double b, const Lay& L, cudaStream_t s);
 template <class T> void add_const_faces(T* f, const Lay& L, int axis, double value, int skip_walls, cudaStream_t s);
 template <class T> void zero_walls(T* f, const Lay& L, int axis, cudaStream_t s);

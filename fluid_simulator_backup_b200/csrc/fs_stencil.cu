@@ -4,22 +4,31 @@
 // (EULERIAN_FLUID_SOLVER_3D.h:886-1109), templated on the storage/arithmetic
 // type (double for the FP64 path, float for FP32_REFINE).
 //
-// Staging.  The four seven-point stencil kernels (WENO5 level set, WENO5 and
-// ENO3 MAC components, Sussman) run on 32 x 8 column tiles that march up a
-// chunk of z planes: the stencil field is staged in shared memory as a ring of
-// seven (32+6) x (8+6) planes (the tile and its three-cell halo), one new
-// plane loaded per output plane with row-contiguous (coalesced) loads, and
-// every x, y and z sample of the stencil is read from that ring.  HBM then
-// carries each field element about once per kernel instead of up to 19
-// times through L1/L2.  The ghost ring of the padded layout supplies the halo
-// at the box boundary.
-//
-// These kernels are FP32/FP64-issue bound rather than HBM bound (about 440
-// flops per cell per WENO5 update), so the WENO weights are evaluated with one
-// division per side: w_k = d_k prod_{j!=k} q_j / sum_m d_m prod_{j!=m} q_j
-// with q = (eps + IS)^2, algebraically equal to the reference's
-// (d_k/q_k)/sum(d_m/q_m).  The substencil constants 1/3, 7/6, ... are applied
-// as multiplications.  Both change results only at the level of rounding.
+// The seven-point stencil kernels (WENO5 level set, WENO5 and ENO3 MAC
+// components, Sussman) take one column of a z chunk per thread and march up
+// it.  The seven samples along z slide through registers (one new load per
+// cell); the x and y samples are read at fixed offsets and hit L1, where the
+// neighbouring threads of the block have just read them.  A shared-memory
+// ring of seven planes, as these kernels used before, spends more on staging
+// the planes, two barriers per plane and the ring's index arithmetic than it
+// saves: they are bound by instruction issue, not by HBM (12 to 20 bytes per
+// cell in FP32).  What cut the time is fewer instructions per cell:
+//   - the two one-sided WENO5 derivatives share their differences, second
+//     differences and the squares of these; an advection, which uses only the
+//     upwind side, evaluates only that one;
+//   - each side is its middle difference plus a weighted correction,
+//     D = r3 + (b1 v1 + b2 v2 + b3 v3)/(b1 + b2 + b3), b_k = d_k prod_{j!=k}
+//     q_j, q = (eps + IS)^2: algebraically the reference's
+//     sum (d_k/q_k) u_k / sum (d_k/q_k) with one reciprocal per side, which in
+//     FP32 may be the hardware's (1 ulp, of a term that only corrects r3);
+//   - level-set ghosts are the linear extrapolation the ghost fill would
+//     store, formed in registers by the threads next to a wall, so no fill
+//     precedes the kernel (and the first Sussman step writes the sign field
+//     it is the first to need).
+// Measured (B200), before -> after, per launch with its ghost fill: Sussman
+// step 256^3 FP32 516 -> 256 us, 33 x 47 x 29 FP64 17.8 -> 4.3 us; level set
+// 256^3 FP32 533 -> 239 us; WENO5 component 200 x 136 x 267 FP32 285 -> 106 us;
+// ENO3 component 65 x 97 x 41 FP64 25.4 -> 11.4 us.
 #include <algorithm>
 
 #include "fs_kernels.h"
@@ -129,24 +138,26 @@ void fill_extrap(T* f, const Lay& L, cudaStream_t s) {
 // WENO5
 // ---------------------------------------------------------------------------
 
+__device__ __forceinline__ float reciprocal(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ double reciprocal(double x) { return 1.0 / x; }
+
+// One side from its middle difference r3, its differences' differences e1 ..
+// e4 (e_k = r_{k+1} - r_k) and the scaled squares T_k = eps + 13/12 (e_{k+1}
+// - e_k)^2 of its three substencils.
 template <class T>
-__device__ __forceinline__ T weno_side(T r1, T r2, T r3, T r4, T r5, T eps) {
-  const T c1312 = T(13.0 / 12.0);
-  T t = (r1 - T(2) * r2) + r3, q = (r1 - T(4) * r2) + T(3) * r3;
-  const T s1 = (c1312 * t) * t + (T(0.25) * q) * q;
-  t = (r2 - T(2) * r3) + r4; q = r2 - r4;
-  const T s2 = (c1312 * t) * t + (T(0.25) * q) * q;
-  t = (r3 - T(2) * r4) + r5; q = (T(3) * r3 - T(4) * r4) + r5;
-  const T s3 = (c1312 * t) * t + (T(0.25) * q) * q;
-  const T e1 = eps + s1, e2 = eps + s2, e3 = eps + s3;
-  const T q1 = e1 * e1, q2 = e2 * e2, q3 = e3 * e3;
+__device__ __forceinline__ T weno_from(T r3, T e1, T e2, T e3, T e4, T T1, T T2, T T3) {
+  const T g1 = T(3) * e2 - e1, g2 = e2 + e3, g3 = T(3) * e3 - e4;
+  const T s1 = T1 + (T(0.25) * g1) * g1, s2 = T2 + (T(0.25) * g2) * g2, s3 = T3 + (T(0.25) * g3) * g3;
+  const T q1 = s1 * s1, q2 = s2 * s2, q3 = s3 * s3;
   const T b1 = T(0.1) * (q2 * q3), b2 = T(0.6) * (q1 * q3), b3 = T(0.3) * (q1 * q2);
-  const T inv = T(1) / ((b1 + b2) + b3);
-  const T third = T(1.0 / 3.0), sixth = T(1.0 / 6.0);
-  const T u1 = (r1 * third - r2 * T(7.0 / 6.0)) + r3 * T(11.0 / 6.0);
-  const T u2 = (r2 * (-sixth) + r3 * T(5.0 / 6.0)) + r4 * third;
-  const T u3 = (r3 * third + r4 * T(5.0 / 6.0)) - r5 * sixth;
-  return ((b1 * u1 + b2 * u2) + b3 * u3) * inv;
+  // six times the substencil values less r3
+  const T v1 = T(5) * e2 - T(2) * e1, v2 = T(2) * e3 + e2, v3 = T(4) * e3 - e4;
+  const T num = (b1 * v1 + b2 * v2) + b3 * v3;
+  return r3 + (num * T(1.0 / 6.0)) * reciprocal((b1 + b2) + b3);
 }
 
 // D- and D+ from the 7 samples v[0..6] = f[-3..3] along one axis.
@@ -154,106 +165,142 @@ template <class T>
 __device__ __forceinline__ void weno_pair7(const T v[7], T inv_h, T eps, T& dm, T& dp) {
   const T d1 = inv_h * (v[1] - v[0]), d2 = inv_h * (v[2] - v[1]), d3 = inv_h * (v[3] - v[2]),
           d4 = inv_h * (v[4] - v[3]), d5 = inv_h * (v[5] - v[4]), d6 = inv_h * (v[6] - v[5]);
-  dm = weno_side(d1, d2, d3, d4, d5, eps);
-  dp = weno_side(d6, d5, d4, d3, d2, eps);
+  const T e1 = d2 - d1, e2 = d3 - d2, e3 = d4 - d3, e4 = d5 - d4, e5 = d6 - d5;
+  const T c1312 = T(13.0 / 12.0);
+  const T t1 = e2 - e1, t2 = e3 - e2, t3 = e4 - e3, t4 = e5 - e4;
+  const T T1 = eps + (c1312 * t1) * t1, T2 = eps + (c1312 * t2) * t2, T3 = eps + (c1312 * t3) * t3,
+          T4 = eps + (c1312 * t4) * t4;
+  dm = weno_from(d3, e1, e2, e3, e4, T1, T2, T3);
+  dp = weno_from(d4, -e5, -e4, -e3, -e2, T4, T3, T2);
+}
+
+// The upwind one of the two: D- for a positive velocity, else D+, which is
+// the same function of the differences in reverse order.
+template <class T>
+__device__ __forceinline__ T weno_upwind7(const T v[7], T inv_h, T eps, bool minus) {
+  const T d1 = inv_h * (v[1] - v[0]), d2 = inv_h * (v[2] - v[1]), d3 = inv_h * (v[3] - v[2]),
+          d4 = inv_h * (v[4] - v[3]), d5 = inv_h * (v[5] - v[4]), d6 = inv_h * (v[6] - v[5]);
+  const T r1 = minus ? d1 : d6, r2 = minus ? d2 : d5, r3 = minus ? d3 : d4, r4 = minus ? d4 : d3,
+          r5 = minus ? d5 : d2;
+  const T e1 = r2 - r1, e2 = r3 - r2, e3 = r4 - r3, e4 = r5 - r4;
+  const T c1312 = T(13.0 / 12.0);
+  const T t1 = e2 - e1, t2 = e3 - e2, t3 = e4 - e3;
+  return weno_from(r3, e1, e2, e3, e4, eps + (c1312 * t1) * t1, eps + (c1312 * t2) * t2, eps + (c1312 * t3) * t3);
 }
 
 // ---------------------------------------------------------------------------
-// shared-memory plane ring of the staged stencil kernels
+// columns of the stencil kernels
 // ---------------------------------------------------------------------------
-constexpr int kTX = 32, kTY = 8;                     // tile (threads) in x and y
-constexpr int kRW = kTX + 2 * GH, kRH = kTY + 2 * GH;  // staged plane: tile + halo
-constexpr int kRing = 2 * GH + 1;                    // planes k-3 .. k+3
+constexpr int kTX = 32, kTY = 8, kColThreads = kTX * kTY;
 
-__device__ __forceinline__ int ring_slot(int k) { return ((k % kRing) + kRing) % kRing; }
-
-// Plane k of f (halo included) into its ring slot: row-contiguous loads of
-// the (32+6) x (8+6) window; halo cells beyond the ghost ring (i >= nx+3 or
-// j >= ny+3, only at the tile past the box edge) are not needed and skipped.
-template <class T>
-__device__ __forceinline__ void stage_plane(T* ring, const T* __restrict__ f, const Lay& L, int i0, int j0, int k) {
-  T* dst = ring + ring_slot(k) * (kRW * kRH);
-  const int tid = threadIdx.x + kTX * threadIdx.y;
-  for (int t = tid; t < kRW * kRH; t += kTX * kTY) {
-    const int x = t % kRW, y = t / kRW;
-    const int gi = i0 - GH + x, gj = j0 - GH + y;
-    if (gi < L.nx + GH && gj < L.ny + GH) dst[t] = f[L.at(gi, gj, k)];
-  }
-}
-
-// The seven samples of (tx, ty) in plane k along x, y and z from the ring.
-template <class T>
-__device__ __forceinline__ void ring_samples(const T* ring, int k, T vx[7], T vy[7], T vz[7]) {
-  const int tx = threadIdx.x + GH, ty = threadIdx.y + GH;
-  const T* pc = ring + ring_slot(k) * (kRW * kRH);
-#pragma unroll
-  for (int o = 0; o < 7; ++o) {
-    vx[o] = pc[ty * kRW + tx + o - GH];
-    vy[o] = pc[(ty + o - GH) * kRW + tx];
-    vz[o] = ring[ring_slot(k + o - GH) * (kRW * kRH) + ty * kRW + tx];
-  }
-}
-
-// Grid of a staged kernel: xy tiles times z chunks, enough blocks to fill
-// the GPU a few times over (each chunk re-stages six halo planes).
-struct StagedGrid {
+// Thread -> column (i, j) of a layout: 32 x 8 tiles, or, where those would
+// leave more than an eighth of their threads without a column (rows a little
+// longer than a multiple of 32, small ragged boxes), 256 consecutive columns
+// of the plane.  Tiles read fewer rows per block, so they are the rule.
+struct ColumnGrid {
   dim3 grid;
-  int kchunk;
+  int kchunk, flat;
 };
-inline StagedGrid staged_grid(const Lay& L) {
+inline ColumnGrid column_grid(const Lay& L) {
   static int sms = 0;
   if (sms <= 0) {
-    int dev = 0;
+    int dev = 0, n = 0;
     cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    sms = n;
   }
   const int tx = (L.nx + kTX - 1) / kTX, ty = (L.ny + kTY - 1) / kTY;
-  const int want = 8 * sms;
-  const int chunks = std::max(1, std::min(L.nz, (want + tx * ty - 1) / (tx * ty)));
-  const int kchunk = (L.nz + chunks - 1) / chunks;
-  StagedGrid g;
-  g.grid = dim3(tx, ty, (L.nz + kchunk - 1) / kchunk);
-  g.kchunk = kchunk;
+  const int64_t cols = (int64_t)L.nx * L.ny;
+  ColumnGrid g;
+  g.flat = (int64_t)tx * ty * kColThreads * 7 > cols * 8 ? 1 : 0;
+  const int bx = g.flat ? (int)((cols + kColThreads - 1) / kColThreads) : tx, by = g.flat ? 1 : ty;
+  // about 16 blocks per SM: several waves, so that the last one is short; a
+  // chunk's start costs its six extra z samples only
+  const int64_t want = (int64_t)16 * sms;
+  const int chunks = (int)std::max<int64_t>(1, std::min<int64_t>(L.nz, (want + (int64_t)bx * by - 1) / ((int64_t)bx * by)));
+  g.kchunk = (L.nz + chunks - 1) / chunks;
+  g.grid = dim3(bx, by, (L.nz + g.kchunk - 1) / g.kchunk);
   return g;
+}
+
+__device__ __forceinline__ bool column_of(const Lay& L, int flat, int& i, int& j) {
+  if (flat) {
+    const unsigned t = blockIdx.x * (unsigned)kColThreads + threadIdx.x;  // at most 4097^2 columns
+    j = (int)(t / (unsigned)L.nx);
+    i = (int)(t - (unsigned)j * (unsigned)L.nx);
+    return j < L.ny;
+  }
+  i = blockIdx.x * kTX + (threadIdx.x & (kTX - 1));
+  j = blockIdx.y * kTY + threadIdx.x / kTX;
+  return i < L.nx && j < L.ny;
+}
+
+// Samples outside [0, n) replaced by the recursion of extrap_layer.
+template <class T>
+__device__ __forceinline__ void extrapolate7(T v[7], int e, int n) {
+#pragma unroll
+  for (int m = 1; m <= 3; ++m) {
+    if (e - m < 0) v[3 - m] = T(2) * v[4 - m] - v[5 - m];
+    if (e + m >= n) v[3 + m] = T(2) * v[2 + m] - v[1 + m];
+  }
+}
+
+// The seven samples around c along one axis (stride st, coordinate e of n).
+template <class T>
+__device__ __forceinline__ void samples7(T v[7], const T* __restrict__ f, int64_t c, int64_t st, T centre, int e, int n,
+                                         bool extrapolate) {
+#pragma unroll
+  for (int m = 1; m <= 3; ++m) {
+    v[3 - m] = f[c - m * st];
+    v[3 + m] = f[c + m * st];
+  }
+  v[3] = centre;
+  if (extrapolate && (e < 3 || e >= n - 3)) extrapolate7(v, e, n);
+}
+
+// The sliding window along z: advance to the next plane.  `next` is
+// f[c + 4 slab] of the plane just done, loaded early; past the box it is
+// extrapolated instead.
+template <class T>
+__device__ __forceinline__ void slide7(T v[7], T next, int k, int nz, bool extrapolate) {
+  const T n = extrapolate && k + 4 >= nz ? T(2) * v[6] - v[5] : next;
+#pragma unroll
+  for (int m = 0; m < 6; ++m) v[m] = v[m + 1];
+  v[6] = n;
 }
 
 // out = c0*base + c1*(src - dt*(u.grad src)), the level-set update at cell
 // centres; u, v, w are the MAC faces (zero ghosts).  With c0 == 0 the
 // combination is skipped and out is the forward-Euler value.
 template <class T>
-__global__ void __launch_bounds__(kTX * kTY) k_weno5_levelset(const T* __restrict__ src, const T* __restrict__ base,
+__global__ void __launch_bounds__(kColThreads) k_weno5_levelset(const T* __restrict__ src, const T* __restrict__ base,
                                                            T* __restrict__ out, const T* __restrict__ u,
                                                            const T* __restrict__ v, const T* __restrict__ w, Lay L,
                                                            Lay Lu, Lay Lv, Lay Lw, T inv_h, T eps, T dt, T c0, T c1,
-                                                           int kchunk, PipeGeom pipe) {
-  __shared__ T ring[kRing * kRW * kRH];
-  const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTY;
-  const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+                                                           int kchunk, int flat, PipeGeom pipe) {
+  int i, j;
+  if (!column_of(L, flat, i, j)) return;
   const int k0 = blockIdx.z * kchunk, k1 = min(L.nz, k0 + kchunk);
-  const bool valid = i < L.nx && j < L.ny;
-  for (int kk = k0 - GH; kk < k0 + GH; ++kk) stage_plane(ring, src, L, i0, j0, kk);
-  for (int k = k0; k < k1; ++k) {
-    stage_plane(ring, src, L, i0, j0, k + GH);
-    __syncthreads();
-    if (valid) {
-      T vx[7], vy[7], vz[7];
-      ring_samples(ring, k, vx, vy, vz);
-      T dxm, dxp, dym, dyp, dzm, dzp;
-      weno_pair7(vx, inv_h, eps, dxm, dxp);
-      weno_pair7(vy, inv_h, eps, dym, dyp);
-      weno_pair7(vz, inv_h, eps, dzm, dzp);
-      const int64_t c = L.at(i, j, k);
-      const T uc = (u[Lu.at(i + 1, j, k)] + u[Lu.at(i, j, k)]) * T(0.5);
-      const T vc = (v[Lv.at(i, j + 1, k)] + v[Lv.at(i, j, k)]) * T(0.5);
-      const T wc = (w[Lw.at(i, j, k + 1)] + w[Lw.at(i, j, k)]) * T(0.5);
-      T fe =
-          vx[3] - dt * ((uc * (uc > T(0) ? dxm : dxp) + vc * (vc > T(0) ? dym : dyp)) + wc * (wc > T(0) ? dzm : dzp));
-      // pipe mode: cells outside the pipe keep their value
-      // (ADVECTION_METHOD_3D.h:293-296)
-      if (pipe.on && pipe_wall_distance(pipe, 0, i, k) > 0.0) fe = vx[3];
-      out[c] = c0 == T(0) ? fe : c0 * base[c] + c1 * fe;
-    }
-    __syncthreads();
+  const bool ex = !pipe.on;  // the pipe's ghosts are periodic, filled by the caller
+  int64_t c = L.at(i, j, k0), cu = Lu.at(i, j, k0), cv = Lv.at(i, j, k0), cw = Lw.at(i, j, k0);
+  T vx[7], vy[7], vz[7];
+  samples7(vz, src, c, L.slab, src[c], k0, L.nz, ex);
+  for (int k = k0; k < k1; ++k, c += L.slab, cu += Lu.slab, cv += Lv.slab, cw += Lw.slab) {
+    const T next = k + 1 < k1 ? src[c + 4 * L.slab] : T(0);
+    samples7(vx, src, c, 1, vz[3], i, L.nx, ex);
+    samples7(vy, src, c, L.px, vz[3], j, L.ny, ex);
+    const T uc = (u[cu + 1] + u[cu]) * T(0.5);
+    const T vc = (v[cv + Lv.px] + v[cv]) * T(0.5);
+    const T wc = (w[cw + Lw.slab] + w[cw]) * T(0.5);
+    const T dx = weno_upwind7(vx, inv_h, eps, uc > T(0));
+    const T dy = weno_upwind7(vy, inv_h, eps, vc > T(0));
+    const T dz = weno_upwind7(vz, inv_h, eps, wc > T(0));
+    T fe = vz[3] - dt * ((uc * dx + vc * dy) + wc * dz);
+    // pipe mode: cells outside the pipe keep their value
+    // (ADVECTION_METHOD_3D.h:293-296)
+    if (pipe.on && pipe_wall_distance(pipe, 0, i, k) > 0.0) fe = vz[3];
+    out[c] = c0 == T(0) ? fe : c0 * base[c] + c1 * fe;
+    slide7(vz, next, k, L.nz, ex);
   }
 }
 
@@ -281,32 +328,27 @@ __device__ __forceinline__ void mac_velocity(const T* __restrict__ u, const T* _
 // MAC component self-advection on every face of component `axis` (wall
 // faces included, as the reference's loop covers the whole face grid).
 template <class T>
-__global__ void __launch_bounds__(kTX * kTY) k_weno5_mac(const T* __restrict__ comp, T* __restrict__ out,
+__global__ void __launch_bounds__(kColThreads) k_weno5_mac(const T* __restrict__ comp, T* __restrict__ out,
                                                       const T* __restrict__ u, const T* __restrict__ v,
                                                       const T* __restrict__ w, Lay Lc, Lay Lu, Lay Lv, Lay Lw,
-                                                      int axis, T inv_h, T eps, T dt, int kchunk) {
-  __shared__ T ring[kRing * kRW * kRH];
-  const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTY;
-  const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+                                                      int axis, T inv_h, T eps, T dt, int kchunk, int flat) {
+  int i, j;
+  if (!column_of(Lc, flat, i, j)) return;
   const int k0 = blockIdx.z * kchunk, k1 = min(Lc.nz, k0 + kchunk);
-  const bool valid = i < Lc.nx && j < Lc.ny;
-  for (int kk = k0 - GH; kk < k0 + GH; ++kk) stage_plane(ring, comp, Lc, i0, j0, kk);
-  for (int k = k0; k < k1; ++k) {
-    stage_plane(ring, comp, Lc, i0, j0, k + GH);
-    __syncthreads();
-    if (valid) {
-      T uvel, vvel, wvel;
-      mac_velocity(u, v, w, Lu, Lv, Lw, axis, i, j, k, uvel, vvel, wvel);
-      T vx[7], vy[7], vz[7];
-      ring_samples(ring, k, vx, vy, vz);
-      T dxm, dxp, dym, dyp, dzm, dzp;
-      weno_pair7(vx, inv_h, eps, dxm, dxp);
-      weno_pair7(vy, inv_h, eps, dym, dyp);
-      weno_pair7(vz, inv_h, eps, dzm, dzp);
-      out[Lc.at(i, j, k)] = vx[3] - dt * ((uvel * (uvel > T(0) ? dxm : dxp) + vvel * (vvel > T(0) ? dym : dyp)) +
-                                          wvel * (wvel > T(0) ? dzm : dzp));
-    }
-    __syncthreads();
+  int64_t c = Lc.at(i, j, k0);
+  T vx[7], vy[7], vz[7];
+  samples7(vz, comp, c, Lc.slab, comp[c], k0, Lc.nz, false);
+  for (int k = k0; k < k1; ++k, c += Lc.slab) {
+    const T next = k + 1 < k1 ? comp[c + 4 * Lc.slab] : T(0);
+    T uvel, vvel, wvel;
+    mac_velocity(u, v, w, Lu, Lv, Lw, axis, i, j, k, uvel, vvel, wvel);
+    samples7(vx, comp, c, 1, vz[3], i, Lc.nx, false);
+    samples7(vy, comp, c, Lc.px, vz[3], j, Lc.ny, false);
+    const T dx = weno_upwind7(vx, inv_h, eps, uvel > T(0));
+    const T dy = weno_upwind7(vy, inv_h, eps, vvel > T(0));
+    const T dz = weno_upwind7(vz, inv_h, eps, wvel > T(0));
+    out[c] = vz[3] - dt * ((uvel * dx + vvel * dy) + wvel * dz);
+    slide7(vz, next, k, Lc.nz, false);
   }
 }
 
@@ -344,33 +386,30 @@ __device__ __forceinline__ void eno3_pair7(const T v[7], T h, T inv, T o2, T o3,
 // MAC component self-advection with ENO3 (the reference's use_3rd_eno_v,
 // ADVECTION_3D.h:323-325), every face of component `axis`.
 template <class T>
-__global__ void __launch_bounds__(kTX * kTY) k_eno3_mac(const T* __restrict__ comp, T* __restrict__ out,
+__global__ void __launch_bounds__(kColThreads) k_eno3_mac(const T* __restrict__ comp, T* __restrict__ out,
                                                      const T* __restrict__ u, const T* __restrict__ v,
                                                      const T* __restrict__ w, Lay Lc, Lay Lu, Lay Lv, Lay Lw,
-                                                     int axis, T h, T dt, int kchunk) {
-  __shared__ T ring[kRing * kRW * kRH];
-  const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTY;
-  const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+                                                     int axis, T h, T dt, int kchunk, int flat) {
+  int i, j;
+  if (!column_of(Lc, flat, i, j)) return;
   const int k0 = blockIdx.z * kchunk, k1 = min(Lc.nz, k0 + kchunk);
-  const bool valid = i < Lc.nx && j < Lc.ny;
   const T inv = T(1) / h, o2 = T(0.5) / h, o3 = inv * T(1) / T(3);
-  for (int kk = k0 - GH; kk < k0 + GH; ++kk) stage_plane(ring, comp, Lc, i0, j0, kk);
-  for (int k = k0; k < k1; ++k) {
-    stage_plane(ring, comp, Lc, i0, j0, k + GH);
-    __syncthreads();
-    if (valid) {
-      T uvel, vvel, wvel;
-      mac_velocity(u, v, w, Lu, Lv, Lw, axis, i, j, k, uvel, vvel, wvel);
-      T vx[7], vy[7], vz[7];
-      ring_samples(ring, k, vx, vy, vz);
-      T dxm, dxp, dym, dyp, dzm, dzp;
-      eno3_pair7(vx, h, inv, o2, o3, dxm, dxp);
-      eno3_pair7(vy, h, inv, o2, o3, dym, dyp);
-      eno3_pair7(vz, h, inv, o2, o3, dzm, dzp);
-      out[Lc.at(i, j, k)] = vx[3] - dt * ((uvel * (uvel > T(0) ? dxm : dxp) + vvel * (vvel > T(0) ? dym : dyp)) +
-                                          wvel * (wvel > T(0) ? dzm : dzp));
-    }
-    __syncthreads();
+  int64_t c = Lc.at(i, j, k0);
+  T vx[7], vy[7], vz[7];
+  samples7(vz, comp, c, Lc.slab, comp[c], k0, Lc.nz, false);
+  for (int k = k0; k < k1; ++k, c += Lc.slab) {
+    const T next = k + 1 < k1 ? comp[c + 4 * Lc.slab] : T(0);
+    T uvel, vvel, wvel;
+    mac_velocity(u, v, w, Lu, Lv, Lw, axis, i, j, k, uvel, vvel, wvel);
+    samples7(vx, comp, c, 1, vz[3], i, Lc.nx, false);
+    samples7(vy, comp, c, Lc.px, vz[3], j, Lc.ny, false);
+    T dxm, dxp, dym, dyp, dzm, dzp;
+    eno3_pair7(vx, h, inv, o2, o3, dxm, dxp);
+    eno3_pair7(vy, h, inv, o2, o3, dym, dyp);
+    eno3_pair7(vz, h, inv, o2, o3, dzm, dzp);
+    out[c] = vz[3] - dt * ((uvel * (uvel > T(0) ? dxm : dxp) + vvel * (vvel > T(0) ? dym : dyp)) +
+                           wvel * (wvel > T(0) ? dzm : dzp));
+    slide7(vz, next, k, Lc.nz, false);
   }
 }
 
@@ -441,43 +480,49 @@ __device__ __forceinline__ T godunov(T s, T dm, T dp, int& code, bool& shock) {
 
 // One pseudo-step phi - dtau*S*(|grad phi|_G - 1) with the sign-preserving
 // clamp; out = c0*base + c1*(that) when c0 != 0 (RK block combination).
+// first: the block's first step, whose src is the field S comes from: S is
+// formed here and stored in sgn for the steps that follow.
 template <class T>
-__global__ void __launch_bounds__(kTX * kTY) k_sussman(const T* __restrict__ src, const T* __restrict__ sgn,
-                                                    const T* __restrict__ base, T* __restrict__ out, Lay L, T inv_h,
-                                                    T eps, T dtau, T c0, T c1, int typo, int kchunk) {
-  __shared__ T ring[kRing * kRW * kRH];
-  const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTY;
-  const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+__global__ void __launch_bounds__(kColThreads) k_sussman(const T* __restrict__ src, T* __restrict__ sgn,
+                                                    const T* __restrict__ base, T* __restrict__ out, Lay L, T dx,
+                                                    T inv_h, T eps, T dtau, T c0, T c1, int typo, int first,
+                                                    int extrapolate, int kchunk, int flat) {
+  int i, j;
+  if (!column_of(L, flat, i, j)) return;
   const int k0 = blockIdx.z * kchunk, k1 = min(L.nz, k0 + kchunk);
-  const bool valid = i < L.nx && j < L.ny;
-  for (int kk = k0 - GH; kk < k0 + GH; ++kk) stage_plane(ring, src, L, i0, j0, kk);
-  for (int k = k0; k < k1; ++k) {
-    stage_plane(ring, src, L, i0, j0, k + GH);
-    __syncthreads();
-    if (valid) {
-      const int64_t c = L.at(i, j, k);
-      T vx[7], vy[7], vz[7];
-      ring_samples(ring, k, vx, vy, vz);
-      T dxm, dxp, dym, dyp, dzm, dzp;
-      weno_pair7(vx, inv_h, eps, dxm, dxp);
-      weno_pair7(vy, inv_h, eps, dym, dyp);
-      weno_pair7(vz, inv_h, eps, dzm, dzp);
-      const T s = sgn[c];
-      int cx, cy, cz;
-      bool shx, shy, shz;
-      const T gx = godunov(s, dxm, dxp, cx, shx);
-      const T gy = godunov(s, dym, dyp, cy, shy);
-      const T gz = godunov(s, dzm, dzp, cz, shz);
-      T mag = sqrt((gx * gx + gy * gy) + gz * gz) - T(1);
-      if (typo && shx && shy && cy == 1 && cz == 2) mag = (sqrt(gx * gx) + gy * gy) - T(1);
-      T r = vx[3] - dtau * s * mag;
-      if (s * r < T(0)) {
-        if (s < T(0)) r = -eps;
-        if (s > T(0)) r = eps;
-      }
-      out[c] = c0 == T(0) ? r : c0 * base[c] + c1 * r;
+  const bool ex = extrapolate != 0;
+  int64_t c = L.at(i, j, k0);
+  T vx[7], vy[7], vz[7];
+  samples7(vz, src, c, L.slab, src[c], k0, L.nz, ex);
+  for (int k = k0; k < k1; ++k, c += L.slab) {
+    const T next = k + 1 < k1 ? src[c + 4 * L.slab] : T(0);
+    T s;
+    if (first) {
+      s = vz[3] / sqrt(vz[3] * vz[3] + dx * dx);
+      sgn[c] = s;
+    } else {
+      s = sgn[c];
     }
-    __syncthreads();
+    samples7(vx, src, c, 1, vz[3], i, L.nx, ex);
+    samples7(vy, src, c, L.px, vz[3], j, L.ny, ex);
+    T dxm, dxp, dym, dyp, dzm, dzp;
+    weno_pair7(vx, inv_h, eps, dxm, dxp);
+    weno_pair7(vy, inv_h, eps, dym, dyp);
+    weno_pair7(vz, inv_h, eps, dzm, dzp);
+    int cx, cy, cz;
+    bool shx, shy, shz;
+    const T gx = godunov(s, dxm, dxp, cx, shx);
+    const T gy = godunov(s, dym, dyp, cy, shy);
+    const T gz = godunov(s, dzm, dzp, cz, shz);
+    T mag = sqrt((gx * gx + gy * gy) + gz * gz) - T(1);
+    if (typo && shx && shy && cy == 1 && cz == 2) mag = (sqrt(gx * gx) + gy * gy) - T(1);
+    T r = vz[3] - dtau * s * mag;
+    if (s * r < T(0)) {
+      if (s < T(0)) r = -eps;
+      if (s > T(0)) r = eps;
+    }
+    out[c] = c0 == T(0) ? r : c0 * base[c] + c1 * r;
+    slide7(vz, next, k, L.nz, ex);
   }
 }
 
@@ -523,27 +568,26 @@ template <class T>
 void weno5_levelset(const T* src, const T* base, T* out, const T* u, const T* v, const T* w, const Lay& L,
                     const Lay& Lu, const Lay& Lv, const Lay& Lw, double dx, double eps, double dt, double c0, double c1,
                     cudaStream_t s, const PipeGeom* pipe) {
-  const StagedGrid g = staged_grid(L);
+  const ColumnGrid g = column_grid(L);
   PipeGeom none{};
-  k_weno5_levelset<T><<<g.grid, dim3(kTX, kTY, 1), 0, s>>>(src, base, out, u, v, w, L, Lu, Lv, Lw, T(1.0 / dx),
-                                                           T(eps), T(dt), T(c0), T(c1), g.kchunk,
-                                                           pipe ? *pipe : none);
+  k_weno5_levelset<T><<<g.grid, kColThreads, 0, s>>>(src, base, out, u, v, w, L, Lu, Lv, Lw, T(1.0 / dx), T(eps),
+                                                     T(dt), T(c0), T(c1), g.kchunk, g.flat, pipe ? *pipe : none);
 }
 
 template <class T>
 void weno5_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
                const Lay& Lw, int axis, double dx, double eps, double dt, cudaStream_t s) {
-  const StagedGrid g = staged_grid(Lc);
-  k_weno5_mac<T><<<g.grid, dim3(kTX, kTY, 1), 0, s>>>(comp, out, u, v, w, Lc, Lu, Lv, Lw, axis, T(1.0 / dx), T(eps),
-                                                      T(dt), g.kchunk);
+  const ColumnGrid g = column_grid(Lc);
+  k_weno5_mac<T><<<g.grid, kColThreads, 0, s>>>(comp, out, u, v, w, Lc, Lu, Lv, Lw, axis, T(1.0 / dx), T(eps), T(dt),
+                                                g.kchunk, g.flat);
 }
 
 template <class T>
 void eno3_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
               const Lay& Lw, int axis, double dx, double dt, cudaStream_t s) {
-  const StagedGrid g = staged_grid(Lc);
-  k_eno3_mac<T><<<g.grid, dim3(kTX, kTY, 1), 0, s>>>(comp, out, u, v, w, Lc, Lu, Lv, Lw, axis, T(dx), T(dt),
-                                                     g.kchunk);
+  const ColumnGrid g = column_grid(Lc);
+  k_eno3_mac<T><<<g.grid, kColThreads, 0, s>>>(comp, out, u, v, w, Lc, Lu, Lv, Lw, axis, T(dx), T(dt), g.kchunk,
+                                               g.flat);
 }
 
 template <class T>
@@ -569,11 +613,11 @@ void sign_function(const T* phi, T* sgn, const Lay& L, double dx, cudaStream_t s
 }
 
 template <class T>
-void sussman_step(const T* src, const T* sgn, const T* base, T* out, const Lay& L, double dx, double eps, double dtau,
-                  double c0, double c1, int typo, cudaStream_t s) {
-  const StagedGrid g = staged_grid(L);
-  k_sussman<T><<<g.grid, dim3(kTX, kTY, 1), 0, s>>>(src, sgn, base, out, L, T(1.0 / dx), T(eps), T(dtau), T(c0),
-                                                    T(c1), typo, g.kchunk);
+void sussman_step(const T* src, T* sgn, const T* base, T* out, const Lay& L, double dx, double eps, double dtau,
+                  double c0, double c1, int typo, int first, int extrapolate, cudaStream_t s) {
+  const ColumnGrid g = column_grid(L);
+  k_sussman<T><<<g.grid, kColThreads, 0, s>>>(src, sgn, base, out, L, T(dx), T(1.0 / dx), T(eps), T(dtau), T(c0),
+                                              T(c1), typo, first, extrapolate, g.kchunk, g.flat);
 }
 
 template <class T>
@@ -606,8 +650,8 @@ void zero_walls(T* f, const Lay& L, int axis, cudaStream_t s) {
   template void eno3_mac<T>(const T*, T*, const T*, const T*, const T*, const Lay&, const Lay&, const Lay&,           \
                             const Lay&, int, double, double, cudaStream_t);                                          \
   template void sign_function<T>(const T*, T*, const Lay&, double, cudaStream_t);                                    \
-  template void sussman_step<T>(const T*, const T*, const T*, T*, const Lay&, double, double, double, double, double, \
-                                int, cudaStream_t);                                                                   \
+  template void sussman_step<T>(const T*, T*, const T*, T*, const Lay&, double, double, double, double, double, int, \
+                                int, int, cudaStream_t);                                                                   \
   template void axpby<T>(T*, const T*, const T*, double, double, const Lay&, cudaStream_t);                          \
   template void add_const_faces<T>(T*, const Lay&, int, double, int, cudaStream_t);                                  \
   template void zero_walls<T>(T*, const Lay&, int, cudaStream_t);
