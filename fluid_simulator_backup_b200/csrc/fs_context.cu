@@ -612,6 +612,13 @@ fs_status advect_levelset_t(fs_ctx* c, double dt, Tape* tp = nullptr) {
       fill_periodic_y<S>(src, c->Lc, s);
       c->launches += 1;
     }
+    if (tp) {
+      // a taped forward keeps its own evaluation order (fs_taped.cu)
+      fill_extrap<S>(src, c->Lc, s);
+      taped_levelset<S>(src, base, out, u, v, w, c->Lc, c->Lu, c->Lv, c->Lw, dx, eps, dt, c0, c1, s);
+      c->launches += 2;
+      return;
+    }
     weno5_levelset<S>(src, base, out, u, v, w, c->Lc, c->Lu, c->Lv, c->Lw, dx, eps, dt, c0, c1, s, pg);
     c->launches += 1;
   };
@@ -639,7 +646,7 @@ static double velocity_epsilon(const fs_ctx* c) {
 }
 
 template <class S>
-fs_status advect_velocity_t(fs_ctx* c, double dt) {
+fs_status advect_velocity_t(fs_ctx* c, double dt, bool taped = false) {
   const double eps = velocity_epsilon(c), dx = c->grid.dx;
   S *u = F<S>(c->u), *v = F<S>(c->v), *w = F<S>(c->w);
   if (c->pipe.on) {
@@ -666,6 +673,10 @@ fs_status advect_velocity_t(fs_ctx* c, double dt) {
     eno3_mac<S>(u, F<S>(c->ua), u, v, w, c->Lu, c->Lu, c->Lv, c->Lw, 0, dx, dt, c->stream);
     eno3_mac<S>(v, F<S>(c->va), u, v, w, c->Lv, c->Lu, c->Lv, c->Lw, 1, dx, dt, c->stream);
     eno3_mac<S>(w, F<S>(c->wa), u, v, w, c->Lw, c->Lu, c->Lv, c->Lw, 2, dx, dt, c->stream);
+  } else if (taped) {
+    taped_mac<S>(u, F<S>(c->ua), u, v, w, c->Lu, c->Lu, c->Lv, c->Lw, 0, dx, eps, dt, c->stream);
+    taped_mac<S>(v, F<S>(c->va), u, v, w, c->Lv, c->Lu, c->Lv, c->Lw, 1, dx, eps, dt, c->stream);
+    taped_mac<S>(w, F<S>(c->wa), u, v, w, c->Lw, c->Lu, c->Lv, c->Lw, 2, dx, eps, dt, c->stream);
   } else {
     weno5_mac<S>(u, F<S>(c->ua), u, v, w, c->Lu, c->Lu, c->Lv, c->Lw, 0, dx, eps, dt, c->stream);
     weno5_mac<S>(v, F<S>(c->va), u, v, w, c->Lv, c->Lu, c->Lv, c->Lw, 1, dx, eps, dt, c->stream);
@@ -722,16 +733,27 @@ fs_status reinit_block_t(fs_ctx* c, void* in, void* out, void* base, double c0, 
     else if (out != in) CK(cudaMemcpyAsync(out, in, c->Lc.total * c->S(), cudaMemcpyDeviceToDevice, s));
     return FS_OK;
   }
-  c->launches += (c->pipe.on ? 2 : 1) * n;
+  c->launches += (c->pipe.on || tape ? 2 : 1) * n;
+  if (tape) {
+    sign_function<S>(F<S>(in), F<S>(c->sgn), c->Lc, dx, s);
+    c->launches += 1;
+  }
   void* cur = in;
   for (int it = 0; it < n; ++it) {
     const bool last = it == n - 1;
     void* dst = last ? out : (cur == scrA ? scrB : scrA);
     if (tape) CK(cudaMemcpyAsync((*tape)[it], cur, c->Lc.total * c->S(), cudaMemcpyDeviceToDevice, s));
     if (c->pipe.on) fill_periodic_y<S>(F<S>(cur), c->Lc, s);  // ADVECTION_3D.h:360-378
-    sussman_step<S>(F<S>(cur), F<S>(c->sgn), F<S>(base), F<S>(dst), c->Lc, dx, P.weno_epsilon, dtau,
-                    last ? c0 : 0.0, last ? c1 : 1.0, (P.flags & FS_FLAG_REINIT_TYPO) ? 1 : 0, it == 0 ? 1 : 0,
-                    c->pipe.on ? 0 : 1, s);
+    const double a0 = last ? c0 : 0.0, a1 = last ? c1 : 1.0;
+    const int typo = (P.flags & FS_FLAG_REINIT_TYPO) ? 1 : 0;
+    if (tape) {
+      fill_extrap<S>(F<S>(cur), c->Lc, s);
+      taped_sussman<S>(F<S>(cur), F<S>(c->sgn), F<S>(base), F<S>(dst), c->Lc, dx, P.weno_epsilon, dtau, a0, a1, typo,
+                       s);
+    } else {
+      sussman_step<S>(F<S>(cur), F<S>(c->sgn), F<S>(base), F<S>(dst), c->Lc, dx, P.weno_epsilon, dtau, a0, a1, typo,
+                      it == 0 ? 1 : 0, c->pipe.on ? 0 : 1, s);
+    }
     cur = dst;
   }
   CK(cudaGetLastError());
@@ -1240,7 +1262,7 @@ template <class S>
 fs_status stage_t(fs_ctx* c, double dt, double c0, double c1, fs_step_report* rep, Tape* tp = nullptr,
                   int stage = 0) {
   if (tp) CKS(tape_velocity(c, tp->vel[stage][0]));
-  CKS(advect_velocity_t<S>(c, dt));
+  CKS(advect_velocity_t<S>(c, dt, tp != nullptr));
   const Lay* lays[3] = {&c->Lu, &c->Lv, &c->Lw};
   if (!(c->prm.flags & FS_FLAG_FAITHFUL_PROJECTION) && !c->pipe.on) {
     // no penetration: advection also updates the wall faces, which hold zero

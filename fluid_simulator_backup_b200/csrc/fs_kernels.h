@@ -106,6 +106,18 @@ int fast_sweeping(const T* in, T* out, unsigned char* fixed, const Lay& L, doubl
 template <class T>
 void sussman_step(const T* src, T* sgn, const T* base, T* out, const Lay& L, double dx, double eps, double dtau,
                   double c0, double c1, int typo, int first, int extrapolate, cudaStream_t s);
+// these in the fixed evaluation order of a taped forward (fs_taped.cu);
+// level-set ghosts and the sign field are read
+template <class T>
+void taped_levelset(const T* src, const T* base, T* out, const T* u, const T* v, const T* w, const Lay& L,
+                    const Lay& Lu, const Lay& Lv, const Lay& Lw, double dx, double eps, double dt, double c0, double c1,
+                    cudaStream_t s);
+template <class T>
+void taped_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
+               const Lay& Lw, int axis, double dx, double eps, double dt, cudaStream_t s);
+template <class T>
+void taped_sussman(const T* src, const T* sgn, const T* base, T* out, const Lay& L, double dx, double eps, double dtau,
+                   double c0, double c1, int typo, cudaStream_t s);
 template <class T> void axpby(T* out, const T* x, const T* y, double a, double b, const Lay& L, cudaStream_t s);
 template <class T> void add_const_faces(T* f, const Lay& L, int axis, double value, int skip_walls, cudaStream_t s);
 template <class T> void zero_walls(T* f, const Lay& L, int axis, cudaStream_t s);
