@@ -111,6 +111,13 @@ __device__ __forceinline__ double face_coef(double pc, double pn, double vneg, d
   return vc * vn * (an + ac) / (vn * ac + vc * an);
 }
 
+// One field of a solver state at the start of a kernel: written by an earlier
+// kernel, so an L1-cached read is current, and all warps of an SM share one
+// fetch.  (Read as volatile, every warp of the grid fetches the same L2 line:
+// 40 us for the 32,768 warps of a 256^3 kernel that has nothing else to do.)
+template <class T>
+__device__ __forceinline__ T state_read(const T* p) { return __ldca(p); }
+
 // Block-wide sum of a double (any block size that is a multiple of 32, up
 // to 1024).  Result valid in thread 0.
 __device__ __forceinline__ double warp_sum(double v) {

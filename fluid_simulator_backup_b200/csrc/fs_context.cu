@@ -222,6 +222,7 @@ fs_status mg_alloc(fs_ctx* c) {
       }
       if (l < M.top)
         for (unsigned char** p : {&m.cls[0], &m.cls[1]}) take((void**)p, m.H.total);
+      if (l == 0) take((void**)&m.ccls, m.L.total);
     }
     if (!pass) CKS(dalloc(c, (void**)&base, off));
   }
@@ -1922,7 +1923,7 @@ fs_status fs_create(const fs_grid_desc* grid, const fs_params* params, fs_ctx** 
   cg_prepare<float, float>();
   int nblk = std::max(pcg_blocks(c->Lu), std::max(pcg_blocks(c->Lv), pcg_blocks(c->Lw))) * 2 + 64;
   for (const Lay* L : {&c->Lc, &c->Lu, &c->Lv, &c->Lw}) nblk = std::max(nblk, cg_max_blocks(*L));
-  if (c->fp32) nblk = std::max(nblk, std::max(rb_blocks(c->Lh), mg_max_blocks(c->Lh)));
+  if (c->fp32) nblk = std::max(nblk, std::max(rb_blocks(c->Lh), mg_max_blocks(c->Lc)));
   if ((s = dalloc(c, (void**)&c->partials, (size_t)nblk * 3 * sizeof(double))) != FS_OK) return fail(s);
   if ((s = dalloc(c, (void**)&c->tickets, 8 * sizeof(unsigned int))) != FS_OK) return fail(s);
   if ((s = dalloc(c, (void**)&c->scalars, 16 * sizeof(double))) != FS_OK) return fail(s);

@@ -244,6 +244,7 @@ struct MgLevel {
   Lay L, H;                            // cell layout of the couplings, packed layout of each colour
   float *ax = nullptr, *ay = nullptr, *az = nullptr;
   unsigned char* cls[2] = {};          // per colour: 1 or 2, the phase whose uniform coupling all faces carry; 0: mixed
+  unsigned char* ccls = nullptr;       // level 0: the classes in the cell layout too
   float* x[2] = {};                    // by colour (0 red, 1 black): the cycle's solution (level 0: z)
   float* b[2] = {};                    // and right-hand side (level 0: the residual r)
   float a[2] = {};                     // the uniform couplings of the two phases
@@ -270,7 +271,7 @@ struct MgState {
 };
 int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top);
 cudaError_t mg_prepare();
-int mg_max_blocks(const Lay& H);
+int mg_max_blocks(const Lay& L);
 // Each returns the number of kernels launched.  mg_build: the operator of
 // every level from st->phi.  mg_start: true residual, first cycle and
 // direction.  mg_iteration: one CG iteration; with `loop` its last kernel

@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_init(Op7<V> A, const RT* b,
 template <class V, class RT>
 __global__ void __launch_bounds__(kRedThreads) k_pcg_pupdate(Op7<V> A, const RT* __restrict__ r, V* __restrict__ p,
                                                              PcgState* st) {
-  if (((volatile PcgState*)st)->done) return;
-  const RT beta = (RT)((volatile PcgState*)st)->beta;
+  if (state_read(&st->done)) return;
+  const RT beta = (RT)state_read(&st->beta);
   Cursor cur;
   for (cur.init(A.L); cur.valid(A.L); cur.next(A.L)) {
     const int64_t c = A.L.at(cur.i, cur.j, cur.k);
@@ -406,7 +406,7 @@ __device__ __forceinline__ void spmv_alpha(double pq, PcgState* st, double* part
 template <class V, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_cg_spmv(Op7<V> A, const V* __restrict__ p, V* __restrict__ q,
                                                  PcgState* st, double* partials, int kchunk) {
-  if (((volatile PcgState*)st)->done) return;
+  if (state_read(&st->done)) return;
   const Lay& L = A.L;
   const int w = blockIdx.x * 32 + threadIdx.x;  // vector index along x
   const int j = blockIdx.y * 8 + threadIdx.y;
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256, MINB) k_cg_spmv(Op7<V> A, const V* __rest
 template <class V>
 __global__ void __launch_bounds__(kRedThreads) k_pq_alpha(Op7<V> A, const V* __restrict__ p, const V* __restrict__ q,
                                                           PcgState* st, double* partials) {
-  if (((volatile PcgState*)st)->done) return;
+  if (state_read(&st->done)) return;
   double pq = 0.0;
   VecCursor vc;
   for (vc.init(A.L); vc.valid(); vc.next()) {
@@ -472,8 +472,8 @@ __global__ void __launch_bounds__(kRedThreads) k_pq_alpha(Op7<V> A, const V* __r
 template <class V>
 __global__ void __launch_bounds__(kRedThreads) k_cg_update(Op7<V> A, V* __restrict__ r, const V* __restrict__ q,
                                                            PcgState* st, double* partials) {
-  if (((volatile PcgState*)st)->done) return;
-  const V alpha = (V)((volatile PcgState*)st)->alpha;
+  if (state_read(&st->done)) return;
+  const V alpha = (V)state_read(&st->alpha);
   double rz = 0.0, rr = 0.0;
   VecCursor vc;
   for (vc.init(A.L); vc.valid(); vc.next()) {
@@ -542,12 +542,11 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(Op7<V> A, V* __restri
 template <class V, class X>
 __global__ void __launch_bounds__(kRedThreads) k_cg_pupdate(Op7<V> A, X* __restrict__ x, const V* __restrict__ r,
                                                             V* __restrict__ p, PcgState* st) {
-  const volatile PcgState* vs = (volatile PcgState*)st;
-  const bool move_x = vs->x_pending != 0;
-  const bool move_p = vs->done == 0;
+  const bool move_x = state_read(&st->x_pending) != 0;
+  const bool move_p = state_read(&st->done) == 0;
   if (!move_x && !move_p) return;  // uniform: every block reads the same state
-  const double alpha = vs->alpha;
-  const V beta = (V)vs->beta;
+  const double alpha = state_read(&st->alpha);
+  const V beta = (V)state_read(&st->beta);
   VecCursor vc;
   for (vc.init(A.L); vc.valid(); vc.next()) {
     const int i0 = 4 * vc.cur.i;

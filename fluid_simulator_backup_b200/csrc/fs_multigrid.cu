@@ -47,8 +47,7 @@
 // r and z are stored by colour in the packed half layout of fs_redblack.cu
 // (slot (h, j, k): red cell at i = 2h + ((j+k)&1), black at 2h + ((j+k+1)&1)),
 // so that a half sweep reads and writes contiguous rows; x, p and q are in
-// the cell layout.  The kernels of the iteration take one slot (two cells)
-// per thread and move along z.
+// the cell layout.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -59,13 +58,14 @@ namespace fsb {
 
 namespace {
 
-constexpr int kBX = 32, kBY = 8;
+constexpr int kThreads = 256;
 
 // one level as the kernels see it
 struct Lev {
   Lay L, H;
   const float *ax, *ay, *az;
   const unsigned char* cls[2];
+  const unsigned char* ccls;  // finest level: the same classes in the cell layout
   float* x[2];
   float* b[2];
   float a[3];   // the uniform coupling of class 1 and 2 (index 0 unused)
@@ -79,6 +79,7 @@ Lev lev_of(const MgLevel& m) {
   v.ax = m.ax;
   v.ay = m.ay;
   v.az = m.az;
+  v.ccls = m.ccls;
   for (int c = 0; c < 2; ++c) {
     v.cls[c] = m.cls[c];
     v.x[c] = m.x[c];
@@ -92,17 +93,39 @@ Lev lev_of(const MgLevel& m) {
   return v;
 }
 
-// planes per block: up to 8, fewer where that would leave the GPU idle
-int chunk_of(const Lay& H) {
-  const int64_t tiles = (int64_t)((H.nx + kBX - 1) / kBX) * ((H.ny + kBY - 1) / kBY);
-  int c = (int)(tiles * H.nz / (148 * 8));
-  return c < 1 ? 1 : (c > 8 ? 8 : c);
-}
-dim3 grid_of(const Lay& H, int chunk) {
-  return dim3((H.nx + kBX - 1) / kBX, (H.ny + kBY - 1) / kBY, (H.nz + chunk - 1) / chunk);
+// Launch of a kernel whose threads walk the columns of a plane (x fastest,
+// `per` items along x each) up chunks of z planes.  Consecutive columns
+// instead of tiles: no thread is left over at the row ends, and a thread's
+// neighbours come from L1 either way.  Chunks of up to 8 planes, fewer where
+// that would leave the GPU idle.
+struct Columns {
+  dim3 grid;
+  int w, chunk;  // items per row, planes per block
+};
+Columns columns(int nx, int ny, int nz, int per) {
+  Columns c;
+  c.w = (nx + per - 1) / per;
+  const int64_t bx = ((int64_t)c.w * ny + kThreads - 1) / kThreads;
+  const int64_t ch = bx * nz / (148 * 12);
+  c.chunk = (int)(ch < 1 ? 1 : (ch > 8 ? 8 : ch));
+  c.grid = dim3((unsigned)bx, (unsigned)((nz + c.chunk - 1) / c.chunk), 1);
+  return c;
 }
 
-__device__ __forceinline__ bool stopped(const MgState* st) { return ((const volatile MgState*)st)->done != 0; }
+struct Column {
+  int i, j, k0, k1;  // i: the first of the thread's items, in items
+  bool ok;
+  __device__ __forceinline__ Column(int w, int ny, int nz, int chunk) {
+    const unsigned t = blockIdx.x * (unsigned)kThreads + threadIdx.x;
+    j = (int)(t / (unsigned)w);
+    i = (int)(t - (unsigned)j * (unsigned)w);
+    k0 = blockIdx.y * chunk;
+    k1 = min(nz, k0 + chunk);
+    ok = j < ny;
+  }
+};
+
+__device__ __forceinline__ bool stopped(const MgState* st) { return state_read(&st->done) != 0; }
 
 __device__ __forceinline__ int faces_inside(const Lay& L, int i, int j, int k) {
   return (i > 0) + (i < L.nx - 1) + (j > 0) + (j < L.ny - 1) + (k > 0) + (k < L.nz - 1);
@@ -124,117 +147,264 @@ __device__ __forceinline__ float first_sweep(const Lev& v, int cl, float b, int 
   return d > 0.0f ? b / d : 0.0f;
 }
 
-// the coarse value under fine cell (i, j, k)
-__device__ __forceinline__ float coarse_at(const Lev& e, int i, int j, int k) {
-  const int I = i >> 1, J = j >> 1, K = k >> 1;
+struct F4 {
+  float v[4];
+};
+__device__ __forceinline__ F4 load4(const float* p) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  return {{q.x, q.y, q.z, q.w}};
+}
+__device__ __forceinline__ void store4(float* p, const F4& a) {
+  *reinterpret_cast<float4*>(p) = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
+}
+
+// The coarse values over slots h .. h+3 (coarse cells I = h .. h+3, h a
+// multiple of 4) of a row in coarse row (J, K): two of each colour.  Coarse
+// ghosts hold 0.
+__device__ __forceinline__ F4 coarse4(const Lev& e, int h, int J, int K) {
+  const int g = (J + K) & 1;  // the colour of the even ones
+  const int64_t s = e.H.at(h >> 1, J, K);
+  const float2 a = *reinterpret_cast<const float2*>(e.x[g] + s), b = *reinterpret_cast<const float2*>(e.x[1 - g] + s);
+  return {{a.x, b.x, a.y, b.y}};
+}
+__device__ __forceinline__ float coarse1(const Lev& e, int I, int J, int K) {
   return e.x[(I + J + K) & 1][e.H.at(I >> 1, J, K)];
 }
 
 // ---------------------------------------------------------------------------
-// Half sweep of one colour.  CORRECT: the first sweep after the coarse
-// correction; the other colour's values are read as x + e, which is all the
-// correction has to do (the swept colour's old values are not used, the
-// other colour is swept next).
+// Half sweep of one colour, four slots per thread.  The other colour's values
+// in the thread's row are one vector (slot h holds the x neighbours of slots h
+// and h -+ 1) and, plane by plane, also its z neighbours: marching up, a plane
+// costs one new vector of them, the two y rows, b, one neighbouring slot and
+// four class bytes.  Measured at 256^3 against one slot per thread (whose
+// loads waited on the class byte, 30 % of HBM) and a dot product of its own:
+// the last black and red sweep and r.z 41 + 41 + 39 -> 32 + 39 us, the
+// restriction 71 -> 48, the SpMV (likewise four cells) 77 -> 52, the update
+// 153 -> 112.
+//
+// CORRECT: the first sweep after the coarse correction; the other colour's
+// values are read as x + e, which is all the correction has to do (the swept
+// colour's old values are not used, the other colour is swept next).  Values
+// past the box stay 0.
+// DOT: the last black (1) and red (2) sweep on the finest level also sum r.z;
+// the red one's last block adds both up and sets beta.
 // ---------------------------------------------------------------------------
-template <bool CORRECT>
-__global__ void __launch_bounds__(kBX * kBY) k_mg_sweep(Lev v, Lev e, int color, const MgState* st, int kchunk) {
+template <bool CORRECT, int DOT>
+__global__ void __launch_bounds__(kThreads) k_mg_sweep(Lev v, Lev e, int color, MgState* st, double* partials, int w,
+                                                       int chunk) {
   if (stopped(st)) return;
   const Lay &L = v.L, &H = v.H;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  if (h >= H.nx || j >= H.ny) return;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
-  const float* __restrict__ xo = v.x[1 - color];
-  const float* __restrict__ b = v.b[color];
-  const unsigned char* __restrict__ cls = v.cls[color];
-  float* __restrict__ x = v.x[color];
-  int64_t s = H.at(h, j, k0);
-  for (int k = k0; k < k1; ++k, s += H.slab) {
-    const int par = (j + k + color) & 1, i = 2 * h + par;
-    if (i >= L.nx) continue;
-    const int cl = cls[s];
-    const float bv = b[s];
-    float xm = xo[s + par - 1], xp = xo[s + par];
-    float ym = xo[s - H.px], yp = xo[s + H.px];
-    float zm = xo[s - H.slab], zp = xo[s + H.slab];
+  const Column q(w, H.ny, H.nz, chunk);
+  double rz = 0.0;
+  if (q.ok) {
+    const int h = 4 * q.i, j = q.j;
+    const float* __restrict__ xo = v.x[1 - color];
+    const float* __restrict__ b = v.b[color];
+    const unsigned char* __restrict__ cls = v.cls[color];
+    float* __restrict__ x = v.x[color];
+    int64_t s = H.at(h, j, q.k0);
+    const int fyz0 = (j > 0) + (j < L.ny - 1);
+    // other colour's row at plane k: x + e, zero in slots without a cell.
+    // Slot m's cell of that colour is at i = 2 (h + m) + (1 - par).
+    auto correct = [&](F4& r, int par, int k) {
+      const F4 c = coarse4(e, h, j >> 1, k >> 1);
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (2 * (h + m) + 1 - par < L.nx) r.v[m] += c.v[m];
+    };
+    const int p0 = (j + q.k0 + color) & 1;
+    F4 zm = load4(xo + s - H.slab), xc = load4(xo + s);
     if (CORRECT) {
-      if (i > 0) xm += coarse_at(e, i - 1, j, k);
-      if (i < L.nx - 1) xp += coarse_at(e, i + 1, j, k);
-      if (j > 0) ym += coarse_at(e, i, j - 1, k);
-      if (j < L.ny - 1) yp += coarse_at(e, i, j + 1, k);
-      if (k > 0) zm += coarse_at(e, i, j, k - 1);
-      if (k < L.nz - 1) zp += coarse_at(e, i, j, k + 1);
+      if (q.k0 > 0) correct(zm, 1 - p0, q.k0 - 1);
+      correct(xc, p0, q.k0);
     }
-    float out;
-    if (cl) {
-      // neighbours beyond a wall hold 0 and are not counted
-      out = over_faces(fmaf(bv, v.ia[cl], ((xm + xp) + (ym + yp)) + (zm + zp)), faces_inside(L, i, j, k));
-    } else {
-      const Couplings a = couplings_at(v, L.at(i, j, k));
-      float num = a.xm * xm + a.xp * xp;
-      num += a.ym * ym + a.yp * yp;
-      num += a.zm * zm + a.zp * zp;
-      const float d = a.sum();
-      out = d > 0.0f ? (bv + num) / d : 0.0f;
+    for (int k = q.k0; k < q.k1; ++k, s += H.slab) {
+      const int par = (j + k + color) & 1;
+      F4 zp = load4(xo + s + H.slab);
+      F4 ym = load4(xo + s - H.px), yp = load4(xo + s + H.px);
+      const F4 bv = load4(b + s);
+      const unsigned cl = *reinterpret_cast<const unsigned*>(cls + s);
+      float side = xo[par ? s + 4 : s - 1];
+      if (CORRECT) {
+        if (k < L.nz - 1) correct(zp, 1 - par, k + 1);
+        const F4 cm = coarse4(e, h, (j - 1) >> 1, k >> 1);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) ym.v[m] += cm.v[m];  // (a ghost row's coarse row is a ghost too)
+        if (j < L.ny - 1) {
+          const F4 cp = coarse4(e, h, (j + 1) >> 1, k >> 1);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) yp.v[m] += cp.v[m];
+        }
+        if (par) {
+          if (2 * (h + 4) < L.nx) side += coarse1(e, h + 4, j >> 1, k >> 1);
+        } else if (h > 0) {
+          side += coarse1(e, h - 1, j >> 1, k >> 1);
+        }
+      }
+      const int fyz = fyz0 + (k > 0) + (k < L.nz - 1);
+      F4 out;
+      const int c0 = cl & 255u;
+      if (c0 && cl == 0x01010101u * c0) {
+        const float ia = v.ia[c0];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const int i = 2 * (h + m) + par;
+          const float xs = par ? (m < 3 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
+          // neighbours beyond a wall hold 0 and are not counted
+          const float sum = fmaf(bv.v[m], ia, ((xc.v[m] + xs) + (ym.v[m] + yp.v[m])) + (zm.v[m] + zp.v[m]));
+          out.v[m] = over_faces(sum, fyz + (i > 0) + (i < L.nx - 1));
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const int i = 2 * (h + m) + par;
+          out.v[m] = 0.0f;
+          if (i >= L.nx) continue;
+          const float xs = par ? (m < 3 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
+          const int cm = (cl >> (8 * m)) & 255u;
+          if (cm) {
+            const float sum = fmaf(bv.v[m], v.ia[cm], ((xc.v[m] + xs) + (ym.v[m] + yp.v[m])) + (zm.v[m] + zp.v[m]));
+            out.v[m] = over_faces(sum, fyz + (i > 0) + (i < L.nx - 1));
+          } else {
+            const Couplings a = couplings_at(v, L.at(i, j, k));
+            float num = par ? a.xm * xc.v[m] + a.xp * xs : a.xm * xs + a.xp * xc.v[m];
+            num += a.ym * ym.v[m] + a.yp * yp.v[m];
+            num += a.zm * zm.v[m] + a.zp * zp.v[m];
+            const float d = a.sum();
+            out.v[m] = d > 0.0f ? (bv.v[m] + num) / d : 0.0f;
+          }
+        }
+      }
+      store4(x + s, out);
+      if (DOT) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) rz += (double)bv.v[m] * (double)out.v[m];
+      }
+      zm = xc;
+      xc = zp;
     }
-    x[s] = out;
+  }
+  if (DOT) {
+    rz = block_sum(rz);
+    const int nb = num_blocks();
+    if (DOT == 1) {
+      if (thread0()) partials[flat_block()] = rz;
+      return;
+    }
+    // two ranges of partial sums: the black sweep's, then this one's
+    __shared__ bool is_last;
+    if (thread0()) {
+      partials[nb + flat_block()] = rz;
+      __threadfence();
+      is_last = atomicAdd(&st->ticket, 1u) == (unsigned)(nb - 1);
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    double sum = 0.0;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < 2 * nb; t += kThreads) sum += __ldcg(partials + t);
+    sum = block_sum(sum);
+    if (thread0()) {
+      st->ticket = 0u;
+      const double old = st->rz;
+      st->beta = (st->restart || !(old > 0.0)) ? 0.0 : sum / old;
+      st->restart = 0;
+      st->rz = sum;
+      if (!isfinite(sum) || !(sum > 0.0)) {
+        st->status = PCG_STAGNATED;
+        st->done = 1;
+      }
+    }
   }
 }
 
-// residual of one cell (slot s of colour `color`) for the restriction
-__device__ __forceinline__ float residual_at(const Lev& v, int color, int h, int j, int k) {
+// Residual of four slots of one row (colour `color`, the one not swept last),
+// zero in slots without a cell.
+__device__ __forceinline__ F4 residual4(const Lev& v, int color, int h, int j, int k) {
+  F4 r = {{0.0f, 0.0f, 0.0f, 0.0f}};
   const Lay &L = v.L, &H = v.H;
-  const int par = (j + k + color) & 1, i = 2 * h + par;
-  if (i >= L.nx || j >= L.ny || k >= L.nz) return 0.0f;
+  if (j >= L.ny || k >= L.nz) return r;
+  const int par = (j + k + color) & 1;
   const int64_t s = H.at(h, j, k);
   const float* __restrict__ xo = v.x[1 - color];
-  const int cl = v.cls[color][s];
-  const float xc = v.x[color][s], b = v.b[color][s];
-  const float xm = xo[s + par - 1], xp = xo[s + par];
-  const float ym = xo[s - H.px], yp = xo[s + H.px];
-  const float zm = xo[s - H.slab], zp = xo[s + H.slab];
-  if (cl) {
-    const float n = (float)faces_inside(L, i, j, k);
-    return fmaf(v.a[cl], (((xm + xp) + (ym + yp)) + (zm + zp)) - n * xc, b);
+  const F4 xc = load4(xo + s), ym = load4(xo + s - H.px), yp = load4(xo + s + H.px), zm = load4(xo + s - H.slab),
+           zp = load4(xo + s + H.slab), own = load4(v.x[color] + s), b = load4(v.b[color] + s);
+  const unsigned cl = *reinterpret_cast<const unsigned*>(v.cls[color] + s);
+  const float side = xo[par ? s + 4 : s - 1];
+  const int fyz = (j > 0) + (j < L.ny - 1) + (k > 0) + (k < L.nz - 1);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int i = 2 * (h + m) + par;
+    if (i >= L.nx) continue;
+    const float xs = par ? (m < 3 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
+    const float o = own.v[m];
+    const int cm = (cl >> (8 * m)) & 255u;
+    if (cm) {
+      const float n = (float)(fyz + (i > 0) + (i < L.nx - 1));
+      r.v[m] = fmaf(v.a[cm], (((xc.v[m] + xs) + (ym.v[m] + yp.v[m])) + (zm.v[m] + zp.v[m])) - n * o, b.v[m]);
+    } else {
+      // a wall's coupling is zero, so its neighbour value does not matter
+      const Couplings a = couplings_at(v, L.at(i, j, k));
+      float q = par ? a.xm * (xc.v[m] - o) + a.xp * (xs - o) : a.xm * (xs - o) + a.xp * (xc.v[m] - o);
+      q += a.ym * (ym.v[m] - o) + a.yp * (yp.v[m] - o);
+      q += a.zm * (zm.v[m] - o) + a.zp * (zp.v[m] - o);
+      r.v[m] = b.v[m] + q;
+    }
   }
-  const Couplings a = couplings_at(v, L.at(i, j, k));
-  float q = a.xm * (xm - xc) + a.xp * (xp - xc);
-  // a wall's coupling is zero, so its neighbour value does not matter
-  q += a.ym * (ym - xc) + a.yp * (yp - xc);
-  q += a.zm * (zm - xc) + a.zp * (zp - xc);
-  return b + q;
+  return r;
 }
 
 // Restriction: the residual of the colour that was not swept last (the other
 // one's is zero) summed over each aggregate into the coarse right-hand side,
 // and the coarse level's first red sweep.  The packed slots of coarse cell
-// (I, J, K) are (I, 2J..2J+1, 2K..2K+1): contiguous across the warp.
-__global__ void __launch_bounds__(kBX * kBY) k_mg_restrict(Lev v, Lev e, int color, const MgState* st, int kchunk) {
+// (I, J, K) are (I, 2J..2J+1, 2K..2K+1): a thread takes four coarse cells.
+__global__ void __launch_bounds__(kThreads) k_mg_restrict(Lev v, Lev e, int color, const MgState* st, int w,
+                                                          int chunk) {
   if (stopped(st)) return;
-  const int I = blockIdx.x * kBX + threadIdx.x, J = blockIdx.y * kBY + threadIdx.y;
-  if (I >= e.L.nx || J >= e.L.ny) return;
-  const int K0 = blockIdx.z * kchunk, K1 = min(e.L.nz, K0 + kchunk);
-  for (int K = K0; K < K1; ++K) {
-    float r = residual_at(v, color, I, 2 * J, 2 * K) + residual_at(v, color, I, 2 * J + 1, 2 * K);
-    r += residual_at(v, color, I, 2 * J, 2 * K + 1) + residual_at(v, color, I, 2 * J + 1, 2 * K + 1);
-    const int cc = (I + J + K) & 1;
+  const Column q(w, e.L.ny, e.L.nz, chunk);
+  if (!q.ok) return;
+  const int I = 4 * q.i, J = q.j;
+  for (int K = q.k0; K < q.k1; ++K) {
+    const F4 a = residual4(v, color, I, 2 * J, 2 * K), b = residual4(v, color, I, 2 * J + 1, 2 * K),
+             c = residual4(v, color, I, 2 * J, 2 * K + 1), d = residual4(v, color, I, 2 * J + 1, 2 * K + 1);
+    F4 r;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) r.v[m] = (a.v[m] + b.v[m]) + (c.v[m] + d.v[m]);
+    const int g = (J + K) & 1;  // the colour of the even coarse cells; cells past the box got 0
     const int64_t s = e.H.at(I >> 1, J, K);
-    e.b[cc][s] = r;
+    *reinterpret_cast<float2*>(e.b[g] + s) = make_float2(r.v[0], r.v[2]);
+    *reinterpret_cast<float2*>(e.b[1 - g] + s) = make_float2(r.v[1], r.v[3]);
     // (the one-block levels start from zero themselves and have no classes)
-    if (cc == 0 && e.cls[0]) e.x[0][s] = first_sweep(e, e.cls[0][s], r, I, J, K);
+    if (e.cls[0]) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int Ir = I + 2 * m + g;  // red: even when g = 0, odd when g = 1
+        if (Ir < e.L.nx) e.x[0][s + m] = first_sweep(e, e.cls[0][s + m], g ? r.v[2 * m + 1] : r.v[2 * m], Ir, J, K);
+      }
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
 // The small levels in one block: a whole V-cycle in shared memory.  Every
-// level's arrays are padded by one cell (x and the couplings 0 there), five
-// per level: x, b and the three couplings.
+// level's arrays are padded by one cell (x and the couplings 0 there): x, b,
+// 1/d and the three couplings.  A half sweep is bound by shared-memory reads
+// (14 per cell), so the slots' positions are found once per level, the
+// diagonal is inverted once, and levels of at most 32 cells a colour run in
+// the first warp alone, without block barriers.  Measured at 256^3 (16^3 and
+// below in the block): 42 us with positions, sums and a division in every
+// sweep and a barrier after each, 36 us so.
 // ---------------------------------------------------------------------------
 constexpr int kCoarseThreads = 1024;
 constexpr int kCoarseSweeps = 4;
+constexpr int kCoarseItems = 4;      // slots of one colour per thread: up to 4096
+constexpr int kWarpCells = 32;       // of one colour: levels of one warp
+constexpr int kCoarseArrays = 6;
 
 struct CoarseLev {
   int nx, ny, nz, sy, sz, n;  // extents; strides and size of the padded arrays
-  int off;                    // of x in shared memory; b, ax, ay, az follow
+  int off;                    // of x in shared memory; b, 1/d, ax, ay, az follow
   const float *ax, *ay, *az;
   Lay L;
 };
@@ -246,32 +416,91 @@ struct CoarseArgs {
   Lay H;  // packed layout of the top level
 };
 
-__device__ __forceinline__ void coarse_sweep(const CoarseLev& v, float* sm, int color) {
-  float* x = sm + v.off;
-  const float *b = x + v.n, *ax = b + v.n, *ay = ax + v.n, *az = ay + v.n;
-  const int hx = (v.nx + 1) >> 1, count = hx * v.ny * v.nz;
-  for (int t = threadIdx.x; t < count; t += kCoarseThreads) {
-    const int h = t % hx, row = t / hx, j = row % v.ny, k = row / v.ny;
-    const int i = 2 * h + ((j + k + color) & 1);
-    if (i >= v.nx) continue;
-    const int c = (k + 1) * v.sz + (j + 1) * v.sy + i + 1;
-    const float xm = ax[c], xp = ax[c + 1], ym = ay[c], yp = ay[c + v.sy], zm = az[c], zp = az[c + v.sz];
-    const float d = ((xm + xp) + (ym + yp)) + (zm + zp);
-    const float num = b[c] + (((xm * x[c - 1] + xp * x[c + 1]) + (ym * x[c - v.sy] + yp * x[c + v.sy])) +
-                              (zm * x[c - v.sz] + zp * x[c + v.sz]));
-    x[c] = d > 0.0f ? num / d : 0.0f;
+__device__ __forceinline__ int coarse_slots(const CoarseLev& v) { return ((v.nx + 1) >> 1) * v.ny * v.nz; }
+
+__device__ __forceinline__ void coarse_relax(const CoarseLev& v, float* x, int c) {
+  const float *b = x + v.n, *di = b + v.n, *ax = di + v.n, *ay = ax + v.n, *az = ay + v.n;
+  const float num = b[c] + (((ax[c] * x[c - 1] + ax[c + 1] * x[c + 1]) + (ay[c] * x[c - v.sy] + ay[c + v.sy] * x[c + v.sy])) +
+                            (az[c] * x[c - v.sz] + az[c + v.sz] * x[c + v.sz]));
+  x[c] = num * di[c];
+}
+__device__ __forceinline__ float coarse_residual(const CoarseLev& v, const float* x, int c) {
+  const float *b = x + v.n, *ax = b + 2 * v.n, *ay = ax + v.n, *az = ay + v.n;
+  const float xc = x[c];
+  float s = b[c] + (ax[c] * (x[c - 1] - xc) + ax[c + 1] * (x[c + 1] - xc));
+  s += ay[c] * (x[c - v.sy] - xc) + ay[c + v.sy] * (x[c + v.sy] - xc);
+  s += az[c] * (x[c - v.sz] - xc) + az[c + v.sz] * (x[c + v.sz] - xc);
+  return s;
+}
+
+// The slots a thread owns on a level: the padded index of the cell at i = 2h
+// in the low bits, and whether the slot's cells exist (a half slot at the end
+// of an odd row has one cell only, marked).
+struct CoarseItems {
+  int c[kCoarseItems];     // index of cell 2h, -1: none
+  unsigned par, half;      // bit m: (j + k) & 1; cell 2h + 1 does not exist
+  __device__ __forceinline__ void init(const CoarseLev& v, int tid, int threads) {
+    const int hx = (v.nx + 1) >> 1, count = hx * v.ny * v.nz;
+    par = half = 0u;
+#pragma unroll
+    for (int m = 0; m < kCoarseItems; ++m) {
+      const int t = tid + m * threads;
+      c[m] = -1;
+      if (t < count) {
+        const int h = t % hx, row = t / hx, j = row % v.ny, k = row / v.ny;
+        c[m] = (k + 1) * v.sz + (j + 1) * v.sy + 2 * h + 1;
+        par |= (unsigned)((j + k) & 1) << m;
+        half |= (unsigned)(2 * h + 1 >= v.nx) << m;
+      }
+    }
   }
-  __syncthreads();
+  __device__ __forceinline__ void sweep(const CoarseLev& v, float* x, int color) const {
+#pragma unroll
+    for (int m = 0; m < kCoarseItems; ++m) {
+      if (c[m] < 0) continue;
+      const int o = ((par >> m) ^ color) & 1;
+      if (o && ((half >> m) & 1)) continue;
+      coarse_relax(v, x, c[m] + o);
+    }
+  }
+};
+
+// restrict from level v into w, by threads tid of `threads`
+__device__ __forceinline__ void coarse_restrict(const CoarseLev& v, const CoarseLev& w, float* sm, int tid, int threads) {
+  const float* x = sm + v.off;
+  float* wb = sm + w.off + w.n;
+  const int count = w.nx * w.ny * w.nz;
+  // the residual is zero in the colour swept last (black): only the four red cells count
+  for (int t = tid; t < count; t += threads) {
+    const int I = t % w.nx, row = t / w.nx, J = row % w.ny, K = row / w.ny;
+    float r = 0.0f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int j = 2 * J + (m & 1), k = 2 * K + (m >> 1), i = 2 * I + ((j + k) & 1);
+      if (i < v.nx && j < v.ny && k < v.nz) r += coarse_residual(v, x, (k + 1) * v.sz + (j + 1) * v.sy + i + 1);
+    }
+    wb[(K + 1) * w.sz + (J + 1) * w.sy + I + 1] = r;
+  }
+}
+__device__ __forceinline__ void coarse_prolong(const CoarseLev& v, const CoarseLev& w, float* sm, int tid, int threads) {
+  float* x = sm + v.off;
+  const float* wx = sm + w.off;
+  const int count = v.nx * v.ny * v.nz;
+  for (int t = tid; t < count; t += threads) {
+    const int i = t % v.nx, row = t / v.nx, j = row % v.ny, k = row / v.ny;
+    x[(k + 1) * v.sz + (j + 1) * v.sy + i + 1] += wx[((k >> 1) + 1) * w.sz + ((j >> 1) + 1) * w.sy + (i >> 1) + 1];
+  }
 }
 
 __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(CoarseArgs A, const MgState* st) {
   if (stopped(st)) return;
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x;
   {
     const CoarseLev& last = A.l[A.levels - 1];
-    const int total = last.off + 5 * last.n;
-    for (int t = tid; t < total; t += kCoarseThreads) sm[t] = 0.0f;
+    const int total4 = (last.off + kCoarseArrays * last.n + 3) >> 2;
+    for (int t = tid; t < total4; t += kCoarseThreads)
+      reinterpret_cast<float4*>(sm)[t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   __syncthreads();
   for (int q = 0; q < A.levels; ++q) {
@@ -282,57 +511,73 @@ __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(CoarseArgs A, cons
       const int i = t % v.nx, row = t / v.nx, j = row % v.ny, k = row / v.ny;
       const int c = (k + 1) * v.sz + (j + 1) * v.sy + i + 1;
       const int64_t g = v.L.at(i, j, k);
-      x[2 * v.n + c] = v.ax[g];  // the low faces; the high walls stay 0
-      x[3 * v.n + c] = v.ay[g];
-      x[4 * v.n + c] = v.az[g];
+      // the low faces, then 1/d (the high walls' couplings are ghosts, 0)
+      const float xm = v.ax[g], ym = v.ay[g], zm = v.az[g];
+      const float d = ((xm + v.ax[g + 1]) + (ym + v.ay[g + v.L.px])) + (zm + v.az[g + v.L.slab]);
+      x[2 * v.n + c] = d > 0.0f ? 1.0f / d : 0.0f;
+      x[3 * v.n + c] = xm;
+      x[4 * v.n + c] = ym;
+      x[5 * v.n + c] = zm;
       if (q == 0) x[v.n + c] = A.b[(i + j + k) & 1][A.H.at(i >> 1, j, k)];
     }
   }
   __syncthreads();
-  for (int q = 0; q < A.levels; ++q) {
+  // levels 0 .. big-1 by the block, the rest by one warp
+  int big = 0;
+  while (big < A.levels && coarse_slots(A.l[big]) > kWarpCells) ++big;
+  for (int q = 0; q < big; ++q) {
     const CoarseLev& v = A.l[q];
-    if (q == A.levels - 1) break;
-    for (int m = 0; m < kCoarseSweeps; ++m) coarse_sweep(v, sm, m & 1);
-    // restrict the residual
-    const CoarseLev& w = A.l[q + 1];
-    const float *x = sm + v.off, *b = x + v.n, *ax = b + v.n, *ay = ax + v.n, *az = ay + v.n;
-    float* wb = sm + w.off + w.n;
-    const int count = w.nx * w.ny * w.nz;
-    for (int t = tid; t < count; t += kCoarseThreads) {
-      const int I = t % w.nx, row = t / w.nx, J = row % w.ny, K = row / w.ny;
-      float r = 0.0f;
-      for (int m = 0; m < 8; ++m) {
-        const int i = 2 * I + (m & 1), j = 2 * J + ((m >> 1) & 1), k = 2 * K + (m >> 2);
-        if (i >= v.nx || j >= v.ny || k >= v.nz) continue;
-        const int c = (k + 1) * v.sz + (j + 1) * v.sy + i + 1;
-        const float xc = x[c];
-        float s = b[c] + (ax[c] * (x[c - 1] - xc) + ax[c + 1] * (x[c + 1] - xc));
-        s += ay[c] * (x[c - v.sy] - xc) + ay[c + v.sy] * (x[c + v.sy] - xc);
-        s += az[c] * (x[c - v.sz] - xc) + az[c + v.sz] * (x[c + v.sz] - xc);
-        r += s;
-      }
-      wb[(K + 1) * w.sz + (J + 1) * w.sy + I + 1] = r;
+    CoarseItems it;
+    it.init(v, tid, kCoarseThreads);
+    for (int m = 0; m < kCoarseSweeps; ++m) {
+      it.sweep(v, sm + v.off, m & 1);
+      __syncthreads();
     }
-    __syncthreads();
+    if (q + 1 < A.levels) {
+      coarse_restrict(v, A.l[q + 1], sm, tid, kCoarseThreads);
+      __syncthreads();
+    }
   }
-  for (int q = A.levels - 1; q >= 0; --q) {
+  if (tid < 32) {
+    for (int q = big; q < A.levels; ++q) {
+      const CoarseLev& v = A.l[q];
+      CoarseItems it;
+      it.init(v, tid, 32);
+      // the coarsest level (at most 2 cells a side) is swept to a solve
+      const int sweeps = q == A.levels - 1 ? 2 * kCoarseSweeps : kCoarseSweeps;
+      for (int m = 0; m < sweeps; ++m) {
+        it.sweep(v, sm + v.off, m & 1);
+        __syncwarp();
+      }
+      if (q + 1 < A.levels) coarse_restrict(v, A.l[q + 1], sm, tid, 32);
+      __syncwarp();
+    }
+    for (int q = A.levels - 1; q >= big; --q) {
+      const CoarseLev& v = A.l[q];
+      CoarseItems it;
+      it.init(v, tid, 32);
+      if (q + 1 < A.levels) coarse_prolong(v, A.l[q + 1], sm, tid, 32);
+      __syncwarp();
+      const int sweeps = q == A.levels - 1 ? 2 * kCoarseSweeps : kCoarseSweeps;
+      for (int m = sweeps - 1; m >= 0; --m) {
+        it.sweep(v, sm + v.off, m & 1);
+        __syncwarp();
+      }
+    }
+  }
+  __syncthreads();
+  for (int q = big - 1; q >= 0; --q) {
     const CoarseLev& v = A.l[q];
-    if (q == A.levels - 1) {
-      // the coarsest level (at most 2 cells a side): sweeps to a solve
-      for (int m = 0; m < 8; ++m) coarse_sweep(v, sm, m & 1);
-      for (int m = 7; m >= 0; --m) coarse_sweep(v, sm, m & 1);
-      continue;
+    CoarseItems it;
+    it.init(v, tid, kCoarseThreads);
+    if (q + 1 < A.levels) {
+      coarse_prolong(v, A.l[q + 1], sm, tid, kCoarseThreads);
+      __syncthreads();
     }
-    const CoarseLev& w = A.l[q + 1];
-    float* x = sm + v.off;
-    const float* wx = sm + w.off;
-    const int count = v.nx * v.ny * v.nz;
-    for (int t = tid; t < count; t += kCoarseThreads) {
-      const int i = t % v.nx, row = t / v.nx, j = row % v.ny, k = row / v.ny;
-      x[(k + 1) * v.sz + (j + 1) * v.sy + i + 1] += wx[((k >> 1) + 1) * w.sz + ((j >> 1) + 1) * w.sy + (i >> 1) + 1];
+    for (int m = kCoarseSweeps - 1; m >= 0; --m) {
+      it.sweep(v, sm + v.off, m & 1);
+      __syncthreads();
     }
-    __syncthreads();
-    for (int m = kCoarseSweeps - 1; m >= 0; --m) coarse_sweep(v, sm, m & 1);
   }
   {
     const CoarseLev& v = A.l[0];
@@ -352,13 +597,15 @@ __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(CoarseArgs A, cons
 // Couplings of the low faces of each cell (FP64 from phi, stored FP32; the
 // expression of the projection's coupling kernel) and the cell's class.
 template <class T>
-__global__ void __launch_bounds__(kBX * kBY) k_mg_build(const MgState* st, Lay L, Lay H, double rn, double rp,
-                                                        double inv2, float* __restrict__ ax, float* __restrict__ ay,
-                                                        float* __restrict__ az, unsigned char* __restrict__ cls0,
-                                                        unsigned char* __restrict__ cls1, double* extra0, int kchunk) {
-  const int i = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  if (i >= L.nx || j >= L.ny) return;
-  const int k0 = blockIdx.z * kchunk, k1 = min(L.nz, k0 + kchunk);
+__global__ void __launch_bounds__(kThreads) k_mg_build(const MgState* st, Lay L, Lay H, double rn, double rp,
+                                                       double inv2, float* __restrict__ ax, float* __restrict__ ay,
+                                                       float* __restrict__ az, unsigned char* __restrict__ cls0,
+                                                       unsigned char* __restrict__ cls1,
+                                                       unsigned char* __restrict__ ccls, double* extra0, int w,
+                                                       int chunk) {
+  const Column col(w, L.ny, L.nz, chunk);
+  if (!col.ok) return;
+  const int i = col.i, j = col.j, k0 = col.k0, k1 = col.k1;
   const T* __restrict__ phi = (const T*)st->phi;
   const double vneg = 1.0 / rn, vpos = 1.0 / rp;
   if (i == 0 && j == 0 && k0 == 0) *extra0 = 0.0;  // no deflation
@@ -382,19 +629,22 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_build(const MgState* st, Lay L
     const bool n = p <= T(0);
     const bool same = (xm <= T(0)) == n && (xp <= T(0)) == n && (ym <= T(0)) == n && (yp <= T(0)) == n &&
                       (down <= T(0)) == n && (up <= T(0)) == n;
-    (((i + j + k) & 1) ? cls1 : cls0)[H.at(i >> 1, j, k)] = same ? (n ? 1 : 2) : 0;
+    const unsigned char cl = same ? (n ? 1 : 2) : 0;
+    (((i + j + k) & 1) ? cls1 : cls0)[H.at(i >> 1, j, k)] = cl;
+    ccls[c] = cl;
     down = p;
     p = up;
   }
 }
 
 // coarse couplings: half the sum of the fine couplings across the face
-__global__ void __launch_bounds__(kBX * kBY) k_mg_coarsen(Lay Lf, const float* __restrict__ fx,
-                                                          const float* __restrict__ fy, const float* __restrict__ fz,
-                                                          Lay L, float* __restrict__ ax, float* __restrict__ ay,
-                                                          float* __restrict__ az) {
-  const int I = blockIdx.x * kBX + threadIdx.x, J = blockIdx.y * kBY + threadIdx.y, K = blockIdx.z;
-  if (I >= L.nx || J >= L.ny) return;
+__global__ void __launch_bounds__(kThreads) k_mg_coarsen(Lay Lf, const float* __restrict__ fx,
+                                                         const float* __restrict__ fy, const float* __restrict__ fz,
+                                                         Lay L, float* __restrict__ ax, float* __restrict__ ay,
+                                                         float* __restrict__ az) {
+  const Column col(L.nx, L.ny, L.nz, 1);
+  if (!col.ok) return;
+  const int I = col.i, J = col.j, K = col.k0;
   // cells past an odd extent are ghosts, whose couplings are zero
   const int64_t c = L.at(I, J, K), f = Lf.at(2 * I, 2 * J, 2 * K);
   ax[c] = 0.5f * ((fx[f] + fx[f + Lf.px]) + (fx[f + Lf.slab] + fx[f + Lf.slab + Lf.px]));
@@ -404,11 +654,12 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_coarsen(Lay Lf, const float* _
 
 // classes of a coarse level: every face inside the box carries the same
 // phase's uniform coupling
-__global__ void __launch_bounds__(kBX * kBY) k_mg_class(Lev v, unsigned char* __restrict__ cls0,
-                                                        unsigned char* __restrict__ cls1) {
-  const int i = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y, k = blockIdx.z;
+__global__ void __launch_bounds__(kThreads) k_mg_class(Lev v, unsigned char* __restrict__ cls0,
+                                                       unsigned char* __restrict__ cls1) {
   const Lay& L = v.L;
-  if (i >= L.nx || j >= L.ny) return;
+  const Column col(L.nx, L.ny, L.nz, 1);
+  if (!col.ok) return;
+  const int i = col.i, j = col.j, k = col.k0;
   const Couplings a = couplings_at(v, L.at(i, j, k));
   int cl = 0;
   for (int q = 1; q < 3; ++q) {
@@ -423,61 +674,58 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_class(Lev v, unsigned char* __
 }
 
 // ---------------------------------------------------------------------------
-// The iteration on the finest level: one packed slot (cells i0 = 2h, i0 + 1)
-// per thread; red is cell i0 + ((j+k)&1).
+// The iteration on the finest level.  x, p and q are in the cell layout; four
+// cells i0 .. i0+3 per thread (slots i0/2, i0/2 + 1 of each colour; cell i0 +
+// m is red when (m + j + k) is even), two in the FP64 residual.
 // ---------------------------------------------------------------------------
+
+// r, z or the red iterate of four cells from / to the packed colours.
+__device__ __forceinline__ F4 unpack4(const float* const a[2], int64_t s, int par) {
+  const float2 e = *reinterpret_cast<const float2*>(a[par] + s), o = *reinterpret_cast<const float2*>(a[1 - par] + s);
+  return {{e.x, o.x, e.y, o.y}};
+}
 
 // q = A p in flux form (FP32 arithmetic, each flux exact to 2 eps32 of
 // itself), p.q and alpha = r.z / p.q.
-__global__ void __launch_bounds__(kBX * kBY) k_mg_spmv(Lev v, const float* __restrict__ p, float* __restrict__ q,
-                                                       MgState* st, double* partials, int kchunk) {
+__global__ void __launch_bounds__(kThreads) k_mg_spmv(Lev v, const float* __restrict__ p, float* __restrict__ q,
+                                                      MgState* st, double* partials, int w, int chunk) {
   if (stopped(st)) return;
-  const Lay &L = v.L, &H = v.H;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
+  const Lay& L = v.L;
+  const Column col(w, L.ny, L.nz, chunk);
   double pq = 0.0;
-  if (h < H.nx && j < H.ny) {
-    const int i0 = 2 * h;
-    const bool two = i0 + 1 < L.nx;
-    int64_t c = L.at(i0, j, k0), s = H.at(h, j, k0);
-    auto ld2 = [&](int64_t o) { return *reinterpret_cast<const float2*>(p + o); };
-    float2 dn = ld2(c - L.slab), pc = ld2(c);
-    for (int k = k0; k < k1; ++k, c += L.slab, s += H.slab) {
-      const float2 up = ld2(c + L.slab);
-      float2 ym = ld2(c - L.px), yp = ld2(c + L.px);
-      const float xl = p[c - 1], xr = p[c + 2];
-      const int par = (j + k) & 1;
-      const int c0 = v.cls[par][s], c1 = v.cls[1 - par][s];
-      float q0, q1 = 0.0f;
-      if (c0) {
-        // a face on a wall carries no flux: its neighbour is read as p itself
-        float f = (i0 > 0 ? pc.x - xl : 0.0f) + (two ? pc.x - pc.y : 0.0f);
-        f += (j > 0 ? pc.x - ym.x : 0.0f) + (j < L.ny - 1 ? pc.x - yp.x : 0.0f);
-        f += (k > 0 ? pc.x - dn.x : 0.0f) + (k < L.nz - 1 ? pc.x - up.x : 0.0f);
-        q0 = v.a[c0] * f;
-      } else {
-        const Couplings a = couplings_at(v, c);
-        q0 = a.xm * (pc.x - xl) + a.xp * (pc.x - pc.y);
-        q0 += a.ym * (pc.x - ym.x) + a.yp * (pc.x - yp.x);
-        q0 += a.zm * (pc.x - dn.x) + a.zp * (pc.x - up.x);
-      }
-      if (two) {
-        if (c1) {
-          float f = (pc.y - pc.x) + (i0 + 2 < L.nx ? pc.y - xr : 0.0f);
-          f += (j > 0 ? pc.y - ym.y : 0.0f) + (j < L.ny - 1 ? pc.y - yp.y : 0.0f);
-          f += (k > 0 ? pc.y - dn.y : 0.0f) + (k < L.nz - 1 ? pc.y - up.y : 0.0f);
-          q1 = v.a[c1] * f;
+  if (col.ok) {
+    const int i0 = 4 * col.i, j = col.j;
+    const int valid = min(4, L.nx - i0);
+    int64_t c = L.at(i0, j, col.k0);
+    F4 dn = load4(p + c - L.slab), pc = load4(p + c);
+    for (int k = col.k0; k < col.k1; ++k, c += L.slab) {
+      const F4 up = load4(p + c + L.slab), ym = load4(p + c - L.px), yp = load4(p + c + L.px);
+      const float xl = p[c - 1], xr = p[c + 4];
+      const unsigned cl = *reinterpret_cast<const unsigned*>(v.ccls + c);
+      const bool b0 = j > 0, b1 = j < L.ny - 1, d0 = k > 0, d1 = k < L.nz - 1;
+      F4 out;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        out.v[m] = 0.0f;
+        if (m >= valid) continue;
+        const int cm = (cl >> (8 * m)) & 255u;
+        const float pm = pc.v[m], l = m ? pc.v[m - 1] : xl, r = m < 3 ? pc.v[m + 1] : xr;
+        if (cm) {
+          // a face on a wall carries no flux
+          float f = (i0 + m > 0 ? pm - l : 0.0f) + (i0 + m < L.nx - 1 ? pm - r : 0.0f);
+          f += (b0 ? pm - ym.v[m] : 0.0f) + (b1 ? pm - yp.v[m] : 0.0f);
+          f += (d0 ? pm - dn.v[m] : 0.0f) + (d1 ? pm - up.v[m] : 0.0f);
+          out.v[m] = v.a[cm] * f;
         } else {
-          const Couplings a = couplings_at(v, c + 1);
-          q1 = a.xm * (pc.y - pc.x) + a.xp * (pc.y - xr);
-          q1 += a.ym * (pc.y - ym.y) + a.yp * (pc.y - yp.y);
-          q1 += a.zm * (pc.y - dn.y) + a.zp * (pc.y - up.y);
+          const Couplings a = couplings_at(v, c + m);
+          float f = a.xm * (pm - l) + a.xp * (pm - r);
+          f += a.ym * (pm - ym.v[m]) + a.yp * (pm - yp.v[m]);
+          f += a.zm * (pm - dn.v[m]) + a.zp * (pm - up.v[m]);
+          out.v[m] = f;
         }
-        *reinterpret_cast<float2*>(q + c) = make_float2(q0, q1);
-      } else {
-        q[c] = q0;
+        pq += (double)pm * (double)out.v[m];
       }
-      pq += (double)pc.x * (double)q0 + (double)pc.y * (double)q1;  // q1 = 0 past an odd extent
+      store4(q + c, out);  // (0 in ghosts past the row's end)
       dn = pc;
       pc = up;
     }
@@ -499,42 +747,55 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_spmv(Lev v, const float* __res
 // next cycle.  The last block asks for the true residual (pause) when the
 // recursive one meets the tolerance, has dropped by reliable_delta since the
 // last true one, or the iteration cap is reached.
-__global__ void __launch_bounds__(kBX * kBY) k_mg_update(Lev v, const float* __restrict__ p,
-                                                         const float* __restrict__ q, MgState* st, double* partials,
-                                                         int kchunk) {
+__global__ void __launch_bounds__(kThreads) k_mg_update(Lev v, const float* __restrict__ p,
+                                                        const float* __restrict__ q, MgState* st, double* partials,
+                                                        int w, int chunk) {
   if (stopped(st)) return;
   const Lay &L = v.L, &H = v.H;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
-  const double alpha = ((const volatile MgState*)st)->alpha;
+  const Column col(w, L.ny, L.nz, chunk);
+  const double alpha = state_read(&st->alpha);
   const float al = (float)alpha;
   double* __restrict__ x = st->x;
+  float* __restrict__ rr_ = v.b[0];
+  float* __restrict__ rb_ = v.b[1];
+  float* __restrict__ xr_ = v.x[0];
   double rr = 0.0;
-  if (h < H.nx && j < H.ny) {
-    const int i0 = 2 * h;
-    const bool two = i0 + 1 < L.nx;
-    int64_t c = L.at(i0, j, k0), s = H.at(h, j, k0);
-    for (int k = k0; k < k1; ++k, c += L.slab, s += H.slab) {
-      const float2 pv = *reinterpret_cast<const float2*>(p + c), qv = *reinterpret_cast<const float2*>(q + c);
-      double2 xv = *reinterpret_cast<const double2*>(x + c);
-      xv.x += alpha * (double)pv.x;
-      xv.y += alpha * (double)pv.y;
-      if (two) *reinterpret_cast<double2*>(x + c) = xv;
-      else x[c] = xv.x;
-      const int par = (j + k) & 1;  // the colour of cell i0; cell i0 + 1 has the other
-      float* r0 = v.b[par];
-      float* r1 = v.b[1 - par];
-      const float ra = r0[s] - al * qv.x;
-      r0[s] = ra;
-      rr += (double)ra * (double)ra;
-      float rb = 0.0f;
-      if (two) {
-        rb = r1[s] - al * qv.y;
-        r1[s] = rb;
-        rr += (double)rb * (double)rb;
+  if (col.ok) {
+    const int i0 = 4 * col.i, j = col.j;
+    const int valid = min(4, L.nx - i0);
+    int64_t c = L.at(i0, j, col.k0), s = H.at(i0 >> 1, j, col.k0);
+    for (int k = col.k0; k < col.k1; ++k, c += L.slab, s += H.slab) {
+      const int par = (j + k) & 1;
+      const F4 pv = load4(p + c), qv = load4(q + c);
+      double2 x0 = *reinterpret_cast<const double2*>(x + c), x1 = *reinterpret_cast<const double2*>(x + c + 2);
+      const float2 red = *reinterpret_cast<const float2*>(rr_ + s), black = *reinterpret_cast<const float2*>(rb_ + s);
+      const unsigned cl = *reinterpret_cast<const unsigned*>(v.ccls + c);
+      x0.x += alpha * (double)pv.v[0];
+      x0.y += alpha * (double)pv.v[1];
+      x1.x += alpha * (double)pv.v[2];
+      x1.y += alpha * (double)pv.v[3];
+      if (valid == 4) {
+        *reinterpret_cast<double2*>(x + c) = x0;
+        *reinterpret_cast<double2*>(x + c + 2) = x1;
+      } else {
+        x[c] = x0.x;
+        if (valid > 1) x[c + 1] = x0.y;
+        if (valid > 2) x[c + 2] = x1.x;
       }
-      if (par == 0) v.x[0][s] = first_sweep(v, v.cls[0][s], ra, i0, j, k);
-      else if (two) v.x[0][s] = first_sweep(v, v.cls[0][s], rb, i0 + 1, j, k);
+      // past the row's end q and r are 0
+      float2 nr, nb;  // red: cells par and par + 2
+      nr.x = red.x - al * (par ? qv.v[1] : qv.v[0]);
+      nr.y = red.y - al * (par ? qv.v[3] : qv.v[2]);
+      nb.x = black.x - al * (par ? qv.v[0] : qv.v[1]);
+      nb.y = black.y - al * (par ? qv.v[2] : qv.v[3]);
+      *reinterpret_cast<float2*>(rr_ + s) = nr;
+      *reinterpret_cast<float2*>(rb_ + s) = nb;
+      rr += ((double)nr.x * (double)nr.x + (double)nr.y * (double)nr.y) +
+            ((double)nb.x * (double)nb.x + (double)nb.y * (double)nb.y);
+      float2 xr = make_float2(0.0f, 0.0f);
+      if (par < valid) xr.x = first_sweep(v, (cl >> (8 * par)) & 255u, nr.x, i0 + par, j, k);
+      if (par + 2 < valid) xr.y = first_sweep(v, (cl >> (8 * par + 16)) & 255u, nr.y, i0 + par + 2, j, k);
+      *reinterpret_cast<float2*>(xr_ + s) = xr;
     }
   }
   rr = block_sum(rr);
@@ -551,67 +812,78 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_update(Lev v, const float* __r
   }
 }
 
+// Flux sum of a cell near the interface, its face coefficients from phi in
+// FP64; d holds x_c - x_nb per face (l, r, b, t, d, u), 0 on walls.
+template <class T>
+__device__ __noinline__ double mixed_flux(const T* phi, const Lay& L, int64_t c, int i, int j, int k, double vneg,
+                                          double vpos, double dl, double dr, double db, double dt, double dd,
+                                          double du) {
+  const double pc = (double)phi[c];
+  double flux = 0.0;
+  if (i > 0) flux += face_coef(pc, (double)phi[c - 1], vneg, vpos) * dl;
+  if (i < L.nx - 1) flux += face_coef(pc, (double)phi[c + 1], vneg, vpos) * dr;
+  if (j > 0) flux += face_coef(pc, (double)phi[c - L.px], vneg, vpos) * db;
+  if (j < L.ny - 1) flux += face_coef(pc, (double)phi[c + L.px], vneg, vpos) * dt;
+  if (k > 0) flux += face_coef(pc, (double)phi[c - L.slab], vneg, vpos) * dd;
+  if (k < L.nz - 1) flux += face_coef(pc, (double)phi[c + L.slab], vneg, vpos) * du;
+  return flux;
+}
+
 // The true residual r = b - A x in FP64 (A from phi in FP64), its norm, the
 // first red half sweep, and the decisions that rest on it.  INIT: the start
 // of a solve (unconditional; also keeps the initial guess in st->bak).
 template <class T, bool INIT>
-__global__ void __launch_bounds__(kBX * kBY) k_mg_defect(Lev v, MgState* st, double* partials, double rn, double rp,
-                                                         double inv2, int kchunk) {
-  if (!INIT && (stopped(st) || !((const volatile MgState*)st)->pause)) return;
+__global__ void __launch_bounds__(kThreads, 3) k_mg_defect(Lev v, MgState* st, double* partials, double rn, double rp,
+                                                           double inv2, int w, int chunk) {
+  if (!INIT && (stopped(st) || !state_read(&st->pause))) return;
   const Lay &L = v.L, &H = v.H;
+  const Column col(w, H.ny, H.nz, chunk);
   const T* __restrict__ phi = (const T*)st->phi;
   const double* __restrict__ x = st->x;
   const double* __restrict__ b = st->b;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
   const double vneg = 1.0 / rn, vpos = 1.0 / rp;
   double rr = 0.0;
-  if (h < H.nx && j < H.ny) {
-    const int i0 = 2 * h;
+  if (col.ok) {
+    const int h = col.i, i0 = 2 * h, j = col.j;
     const bool two = i0 + 1 < L.nx;
-    int64_t c = L.at(i0, j, k0), s = H.at(h, j, k0);
-    auto ld2 = [&](int64_t o) { return *reinterpret_cast<const double2*>(x + o); };
-    double2 dn = ld2(c - L.slab), xc = ld2(c);
-    // flux sum of one cell whose faces all carry its phase's 1/rho
-    for (int k = k0; k < k1; ++k, c += L.slab, s += H.slab) {
-      const double2 up = ld2(c + L.slab), ym = ld2(c - L.px), yp = ld2(c + L.px);
+    int64_t c = L.at(i0, j, col.k0), s = H.at(h, j, col.k0);
+    auto ld2 = [&](const double* a, int64_t o) { return *reinterpret_cast<const double2*>(a + o); };
+    double2 dn = ld2(x, c - L.slab), xc = ld2(x, c);
+    const bool okl = i0 > 0, okr = i0 + 2 < L.nx, okb = j > 0, okt = j < L.ny - 1;
+    for (int k = col.k0; k < col.k1; ++k, c += L.slab, s += H.slab) {
+      const double2 up = ld2(x, c + L.slab), ym = ld2(x, c - L.px), yp = ld2(x, c + L.px);
       const double xl = x[c - 1], xr = x[c + 2];
-      const double2 bv = *reinterpret_cast<const double2*>(b + c);
+      const double2 bv = ld2(b, c);
+      const uchar2 cl = *reinterpret_cast<const uchar2*>(v.ccls + c);
+      const int par = (j + k) & 1;
+      const bool okd = k > 0, oku = k < L.nz - 1;
       if (INIT) {
         if (two) *reinterpret_cast<double2*>(st->bak + c) = xc;
         else st->bak[c] = xc.x;
       }
-      const int par = (j + k) & 1;
-      double r[2] = {0.0, 0.0};
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        if (m == 1 && !two) break;
-        const int i = i0 + m;
-        const int cl = v.cls[par ^ m][s];
-        const double xv = m ? xc.y : xc.x;
-        const bool okl = i > 0, okr = i < L.nx - 1, okb = j > 0, okt = j < L.ny - 1, okd = k > 0, oku = k < L.nz - 1;
-        const double dl = okl ? xv - (m ? xc.x : xl) : 0.0, dr = okr ? xv - (m ? xr : xc.y) : 0.0;
-        const double db = okb ? xv - (m ? ym.y : ym.x) : 0.0, dt = okt ? xv - (m ? yp.y : yp.x) : 0.0;
-        const double dd = okd ? xv - (m ? dn.y : dn.x) : 0.0, du = oku ? xv - (m ? up.y : up.x) : 0.0;
-        double flux;
-        if (cl) {
-          flux = (cl == 1 ? vneg : vpos) * (((dl + dr) + (db + dt)) + (dd + du));
-        } else {
-          const int64_t cc = c + m;
-          const double pc = (double)phi[cc];
-          flux = 0.0;
-          if (okl) flux += face_coef(pc, (double)phi[cc - 1], vneg, vpos) * dl;
-          if (okr) flux += face_coef(pc, (double)phi[cc + 1], vneg, vpos) * dr;
-          if (okb) flux += face_coef(pc, (double)phi[cc - L.px], vneg, vpos) * db;
-          if (okt) flux += face_coef(pc, (double)phi[cc + L.px], vneg, vpos) * dt;
-          if (okd) flux += face_coef(pc, (double)phi[cc - L.slab], vneg, vpos) * dd;
-          if (oku) flux += face_coef(pc, (double)phi[cc + L.slab], vneg, vpos) * du;
-        }
-        r[m] = (m ? bv.y : bv.x) - inv2 * flux;
-        rr += r[m] * r[m];
-        const float rf = (float)r[m];
-        v.b[par ^ m][s] = rf;
-        if ((par ^ m) == 0) v.x[0][s] = first_sweep(v, cl, rf, i, j, k);
+      const double dx = two ? xc.x - xc.y : 0.0;  // across the pair
+      double f0, f1;
+      {
+        const double dl = okl ? xc.x - xl : 0.0, db = okb ? xc.x - ym.x : 0.0, dt = okt ? xc.x - yp.x : 0.0,
+                     dd = okd ? xc.x - dn.x : 0.0, du = oku ? xc.x - up.x : 0.0;
+        if (cl.x) f0 = (cl.x == 1 ? vneg : vpos) * (((dl + dx) + (db + dt)) + (dd + du));
+        else f0 = mixed_flux<T>(phi, L, c, i0, j, k, vneg, vpos, dl, dx, db, dt, dd, du);
+      }
+      const double r0 = bv.x - inv2 * f0;
+      rr += r0 * r0;
+      const float a0 = (float)r0;
+      v.b[par][s] = a0;
+      if (par == 0) v.x[0][s] = first_sweep(v, cl.x, a0, i0, j, k);
+      if (two) {
+        const double dr = okr ? xc.y - xr : 0.0, db = okb ? xc.y - ym.y : 0.0, dt = okt ? xc.y - yp.y : 0.0,
+                     dd = okd ? xc.y - dn.y : 0.0, du = oku ? xc.y - up.y : 0.0;
+        if (cl.y) f1 = (cl.y == 1 ? vneg : vpos) * (((dr - dx) + (db + dt)) + (dd + du));
+        else f1 = mixed_flux<T>(phi, L, c + 1, i0 + 1, j, k, vneg, vpos, -dx, dr, db, dt, dd, du);
+        const double r1 = bv.y - inv2 * f1;
+        rr += r1 * r1;
+        const float a1 = (float)r1;
+        v.b[1 - par][s] = a1;
+        if (par == 1) v.x[0][s] = first_sweep(v, cl.y, a1, i0 + 1, j, k);
       }
       dn = xc;
       xc = up;
@@ -664,64 +936,33 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_defect(Lev v, MgState* st, dou
   }
 }
 
-// r.z over both colours and beta.  The packed arrays are walked whole: z is
-// zero in every slot without a cell.
-__global__ void __launch_bounds__(256) k_mg_dot(Lev v, MgState* st, double* partials) {
-  if (stopped(st)) return;
-  const int64_t n4 = v.H.total >> 2;
-  double rz = 0.0;
-  for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < n4; t += (int64_t)gridDim.x * 256) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const float4 a = reinterpret_cast<const float4*>(v.b[c])[t], z = reinterpret_cast<const float4*>(v.x[c])[t];
-      rz += ((double)a.x * (double)z.x + (double)a.y * (double)z.y) +
-            ((double)a.z * (double)z.z + (double)a.w * (double)z.w);
-    }
-  }
-  rz = block_sum(rz);
-  double tot;
-  if (grid_reduce_sum(rz, partials, &st->ticket, &tot)) {
-    const double old = st->rz;
-    st->beta = (st->restart || !(old > 0.0)) ? 0.0 : tot / old;
-    st->restart = 0;
-    st->rz = tot;
-    if (!isfinite(tot) || !(tot > 0.0)) {
-      st->status = PCG_STAGNATED;
-      st->done = 1;
-    }
-  }
-}
-
 // p = z + beta p.  With a loop handle one thread also continues the graph's
 // loop while the solve runs (bounded by the iteration cap whatever the
 // state says).
-__global__ void __launch_bounds__(kBX * kBY) k_mg_direction(Lev v, float* __restrict__ p, MgState* st, int kchunk,
-                                                            int loop, cudaGraphConditionalHandle handle) {
+__global__ void __launch_bounds__(kThreads) k_mg_direction(Lev v, float* __restrict__ p, MgState* st, int w, int chunk,
+                                                           int loop, cudaGraphConditionalHandle handle) {
   const bool stop = stopped(st);
-  if (loop && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+  if (loop && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     const unsigned int n = st->batches + 1u;
     st->batches = n;
     cudaGraphSetConditional(handle, (!stop && n < (unsigned int)st->max_iter + 2u) ? 1u : 0u);
   }
   if (stop) return;
   const Lay &L = v.L, &H = v.H;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  if (h >= H.nx || j >= H.ny) return;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
-  const float beta = (float)((const volatile MgState*)st)->beta;
-  const int i0 = 2 * h;
-  const bool two = i0 + 1 < L.nx;
-  int64_t c = L.at(i0, j, k0), s = H.at(h, j, k0);
-  for (int k = k0; k < k1; ++k, c += L.slab, s += H.slab) {
-    const int par = (j + k) & 1;
-    float2 pv = make_float2(v.x[par][s], v.x[1 - par][s]);
+  const Column col(w, L.ny, L.nz, chunk);
+  if (!col.ok) return;
+  const float beta = (float)state_read(&st->beta);
+  const int i0 = 4 * col.i, j = col.j;
+  int64_t c = L.at(i0, j, col.k0), s = H.at(i0 >> 1, j, col.k0);
+  const float* const z[2] = {v.x[0], v.x[1]};
+  for (int k = col.k0; k < col.k1; ++k, c += L.slab, s += H.slab) {
+    F4 pv = unpack4(z, s, (j + k) & 1);  // (0 past the row's end)
     if (beta != 0.0f) {  // a restart does not read the old direction
-      const float2 po = *reinterpret_cast<const float2*>(p + c);
-      pv.x += beta * po.x;
-      pv.y += beta * po.y;
+      const F4 po = load4(p + c);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) pv.v[m] += beta * po.v[m];
     }
-    if (two) *reinterpret_cast<float2*>(p + c) = pv;
-    else p[c] = pv.x;
+    store4(p + c, pv);
   }
 }
 
@@ -732,17 +973,16 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_direction(Lev v, float* __rest
 // one pressure.
 // Sums over the black cells: sum(x / dinv) and sum(1 / dinv), dinv the bf16
 // 1/diag(S) of the red-black solve (fs_redblack.cu).
-__global__ void __launch_bounds__(kBX * kBY) k_mg_anchor(Lay L, Lay H,
-                                                         const unsigned short* __restrict__ dinv, MgState* st,
-                                                         double* partials, int after, int kchunk) {
-  if (after && ((const volatile MgState*)st)->status == PCG_STAGNATED) return;
+__global__ void __launch_bounds__(kThreads) k_mg_anchor(Lay L, Lay H, const unsigned short* __restrict__ dinv,
+                                                        MgState* st, double* partials, int after, int w, int chunk) {
+  if (after && state_read(&st->status) == PCG_STAGNATED) return;
   const double* __restrict__ x = st->x;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
+  const Column col(w, H.ny, H.nz, chunk);
   double sx = 0.0, sw = 0.0;
-  if (h < H.nx && j < H.ny) {
-    int64_t s = H.at(h, j, k0);
-    for (int k = k0; k < k1; ++k, s += H.slab) {
+  if (col.ok) {
+    const int h = col.i, j = col.j;
+    int64_t s = H.at(h, j, col.k0);
+    for (int k = col.k0; k < col.k1; ++k, s += H.slab) {
       const int i = 2 * h + ((j + k + 1) & 1);
       if (i >= L.nx) continue;
       const double w = (double)(1.0f / __uint_as_float((unsigned)dinv[s] << 16));
@@ -764,32 +1004,30 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_anchor(Lay L, Lay H,
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  const int tid = threadIdx.x + kBX * threadIdx.y;
-  double a = 0.0, w = 0.0;
-  for (int t = tid; t < nb; t += kBX * kBY) {
+  double a = 0.0, ws = 0.0;
+  for (int t = threadIdx.x; t < nb; t += kThreads) {
     a += __ldcg(partials + t);
-    w += __ldcg(partials + nb + t);
+    ws += __ldcg(partials + nb + t);
   }
   a = block_sum(a);
   __syncthreads();
-  w = block_sum(w);
+  ws = block_sum(ws);
   if (thread0()) {
-    if (after) st->shift = w > 0.0 ? (st->anchor - a) / w : 0.0;
+    if (after) st->shift = ws > 0.0 ? (st->anchor - a) / ws : 0.0;
     else st->anchor = a;
     st->ticket = 0u;
   }
 }
 
-__global__ void __launch_bounds__(kBX * kBY) k_mg_shift(Lay L, Lay H, const MgState* st, int kchunk) {
+__global__ void __launch_bounds__(kThreads) k_mg_shift(Lay L, const MgState* st, int w, int chunk) {
   const double d = st->shift;
   if (st->status == PCG_STAGNATED || d == 0.0) return;
+  const Column col(w, L.ny, L.nz, chunk);
+  if (!col.ok) return;
   double* __restrict__ x = st->x;
-  const int h = blockIdx.x * kBX + threadIdx.x, j = blockIdx.y * kBY + threadIdx.y;
-  if (h >= H.nx || j >= H.ny) return;
-  const int k0 = blockIdx.z * kchunk, k1 = min(H.nz, k0 + kchunk);
-  const bool two = 2 * h + 1 < L.nx;
-  int64_t c = L.at(2 * h, j, k0);
-  for (int k = k0; k < k1; ++k, c += L.slab) {
+  const bool two = 2 * col.i + 1 < L.nx;
+  int64_t c = L.at(2 * col.i, col.j, col.k0);
+  for (int k = col.k0; k < col.k1; ++k, c += L.slab) {
     if (two) {
       double2 v = *reinterpret_cast<double2*>(x + c);
       v.x += d;
@@ -801,7 +1039,10 @@ __global__ void __launch_bounds__(kBX * kBY) k_mg_shift(Lay L, Lay H, const MgSt
   }
 }
 
-size_t coarse_floats(int nx, int ny, int nz) { return (size_t)5 * (nx + 2) * (ny + 2) * (nz + 2); }
+// shared floats of one level, rounded up to a float4
+size_t coarse_floats(int nx, int ny, int nz) {
+  return ((size_t)kCoarseArrays * (nx + 2) * (ny + 2) * (nz + 2) + 3) / 4 * 4;
+}
 constexpr size_t kCoarseBytes = 220 * 1024;  // of the 227 KB a block may have
 
 }  // namespace
@@ -835,28 +1076,30 @@ cudaError_t mg_prepare() {
   return cudaFuncSetAttribute(k_mg_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseBytes);
 }
 
-int mg_max_blocks(const Lay& H) {
-  const dim3 g = grid_of(H, chunk_of(H));
-  return (int)std::max<int64_t>((int64_t)g.x * g.y * g.z, reduction_blocks((int64_t)1 << 40));
+int mg_max_blocks(const Lay& L) {
+  int64_t most = 0;
+  for (int per : {1, 2, 4}) {
+    const Columns c = columns(L.nx, L.ny, L.nz, per);
+    most = std::max(most, (int64_t)c.grid.x * c.grid.y);
+  }
+  return (int)most;
 }
 
 template <class T>
 int mg_build(const Multigrid& M, const MgState* st, double dx, double rho_neg, double rho_pos, double* extra0,
              cudaStream_t s) {
   const MgLevel& f = M.level[0];
-  {
-    const int ch = chunk_of(f.L);
-    k_mg_build<T><<<grid_of(f.L, ch), dim3(kBX, kBY, 1), 0, s>>>(st, f.L, f.H, rho_neg, rho_pos, 1.0 / (dx * dx),
-                                                                 f.ax, f.ay, f.az, f.cls[0], f.cls[1], extra0, ch);
-  }
+  const Columns g = columns(f.L.nx, f.L.ny, f.L.nz, 1);
+  k_mg_build<T><<<g.grid, kThreads, 0, s>>>(st, f.L, f.H, rho_neg, rho_pos, 1.0 / (dx * dx), f.ax, f.ay, f.az,
+                                            f.cls[0], f.cls[1], f.ccls, extra0, g.w, g.chunk);
   int launches = 1;
   for (int l = 1; l < M.levels; ++l) {
     const MgLevel &a = M.level[l - 1], &b = M.level[l];
-    const dim3 g = grid_of(b.L, 1);
-    k_mg_coarsen<<<g, dim3(kBX, kBY, 1), 0, s>>>(a.L, a.ax, a.ay, a.az, b.L, b.ax, b.ay, b.az);
+    const dim3 grid((unsigned)(((int64_t)b.L.nx * b.L.ny + kThreads - 1) / kThreads), (unsigned)b.L.nz, 1);
+    k_mg_coarsen<<<grid, kThreads, 0, s>>>(a.L, a.ax, a.ay, a.az, b.L, b.ax, b.ay, b.az);
     ++launches;
     if (l < M.top) {
-      k_mg_class<<<g, dim3(kBX, kBY, 1), 0, s>>>(lev_of(b), b.cls[0], b.cls[1]);
+      k_mg_class<<<grid, kThreads, 0, s>>>(lev_of(b), b.cls[0], b.cls[1]);
       ++launches;
     }
   }
@@ -865,18 +1108,16 @@ int mg_build(const Multigrid& M, const MgState* st, double dx, double rho_neg, d
 
 namespace {
 
-// z = M r: the V-cycle on the residual in level 0's b (x's first red sweep done)
-int cycle(const Multigrid& M, const MgState* st, cudaStream_t s) {
+// z = M r: the V-cycle on the residual in level 0's b (x's first red sweep
+// done), and r.z with beta
+int cycle(const Multigrid& M, MgState* st, double* partials, cudaStream_t s) {
   int launches = 0;
-  const dim3 blk(kBX, kBY, 1);
   for (int l = 0; l < M.top; ++l) {
     const Lev v = lev_of(M.level[l]), e = lev_of(M.level[l + 1]);
-    const int ch = chunk_of(v.H);
-    const dim3 g = grid_of(v.H, ch);
-    k_mg_sweep<false><<<g, blk, 0, s>>>(v, e, 1, st, ch);
-    k_mg_sweep<false><<<g, blk, 0, s>>>(v, e, 0, st, ch);
-    const int ce = chunk_of(e.L);
-    k_mg_restrict<<<grid_of(e.L, ce), blk, 0, s>>>(v, e, 1, st, ce);
+    const Columns g = columns(v.H.nx, v.H.ny, v.H.nz, 4), ge = columns(e.L.nx, e.L.ny, e.L.nz, 4);
+    k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 1, st, partials, g.w, g.chunk);
+    k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+    k_mg_restrict<<<ge.grid, kThreads, 0, s>>>(v, e, 1, st, ge.w, ge.chunk);
     launches += 3;
   }
   CoarseArgs A{};
@@ -896,7 +1137,7 @@ int cycle(const Multigrid& M, const MgState* st, cudaStream_t s) {
     w.ay = m.ay;
     w.az = m.az;
     w.L = m.L;
-    floats += 5 * (size_t)w.n;
+    floats += coarse_floats(w.nx, w.ny, w.nz);
   }
   const MgLevel& t = M.level[M.top];
   for (int c = 0; c < 2; ++c) {
@@ -908,23 +1149,26 @@ int cycle(const Multigrid& M, const MgState* st, cudaStream_t s) {
   ++launches;
   for (int l = M.top - 1; l >= 0; --l) {
     const Lev v = lev_of(M.level[l]), e = lev_of(M.level[l + 1]);
-    const int ch = chunk_of(v.H);
-    const dim3 g = grid_of(v.H, ch);
-    k_mg_sweep<true><<<g, blk, 0, s>>>(v, e, 0, st, ch);
-    k_mg_sweep<false><<<g, blk, 0, s>>>(v, e, 1, st, ch);
-    k_mg_sweep<false><<<g, blk, 0, s>>>(v, e, 0, st, ch);
+    const Columns g = columns(v.H.nx, v.H.ny, v.H.nz, 4);
+    k_mg_sweep<true, 0><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+    if (l == 0) {
+      k_mg_sweep<false, 1><<<g.grid, kThreads, 0, s>>>(v, e, 1, st, partials, g.w, g.chunk);
+      k_mg_sweep<false, 2><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+    } else {
+      k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 1, st, partials, g.w, g.chunk);
+      k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+    }
     launches += 3;
   }
   return launches;
 }
 
-int direction(const Multigrid& M, float* p, MgState* st, double* partials, bool loop,
-              cudaGraphConditionalHandle handle, cudaStream_t s) {
+int direction(const Multigrid& M, float* p, MgState* st, bool loop, cudaGraphConditionalHandle handle,
+              cudaStream_t s) {
   const Lev v = lev_of(M.level[0]);
-  const int ch = chunk_of(v.H);
-  k_mg_dot<<<reduction_blocks(v.H.total >> 2), 256, 0, s>>>(v, st, partials);
-  k_mg_direction<<<grid_of(v.H, ch), dim3(kBX, kBY, 1), 0, s>>>(v, p, st, ch, loop ? 1 : 0, handle);
-  return 2;
+  const Columns g = columns(v.L.nx, v.L.ny, v.L.nz, 4);
+  k_mg_direction<<<g.grid, kThreads, 0, s>>>(v, p, st, g.w, g.chunk, loop ? 1 : 0, handle);
+  return 1;
 }
 
 }  // namespace
@@ -933,33 +1177,31 @@ template <class T>
 int mg_start(const Multigrid& M, float* p, MgState* st, double* partials, double dx, double rho_neg, double rho_pos,
              cudaStream_t s) {
   const Lev v = lev_of(M.level[0]);
-  const int ch = chunk_of(v.H);
-  k_mg_defect<T, true><<<grid_of(v.H, ch), dim3(kBX, kBY, 1), 0, s>>>(v, st, partials, rho_neg, rho_pos,
-                                                                     1.0 / (dx * dx), ch);
-  int n = 1 + cycle(M, st, s);
-  return n + direction(M, p, st, partials, false, cudaGraphConditionalHandle{}, s);
+  const Columns g = columns(v.H.nx, v.H.ny, v.H.nz, 1);
+  k_mg_defect<T, true><<<g.grid, kThreads, 0, s>>>(v, st, partials, rho_neg, rho_pos, 1.0 / (dx * dx), g.w, g.chunk);
+  int n = 1 + cycle(M, st, partials, s);
+  return n + direction(M, p, st, false, cudaGraphConditionalHandle{}, s);
 }
 
 template <class T>
 int mg_iteration(const Multigrid& M, float* p, float* q, MgState* st, double* partials, double dx, double rho_neg,
                  double rho_pos, bool loop, cudaGraphConditionalHandle handle, cudaStream_t s) {
   const Lev v = lev_of(M.level[0]);
-  const int ch = chunk_of(v.H);
-  const dim3 g = grid_of(v.H, ch), blk(kBX, kBY, 1);
-  k_mg_spmv<<<g, blk, 0, s>>>(v, p, q, st, partials, ch);
-  k_mg_update<<<g, blk, 0, s>>>(v, p, q, st, partials, ch);
-  k_mg_defect<T, false><<<g, blk, 0, s>>>(v, st, partials, rho_neg, rho_pos, 1.0 / (dx * dx), ch);
-  int n = 3 + cycle(M, st, s);
-  return n + direction(M, p, st, partials, loop, handle, s);
+  const Columns g = columns(v.L.nx, v.L.ny, v.L.nz, 4), gd = columns(v.H.nx, v.H.ny, v.H.nz, 1);
+  k_mg_spmv<<<g.grid, kThreads, 0, s>>>(v, p, q, st, partials, g.w, g.chunk);
+  k_mg_update<<<g.grid, kThreads, 0, s>>>(v, p, q, st, partials, g.w, g.chunk);
+  k_mg_defect<T, false><<<gd.grid, kThreads, 0, s>>>(v, st, partials, rho_neg, rho_pos, 1.0 / (dx * dx), gd.w,
+                                                     gd.chunk);
+  int n = 3 + cycle(M, st, partials, s);
+  return n + direction(M, p, st, loop, handle, s);
 }
 
 void mg_anchor(const Multigrid& M, const unsigned short* dinv, MgState* st, double* partials, bool after,
                cudaStream_t s) {
   const MgLevel& f = M.level[0];
-  const int ch = chunk_of(f.H);
-  const dim3 g = grid_of(f.H, ch), blk(kBX, kBY, 1);
-  k_mg_anchor<<<g, blk, 0, s>>>(f.L, f.H, dinv, st, partials, after ? 1 : 0, ch);
-  if (after) k_mg_shift<<<g, blk, 0, s>>>(f.L, f.H, st, ch);
+  const Columns g = columns(f.H.nx, f.H.ny, f.H.nz, 1);
+  k_mg_anchor<<<g.grid, kThreads, 0, s>>>(f.L, f.H, dinv, st, partials, after ? 1 : 0, g.w, g.chunk);
+  if (after) k_mg_shift<<<g.grid, kThreads, 0, s>>>(f.L, st, g.w, g.chunk);
 }
 
 __global__ void k_mg_loop_start(cudaGraphConditionalHandle handle, const MgState* st) {

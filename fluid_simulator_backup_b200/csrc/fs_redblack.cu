@@ -99,7 +99,7 @@ __device__ __forceinline__ float rb_tau(const RbOp& A, const float* __restrict__
 
 __global__ void __launch_bounds__(32 * kRbBY) k_rb_red(RbOp A, const float* __restrict__ p, float* __restrict__ tau,
                                                       const PcgState* st, int kchunk) {
-  if (((volatile const PcgState*)st)->done) return;
+  if (state_read(&st->done)) return;
   const int h = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kRbBY + threadIdx.y;
   if (h >= A.Lh.nx || j >= A.Lh.ny) return;
   const int k0 = blockIdx.z * kchunk, k1 = min(A.Lh.nz, k0 + kchunk);
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(32 * kRbBY) k_rb_red(RbOp A, const float* __re
 __global__ void __launch_bounds__(32 * kRbBY) k_rb_black(RbOp A, const float* __restrict__ p,
                                                         const float* __restrict__ tau, float* __restrict__ q,
                                                         const PcgState* st, int kchunk) {
-  if (((volatile const PcgState*)st)->done) return;
+  if (state_read(&st->done)) return;
   const Lay& L = A.L;
   const Lay& H = A.Lh;
   const int h = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * kRbBY + threadIdx.y;
