@@ -98,6 +98,9 @@ struct fs_ctx {
   MgState *mgst = nullptr, *mgst_host = nullptr;  // device, pinned
   cudaGraphExec_t mg_graph = nullptr;
   int mg_launches[3] = {0, 0, 0};  // kernels of its start, of one iteration, of its end
+  // resident FP64 pressure solve of small boxes (fs_brick.cu)
+  BrickPlan brick;
+  void* brick_slots = nullptr;
   PipeGeom pipe{};  // the oil/water pipe's geometry (pipe.on = 0: the box)
   void* pgen[3] = {nullptr, nullptr, nullptr};  // pipe: masked periodic velocity copies
   void* pgx[3] = {nullptr, nullptr, nullptr};   // pipe: their ENO3-guarded copies along x
@@ -542,7 +545,7 @@ fs_status drive_pcg(fs_ctx* c, std::pair<int, const void*> key, F&& enqueue_iter
 
 template <class V>
 fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, V* x, V* r, V* p, V* q, double tol, int max_iter,
-                  int criterion, int* iterations, double* rel, int* status) {
+                  int criterion, int* iterations, double* rel, int* status, const void* phi = nullptr) {
   PcgState init{};
   init.tol = tol;
   init.max_iter = max_iter;
@@ -553,11 +556,27 @@ fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, V* x, V* r, V
   const bool timed = key < 100;  // pressure solves
   CK(cudaMemcpyAsync(c->st, c->st_host, sizeof(PcgState), cudaMemcpyHostToDevice, c->stream));
   if (timed) CK(cudaEventRecord(c->evp0, c->stream));
-  pcg_init<V>(A, b, x, r, p, c->st, c->partials, c->stream);
-  c->launches += 1;
-  CK(cudaGetLastError());
-  CKS(drive_pcg(c, std::make_pair(key, (const void*)nullptr),
-                [&] { cg_iteration<V, V>(A, x, r, p, q, c->st, c->partials, c->stream); }, max_iter, timed));
+  bool resident = false;
+  if constexpr (sizeof(V) == sizeof(double)) {
+    // an FP64 pressure solve (phi given) of a box that fits the SMs: one
+    // resident kernel
+    resident = phi && c->brick.gx > 0;
+    if (resident) {
+      CK(brick_solve(c->brick, A, (const double*)phi, b, x, q, c->brick_slots, c->st, c->grid.dx, c->prm.rho_neg,
+                     c->prm.rho_pos, c->stream));
+      CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(PcgState), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      c->launches += 1;
+      if (timed) c->pcg_launched_iterations += c->st_host->iter;
+    }
+  }
+  if (!resident) {
+    pcg_init<V>(A, b, x, r, p, c->st, c->partials, c->stream);
+    c->launches += 1;
+    CK(cudaGetLastError());
+    CKS(drive_pcg(c, std::make_pair(key, (const void*)nullptr),
+                  [&] { cg_iteration<V, V>(A, x, r, p, q, c->st, c->partials, c->stream); }, max_iter, timed));
+  }
   if (timed) {
     CK(cudaEventRecord(c->evp1, c->stream));
     CK(cudaEventSynchronize(c->evp1));
@@ -572,6 +591,10 @@ fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, V* x, V* r, V
   if (c->debug)
     std::fprintf(stderr, "[fs] pcg key %d: %d iterations, status %d, rel %.3e\n", key, s.iter, s.status,
                  s.bb > 0 ? std::sqrt(s.rr / s.bb) : 0.0);
+  if (s.status == PCG_TIMEOUT) {
+    set_error("a block of the resident pressure solve did not answer (key %d, iteration %d)", key, s.iter);
+    return FS_TIMEOUT;
+  }
   if (s.status == PCG_NONFINITE) {
     set_error("non-finite residual in a PCG solve (key %d, iteration %d)", key, s.iter);
     return FS_NONFINITE;
@@ -1185,7 +1208,7 @@ fs_status project_t(fs_ctx* c, double dt, double c0, double c1, fs_solve_report*
     Op7<double> A{(double*)c->pax, (double*)c->pay, (double*)c->paz, (double*)c->pdiag, c->Lc, 1, c->scalars + 12};
     A.c_extra = deflated_cell(c);
     CKS(run_pcg<double>(c, 1, A, c->b64, c->p64, (double*)c->pr, (double*)c->pp, (double*)c->pq, P.tolerance,
-                        P.max_iteration, P.stop, &iters, &rel, &st));
+                        P.max_iteration, P.stop, &iters, &rel, &st, phi));
     outer = 1;
   } else {
     CKS(mixed_solve<S>(c, phi, c->b64, c->p64, &iters, &outer, &rel, &st));
@@ -1579,7 +1602,7 @@ fs_status adj_projection(fs_ctx* c, void* phi, void* const ustar[3], const doubl
                                        c->a_diag, c->scalars + 12, deflate(c), s);
     Op7<double> A{c->a_ax, c->a_ay, c->a_az, c->a_diag, c->Lc, 1, c->scalars + 12};
     CKS(run_pcg<double>(c, 3, A, pbar, lam, c->a_r, c->a_p, c->a_q, P.tolerance, std::max(P.max_iteration, 1),
-                        FS_STOP_RELATIVE, &it, &rel, &st));
+                        FS_STOP_RELATIVE, &it, &rel, &st, phi));
   }
   if (st != PCG_CONVERGED) {
     c->adj_unconverged += 1;
@@ -1928,6 +1951,12 @@ fs_status fs_create(const fs_grid_desc* grid, const fs_params* params, fs_ctx** 
   if ((s = dalloc(c, (void**)&c->tickets, 8 * sizeof(unsigned int))) != FS_OK) return fail(s);
   if ((s = dalloc(c, (void**)&c->scalars, 16 * sizeof(double))) != FS_OK) return fail(s);
   if ((s = dalloc(c, (void**)&c->st, sizeof(PcgState))) != FS_OK) return fail(s);
+  if (!c->fp32 && !prm.pipe) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) == cudaSuccess)
+      c->brick = brick_plan(c->Lc, sms);
+    if (c->brick.gx > 0 && (s = dalloc(c, &c->brick_slots, brick_slots_bytes())) != FS_OK) return fail(s);
+  }
   const int64_t maxf = std::max(std::max(c->Lu.total, c->Lv.total), std::max(c->Lw.total, c->Lc.total));
   if ((s = dalloc(c, (void**)&c->staging, (size_t)maxf * sizeof(double))) != FS_OK) return fail(s);
   if (cudaMallocHost((void**)&c->st_host, sizeof(PcgState)) != cudaSuccess ||

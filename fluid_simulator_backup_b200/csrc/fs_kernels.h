@@ -141,8 +141,9 @@ struct PcgState {
 // (p.Ap <= 0 or no improvement for stall_limit iterations); the iterate is
 // kept and the caller decides.  RELIABLE_UPDATE: paused (done = 2) for the
 // caller to replace the recursive residual by the true one.
+// TIMEOUT: a wait of the resident solve (fs_brick.cu) ran out.
 enum { PCG_RUNNING = 0, PCG_CONVERGED = 1, PCG_MAXITER = 2, PCG_NONFINITE = 3, PCG_STAGNATED = 4,
-       PCG_RELIABLE_UPDATE = 5 };
+       PCG_RELIABLE_UPDATE = 5, PCG_TIMEOUT = 6 };
 
 // Seven-point symmetric operator on a padded layout:
 // (A x)_c = diag_c x_c - sum_d (a_d[c] x_{c-e_d} + a_d[c+e_d] x_{c+e_d});
@@ -237,6 +238,23 @@ template <class S, class D> void rb_gather(const S* full, D* half, const Lay& L,
 template <class V, class R = V>
 void pcg_resume(const Op7<V>& A, const R* r, V* p, PcgState* st, double* partials, int restart, cudaStream_t s);
 int pcg_blocks(const Lay& L);
+
+// ---- resident FP64 pressure solve (fs_brick.cu)
+struct BrickPlan {
+  int gx = 0, gy = 0, gz = 0;  // bricks along each axis; gx = 0: the grid does not fit
+  int per_thread = 0;
+  bool xg = false;             // the iterate stays in global memory
+  size_t smem = 0;
+  int cap = 0;                 // cells next to the interface listed in shared memory
+};
+BrickPlan brick_plan(const Lay& L, int sms);
+size_t brick_slots_bytes();
+// The whole solve in one cooperative launch: the iteration of run_pcg with its
+// tests and its final state in st (tol, criterion and max_iter set by the
+// caller).  zx: a cell field for the exchanged z.
+cudaError_t brick_solve(const BrickPlan& P, const Op7<double>& A, const double* phi, const double* b, double* x,
+                        double* zx, void* slots, PcgState* st, double dx, double rho_neg, double rho_pos,
+                        cudaStream_t s);
 
 // ---- multigrid-preconditioned pressure solve (fs_multigrid.cu)
 constexpr int kMgMaxLevels = 14;
