@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
                     (k < L.nz - 1) << 5;
       const double* ph = A.phi + base + o;
       const bool n = ph[0] <= 0.0;
-      const bool same = (!(f & 1) || (ph[-1] <= 0.0) == n) && (!(f & 2) || (ph[1] <= 0.0) == n) &&
+      const bool same = ph[0] == ph[0] && (!(f & 1) || (ph[-1] <= 0.0) == n) && (!(f & 2) || (ph[1] <= 0.0) == n) &&
                         (!(f & 4) || (ph[-L.px] <= 0.0) == n) && (!(f & 8) || (ph[L.px] <= 0.0) == n) &&
                         (!(f & 16) || (ph[-L.slab] <= 0.0) == n) && (!(f & 32) || (ph[L.slab] <= 0.0) == n);
       const bool extra = base + o == A.c_extra;

@@ -51,6 +51,9 @@ void set_error(const char* fmt, ...) {
   } while (0)
 
 constexpr int kGraphIters = 16;
+// the viscosity solves converge in 1 to 10 iterations: a batch of 16 would
+// mostly be launches of kernels that return at once
+constexpr int kViscosityIters = 4;
 
 // A device buffer typed at run time (float or double storage).
 struct Buf {
@@ -116,10 +119,9 @@ struct fs_ctx {
   PcgState* st_host = nullptr;      // pinned
   double* sc_host = nullptr;        // pinned [16]
   double* staging = nullptr;        // packed FP64 transfer buffer
-  // captured solver graphs keyed by solve kind and the one operand whose
-  // buffer rotates between calls (the level set); kernel arguments are
-  // baked into a graph, so a different buffer needs its own graph
-  std::map<std::pair<int, const void*>, cudaGraphExec_t> graphs;
+  // captured solver graphs keyed by solve kind; kernel arguments are baked
+  // into a graph, what changes between calls is in the device state
+  std::map<int, cudaGraphExec_t> graphs;
   // accounting for fs_step_report
   int64_t launches = 0;
   float pcg_ms = 0.0f;
@@ -459,46 +461,46 @@ fs_status box_only(const fs_ctx* c, const char* what) {
 
 // The loop control of a captured solve: before the loop it clears the batch
 // counter and lets the loop start only if the solve is still running; after
-// each batch of kGraphIters iterations it continues the loop while the solve
-// runs and fewer than max_iter / kGraphIters + 2 batches have run (the
+// each batch of iterations it continues the loop while the solve
+// runs and fewer than max_iter / batch + 2 batches have run (the
 // bound that guarantees the loop ends whatever the state says).
 __global__ void k_loop_start(cudaGraphConditionalHandle h, const PcgState* st, unsigned int* batches) {
   *batches = 0u;
   cudaGraphSetConditional(h, ((volatile const PcgState*)st)->done == 0 ? 1u : 0u);
 }
-__global__ void k_loop_next(cudaGraphConditionalHandle h, const PcgState* st, unsigned int* batches) {
+__global__ void k_loop_next(cudaGraphConditionalHandle h, const PcgState* st, unsigned int* batches, int batch) {
   const volatile PcgState* vs = (volatile const PcgState*)st;
   const unsigned int n = *batches + 1u;
   *batches = n;
-  const unsigned int cap = (unsigned int)(vs->max_iter / kGraphIters + 2);
+  const unsigned int cap = (unsigned int)(vs->max_iter / batch + 2);
   cudaGraphSetConditional(h, (vs->done == 0 && n < cap) ? 1u : 0u);
 }
 
 // Run the iterations of a solve until its state says stop (done != 0), as
 // ONE graph launch: a captured CUDA graph whose conditional while node
-// repeats a body of kGraphIters iterations plus the loop control above, so
+// repeats a body of `batch` iterations plus the loop control above, so
 // the host waits once per solve (or per reliable update of the mixed
 // solve) instead of once per batch.  The graph is captured on first use per
 // key (kernel arguments are baked into it).
 template <class F>
-fs_status drive_pcg(fs_ctx* c, std::pair<int, const void*> key, F&& enqueue_iteration, int max_iter, bool timed,
-                    int kernels_per_iteration = 3) {
+fs_status drive_pcg(fs_ctx* c, int key, F&& enqueue_iteration, int max_iter, bool timed,
+                    int kernels_per_iteration = 3, int batch = kGraphIters) {
   if (c->prm.host_loop) {
     // the same batches launched from the host, the state polled after each;
     // bounded like the graph's loop
-    const int cap = max_iter / kGraphIters + 2;
+    const int cap = max_iter / batch + 2;
     int nb = 0;
     CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(PcgState), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     while (!c->st_host->done && nb < cap) {
-      for (int n = 0; n < kGraphIters; ++n) enqueue_iteration();
+      for (int n = 0; n < batch; ++n) enqueue_iteration();
       CK(cudaGetLastError());
       ++nb;
       CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(PcgState), cudaMemcpyDeviceToHost, c->stream));
       CK(cudaStreamSynchronize(c->stream));
     }
-    c->launches += (int64_t)nb * kernels_per_iteration * kGraphIters;
-    if (timed) c->pcg_launched_iterations += nb * kGraphIters;
+    c->launches += (int64_t)nb * kernels_per_iteration * batch;
+    if (timed) c->pcg_launched_iterations += nb * batch;
     return FS_OK;
   }
   unsigned int* batches = c->tickets + 6;
@@ -524,8 +526,8 @@ fs_status drive_pcg(fs_ctx* c, std::pair<int, const void*> key, F&& enqueue_iter
     CK(cudaGraphAddNode(&loop, g, &start, 1, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    for (int n = 0; n < kGraphIters; ++n) enqueue_iteration();
-    k_loop_next<<<1, 1, 0, c->stream>>>(h, c->st, batches);
+    for (int n = 0; n < batch; ++n) enqueue_iteration();
+    k_loop_next<<<1, 1, 0, c->stream>>>(h, c->st, batches, batch);
     CK(cudaStreamEndCapture(c->stream, &body));
     cudaGraphExec_t ge;
     CK(cudaGraphInstantiate(&ge, g, 0));
@@ -538,18 +540,19 @@ fs_status drive_pcg(fs_ctx* c, std::pair<int, const void*> key, F&& enqueue_iter
   CK(cudaMemcpyAsync(c->sc_host + 15, batches, sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   std::memcpy(&nb, c->sc_host + 15, sizeof nb);
-  c->launches += 1 + (int64_t)nb * (kernels_per_iteration * kGraphIters + 1);
-  if (timed) c->pcg_launched_iterations += (int)nb * kGraphIters;
+  c->launches += 1 + (int64_t)nb * (kernels_per_iteration * batch + 1);
+  if (timed) c->pcg_launched_iterations += (int)nb * batch;
   return FS_OK;
 }
 
 template <class V>
-fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, V* x, V* r, V* p, V* q, double tol, int max_iter,
-                  int criterion, int* iterations, double* rel, int* status, const void* phi = nullptr) {
+fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, const V* x0, V* x, V* r, V* p, V* q, double tol,
+                  int max_iter, int criterion, int* iterations, double* rel, int* status, const void* phi = nullptr) {
   PcgState init{};
   init.tol = tol;
   init.max_iter = max_iter;
   init.criterion = criterion;
+  init.x = x;
   // FP32 viscosity solves can stall at their rounding floor before a tight tolerance
   init.stall_limit = (c->fp32 && key >= 100 && key < 110) ? 400 : 0;  // the FP32 forward viscosity solves
   *c->st_host = init;
@@ -571,11 +574,11 @@ fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, V* x, V* r, V
     }
   }
   if (!resident) {
-    pcg_init<V>(A, b, x, r, p, c->st, c->partials, c->stream);
+    pcg_init<V>(A, b, x0, x, r, p, c->st, c->partials, c->stream);
     c->launches += 1;
     CK(cudaGetLastError());
-    CKS(drive_pcg(c, std::make_pair(key, (const void*)nullptr),
-                  [&] { cg_iteration<V, V>(A, x, r, p, q, c->st, c->partials, c->stream); }, max_iter, timed));
+    CKS(drive_pcg(c, key, [&] { cg_iteration<V, V>(A, r, p, q, c->st, c->partials, c->stream); }, max_iter, timed, 3,
+                  timed ? kGraphIters : kViscosityIters));
   }
   if (timed) {
     CK(cudaEventRecord(c->evp1, c->stream));
@@ -669,8 +672,11 @@ static double velocity_epsilon(const fs_ctx* c) {
   return c->prm.velocity_epsilon > 0.0 ? c->prm.velocity_epsilon : c->prm.weno_epsilon;
 }
 
+// in_step: followed by the no-penetration zeroing (not in the faithful
+// projection) and gravity, which the box's kernel does in the same pass; a
+// taped forward leaves both to its caller.
 template <class S>
-fs_status advect_velocity_t(fs_ctx* c, double dt, bool taped = false) {
+fs_status advect_velocity_t(fs_ctx* c, double dt, bool taped = false, bool in_step = false) {
   const double eps = velocity_epsilon(c), dx = c->grid.dx;
   S *u = F<S>(c->u), *v = F<S>(c->v), *w = F<S>(c->w);
   if (c->pipe.on) {
@@ -693,20 +699,23 @@ fs_status advect_velocity_t(fs_ctx* c, double dt, bool taped = false) {
     CK(cudaGetLastError());
     return FS_OK;
   }
-  if (c->prm.velocity_scheme == FS_VELOCITY_ENO3) {
-    eno3_mac<S>(u, F<S>(c->ua), u, v, w, c->Lu, c->Lu, c->Lv, c->Lw, 0, dx, dt, c->stream);
-    eno3_mac<S>(v, F<S>(c->va), u, v, w, c->Lv, c->Lu, c->Lv, c->Lw, 1, dx, dt, c->stream);
-    eno3_mac<S>(w, F<S>(c->wa), u, v, w, c->Lw, c->Lu, c->Lv, c->Lw, 2, dx, dt, c->stream);
-  } else if (taped) {
+  if (taped) {
+    // WENO5 (the adjoints cover no other)
     taped_mac<S>(u, F<S>(c->ua), u, v, w, c->Lu, c->Lu, c->Lv, c->Lw, 0, dx, eps, dt, c->stream);
     taped_mac<S>(v, F<S>(c->va), u, v, w, c->Lv, c->Lu, c->Lv, c->Lw, 1, dx, eps, dt, c->stream);
     taped_mac<S>(w, F<S>(c->wa), u, v, w, c->Lw, c->Lu, c->Lv, c->Lw, 2, dx, eps, dt, c->stream);
+    c->launches += 3;
   } else {
-    weno5_mac<S>(u, F<S>(c->ua), u, v, w, c->Lu, c->Lu, c->Lv, c->Lw, 0, dx, eps, dt, c->stream);
-    weno5_mac<S>(v, F<S>(c->va), u, v, w, c->Lv, c->Lu, c->Lv, c->Lw, 1, dx, eps, dt, c->stream);
-    weno5_mac<S>(w, F<S>(c->wa), u, v, w, c->Lw, c->Lu, c->Lv, c->Lw, 2, dx, eps, dt, c->stream);
+    const S* const in[3] = {u, v, w};
+    S* const out[3] = {F<S>(c->ua), F<S>(c->va), F<S>(c->wa)};
+    const Lay* const lays[3] = {&c->Lu, &c->Lv, &c->Lw};
+    double add[3] = {0.0, 0.0, 0.0};
+    if (in_step)
+      for (int a = 0; a < 3; ++a) add[a] = dt * c->prm.gravity[a];
+    mac_advect<S>(in, out, lays, c->prm.velocity_scheme == FS_VELOCITY_ENO3, dx, eps, dt, add,
+                  in_step && !(c->prm.flags & FS_FLAG_FAITHFUL_PROJECTION) ? 1 : 0, c->stream);
+    c->launches += 1;
   }
-  c->launches += 3;
   std::swap(c->u, c->ua);
   std::swap(c->v, c->va);
   std::swap(c->w, c->wa);
@@ -821,29 +830,26 @@ fs_status viscosity_t(fs_ctx* c, double dt, int* iters_out) {
     return FS_OK;
   }
   const Lay* lays[3] = {&c->Lu, &c->Lv, &c->Lw};
-  void* comps[3] = {c->u, c->v, c->w};
+  void** comps[3] = {&c->u, &c->v, &c->w};
   // all three systems from the pre-viscosity velocities
   for (int a = 0; a < 3; ++a) {
     viscosity_system<S>(F<S>(c->phi), F<S>(c->u), F<S>(c->v), F<S>(c->w), c->Lc, c->Lu, c->Lv, c->Lw, a,
                         c->grid.dx, dt, P.rho_neg, P.rho_pos, P.mu_neg, P.mu_pos, F<S>(c->vs[a][0]),
                         F<S>(c->vs[a][1]), F<S>(c->vs[a][2]), F<S>(c->vs[a][3]), F<S>(c->vs[a][4]), c->stream);
     c->launches += 1;
-    CK(cudaMemcpyAsync(c->vs[a][5], comps[a], lays[a]->total * c->S(), cudaMemcpyDeviceToDevice, c->stream));
   }
   CK(cudaGetLastError());
   int total = 0;
   for (int a = 0; a < 3; ++a) {
     Op7<S> A{F<S>(c->vs[a][0]), F<S>(c->vs[a][1]), F<S>(c->vs[a][2]), F<S>(c->vs[a][3]), *lays[a]};
     int it = 0, st = 0;
-    CKS(run_pcg<S>(c, 100 + a, A, F<S>(c->vs[a][4]), F<S>(c->vs[a][5]), F<S>(c->vs[a][6]), F<S>(c->vs[a][7]),
-                   F<S>(c->vs[a][8]), P.viscosity_tolerance, P.viscosity_max_iteration, FS_STOP_RELATIVE, &it,
-                   nullptr, &st));
+    CKS(run_pcg<S>(c, 100 + a, A, F<S>(c->vs[a][4]), F<S>(*comps[a]), F<S>(c->vs[a][5]), F<S>(c->vs[a][6]),
+                   F<S>(c->vs[a][7]), F<S>(c->vs[a][8]), P.viscosity_tolerance, P.viscosity_max_iteration,
+                   FS_STOP_RELATIVE, &it, nullptr, &st));
     total += it;
   }
-  // the solution buffers stay where the captured solver graphs expect them;
-  // copy the result back into the velocity fields
-  for (int a = 0; a < 3; ++a)
-    CK(cudaMemcpyAsync(comps[a], c->vs[a][5], lays[a]->total * c->S(), cudaMemcpyDeviceToDevice, c->stream));
+  // the solutions become the velocity fields (an error above leaves them)
+  for (int a = 0; a < 3; ++a) std::swap(*comps[a], c->vs[a][5]);
   if (iters_out) *iters_out = total;
   return FS_OK;
 }
@@ -1080,6 +1086,7 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     init.tol = P.tolerance * std::sqrt(bb);
     init.max_iter = P.max_iteration;
     init.reliable_delta = c->reliable_delta;
+    init.x = rb ? (void*)c->rb_x : (void*)x;
     init.bb = bb;  // ||b||^2 of the pressure system, for the recursive relative residual
     *c->st_host = init;
     CK(cudaMemcpyAsync(c->st, c->st_host, sizeof(PcgState), cudaMemcpyHostToDevice, s));
@@ -1092,14 +1099,11 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     for (;;) {
       ++passes;  // each pass runs at least one iteration or ends the solve; this bounds the host loop too
       if (rb) {
-        CKS(drive_pcg(c, std::make_pair(4, (const void*)nullptr),
-                      [&] {
-                        rb_iteration(R, Ah, c->rb_x, c->rb_r, c->rb_p, c->rb_q, c->rb_tau, c->st, c->partials, s);
-                      },
-                      P.max_iteration, true, 4));
+        CKS(drive_pcg(c, 4,
+                      [&] { rb_iteration(R, Ah, c->rb_r, c->rb_p, c->rb_q, c->rb_tau, c->st, c->partials, s); },
+                      P.max_iteration, true, 5));
       } else {
-        CKS(drive_pcg(c, std::make_pair(2, (const void*)x),
-                      [&] { cg_iteration<float, double>(A, x, r32, p32, q32, c->st, c->partials, s); },
+        CKS(drive_pcg(c, 2, [&] { cg_iteration<float, double>(A, r32, p32, q32, c->st, c->partials, s); },
                       P.max_iteration, true));
       }
       const int status = c->st_host->status;
@@ -1207,7 +1211,7 @@ fs_status project_t(fs_ctx* c, double dt, double c0, double c1, fs_solve_report*
                                        pipe_of(c));
     Op7<double> A{(double*)c->pax, (double*)c->pay, (double*)c->paz, (double*)c->pdiag, c->Lc, 1, c->scalars + 12};
     A.c_extra = deflated_cell(c);
-    CKS(run_pcg<double>(c, 1, A, c->b64, c->p64, (double*)c->pr, (double*)c->pp, (double*)c->pq, P.tolerance,
+    CKS(run_pcg<double>(c, 1, A, c->b64, c->p64, c->p64, (double*)c->pr, (double*)c->pp, (double*)c->pq, P.tolerance,
                         P.max_iteration, P.stop, &iters, &rel, &st, phi));
     outer = 1;
   } else {
@@ -1220,13 +1224,12 @@ fs_status project_t(fs_ctx* c, double dt, double c0, double c1, fs_solve_report*
                              P.rho_pos, sigma, s);
     c->launches += 4;
   } else {
-    velocity_correct<S>(u, F<S>(c->u0), c->p64, phi, c->Lu, c->Lc, 0, dx, dt, P.rho_neg, P.rho_pos, faithful, c0, c1,
-                        kap, sigma, s);
-    velocity_correct<S>(v, F<S>(c->v0), c->p64, phi, c->Lv, c->Lc, 1, dx, dt, P.rho_neg, P.rho_pos, faithful, c0, c1,
-                        kap, sigma, s);
-    velocity_correct<S>(w, F<S>(c->w0), c->p64, phi, c->Lw, c->Lc, 2, dx, dt, P.rho_neg, P.rho_pos, faithful, c0, c1,
-                        kap, sigma, s);
-    c->launches += 3;
+    S* const vel[3] = {u, v, w};
+    const S* const base[3] = {F<S>(c->u0), F<S>(c->v0), F<S>(c->w0)};
+    const Lay* const lays[3] = {&c->Lu, &c->Lv, &c->Lw};
+    velocity_correct<S>(vel, base, c->p64, phi, lays, c->Lc, dx, dt, P.rho_neg, P.rho_pos, faithful, c0, c1, kap, sigma,
+                        s);
+    c->launches += faithful ? 3 : 1;
   }
   CK(cudaGetLastError());
   if (rep) {
@@ -1286,16 +1289,17 @@ template <class S>
 fs_status stage_t(fs_ctx* c, double dt, double c0, double c1, fs_step_report* rep, Tape* tp = nullptr,
                   int stage = 0) {
   if (tp) CKS(tape_velocity(c, tp->vel[stage][0]));
-  CKS(advect_velocity_t<S>(c, dt, tp != nullptr));
+  CKS(advect_velocity_t<S>(c, dt, tp != nullptr, true));
   const Lay* lays[3] = {&c->Lu, &c->Lv, &c->Lw};
-  if (!(c->prm.flags & FS_FLAG_FAITHFUL_PROJECTION) && !c->pipe.on) {
+  const bool fused = !c->pipe.on && !tp;  // the advection kernel has zeroed the walls and added gravity
+  if (!(c->prm.flags & FS_FLAG_FAITHFUL_PROJECTION) && !c->pipe.on && !fused) {
     // no penetration: advection also updates the wall faces, which hold zero
     zero_walls<S>(F<S>(c->u), *lays[0], 0, c->stream);
     zero_walls<S>(F<S>(c->v), *lays[1], 1, c->stream);
     zero_walls<S>(F<S>(c->w), *lays[2], 2, c->stream);
     c->launches += 3;
   }
-  CKS(gravity_t<S>(c, dt));
+  if (!fused) CKS(gravity_t<S>(c, dt));
   if (tp) CKS(tape_velocity(c, tp->vel[stage][1]));
   int vit = 0;
   CKS(viscosity_t<S>(c, dt, &vit));
@@ -1601,7 +1605,7 @@ fs_status adj_projection(fs_ctx* c, void* phi, void* const ustar[3], const doubl
     build_pressure_operator<S, double>(F<S>(phi), c->Lc, dx, P.rho_neg, P.rho_pos, c->a_ax, c->a_ay, c->a_az,
                                        c->a_diag, c->scalars + 12, deflate(c), s);
     Op7<double> A{c->a_ax, c->a_ay, c->a_az, c->a_diag, c->Lc, 1, c->scalars + 12};
-    CKS(run_pcg<double>(c, 3, A, pbar, lam, c->a_r, c->a_p, c->a_q, P.tolerance, std::max(P.max_iteration, 1),
+    CKS(run_pcg<double>(c, 3, A, pbar, lam, lam, c->a_r, c->a_p, c->a_q, P.tolerance, std::max(P.max_iteration, 1),
                         FS_STOP_RELATIVE, &it, &rel, &st, phi));
   }
   if (st != PCG_CONVERGED) {
@@ -1648,7 +1652,7 @@ fs_status adj_viscosity(fs_ctx* c, void* phi, void* const ug[3], void* const x[3
     CK(cudaMemsetAsync(c->a_vlam[a], 0, lays[a]->total * sizeof(double), s));
     Op7<double> A{c->a_vs[a][0], c->a_vs[a][1], c->a_vs[a][2], c->a_vs[a][3], *lays[a]};
     int it = 0, st = 0;
-    CKS(run_pcg<double>(c, 120 + a, A, c->a_vxb[a], c->a_vlam[a], c->a_vs[a][6], c->a_vs[a][7], c->a_vs[a][8],
+    CKS(run_pcg<double>(c, 120 + a, A, c->a_vxb[a], c->a_vlam[a], c->a_vlam[a], c->a_vs[a][6], c->a_vs[a][7], c->a_vs[a][8],
                         P.viscosity_tolerance, std::max(P.viscosity_max_iteration, 1), FS_STOP_RELATIVE, &it, nullptr,
                         &st));
     if (st != PCG_CONVERGED) {

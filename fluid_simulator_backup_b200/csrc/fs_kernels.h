@@ -75,12 +75,11 @@ template <class T>
 void weno5_levelset(const T* src, const T* base, T* out, const T* u, const T* v, const T* w, const Lay& L,
                     const Lay& Lu, const Lay& Lv, const Lay& Lw, double dx, double eps, double dt, double c0, double c1,
                     cudaStream_t s, const PipeGeom* pipe = nullptr);
+// self-advection of the three MAC components, WENO5 or ENO3; in a step also
+// add[a] off the component's walls and, with zero_walls, zero on them
 template <class T>
-void weno5_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
-               const Lay& Lw, int axis, double dx, double eps, double dt, cudaStream_t s);
-template <class T>
-void eno3_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
-              const Lay& Lw, int axis, double dx, double dt, cudaStream_t s);
+void mac_advect(const T* const in[3], T* const out[3], const Lay* const L[3], bool eno, double dx, double eps, double dt,
+                const double add[3], int zero_walls, cudaStream_t s);
 template <class T> void sign_function(const T* phi, T* sgn, const Lay& L, double dx, cudaStream_t s);
 // The zero level set as a triangle mesh in device memory (fs_surface.cu).
 struct SurfaceMesh {
@@ -132,6 +131,7 @@ struct PcgState {
   double alpha;           // step length of the current iteration (set by the SpMV)
   int iter, max_iter, done, criterion, status, stall;
   int stall_limit;  // iterations without a 1% improvement of best_rr before giving up (0: never)
+  void* x;          // the iterate (type of the solve), set by the host: one captured graph serves any buffer
   int x_pending;    // alpha is set and x += alpha p is still due (applied by the direction update)
   unsigned int ticket;
   unsigned int ticket2;  // completion count of the direction update
@@ -183,18 +183,20 @@ template <class V> struct Op7 {
   const unsigned short* dinv16 = nullptr;  // bf16 bit patterns of 1/diag
 };
 
-template <class V, class R = V>
-void pcg_init(const Op7<V>& A, const R* b, R* x, R* r, V* p, PcgState* st, double* partials, cudaStream_t s);
+// the start of a solve from the guess x0 (x may be x0)
+template <class V>
+void pcg_init(const Op7<V>& A, const V* b, const V* x0, V* x, V* r, V* p, PcgState* st, double* partials,
+              cudaStream_t s);
 // One iteration with the iterate update deferred into the direction update
-// (x of type X, r, p, q and the operator of type V): SpMV + alpha, residual
+// (st->x of type X, r, p, q and the operator of type V): SpMV + alpha, residual
 // update + beta, then x += alpha p and p = z + beta p in one pass over p.
 template <class V, class X>
-void cg_iteration(const Op7<V>& A, X* x, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s);
+void cg_iteration(const Op7<V>& A, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s);
 // The two pointwise kernels of cg_iteration alone (residual update, then the
 // deferred iterate update and the direction update), after a SpMV that set
 // alpha in the state.
 template <class V, class X>
-void cg_vector_updates(const Op7<V>& A, X* x, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s);
+void cg_vector_updates(const Op7<V>& A, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s);
 // p.q and the step length (alpha, or a stagnation stop) for a SpMV that
 // wrote q without reducing p.q (the red-black black pass)
 template <class V>
@@ -222,7 +224,8 @@ int rb_blocks(const Lay& Lh);
 // One CG iteration on the black Schur complement: red stage (tau), black
 // stage (q = S p, p.q, alpha), then cg_vector_updates on the packed black
 // vectors with Ah (layout Lh, dinv16 the packed black bf16 1/diag).
-void rb_iteration(const RbOp& A, const Op7<float>& Ah, double* xh, float* rh, float* ph, float* qh, float* tau,
+// (the iterate is st->x, packed)
+void rb_iteration(const RbOp& A, const Op7<float>& Ah, float* rh, float* ph, float* qh, float* tau,
                   PcgState* st, double* partials, cudaStream_t s);
 // p64 <- black cells from the packed iterate xh, red cells eliminated in FP64
 // from phi and b (the red rows of b - A p64 vanish)
@@ -338,10 +341,11 @@ void defect_residual(const T* phi, const double* p64, const float* x32, const do
                      const Lay& Lc, double dx, double rho_neg, double rho_pos, double* partials, unsigned int* ticket,
                      double* rr_out, int deflate, cudaStream_t s, const PipeGeom* pipe = nullptr);
 void add_correction(double* p64, const float* e, const Lay& Lc, cudaStream_t s);
+// the pressure-gradient update of the three components, with the RK combination
 template <class T>
-void velocity_correct(T* f, const T* base, const double* p, const T* phi, const Lay& Lf, const Lay& Lc, int axis,
-                      double dx, double dt, double rho_neg, double rho_pos, int faithful, double c0, double c1,
-                      const double* kappa, double sigma, cudaStream_t s);
+void velocity_correct(T* const f[3], const T* const base[3], const double* p, const T* phi, const Lay* const Lf[3],
+                      const Lay& Lc, double dx, double dt, double rho_neg, double rho_pos, int faithful, double c0,
+                      double c1, const double* kappa, double sigma, cudaStream_t s);
 // mean curvature of phi (ghosts must be filled) and max |kappa| near the interface
 template <class T>
 void curvature(const T* phi, double* kappa, const Lay& L, double dx, int typo, double* kmax, cudaStream_t s);

@@ -60,46 +60,33 @@ __device__ __forceinline__ R precond1(const Op7<V>& A, R r, int64_t c) {
   return A.dinv16 ? r * (R)bf16_to_float(A.dinv16[c]) : r / (R)A.diag[c];
 }
 
-// (A x)_c evaluated in the type X of x (the operator's coefficients are
-// converted): FP32 iterates get FP32 arithmetic, FP64 iterates FP64.
-// The flux form is evaluated here in FP64 (loads in their storage type):
-// for smooth x the six fluxes nearly cancel, and FP64 keeps q exact to
-// rounding.  (The iteration's own SpMV, k_cg_spmv, may form FP32 fluxes in
-// FP32: see Op7::flux32.)
-template <class V, class X>
-__device__ __forceinline__ X apply7(const Op7<V>& A, const X* __restrict__ x, int64_t c) {
-  const int64_t sy = A.L.px, sz = A.L.slab;
-  const X xc = x[c];
-  if (A.flux_form) {
-    const double d = (double)xc;
-    double acc = (double)A.ax[c] * (d - (double)x[c - 1]) + (double)A.ax[c + 1] * (d - (double)x[c + 1]);
-    acc += (double)A.ay[c] * (d - (double)x[c - sy]) + (double)A.ay[c + sy] * (d - (double)x[c + sy]);
-    acc += (double)A.az[c] * (d - (double)x[c - sz]) + (double)A.az[c + sz] * (d - (double)x[c + sz]);
-    if (c == (A.c_extra >= 0 ? A.c_extra : A.L.at(0, 0, 0))) acc += (*A.extra0) * d;
-    return (X)acc;
-  }
-  X acc = (X)A.diag[c] * xc;
-  acc -= (X)A.ax[c] * x[c - 1] + (X)A.ax[c + 1] * x[c + 1];
-  acc -= (X)A.ay[c] * x[c - sy] + (X)A.ay[c + sy] * x[c + sy];
-  acc -= (X)A.az[c] * x[c - sz] + (X)A.az[c + sz] * x[c + sz];
-  return acc;
+// Three FP64 sums through one grid reduction: one pass over the warps, the
+// block and the partial sums for all three (three passes of six barriers each
+// cost a residual update of 96^3 black cells 0.9 of its 8.1 us).
+__device__ __forceinline__ void block_sum3(double v[3]) {
+  __shared__ double part[3][32];
+  const int t = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z), lane = t & 31, warp = t >> 5;
+  const int nwarps = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) v[m] = warp_sum(v[m]);
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) part[m][warp] = v[m];
+  __syncthreads();
+  if (warp == 0)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) v[m] = warp_sum(lane < nwarps ? part[m][lane] : 0.0);
 }
-
-// Three FP64 sums through one grid reduction (1-D grids).
 __device__ __forceinline__ bool grid_reduce3(double a, double b, double c, double* partials, unsigned int* ticket,
                                              double out[3]) {
   __shared__ bool is_last;
-  __shared__ double tot[3];
-  a = block_sum(a);
-  __syncthreads();
-  b = block_sum(b);
-  __syncthreads();
-  c = block_sum(c);
-  const int nb = gridDim.x;
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x] = a;
-    partials[nb + blockIdx.x] = b;
-    partials[2 * nb + blockIdx.x] = c;
+  double v[3] = {a, b, c};
+  block_sum3(v);
+  const int nb = num_blocks(), fb = flat_block();
+  if (thread0()) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) partials[m * nb + fb] = v[m];
     __threadfence();
     const unsigned int t = atomicAdd(ticket, 1u);
     is_last = (t == (unsigned int)(nb - 1));
@@ -107,21 +94,20 @@ __device__ __forceinline__ bool grid_reduce3(double a, double b, double c, doubl
   __syncthreads();
   if (!is_last) return false;
   __threadfence();
-  for (int m = 0; m < 3; ++m) {
-    double s = 0.0;
-#pragma unroll 8
-    for (int q = threadIdx.x; q < nb; q += blockDim.x) s += __ldcg(partials + m * nb + q);  // as in grid_reduce_sum
-    s = block_sum(s);
-    if (threadIdx.x == 0) tot[m] = s;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    out[0] = tot[0];
-    out[1] = tot[1];
-    out[2] = tot[2];
+  v[0] = v[1] = v[2] = 0.0;
+  const int nt = blockDim.x * blockDim.y * blockDim.z;
+#pragma unroll 4
+  for (int q = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z); q < nb; q += nt)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) v[m] += __ldcg(partials + m * nb + q);  // as in grid_reduce_sum
+  block_sum3(v);
+  if (thread0()) {
+    out[0] = v[0];
+    out[1] = v[1];
+    out[2] = v[2];
     *ticket = 0u;
   }
-  return threadIdx.x == 0;
+  return thread0();
 }
 
 __device__ __forceinline__ bool stop_test(const PcgState* st, double rz, double rr) {
@@ -129,49 +115,6 @@ __device__ __forceinline__ bool stop_test(const PcgState* st, double rz, double 
     case 1: return rz < st->tol * st->tol;                 // the reference's r.z < tol^2
     case 2: return rr < st->tol * st->tol;                 // absolute 2-norm
     default: return sqrt(rr) <= st->tol * sqrt(st->bb);    // relative 2-norm
-  }
-}
-
-template <class V, class RT>
-__global__ void __launch_bounds__(kRedThreads) k_pcg_init(Op7<V> A, const RT* b, RT* x, RT* r, V* __restrict__ p,
-                                                          PcgState* st, double* partials) {
-  double rz = 0.0, rr = 0.0, bb = 0.0;
-  Cursor cur;
-  for (cur.init(A.L); cur.valid(A.L); cur.next(A.L)) {
-    const int64_t c = A.L.at(cur.i, cur.j, cur.k);
-    const RT bv = b[c];
-    const RT rv = bv - apply7<V, RT>(A, x, c);
-    const RT z = precond1<V, RT>(A, rv, c);
-    r[c] = rv;  // b may alias r: each element is read before it is written
-    p[c] = (V)z;
-    rz += (double)rv * (double)z;
-    rr += (double)rv * (double)rv;
-    bb += (double)bv * (double)bv;
-  }
-  double tot[3];
-  if (grid_reduce3(rz, rr, bb, partials, &st->ticket, tot)) {
-    st->rz = tot[0];
-    st->rr = tot[1];
-    st->bb = tot[2];
-    st->iter = 0;
-    st->beta = 0.0;
-    st->best_rr = tot[1];
-    st->max_rr = tot[1];
-    st->rz_prev = tot[0];
-    st->stall = 0;
-    st->status = PCG_RUNNING;
-    st->done = 0;
-    if (!isfinite(tot[0]) || !isfinite(tot[1])) {
-      st->status = PCG_NONFINITE;
-      st->done = 1;
-    } else if (tot[2] == 0.0 || tot[1] == 0.0 || (st->criterion != 1 && stop_test(st, tot[0], tot[1]))) {
-      // zero right-hand side or an initial guess that already satisfies the test
-      st->status = PCG_CONVERGED;
-      st->done = 1;
-    } else if (st->max_iter <= 0) {
-      st->status = PCG_MAXITER;
-      st->done = 1;
-    }
   }
 }
 
@@ -218,11 +161,6 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_resume(Op7<V> A, const RT* 
       st->done = 1;
     }
   }
-}
-
-template <class V, class RT>
-void pcg_init(const Op7<V>& A, const RT* b, RT* x, RT* r, V* p, PcgState* st, double* partials, cudaStream_t s) {
-  k_pcg_init<V, RT><<<pcg_blocks(A.L), kRedThreads, 0, s>>>(A, b, x, r, p, st, partials);
 }
 
 template <class V, class RT>
@@ -326,21 +264,30 @@ struct VecCursor {
 // block load in the same plane (L1 hits).  Blocks are 32 x 8 threads
 // (128 x 8 cells); the grid is the xy tiles times as many z chunks as fill
 // the resident blocks of the GPU.
-template <class V>
-__device__ __forceinline__ void spmv_row4(const Op7<V>& A, const V* __restrict__ p, int64_t c, int i0,
-                                          const V4<V>& pc, const V4<V>& pdn, const V4<V>& pup, const V4<V>& azc,
-                                          const V4<V>& azu, V4<V>& q) {
+// SHUFFLE: the x neighbours outside the vector come from the adjacent lanes
+// (every thread of the warp takes part; i0 the thread's first column), else from
+// L1.
+template <class V, bool SHUFFLE>
+__device__ __forceinline__ void spmv_row4(const Op7<V>& A, const V* __restrict__ p, int64_t c, int i0, const V4<V>& pc,
+                                          const V4<V>& pdn, const V4<V>& pup, const V4<V>& azc, const V4<V>& azu,
+                                          V4<V>& q) {
   const int64_t sy = A.L.px;
-  const int lane_id = threadIdx.x & 31;
   const V4<V> ps = ld4(p + c - sy), pn = ld4(p + c + sy);
   const V4<V> ayc = ld4(A.ay + c), ayn = ld4(A.ay + c + sy);
   const V4<V> axc = ld4(A.ax + c);
-  // x neighbours: p[i0-1], p[i0+4] and ax[i0+4] from the adjacent lanes
-  V pl = __shfl_up_sync(0xffffffffu, pc.d, 1);
-  V pr = __shfl_down_sync(0xffffffffu, pc.a, 1);
-  V axr = __shfl_down_sync(0xffffffffu, axc.a, 1);
-  if (lane_id == 0) pl = p[c - 1];
-  if (lane_id == 31 || i0 + 4 >= A.L.nx) {  // warp end, or the row ends in this vector
+  V pl, pr, axr;
+  if (SHUFFLE) {
+    const int lane_id = threadIdx.x & 31;
+    pl = __shfl_up_sync(0xffffffffu, pc.d, 1);
+    pr = __shfl_down_sync(0xffffffffu, pc.a, 1);
+    axr = __shfl_down_sync(0xffffffffu, axc.a, 1);
+    if (lane_id == 0) pl = p[c - 1];
+    if (lane_id == 31 || i0 + 4 >= A.L.nx) {  // warp end, or the row ends in this vector
+      pr = p[c + 4];
+      axr = A.ax[c + 4];
+    }
+  } else {
+    pl = p[c - 1];
     pr = p[c + 4];
     axr = A.ax[c + 4];
   }
@@ -365,7 +312,7 @@ __device__ __forceinline__ void spmv_row4(const Op7<V>& A, const V* __restrict__
       if (c + m == c00) acc += (*A.extra0) * (double)xc;
       out = (V)acc;
     } else if (A.flux_form) {
-      // flux form in FP64 arithmetic (see apply7)
+      // flux form in FP64 arithmetic: for smooth x the six fluxes nearly cancel
       const double d = (double)xc;
       double acc = (double)lane(axc, m) * (d - (double)xl) + (double)ar * (d - (double)xr);
       acc += (double)lane(ayc, m) * (d - (double)lane(ps, m)) + (double)lane(ayn, m) * (d - (double)lane(pn, m));
@@ -427,7 +374,7 @@ __global__ void __launch_bounds__(256, MINB) k_cg_spmv(Op7<V> A, const V* __rest
     for (int k = k0; k < k1; ++k, c += sz) {
       const V4<V> pup = ld4(p + c + sz), azu = ld4(A.az + c + sz);
       V4<V> qv;
-      spmv_row4<V>(A, p, c, ii, pc, pdn, pup, azc, azu, qv);
+      spmv_row4<V, true>(A, p, c, ii, pc, pdn, pup, azc, azu, qv);
       if (nvalid > 0) {
         st4(q + c, qv, nvalid);
         pq += (double)pc.a * (double)qv.a;  // p.q of the stored q, as the residual update uses it
@@ -441,6 +388,84 @@ __global__ void __launch_bounds__(256, MINB) k_cg_spmv(Op7<V> A, const V* __rest
     }
   }
   spmv_alpha(pq, st, partials);
+}
+
+// ---- the start of a solve: x <- the initial guess x0, r = b - A x, p = z =
+// M^-1 r, r.z, r.r and b.b.  Four cells per thread up a chunk of planes like the
+// SpMV, on 256 consecutive vectors of the plane (rows of any length fill the
+// blocks; the SpMV's 128 x 8 tiles, which are faster there, idle a third of
+// their threads on the 257 faces of a 256^3 grid).  256^3 in FP32: 132 us, with
+// one cell per thread 187 us and a copy of the guess before it.
+struct RowVectors {  // thread -> vector of the plane, planes of the block
+  int i0, j, k0, k1, nvalid;
+  __device__ __forceinline__ RowVectors(const Lay& L, int kchunk) {
+    const unsigned nv = (unsigned)(L.nx + 3) >> 2;
+    const unsigned t = blockIdx.x * 256u + threadIdx.x;
+    j = (int)(t / nv);
+    i0 = 4 * (int)(t - (unsigned)j * nv);
+    k0 = blockIdx.y * kchunk;
+    k1 = min(L.nz, k0 + kchunk);
+    nvalid = j < L.ny ? min(4, L.nx - i0) : 0;
+  }
+};
+template <class V>
+__global__ void __launch_bounds__(256) k_pcg_init(Op7<V> A, const V* __restrict__ b, const V* __restrict__ x0, V* __restrict__ x,
+                                                  V* __restrict__ r, V* __restrict__ p, PcgState* st, double* partials,
+                                                  int kchunk) {
+  const Lay& L = A.L;
+  const RowVectors R(L, kchunk);
+  const int64_t sz = L.slab;
+  double rz = 0.0, rr = 0.0, bb = 0.0;
+  if (R.nvalid > 0) {
+    int64_t c = L.at(R.i0, R.j, R.k0);
+    V4<V> xdn = ld4(x0 + c - sz), xc = ld4(x0 + c), azc = ld4(A.az + c);
+    for (int k = R.k0; k < R.k1; ++k, c += sz) {
+      const V4<V> xup = ld4(x0 + c + sz), azu = ld4(A.az + c + sz), bv = ld4(b + c);
+      V4<V> qv;
+      spmv_row4<V, false>(A, x0, c, 0, xc, xdn, xup, azc, azu, qv);
+      const V4<V> rv = {bv.a - qv.a, bv.b - qv.b, bv.c - qv.c, bv.d - qv.d};
+      const V4<V> zv = precond4(A, rv, c);
+      st4(r + c, rv, R.nvalid);
+      st4(p + c, zv, R.nvalid);
+      if (x != x0) st4(x + c, xc, R.nvalid);  // (x may be x0, then it is only read)
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (m < R.nvalid) {
+          const double rm = (double)lane(rv, m), bm = (double)lane(bv, m);
+          rz += rm * (double)lane(zv, m);
+          rr += rm * rm;
+          bb += bm * bm;
+        }
+      xdn = xc;
+      xc = xup;
+      azc = azu;
+    }
+  }
+  double tot[3];
+  if (grid_reduce3(rz, rr, bb, partials, &st->ticket, tot)) {
+    st->rz = tot[0];
+    st->rr = tot[1];
+    st->bb = tot[2];
+    st->iter = 0;
+    st->beta = 0.0;
+    st->best_rr = tot[1];
+    st->max_rr = tot[1];
+    st->rz_prev = tot[0];
+    st->stall = 0;
+    st->status = PCG_RUNNING;
+    st->done = 0;
+    if (!isfinite(tot[0]) || !isfinite(tot[1])) {
+      st->status = PCG_NONFINITE;
+      st->done = 1;
+    } else if (tot[2] == 0.0 || tot[1] == 0.0 || (st->criterion != 1 && stop_test(st, tot[0], tot[1]))) {
+      // zero right-hand side or an initial guess that already satisfies the test
+      st->status = PCG_CONVERGED;
+      st->done = 1;
+    } else if (st->max_iter <= 0) {
+      st->status = PCG_MAXITER;
+      st->done = 1;
+    }
+  }
 }
 
 // ---- p.q and the step length of a SpMV that does not reduce (the
@@ -540,8 +565,9 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(Op7<V> A, V* __restri
 
 // ---- direction update: x += alpha p (when pending), p = r/diag + beta p
 template <class V, class X>
-__global__ void __launch_bounds__(kRedThreads) k_cg_pupdate(Op7<V> A, X* __restrict__ x, const V* __restrict__ r,
-                                                            V* __restrict__ p, PcgState* st) {
+__global__ void __launch_bounds__(kRedThreads) k_cg_pupdate(Op7<V> A, const V* __restrict__ r, V* __restrict__ p,
+                                                            PcgState* st) {
+  X* __restrict__ x = (X*)state_read(reinterpret_cast<const unsigned long long*>(&st->x));
   const bool move_x = state_read(&st->x_pending) != 0;
   const bool move_p = state_read(&st->done) == 0;
   if (!move_x && !move_p) return;  // uniform: every block reads the same state
@@ -605,13 +631,33 @@ void cg_prepare() {
   }
 }
 
+// grid of k_pcg_init: the plane's vectors times z chunks, about two waves of
+// resident blocks, at most 16 planes a block
+static dim3 init_grid(const Lay& L, int* kchunk) {
+  const int64_t bx = ((int64_t)((L.nx + 3) >> 2) * L.ny + 255) / 256;
+  const int64_t want = (int64_t)2 * 4 * g_sm_count;
+  const int64_t chunks = std::max<int64_t>((L.nz + 15) / 16, std::min<int64_t>(L.nz, want / bx));
+  *kchunk = (int)((L.nz + chunks - 1) / chunks);
+  return dim3((unsigned)bx, (unsigned)((L.nz + *kchunk - 1) / *kchunk), 1);
+}
+
 int cg_max_blocks(const Lay& L) {
+  int kchunk = 1;
+  const dim3 g = init_grid(L, &kchunk);
   const int tiles = ((L.nx + 127) / 128) * ((L.ny + 7) / 8);
-  return std::max(tiles, reduction_blocks((int64_t)1 << 40));  // the resident-block cap
+  return std::max(std::max(tiles, (int)(g.x * g.y)), reduction_blocks((int64_t)1 << 40));  // the resident-block cap
+}
+
+template <class V>
+void pcg_init(const Op7<V>& A, const V* b, const V* x0, V* x, V* r, V* p, PcgState* st, double* partials,
+              cudaStream_t s) {
+  int kchunk = 1;
+  const dim3 g = init_grid(A.L, &kchunk);
+  k_pcg_init<V><<<g, 256, 0, s>>>(A, b, x0, x, r, p, st, partials, kchunk);
 }
 
 template <class V, class X>
-void cg_iteration(const Op7<V>& A, X* x, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s) {
+void cg_iteration(const Op7<V>& A, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s) {
   const int* slot = g_cg_blocks[sizeof(X) == 8][sizeof(V) == 8];
   const Lay& L = A.L;
   // SpMV grid: xy tiles of 128 x 8 cells times z chunks filling the resident blocks
@@ -621,11 +667,11 @@ void cg_iteration(const Op7<V>& A, X* x, V* r, V* p, V* q, PcgState* st, double*
   const int kchunk = (L.nz + chunks - 1) / chunks;
   const dim3 sg(tx, ty, (L.nz + kchunk - 1) / kchunk);
   k_cg_spmv<V, spmv_minb<V>()><<<sg, dim3(32, 8, 1), 0, s>>>(A, p, q, st, partials, kchunk);
-  cg_vector_updates<V, X>(A, x, r, p, q, st, partials, s);
+  cg_vector_updates<V, X>(A, r, p, q, st, partials, s);
 }
 
 template <class V, class X>
-void cg_vector_updates(const Op7<V>& A, X* x, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s) {
+void cg_vector_updates(const Op7<V>& A, V* r, V* p, V* q, PcgState* st, double* partials, cudaStream_t s) {
   const int* slot = g_cg_blocks[sizeof(X) == 8][sizeof(V) == 8];
   const Lay& L = A.L;
   // pointwise kernels: grid-stride over the vectors, resident blocks only
@@ -638,7 +684,7 @@ void cg_vector_updates(const Op7<V>& A, X* x, V* r, V* p, V* q, PcgState* st, do
   // the direction update on two waves of blocks: measured at 256^3 on the
   // packed black vectors, 48 us against 56 us on one wave (fewer vectors per
   // thread, the second wave fills the first one's tail)
-  k_cg_pupdate<V, X><<<grid(2 * slot[2]), kRedThreads, 0, s>>>(A, x, r, p, st);
+  k_cg_pupdate<V, X><<<grid(2 * slot[2]), kRedThreads, 0, s>>>(A, r, p, st);
 }
 
 template <class V>
@@ -654,21 +700,16 @@ template void pq_alpha<float>(const Op7<float>&, const float*, const float*, Pcg
 template void cg_prepare<float, double>();
 template void cg_prepare<double, double>();
 template void cg_prepare<float, float>();
-template void cg_iteration<float, double>(const Op7<float>&, double*, float*, float*, float*, PcgState*, double*,
-                                          cudaStream_t);
-template void cg_iteration<double, double>(const Op7<double>&, double*, double*, double*, double*, PcgState*,
-                                           double*, cudaStream_t);
-template void cg_iteration<float, float>(const Op7<float>&, float*, float*, float*, float*, PcgState*, double*,
-                                         cudaStream_t);
-template void cg_vector_updates<float, double>(const Op7<float>&, double*, float*, float*, float*, PcgState*, double*,
+template void cg_iteration<float, double>(const Op7<float>&, float*, float*, float*, PcgState*, double*, cudaStream_t);
+template void cg_iteration<double, double>(const Op7<double>&, double*, double*, double*, PcgState*, double*,
+                                           cudaStream_t);
+template void cg_iteration<float, float>(const Op7<float>&, float*, float*, float*, PcgState*, double*, cudaStream_t);
+template void cg_vector_updates<float, double>(const Op7<float>&, float*, float*, float*, PcgState*, double*,
                                                cudaStream_t);
-
-#define FS_KINST(V, RT)                                                                                           \
-  template void pcg_init<V, RT>(const Op7<V>&, const RT*, RT*, RT*, V*, PcgState*, double*, cudaStream_t);       \
-  template void pcg_resume<V, RT>(const Op7<V>&, const RT*, V*, PcgState*, double*, int, cudaStream_t);
-
-FS_KINST(float, float)
-FS_KINST(double, double)
-FS_KINST(float, double)
+template void pcg_init<float>(const Op7<float>&, const float*, const float*, float*, float*, float*, PcgState*, double*,
+                              cudaStream_t);
+template void pcg_init<double>(const Op7<double>&, const double*, const double*, double*, double*, double*, PcgState*,
+                               double*, cudaStream_t);
+template void pcg_resume<float, float>(const Op7<float>&, const float*, float*, PcgState*, double*, int, cudaStream_t);
 
 }  // namespace fsb

@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_build(const MgState* st, Lay L,
   // the face between a cell and its low neighbour
   auto beta = [&](T low, T c) -> double {
     const bool nl = low <= T(0), nc = c <= T(0);
-    if (nl == nc) return nc ? vneg : vpos;
+    if (nl == nc && low == low && c == c) return nc ? vneg : vpos;  // (a NaN goes on into the coupling)
     const double vl = nl ? vneg : vpos, vc = nc ? vneg : vpos, al = fabs((double)low), ac = fabs((double)c);
     return vl * vc * (ac + al) / (vc * al + vl * ac);
   };
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_build(const MgState* st, Lay L,
     ay[c] = j > 0 ? (float)(beta(ym, p) * inv2) : 0.0f;
     az[c] = k > 0 ? (float)(beta(down, p) * inv2) : 0.0f;
     const bool n = p <= T(0);
-    const bool same = (xm <= T(0)) == n && (xp <= T(0)) == n && (ym <= T(0)) == n && (yp <= T(0)) == n &&
+    const bool same = p == p && (xm <= T(0)) == n && (xp <= T(0)) == n && (ym <= T(0)) == n && (yp <= T(0)) == n &&
                       (down <= T(0)) == n && (up <= T(0)) == n;
     const unsigned char cl = same ? (n ? 1 : 2) : 0;
     (((i + j + k) & 1) ? cls1 : cls0)[H.at(i >> 1, j, k)] = cl;

@@ -218,30 +218,103 @@ __device__ __forceinline__ double heaviside_proj(double phi, double e) {
   return (0.5 + phi * ooe * 0.5) + 0.5 * oop * sin(3.14159265358979323846 * phi * ooe);
 }
 
-// Pressure-gradient update of one face component.  Face (i,j,k) of
-// component `axis` lies between cell c = (i,j,k) and the cell n one step
-// back along the axis; wall faces are left alone.  Then the RK combination
-// out = c0*base + c1*f (skipped when c0 == 0).
+// Pressure-gradient update (UpdateVelocityByPressureGradientVariableDensity,
+// PROJECTION_3D.h:1099-1449).  Face (i,j,k) of a component lies between cell c
+// = (i,j,k) and the cell n one step back along its axis; wall faces are left
+// alone.  Then the RK combination out = c0*base + c1*f (skipped when c0 == 0).
 //
 // Corrected (the default): u_f -= dt beta_f (p_c - p_n +- a_f)/dx with the
 // pressure matrix's own face coefficient beta_f (POISSON_SOLVER_3D.h:1080-1085,
-// the same expression and operand order as k_pressure_faces) and, on faces
+// the expression of k_pressure_faces, 1/rho itself inside a phase) and, on faces
 // whose cells lie in different phases, the same interface jump a_f that the
 // right-hand side carries (+ when c is in the phi <= 0 phase).  The update
 // is then the discrete gradient the matrix was built from: the corrected
 // velocity's divergence is dt times the solve's residual, so it is
 // divergence free to the solve tolerance at the interface too.
 //
+// One thread updates the low faces of a cell along all three axes and marches
+// up z, so p and phi are read once for the three components and divisions are
+// left to the interface.  Measured at 256^3, FP32: one kernel per component
+// with three divisions per face 3 x 249 us, this one 241 us.
+template <class T>
+struct Corrected {
+  T* f[3];
+  const T* base[3];
+  Lay L[3];
+};
+template <class T>
+__global__ void __launch_bounds__(256) k_velocity_correct(Corrected<T> V, const double* __restrict__ p,
+                                                          const T* __restrict__ phi, Lay Lc, double inv_h, double dt,
+                                                          double rn, double rp, double c0, double c1,
+                                                          const double* __restrict__ kappa, double sigma, int kchunk) {
+  // faces 0 .. n along each axis: one column more than cells in x and y
+  const int w = Lc.nx + 1;
+  const unsigned t = blockIdx.x * 256u + threadIdx.x;
+  const int j = (int)(t / (unsigned)w), i = (int)(t - (unsigned)j * (unsigned)w);
+  if (j > Lc.ny) return;
+  const int k0 = blockIdx.y * kchunk, k1 = min(Lc.nz + 1, k0 + kchunk);
+  const double vneg = 1.0 / rn, vpos = 1.0 / rp;
+  const bool in_x = i < Lc.nx, in_y = j < Lc.ny;
+  // the value of one face from its own and its base value
+  auto update = [&](double val, double base, bool inside, int64_t c, int64_t step, double phc, double pc, double phn,
+                    double pn) -> double {
+    if (inside) {
+      const bool nc = phc <= 0.0, nn = phn <= 0.0;
+      double dp = pc - pn, beta = nc ? vneg : vpos;
+      if (nc != nn) {
+        const double vc = beta, vn = nn ? vneg : vpos;
+        beta = face_beta(vn, vc, fabs(phn), fabs(phc));
+        if (kappa) {
+          const double jcc = sigma * kappa[c], jcn = sigma * kappa[c - step];
+          const double jump = (jcc * fabs(phn) + jcn * fabs(phc)) / (fabs(phn) + fabs(phc));
+          dp = nc ? dp + jump : dp - jump;
+        }
+      }
+      val -= dt * dp * beta * inv_h;
+    }
+    return c0 == 0.0 ? val : c0 * base + c1 * val;
+  };
+  int64_t c = Lc.at(i, j, k0);
+  int64_t gu = V.L[0].at(i, j, k0), gv = V.L[1].at(i, j, k0), gw = V.L[2].at(i, j, k0);
+  double pd = 0.0, hd = 0.0;
+  if (k0 > 0 && in_x && in_y) {
+    pd = p[c - Lc.slab];
+    hd = (double)phi[c - Lc.slab];
+  }
+  for (int k = k0; k < k1; ++k, c += Lc.slab, gu += V.L[0].slab, gv += V.L[1].slab, gw += V.L[2].slab) {
+    const bool in_z = k < Lc.nz;
+    // which faces exist, and all loads before the first store
+    const bool fu = in_y && in_z, fv = in_x && in_z, fw = in_x && in_y;
+    const double pc = p[c], hc = (double)phi[c];  // (ghosts past the last cell are not used)
+    const double pl = p[c - 1], hl = (double)phi[c - 1], pb = p[c - Lc.px], hb = (double)phi[c - Lc.px];
+    double u = fu ? (double)V.f[0][gu] : 0.0, v = fv ? (double)V.f[1][gv] : 0.0, x = fw ? (double)V.f[2][gw] : 0.0;
+    double bu = 0.0, bv = 0.0, bw = 0.0;
+    if (c0 != 0.0) {
+      if (fu) bu = (double)V.base[0][gu];
+      if (fv) bv = (double)V.base[1][gv];
+      if (fw) bw = (double)V.base[2][gw];
+    }
+    u = update(u, bu, i > 0 && in_x, c, 1, hc, pc, hl, pl);
+    v = update(v, bv, j > 0 && in_y, c, Lc.px, hc, pc, hb, pb);
+    x = update(x, bw, k > 0 && in_z, c, Lc.slab, hc, pc, hd, pd);
+    if (fu) V.f[0][gu] = (T)u;
+    if (fv) V.f[1][gv] = (T)v;
+    if (fw) V.f[2][gw] = (T)x;
+    pd = pc;
+    hd = hc;
+  }
+}
+
 // Faithful (FS_FLAG_FAITHFUL_PROJECTION, PROJECTION_3D.h:1099-1449): same-side
 // faces use the sharp 1/rho of cell c, faces with phi_c phi_n <= 0 the
 // smeared density of the face-averaged phi, only w is updated, and the first
 // cell's bottom face sees the zero ghost pressure.  This is not consistent
 // with the matrix, so the interface keeps a divergence residual there.
 template <class T>
-__global__ void k_velocity_correct(T* __restrict__ f, const T* __restrict__ base, const double* __restrict__ p,
-                                   const T* __restrict__ phi, Lay Lf, Lay Lc, int axis, double inv_h, double dt,
-                                   double rn, double rp, int faithful, double c0, double c1,
-                                   const double* __restrict__ kappa, double sigma) {
+__global__ void k_velocity_correct_faithful(T* __restrict__ f, const T* __restrict__ base, const double* __restrict__ p,
+                                            const T* __restrict__ phi, Lay Lf, Lay Lc, int axis, double inv_h,
+                                            double dt, double rn, double rp, double c0, double c1,
+                                            const double* __restrict__ kappa, double sigma) {
   FS_IJK(Lf);
   const int64_t fc = Lf.at(i, j, k);
   double val = (double)f[fc];
@@ -250,20 +323,7 @@ __global__ void k_velocity_correct(T* __restrict__ f, const T* __restrict__ base
   const bool interior = e > 0 && e < n;
   const int64_t c = Lc.at(i, j, k);
   const int64_t step = axis == 0 ? 1 : (axis == 1 ? Lc.px : Lc.slab);
-  if (!faithful) {
-    if (interior) {
-      const double phc = (double)phi[c], phn = (double)phi[c - step];
-      const double vc = inv_rho(phi[c], rn, rp), vn = inv_rho(phi[c - step], rn, rp);
-      const double beta = face_beta(vn, vc, fabs(phn), fabs(phc));
-      double dp = p[c] - p[c - step];
-      if (kappa && (phc <= 0.0) != (phn <= 0.0)) {
-        const double jcc = sigma * kappa[c], jcn = sigma * kappa[c - step];
-        const double jump = (jcc * fabs(phn) + jcn * fabs(phc)) / (fabs(phn) + fabs(phc));
-        dp = phc <= 0.0 ? dp + jump : dp - jump;
-      }
-      val -= dt * dp * beta * inv_h;
-    }
-  } else if (axis == 2 && (interior || (i == 0 && j == 0 && k == 0))) {
+  if (axis == 2 && (interior || (i == 0 && j == 0 && k == 0))) {
     const double phc = (double)phi[c];
     // across the bottom wall the ghost phi is the linear extrapolation and
     // the ghost pressure is zero
@@ -443,17 +503,46 @@ __global__ void k_convert(D* __restrict__ dst, const S* __restrict__ src, Lay L)
   dst[c] = (D)src[c];
 }
 
-// packed (x fastest, no ghosts) FP64 <-> padded storage
-template <class T>
-__global__ void k_pack(double* __restrict__ dst, const T* __restrict__ src, Lay L) {
-  FS_IJK(L);
-  dst[((int64_t)k * L.ny + j) * L.nx + i] = (double)src[L.at(i, j, k)];
+// packed (x fastest, no ghosts) FP64 <-> padded storage, rows walked by
+// consecutive threads with kRows rows in flight each: a plane's rows are read and
+// written whole whatever their length.  (One value per thread of a 32 x 4 x 2
+// block: 63 us at 256^3 between FP32 storage and FP64, 47 us so.)
+constexpr int kPackRows = 4;
+template <class T, bool PACK>
+__global__ void __launch_bounds__(256) k_transfer(double* __restrict__ packed, T* __restrict__ padded, Lay L) {
+  const int64_t rows = (int64_t)L.ny * L.nz;
+  // threads along a row: the row length rounded up to a power of two, at most the block
+  const int wide = blockDim.x, per = blockDim.y;
+  const int64_t r0 = ((int64_t)blockIdx.x * per + threadIdx.y) * kPackRows;
+  for (int i = threadIdx.x; i < L.nx; i += wide) {
+    T v[kPackRows];
+    double d[kPackRows];
+#pragma unroll
+    for (int m = 0; m < kPackRows; ++m) {
+      const int64_t r = r0 + m;
+      if (r >= rows) continue;
+      const int k = (int)(r / L.ny), j = (int)(r - (int64_t)k * L.ny);
+      if (PACK) v[m] = padded[L.at(i, j, k)];
+      else d[m] = packed[r * L.nx + i];
+    }
+#pragma unroll
+    for (int m = 0; m < kPackRows; ++m) {
+      const int64_t r = r0 + m;
+      if (r >= rows) continue;
+      const int k = (int)(r / L.ny), j = (int)(r - (int64_t)k * L.ny);
+      if (PACK) packed[r * L.nx + i] = (double)v[m];
+      else padded[L.at(i, j, k)] = (T)d[m];
+    }
+  }
 }
 
-template <class T>
-__global__ void k_unpack(T* __restrict__ dst, const double* __restrict__ src, Lay L) {
-  FS_IJK(L);
-  dst[L.at(i, j, k)] = (T)src[((int64_t)k * L.ny + j) * L.nx + i];
+template <class T, bool PACK>
+void transfer(double* packed, T* padded, const Lay& L, cudaStream_t s) {
+  int wide = 32;
+  while (wide < 256 && wide < L.nx) wide *= 2;
+  const dim3 block(wide, 256 / wide, 1);
+  const int64_t rows = (int64_t)L.ny * L.nz, per = (int64_t)block.y * kPackRows;
+  k_transfer<T, PACK><<<(unsigned)((rows + per - 1) / per), block, 0, s>>>(packed, padded, L);
 }
 
 // ---------------------------------------------------------------------------
@@ -500,12 +589,29 @@ void add_correction(double* p64, const float* e, const Lay& Lc, cudaStream_t s) 
 }
 
 template <class T>
-void velocity_correct(T* f, const T* base, const double* p, const T* phi, const Lay& Lf, const Lay& Lc, int axis,
-                      double dx, double dt, double rho_neg, double rho_pos, int faithful, double c0, double c1,
-                      const double* kappa, double sigma, cudaStream_t s) {
-  Launch3 g = launch3(Lf.nx, Lf.ny, Lf.nz);
-  k_velocity_correct<T><<<g.grid, g.block, 0, s>>>(f, base, p, phi, Lf, Lc, axis, 1.0 / dx, dt, rho_neg, rho_pos,
-                                                    faithful, c0, c1, kappa, sigma);
+void velocity_correct(T* const f[3], const T* const base[3], const double* p, const T* phi, const Lay* const Lf[3],
+                      const Lay& Lc, double dx, double dt, double rho_neg, double rho_pos, int faithful, double c0,
+                      double c1, const double* kappa, double sigma, cudaStream_t s) {
+  if (faithful) {
+    for (int a = 0; a < 3; ++a) {
+      Launch3 g = launch3(Lf[a]->nx, Lf[a]->ny, Lf[a]->nz);
+      k_velocity_correct_faithful<T><<<g.grid, g.block, 0, s>>>(f[a], base[a], p, phi, *Lf[a], Lc, a, 1.0 / dx, dt,
+                                                                rho_neg, rho_pos, c0, c1, kappa, sigma);
+    }
+    return;
+  }
+  Corrected<T> V;
+  for (int a = 0; a < 3; ++a) {
+    V.f[a] = f[a];
+    V.base[a] = base[a];
+    V.L[a] = *Lf[a];
+  }
+  const int64_t cols = (int64_t)(Lc.nx + 1) * (Lc.ny + 1), bx = (cols + 255) / 256;
+  const int64_t ch = bx * (Lc.nz + 1) / (148 * 16);
+  const int kchunk = (int)(ch < 1 ? 1 : (ch > 8 ? 8 : ch));
+  const dim3 grid((unsigned)bx, (unsigned)((Lc.nz + kchunk) / kchunk), 1);
+  k_velocity_correct<T><<<grid, 256, 0, s>>>(V, p, phi, Lc, 1.0 / dx, dt, rho_neg, rho_pos, c0, c1, kappa, sigma,
+                                             kchunk);
 }
 
 template <class T>
@@ -548,14 +654,12 @@ void convert_copy(D* dst, const S* src, const Lay& L, cudaStream_t s) {
 
 template <class T>
 void pack_to_double(double* dst, const T* src, const Lay& L, cudaStream_t s) {
-  Launch3 g = launch3(L.nx, L.ny, L.nz);
-  k_pack<T><<<g.grid, g.block, 0, s>>>(dst, src, L);
+  transfer<T, true>(dst, const_cast<T*>(src), L, s);
 }
 
 template <class T>
 void unpack_from_double(T* dst, const double* src, const Lay& L, cudaStream_t s) {
-  Launch3 g = launch3(L.nx, L.ny, L.nz);
-  k_unpack<T><<<g.grid, g.block, 0, s>>>(dst, src, L);
+  transfer<T, false>(const_cast<double*>(src), dst, L, s);
 }
 
 #define FS_PINST(T)                                                                                                  \
@@ -564,9 +668,9 @@ void unpack_from_double(T* dst, const double* src, const Lay& L, cudaStream_t s)
   template void defect_residual<T>(const T*, const double*, const float*, const double*, double*, float*,         \
                                    const Lay&, double, double, double, double*, unsigned int*, double*, int,        \
                                    cudaStream_t, const PipeGeom*);                                                  \
-  template void velocity_correct<T>(T*, const T*, const double*, const T*, const Lay&, const Lay&, int, double,     \
-                                    double, double, double, int, double, double, const double*, double,            \
-                                    cudaStream_t);                                                                  \
+  template void velocity_correct<T>(T* const[3], const T* const[3], const double*, const T*, const Lay* const[3],    \
+                                    const Lay&, double, double, double, double, int, double, double,                \
+                                    const double*, double, cudaStream_t);                                           \
   template void curvature<T>(const T*, double*, const Lay&, double, int, double*, cudaStream_t);                   \
   template void jump_rhs<T>(const T*, const double*, double, double*, const Lay&, double, double, double, int,    \
                             double*, unsigned int*, double*, cudaStream_t, const PipeGeom*);                 \

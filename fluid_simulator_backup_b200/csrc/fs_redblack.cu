@@ -274,12 +274,12 @@ int rb_blocks(const Lay& H) {
   return std::max((int)(g.x * g.y * g.z), reduction_blocks((int64_t)H.nx * H.ny * H.nz));
 }
 
-void rb_iteration(const RbOp& A, const Op7<float>& Ah, double* xh, float* rh, float* ph, float* qh, float* tau,
+void rb_iteration(const RbOp& A, const Op7<float>& Ah, float* rh, float* ph, float* qh, float* tau,
                   PcgState* st, double* partials, cudaStream_t s) {
   k_rb_red<<<rb_red_grid(A.Lh), dim3(32, kRbBY, 1), 0, s>>>(A, ph, tau, st, kRbRedChunk);
   k_rb_black<<<rb_black_grid(A.Lh), dim3(32, kRbBY, 1), 0, s>>>(A, ph, tau, qh, st, kRbChunk);
   pq_alpha<float>(Ah, ph, qh, st, partials, s);
-  cg_vector_updates<float, double>(Ah, xh, rh, ph, qh, st, partials, s);
+  cg_vector_updates<float, double>(Ah, rh, ph, qh, st, partials, s);
 }
 
 template <class T>

@@ -27,8 +27,8 @@
 //     it is the first to need).
 // Measured (B200), before -> after, per launch with its ghost fill: Sussman
 // step 256^3 FP32 516 -> 256 us, 33 x 47 x 29 FP64 17.8 -> 4.3 us; level set
-// 256^3 FP32 533 -> 239 us; WENO5 component 200 x 136 x 267 FP32 285 -> 106 us;
-// ENO3 component 65 x 97 x 41 FP64 25.4 -> 11.4 us.
+// 256^3 FP32 533 -> 239 us; WENO5, three components, 200 x 136 x 267 FP32 855 ->
+// 305 us; ENO3, three components, 65 x 97 x 41 FP64 76 -> 19 us.
 #include <algorithm>
 
 #include "fs_kernels.h"
@@ -325,33 +325,6 @@ __device__ __forceinline__ void mac_velocity(const T* __restrict__ u, const T* _
   }
 }
 
-// MAC component self-advection on every face of component `axis` (wall
-// faces included, as the reference's loop covers the whole face grid).
-template <class T>
-__global__ void __launch_bounds__(kColThreads) k_weno5_mac(const T* __restrict__ comp, T* __restrict__ out,
-                                                      const T* __restrict__ u, const T* __restrict__ v,
-                                                      const T* __restrict__ w, Lay Lc, Lay Lu, Lay Lv, Lay Lw,
-                                                      int axis, T inv_h, T eps, T dt, int kchunk, int flat) {
-  int i, j;
-  if (!column_of(Lc, flat, i, j)) return;
-  const int k0 = blockIdx.z * kchunk, k1 = min(Lc.nz, k0 + kchunk);
-  int64_t c = Lc.at(i, j, k0);
-  T vx[7], vy[7], vz[7];
-  samples7(vz, comp, c, Lc.slab, comp[c], k0, Lc.nz, false);
-  for (int k = k0; k < k1; ++k, c += Lc.slab) {
-    const T next = k + 1 < k1 ? comp[c + 4 * Lc.slab] : T(0);
-    T uvel, vvel, wvel;
-    mac_velocity(u, v, w, Lu, Lv, Lw, axis, i, j, k, uvel, vvel, wvel);
-    samples7(vx, comp, c, 1, vz[3], i, Lc.nx, false);
-    samples7(vy, comp, c, Lc.px, vz[3], j, Lc.ny, false);
-    const T dx = weno_upwind7(vx, inv_h, eps, uvel > T(0));
-    const T dy = weno_upwind7(vy, inv_h, eps, vvel > T(0));
-    const T dz = weno_upwind7(vz, inv_h, eps, wvel > T(0));
-    out[c] = vz[3] - dt * ((uvel * dx + vvel * dy) + wvel * dz);
-    slide7(vz, next, k, Lc.nz, false);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // ENO3 (ADVECTION_METHOD_3D.h:1639-1934)
 // ---------------------------------------------------------------------------
@@ -383,34 +356,77 @@ __device__ __forceinline__ void eno3_pair7(const T v[7], T h, T inv, T o2, T o3,
   }
 }
 
-// MAC component self-advection with ENO3 (the reference's use_3rd_eno_v,
-// ADVECTION_3D.h:323-325), every face of component `axis`.
+// MAC self-advection of the three components, WENO5 or ENO3 (the reference's
+// use_3rd_eno_v, ADVECTION_3D.h:323-325), on every face (wall faces included,
+// as the reference's loop covers the whole face grid).  One launch for the
+// three: blockIdx.z holds the component and the z chunk, so that a small box
+// fills three times as many SMs (65 x 97 x 41 FP64 ENO3: 3 x 11.4 us -> 19.2 us).
+// In a step the kernel also does what follows the advection there: add[a]
+// (dt g_a) on the faces off the component's walls and, with zero_walls, no
+// penetration on them (one pass per component each before).
 template <class T>
-__global__ void __launch_bounds__(kColThreads) k_eno3_mac(const T* __restrict__ comp, T* __restrict__ out,
-                                                     const T* __restrict__ u, const T* __restrict__ v,
-                                                     const T* __restrict__ w, Lay Lc, Lay Lu, Lay Lv, Lay Lw,
-                                                     int axis, T h, T dt, int kchunk, int flat) {
-  int i, j;
-  if (!column_of(Lc, flat, i, j)) return;
-  const int k0 = blockIdx.z * kchunk, k1 = min(Lc.nz, k0 + kchunk);
-  const T inv = T(1) / h, o2 = T(0.5) / h, o3 = inv * T(1) / T(3);
+struct MacFields {
+  const T* in[3];
+  T* out[3];
+  Lay L[3];
+  T add[3];
+  int zero_walls, chunks;
+};
+
+template <class T, bool ENO, int axis>
+__device__ __forceinline__ void mac_column(const MacFields<T>& A, int i, int j, int k0, int k1, T h, T inv_h, T eps,
+                                           T dt) {
+  const Lay& Lc = A.L[axis];
+  const T* __restrict__ comp = A.in[axis];
+  T* __restrict__ out = A.out[axis];
+  const T add = A.add[axis];
+  const T o2 = T(0.5) / h, o3 = inv_h * T(1) / T(3);
   int64_t c = Lc.at(i, j, k0);
   T vx[7], vy[7], vz[7];
   samples7(vz, comp, c, Lc.slab, comp[c], k0, Lc.nz, false);
   for (int k = k0; k < k1; ++k, c += Lc.slab) {
     const T next = k + 1 < k1 ? comp[c + 4 * Lc.slab] : T(0);
     T uvel, vvel, wvel;
-    mac_velocity(u, v, w, Lu, Lv, Lw, axis, i, j, k, uvel, vvel, wvel);
+    mac_velocity(A.in[0], A.in[1], A.in[2], A.L[0], A.L[1], A.L[2], axis, i, j, k, uvel, vvel, wvel);
     samples7(vx, comp, c, 1, vz[3], i, Lc.nx, false);
     samples7(vy, comp, c, Lc.px, vz[3], j, Lc.ny, false);
-    T dxm, dxp, dym, dyp, dzm, dzp;
-    eno3_pair7(vx, h, inv, o2, o3, dxm, dxp);
-    eno3_pair7(vy, h, inv, o2, o3, dym, dyp);
-    eno3_pair7(vz, h, inv, o2, o3, dzm, dzp);
-    out[c] = vz[3] - dt * ((uvel * (uvel > T(0) ? dxm : dxp) + vvel * (vvel > T(0) ? dym : dyp)) +
-                           wvel * (wvel > T(0) ? dzm : dzp));
+    T dx, dy, dz;
+    if (ENO) {
+      T dm, dp;
+      eno3_pair7(vx, h, inv_h, o2, o3, dm, dp);
+      dx = uvel > T(0) ? dm : dp;
+      eno3_pair7(vy, h, inv_h, o2, o3, dm, dp);
+      dy = vvel > T(0) ? dm : dp;
+      eno3_pair7(vz, h, inv_h, o2, o3, dm, dp);
+      dz = wvel > T(0) ? dm : dp;
+    } else {
+      dx = weno_upwind7(vx, inv_h, eps, uvel > T(0));
+      dy = weno_upwind7(vy, inv_h, eps, vvel > T(0));
+      dz = weno_upwind7(vz, inv_h, eps, wvel > T(0));
+    }
+    T r = vz[3] - dt * ((uvel * dx + vvel * dy) + wvel * dz);
+    const int e = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? Lc.nx : (axis == 1 ? Lc.ny : Lc.nz);
+    if (e > 0 && e < n - 1) {
+      if (add != T(0)) r += add;
+    } else if (A.zero_walls) {
+      r = T(0);
+    }
+    out[c] = r;
     slide7(vz, next, k, Lc.nz, false);
   }
+}
+
+template <class T, bool ENO>
+__global__ void __launch_bounds__(kColThreads) k_mac(const __grid_constant__ MacFields<T> A, T h, T inv_h, T eps, T dt,
+                                                     int kchunk, int flat) {
+  const int axis = blockIdx.z / A.chunks;
+  int i, j;
+  if (!column_of(A.L[axis], flat, i, j)) return;
+  const int k0 = (blockIdx.z - axis * A.chunks) * kchunk, k1 = min(A.L[axis].nz, k0 + kchunk);
+  if (k0 >= k1) return;
+  if (axis == 0) mac_column<T, ENO, 0>(A, i, j, k0, k1, h, inv_h, eps, dt);
+  else if (axis == 1) mac_column<T, ENO, 1>(A, i, j, k0, k1, h, inv_h, eps, dt);
+  else mac_column<T, ENO, 2>(A, i, j, k0, k1, h, inv_h, eps, dt);
 }
 
 // The vertical pipe's ENO3 self-advection of component `axis`
@@ -575,19 +591,28 @@ void weno5_levelset(const T* src, const T* base, T* out, const T* u, const T* v,
 }
 
 template <class T>
-void weno5_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
-               const Lay& Lw, int axis, double dx, double eps, double dt, cudaStream_t s) {
-  const ColumnGrid g = column_grid(Lc);
-  k_weno5_mac<T><<<g.grid, kColThreads, 0, s>>>(comp, out, u, v, w, Lc, Lu, Lv, Lw, axis, T(1.0 / dx), T(eps), T(dt),
-                                                g.kchunk, g.flat);
-}
-
-template <class T>
-void eno3_mac(const T* comp, T* out, const T* u, const T* v, const T* w, const Lay& Lc, const Lay& Lu, const Lay& Lv,
-              const Lay& Lw, int axis, double dx, double dt, cudaStream_t s) {
-  const ColumnGrid g = column_grid(Lc);
-  k_eno3_mac<T><<<g.grid, kColThreads, 0, s>>>(comp, out, u, v, w, Lc, Lu, Lv, Lw, axis, T(dx), T(dt), g.kchunk,
-                                               g.flat);
+void mac_advect(const T* const in[3], T* const out[3], const Lay* const L[3], bool eno, double dx, double eps, double dt,
+                const double add[3], int zero_walls, cudaStream_t s) {
+  MacFields<T> A;
+  ColumnGrid g = column_grid(*L[0]);
+  unsigned gx = 0, gy = 0;
+  int nz = 0;
+  for (int a = 0; a < 3; ++a) {
+    A.in[a] = in[a];
+    A.out[a] = out[a];
+    A.L[a] = *L[a];
+    A.add[a] = T(add[a]);
+    nz = std::max(nz, L[a]->nz);
+    const int64_t cols = (int64_t)L[a]->nx * L[a]->ny;
+    gx = std::max(gx, g.flat ? (unsigned)((cols + kColThreads - 1) / kColThreads) : (unsigned)((L[a]->nx + kTX - 1) / kTX));
+    gy = std::max(gy, g.flat ? 1u : (unsigned)((L[a]->ny + kTY - 1) / kTY));
+  }
+  g.kchunk = std::min(nz, 3 * g.kchunk);  // three components share the GPU
+  A.zero_walls = zero_walls;
+  A.chunks = (nz + g.kchunk - 1) / g.kchunk;
+  auto* kernel = eno ? k_mac<T, true> : k_mac<T, false>;
+  kernel<<<dim3(gx, gy, 3 * A.chunks), kColThreads, 0, s>>>(A, T(dx), eno ? T(1) / T(dx) : T(1.0 / dx), T(eps), T(dt),
+                                                            g.kchunk, g.flat);
 }
 
 template <class T>
@@ -643,12 +668,10 @@ void zero_walls(T* f, const Lay& L, int axis, cudaStream_t s) {
   template void weno5_levelset<T>(const T*, const T*, T*, const T*, const T*, const T*, const Lay&, const Lay&,       \
                                   const Lay&, const Lay&, double, double, double, double, double, cudaStream_t,       \
                                   const PipeGeom*);                                                                   \
-  template void weno5_mac<T>(const T*, T*, const T*, const T*, const T*, const Lay&, const Lay&, const Lay&,          \
-                             const Lay&, int, double, double, double, cudaStream_t);                                  \
+  template void mac_advect<T>(const T* const[3], T* const[3], const Lay* const[3], bool, double, double, double,      \
+                              const double[3], int, cudaStream_t);                                                    \
   template void eno3_pipe<T>(T*, const T*, const T*, const T*, const T*, const T*, const T*, const Lay&, const Lay&,  \
                              const Lay&, const Lay&, int, const PipeGeom&, double, double, cudaStream_t);             \
-  template void eno3_mac<T>(const T*, T*, const T*, const T*, const T*, const Lay&, const Lay&, const Lay&,           \
-                            const Lay&, int, double, double, cudaStream_t);                                          \
   template void sign_function<T>(const T*, T*, const Lay&, double, cudaStream_t);                                    \
   template void sussman_step<T>(const T*, T*, const T*, T*, const Lay&, double, double, double, double, double, int, \
                                 int, int, cudaStream_t);                                                                   \
