@@ -74,6 +74,9 @@ struct fs_ctx {
 
   std::vector<Buf> owned;
   int64_t bytes = 0;
+  bool arena_pass = false;  // fs_create's requests: parts of one allocation
+  char* arena = nullptr;    // NULL while they are summed
+  size_t arena_used = 0;
 
   // fields (storage type S)
   void *phi = nullptr, *s1 = nullptr, *s2 = nullptr, *s3 = nullptr, *s4 = nullptr, *sgn = nullptr;
@@ -170,7 +173,16 @@ struct Tape {
   std::vector<void*> re[3];           // [reinit block][pseudo-step]: input of each Sussman step
 };
 
+// A context's buffers come from one allocation: fs_create runs its requests
+// twice, first summing them (each rounded to 256 bytes), then handing out the
+// parts (creating and destroying a 256^3 context took 24 + 21 ms with one
+// cudaMalloc, one memset and one cudaFree each, 2 to 4 + 5 ms so).  Requests after creation (the adjoint's) are allocations of their own.
 fs_status dalloc(fs_ctx* c, void** out, size_t bytes) {
+  if (c->arena_pass) {
+    *out = c->arena ? c->arena + c->arena_used : nullptr;
+    c->arena_used += (bytes + 255) / 256 * 256;
+    return FS_OK;
+  }
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) {
@@ -209,34 +221,18 @@ fs_status mg_alloc(fs_ctx* c) {
       m.x[1] = c->rb_q;
     }
   }
-  // everything else in one allocation, each array 256-byte aligned: first
-  // its size, then the pointers
-  char* base = nullptr;
-  for (int pass = 0; pass < 2; ++pass) {
-    size_t off = 0;
-    auto take = [&](void** p, size_t bytes) {
-      if (pass) *p = base + off;
-      off += (bytes + 255) / 256 * 256;
-    };
-    for (int l = 0; l < M.levels; ++l) {
-      MgLevel& m = M.level[l];
-      if (l > 0) {
-        for (float** p : {&m.ax, &m.ay, &m.az}) take((void**)p, m.L.total * sizeof(float));
-        if (l <= M.top)
-          for (float** p : {&m.x[0], &m.x[1], &m.b[0], &m.b[1]}) take((void**)p, m.H.total * sizeof(float));
-      }
-      if (l < M.top)
-        for (unsigned char** p : {&m.cls[0], &m.cls[1]}) take((void**)p, m.H.total);
-      if (l == 0) take((void**)&m.ccls, m.L.total);
+  for (int l = 0; l < M.levels; ++l) {
+    MgLevel& m = M.level[l];
+    if (l > 0) {
+      for (float** p : {&m.ax, &m.ay, &m.az}) CKS(dalloc(c, (void**)p, m.L.total * sizeof(float)));
+      if (l <= M.top)
+        for (float** p : {&m.x[0], &m.x[1], &m.b[0], &m.b[1]}) CKS(dalloc(c, (void**)p, m.H.total * sizeof(float)));
     }
-    if (!pass) CKS(dalloc(c, (void**)&base, off));
+    if (l < M.top)
+      for (unsigned char** p : {&m.cls[0], &m.cls[1]}) CKS(dalloc(c, (void**)p, m.H.total));
+    if (l == 0) CKS(dalloc(c, (void**)&m.ccls, m.L.total));
   }
   CKS(dalloc(c, (void**)&c->mgst, sizeof(MgState)));
-  if (cudaMallocHost((void**)&c->mgst_host, sizeof(MgState)) != cudaSuccess) {
-    cudaGetLastError();
-    set_error("pinned host allocation failed");
-    return FS_OOM;
-  }
   return FS_OK;
 }
 
@@ -254,8 +250,6 @@ void release(fs_ctx* c) {
   c->owned.clear();
   c->mesh.release();
   if (c->st_host) cudaFreeHost(c->st_host);
-  if (c->sc_host) cudaFreeHost(c->sc_host);
-  if (c->mgst_host) cudaFreeHost(c->mgst_host);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->evp0) cudaEventDestroy(c->evp0);
   if (c->evp1) cudaEventDestroy(c->evp1);
@@ -1897,77 +1891,85 @@ fs_status fs_create(const fs_grid_desc* grid, const fs_params* params, fs_ctx** 
   const size_t c8 = c->Lc.total * sizeof(double);
   const size_t V = c->fp32 ? sizeof(float) : sizeof(double);
   const size_t cv = c->Lc.total * V;
-  fs_status s = FS_OK;
-  void** cell_s[] = {&c->phi, &c->s1, &c->s2, &c->s3, &c->s4, &c->sgn};
-  for (void** p : cell_s) if ((s = dalloc(c, p, cb)) != FS_OK) return fail(s);
-  void** fu[] = {&c->u, &c->u0, &c->ua};
-  void** fv[] = {&c->v, &c->v0, &c->va};
-  void** fw[] = {&c->w, &c->w0, &c->wa};
-  for (void** p : fu) if ((s = dalloc(c, p, ub)) != FS_OK) return fail(s);
-  for (void** p : fv) if ((s = dalloc(c, p, vb)) != FS_OK) return fail(s);
-  for (void** p : fw) if ((s = dalloc(c, p, wb)) != FS_OK) return fail(s);
-  double** d8[] = {&c->p64, &c->b64, &c->div64, &c->kappa};
-  for (double** p : d8) if ((s = dalloc(c, (void**)p, c8)) != FS_OK) return fail(s);
-  if ((s = dalloc(c, (void**)&c->fsfixed, c->Lc.total)) != FS_OK) return fail(s);
-  if ((s = dalloc(c, (void**)&c->fsflag, sizeof(int))) != FS_OK) return fail(s);
-  if (c->fp32 && (s = dalloc(c, (void**)&c->p64bak, c8)) != FS_OK) return fail(s);
-  void** pv[] = {&c->pax, &c->pay, &c->paz, &c->pdiag, &c->pr, &c->pp, &c->pq};
-  for (void** p : pv) if ((s = dalloc(c, p, cv)) != FS_OK) return fail(s);
-  if (c->fp32) {
-    if ((s = dalloc(c, &c->px, cv)) != FS_OK) return fail(s);
-    if ((s = dalloc(c, &c->prhs, cv)) != FS_OK) return fail(s);
-    if ((s = dalloc(c, (void**)&c->pdinv, c->Lc.total * sizeof(unsigned short))) != FS_OK) return fail(s);
-    c->Lh = make_half_lay(c->Lc);
-    const size_t hb = c->Lh.total;
-    if ((s = dalloc(c, (void**)&c->rb_x, hb * sizeof(double))) != FS_OK) return fail(s);
-    float** hv[] = {&c->rb_r, &c->rb_p, &c->rb_q, &c->rb_tau};
-    for (float** p : hv) if ((s = dalloc(c, (void**)p, hb * sizeof(float))) != FS_OK) return fail(s);
-    if ((s = dalloc(c, (void**)&c->rb_dinv, hb * sizeof(unsigned short))) != FS_OK) return fail(s);
-    if (!prm.pipe) {
-      if ((s = mg_alloc(c)) != FS_OK) return fail(s);
-      apply_params(c);  // the levels' uniform couplings
-      if (mg_prepare() != cudaSuccess) {
-        set_error("shared memory of the multigrid cycle: %s", cudaGetErrorString(cudaGetLastError()));
-        return fail(FS_CUDA_ERROR);
-      }
-    }
-  }
-  if (prm.pipe) {
-    const size_t fb[3] = {ub, vb, wb};
-    for (int a = 0; a < 3; ++a)
-      for (void** p : {&c->pgen[a], &c->pgx[a], &c->pgz[a]})
-        if ((s = dalloc(c, p, fb[a])) != FS_OK) return fail(s);
-  }
-  if (prm.viscosity == 1) {
-    const size_t fb[3] = {ub, vb, wb};
-    for (int a = 0; a < 3; ++a)
-      for (int m = 0; m < 9; ++m)
-        if ((s = dalloc(c, &c->vs[a][m], fb[a])) != FS_OK) return fail(s);
-  }
   // grid sizes of the Krylov kernels (occupancy queries; never under capture)
   cg_prepare<double, double>();
   cg_prepare<float, double>();
   cg_prepare<float, float>();
-  int nblk = std::max(pcg_blocks(c->Lu), std::max(pcg_blocks(c->Lv), pcg_blocks(c->Lw))) * 2 + 64;
-  for (const Lay* L : {&c->Lc, &c->Lu, &c->Lv, &c->Lw}) nblk = std::max(nblk, cg_max_blocks(*L));
-  if (c->fp32) nblk = std::max(nblk, std::max(rb_blocks(c->Lh), mg_max_blocks(c->Lc)));
-  if ((s = dalloc(c, (void**)&c->partials, (size_t)nblk * 3 * sizeof(double))) != FS_OK) return fail(s);
-  if ((s = dalloc(c, (void**)&c->tickets, 8 * sizeof(unsigned int))) != FS_OK) return fail(s);
-  if ((s = dalloc(c, (void**)&c->scalars, 16 * sizeof(double))) != FS_OK) return fail(s);
-  if ((s = dalloc(c, (void**)&c->st, sizeof(PcgState))) != FS_OK) return fail(s);
+  if (c->fp32) c->Lh = make_half_lay(c->Lc);
   if (!c->fp32 && !prm.pipe) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) == cudaSuccess)
       c->brick = brick_plan(c->Lc, sms);
-    if (c->brick.gx > 0 && (s = dalloc(c, &c->brick_slots, brick_slots_bytes())) != FS_OK) return fail(s);
   }
-  const int64_t maxf = std::max(std::max(c->Lu.total, c->Lv.total), std::max(c->Lw.total, c->Lc.total));
-  if ((s = dalloc(c, (void**)&c->staging, (size_t)maxf * sizeof(double))) != FS_OK) return fail(s);
-  if (cudaMallocHost((void**)&c->st_host, sizeof(PcgState)) != cudaSuccess ||
-      cudaMallocHost((void**)&c->sc_host, 16 * sizeof(double)) != cudaSuccess) {
+  if (c->fp32 && !prm.pipe && mg_prepare() != cudaSuccess) {
+    set_error("shared memory of the multigrid cycle: %s", cudaGetErrorString(cudaGetLastError()));
+    return fail(FS_CUDA_ERROR);
+  }
+  auto requests = [&]() -> fs_status {
+    void** cell_s[] = {&c->phi, &c->s1, &c->s2, &c->s3, &c->s4, &c->sgn};
+    for (void** p : cell_s) CKS(dalloc(c, p, cb));
+    const size_t fb[3] = {ub, vb, wb};
+    void** faces[3][3] = {{&c->u, &c->u0, &c->ua}, {&c->v, &c->v0, &c->va}, {&c->w, &c->w0, &c->wa}};
+    for (int a = 0; a < 3; ++a)
+      for (void** p : faces[a]) CKS(dalloc(c, p, fb[a]));
+    double** d8[] = {&c->p64, &c->b64, &c->div64, &c->kappa};
+    for (double** p : d8) CKS(dalloc(c, (void**)p, c8));
+    CKS(dalloc(c, (void**)&c->fsfixed, c->Lc.total));
+    CKS(dalloc(c, (void**)&c->fsflag, sizeof(int)));
+    if (c->fp32) CKS(dalloc(c, (void**)&c->p64bak, c8));
+    void** pv[] = {&c->pax, &c->pay, &c->paz, &c->pdiag, &c->pr, &c->pp, &c->pq};
+    for (void** p : pv) CKS(dalloc(c, p, cv));
+    if (c->fp32) {
+      CKS(dalloc(c, &c->px, cv));
+      CKS(dalloc(c, &c->prhs, cv));
+      CKS(dalloc(c, (void**)&c->pdinv, c->Lc.total * sizeof(unsigned short)));
+      const size_t hb = c->Lh.total;
+      CKS(dalloc(c, (void**)&c->rb_x, hb * sizeof(double)));
+      float** hv[] = {&c->rb_r, &c->rb_p, &c->rb_q, &c->rb_tau};
+      for (float** p : hv) CKS(dalloc(c, (void**)p, hb * sizeof(float)));
+      CKS(dalloc(c, (void**)&c->rb_dinv, hb * sizeof(unsigned short)));
+      if (!prm.pipe) CKS(mg_alloc(c));
+    }
+    if (prm.pipe)
+      for (int a = 0; a < 3; ++a)
+        for (void** p : {&c->pgen[a], &c->pgx[a], &c->pgz[a]}) CKS(dalloc(c, p, fb[a]));
+    if (prm.viscosity == 1)
+      for (int a = 0; a < 3; ++a)
+        for (int m = 0; m < 9; ++m) CKS(dalloc(c, &c->vs[a][m], fb[a]));
+    int nblk = std::max(pcg_blocks(c->Lu), std::max(pcg_blocks(c->Lv), pcg_blocks(c->Lw))) * 2 + 64;
+    for (const Lay* L : {&c->Lc, &c->Lu, &c->Lv, &c->Lw}) nblk = std::max(nblk, cg_max_blocks(*L));
+    if (c->fp32) nblk = std::max(nblk, std::max(rb_blocks(c->Lh), mg_max_blocks(c->Lc)));
+    CKS(dalloc(c, (void**)&c->partials, (size_t)nblk * 3 * sizeof(double)));
+    CKS(dalloc(c, (void**)&c->tickets, 8 * sizeof(unsigned int)));
+    CKS(dalloc(c, (void**)&c->scalars, 16 * sizeof(double)));
+    CKS(dalloc(c, (void**)&c->st, sizeof(PcgState)));
+    if (c->brick.gx > 0) CKS(dalloc(c, &c->brick_slots, brick_slots_bytes()));
+    const int64_t maxf = std::max(std::max(c->Lu.total, c->Lv.total), std::max(c->Lw.total, c->Lc.total));
+    CKS(dalloc(c, (void**)&c->staging, (size_t)maxf * sizeof(double)));
+    return FS_OK;
+  };
+  c->arena_pass = true;
+  fs_status s = requests();  // their sum
+  c->arena_pass = false;
+  void* arena = nullptr;
+  if (s != FS_OK || (s = dalloc(c, &arena, c->arena_used)) != FS_OK) return fail(s);
+  c->arena = (char*)arena;
+  c->arena_used = 0;
+  c->arena_pass = true;
+  s = requests();
+  c->arena_pass = false;
+  if (s != FS_OK) return fail(s);
+  apply_params(c);  // the multigrid levels' uniform couplings
+  // pinned host copies of the solver states and the scalars, one allocation
+  constexpr size_t kSt = (sizeof(PcgState) + 63) / 64 * 64, kMg = (sizeof(MgState) + 63) / 64 * 64;
+  char* pinned = nullptr;
+  if (cudaMallocHost((void**)&pinned, kSt + kMg + 16 * sizeof(double)) != cudaSuccess) {
     set_error("pinned host allocation failed");
     return fail(FS_OOM);
   }
+  c->st_host = (PcgState*)pinned;
+  c->mgst_host = (MgState*)(pinned + kSt);
+  c->sc_host = (double*)(pinned + kSt + kMg);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
     set_error("initialisation failed: %s", cudaGetErrorString(cudaGetLastError()));
     return fail(FS_CUDA_ERROR);
