@@ -1,5 +1,6 @@
-// The FP64 Jacobi-PCG of the pressure (PCG_METHOD.cpp:4-126) as one resident
-// kernel, for grids whose vectors fit the GPU's shared memory and registers.
+// Pressure solves of small boxes as one resident kernel: the FP64 Jacobi-PCG
+// (PCG_METHOD.cpp:4-126) below, the red-black iteration of the FP32 contexts after
+// it, for grids whose vectors fit the SMs' shared memory and registers.
 //
 // What bounds it.  At 64^3 and 96^3 an iteration of three kernels (fs_krylov.cu)
 // takes 20 to 31 us, nearly all of it launches, grid-wide reductions and cold
@@ -57,7 +58,8 @@ struct BrickArgs {
 // 1.8 us, against 4.5 us where every block polls the 144 sums themselves (the
 // polls queue in front of the stores they wait for).  `turn` counts the
 // exchanges of the solve from 1.  Returns false when a wait ran out.
-__device__ __forceinline__ bool exchange(const BrickArgs& A, int nb, unsigned turn, bool two, double& v0, double& v1) {
+__device__ __forceinline__ bool exchange(double* all_sums, unsigned* count, int nb, unsigned turn, bool two, double& v0,
+                                         double& v1) {
   __shared__ double part[2][kT / 32];
   __shared__ int bad;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -68,7 +70,7 @@ __device__ __forceinline__ bool exchange(const BrickArgs& A, int nb, unsigned tu
   }
   if (tid == 0) bad = 0;
   __syncthreads();
-  double* sums = A.sums + (turn & 1u) * 2 * kMaxBlocks;  // the other half may still be read
+  double* sums = all_sums + (turn & 1u) * 2 * kMaxBlocks;  // the other half may still be read
   if (warp == 0) {
     const double s0 = warp_sum(lane < kT / 32 ? part[0][lane] : 0.0);
     const double s1 = two ? warp_sum(lane < kT / 32 ? part[1][lane] : 0.0) : 0.0;
@@ -76,11 +78,11 @@ __device__ __forceinline__ bool exchange(const BrickArgs& A, int nb, unsigned tu
       __stcg(sums + blockIdx.x, s0);
       if (two) __stcg(sums + kMaxBlocks + blockIdx.x, s1);
       // release: cumulative over the block's stores (after the barrier above)
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.count) : "memory");
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
       const unsigned want = turn * (unsigned)nb;
       unsigned got = 0, n = 0;
       for (;;) {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(A.count) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(count) : "memory");
         if ((int)(got - want) >= 0) break;
         if (++n >= kSpin) {
           bad = 1;
@@ -311,8 +313,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
       rr += r[m] * r[m];
       bb += bv * bv;
     }
-  bool alive = exchange(A, nb, ++turn, true, rz, rr);
-  alive = exchange(A, nb, ++turn, false, bb, zero) && alive;
+  bool alive = exchange(A.sums, A.count, nb, ++turn, true, rz, rr);
+  alive = exchange(A.sums, A.count, nb, ++turn, false, bb, zero) && alive;
   int iter = 0, status = PCG_RUNNING;
   if (!alive) status = PCG_TIMEOUT;
   else if (!isfinite(rz) || !isfinite(rr)) status = PCG_NONFINITE;
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
         q[m] = apply(m);
         pq += p[pi[m]] * q[m];
       }
-    if (!exchange(A, nb, ++turn, false, pq, zero)) {
+    if (!exchange(A.sums, A.count, nb, ++turn, false, pq, zero)) {
       status = PCG_TIMEOUT;
       break;
     }
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
         rz1 += r[m] * z;
         rr1 += r[m] * r[m];
       }
-    if (!exchange(A, nb, ++turn, true, rz1, rr1)) {
+    if (!exchange(A.sums, A.count, nb, ++turn, true, rz1, rr1)) {
       status = PCG_TIMEOUT;
       break;
     }
@@ -435,6 +437,368 @@ const void* kernel_of(const BrickPlan& P) {
     case 8: return (const void*)k_pcg_brick<8, false>;
     case 12: return (const void*)k_pcg_brick<12, false>;
     default: return (const void*)k_pcg_brick<16, false>;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The red-black iteration of fs_redblack.cu (CG on the black Schur complement:
+// FP32 vectors, FP64 iterate, bf16 pivots) between two reliable updates, as
+// one resident kernel in the manner of the one above.
+//
+// What bounds it: at 96^3 the five kernels of an iteration move a few MB that L2
+// holds, and 26.5 us go into their launches, cold starts and grid-wide
+// reductions.  Here a brick's p and the tau of its red cells live in shared
+// memory, one array per colour (neighbouring threads read neighbouring words; one
+// array of both colours would be read two words apart), p with a halo of two
+// cells and tau with one: each brick computes the tau of the red cells around it
+// itself, so that an iteration still exchanges only twice.  r and q are
+// registers, the FP64 iterate is in shared memory.  Every value is computed by the
+// expressions of fs_redblack.cu and fs_krylov.cu in the same order; only the
+// sums over the grid add in another one.  Measured, a whole projection to 1e-8 with five
+// kernels per iteration -> with this one: 32^3 (120 iterations) 4.0 -> 1.5 ms,
+// 64^3 (218) 7.2 -> 2.6, 96^3 (327) 14.2 -> 5.6, 120^3 (395) 25.3 -> 14.1.
+// ---------------------------------------------------------------------------
+struct RbBrickArgs {
+  Lay L, H;
+  int gx, gy, gz;
+  const float *ax, *ay, *az, *phi;
+  const double* extra0;
+  float *r, *p, *z;
+  const unsigned short* dinv;
+  double* sums;
+  unsigned* count;
+  PcgState* st;
+  float a[3];  // uniform coupling of a phase
+  int cap;     // mixed cells listed in shared memory
+};
+
+struct Six {
+  float xm, xp, ym, yp, zm, zp;
+};
+
+// tau of the red cell in place c of its colour's array; o: its column is the
+// second of its pair; first: it lies in column 0 of the box
+__device__ __forceinline__ float brick_tau(const float* PB, int c, int o, int hy, int hz, bool first, const Six& a,
+                                           float e0) {
+  const float xm = PB[c + o - 1], xp = PB[c + o], ym = PB[c - hy], yp = PB[c + hy], zm = PB[c - hz], zp = PB[c + hz];
+  const float b0 = first ? xp : xm;
+  float num = a.xm * (xm - b0) + a.xp * (xp - b0);
+  num += a.ym * (ym - b0) + a.yp * (yp - b0);
+  num += a.zm * (zm - b0) + a.zp * (zp - b0);
+  float d = ((a.xm + a.xp) + (a.ym + a.yp)) + (a.zm + a.zp);
+  if (e0 != 0.0f) {
+    num -= e0 * b0;
+    d += e0;
+  }
+  return d > 0.0f ? num / d : 0.0f;
+}
+
+// (S p) of the black cell in place c; column: 0, 1 or 2 (any later one)
+__device__ __forceinline__ float brick_schur(const float* PB, const float* PR, int c, int o, int hy, int hz, int column,
+                                             const Six& a) {
+  const float pc = PB[c];
+  const float txm = PR[c + o - 1], txp = PR[c + o], tym = PR[c - hy], typ = PR[c + hy], tzm = PR[c - hz],
+              tzp = PR[c + hz];
+  const int b = column > 0 ? o - 1 : 0;
+  const float dxm = column > 1 ? pc - PB[c - 1] : 0.0f;
+  const float dym = pc - PB[c - hy + b], dyp = pc - PB[c + hy + b];
+  const float dzm = pc - PB[c - hz + b], dzp = pc - PB[c + hz + b];
+  float acc = a.xm * (dxm - txm) + a.xp * (0.0f - txp);
+  acc += a.ym * (dym - tym) + a.yp * (dyp - typ);
+  acc += a.zm * (dzm - tzm) + a.zp * (dzp - tzp);
+  return acc;
+}
+
+// black cells of the halo (two layers on each face, the twelve edges between
+// them; half of each, rounded up) and red cells of the first layer
+__host__ __device__ inline int rb_halo(int bx, int by, int bz) {
+  return 2 * (by * bz + bx * bz + bx * by) + 2 * (bx + by + bz) + 24;
+}
+__host__ __device__ inline int rb_ring(int bx, int by, int bz) { return by * bz + bx * bz + bx * by + 6; }
+
+constexpr int kNotListed = 255;
+
+// K: packed slots (a black and a red cell) per thread
+template <int K>
+__global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBrickArgs A) {
+  extern __shared__ double smem[];
+  const Lay &L = A.L, &H = A.H;
+  const int nb = gridDim.x, tid = threadIdx.x;
+  const int qx = blockIdx.x % A.gx, qy = (blockIdx.x / A.gx) % A.gy, qz = blockIdx.x / (A.gx * A.gy);
+  const int h0 = (int)((int64_t)qx * H.nx / A.gx), h1 = (int)((int64_t)(qx + 1) * H.nx / A.gx);
+  const int j0 = (int)((int64_t)qy * L.ny / A.gy), j1 = (int)((int64_t)(qy + 1) * L.ny / A.gy);
+  const int k0 = (int)((int64_t)qz * L.nz / A.gz), k1 = (int)((int64_t)(qz + 1) * L.nz / A.gz);
+  const int i0 = 2 * h0, bh = h1 - h0, bx = 2 * bh, by = j1 - j0, bz = k1 - k0, slots = bh * by * bz;
+  const int sy = bx + 4, sz = sy * (by + 4), padded = sz * (bz + 4), hy = sy / 2, hz = sz / 2;
+  double* xs = smem;
+  float* PB = (float*)(xs + slots);
+  float* PR = PB + padded / 2;
+  float* ma = PR + padded / 2;  // the list of mixed cells: couplings, q, place
+  float* mq = ma + 6 * (size_t)A.cap;
+  int* list = (int*)(mq + A.cap);
+  int* hp = list + A.cap;  // black halo cells: place and packed offset
+  int* hg = hp + rb_halo(bx, by, bz);
+  int* ring = hg + rb_halo(bx, by, bz);
+  int* go = ring + rb_ring(bx, by, bz);                // a slot's packed offset
+  unsigned short* me = (unsigned short*)(go + slots);  // a listed black cell's entry
+  unsigned short* dv = me + slots;
+  unsigned char* kind = (unsigned char*)(dv + slots);
+  __shared__ int nhalo, nring, nmixed;
+  const PcgState in = *A.st;
+  if (in.done) return;  // the same in every block
+  double* x = (double*)in.x;
+  if (tid == 0) nhalo = nring = nmixed = 0;
+  for (int t = tid; t < padded; t += kT) kind[t] = 0;
+  for (int t = tid; t < padded / 2; t += kT) PB[t] = PR[t] = 0.0f;
+  __syncthreads();
+  const int64_t hbase = H.at(h0, j0, k0);
+  // Every cell of the padded brick that takes part: its place in the lists, and
+  // for a red cell of the brick or its first layer and a black cell of the brick
+  // its kind: bits 0..5 the face lies inside the box, 6 and 7 the phase whose
+  // 1/rho all faces carry.  0: listed (or no cell), kNotListed: the list is full.
+  for (int t = tid; t < padded; t += kT) {
+    const int lz = t / sz - 2, ly = t % sz / sy - 2, lx = t % sy - 2;
+    const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
+    if (i < 0 || i >= L.nx || j < 0 || j >= L.ny || k < 0 || k >= L.nz) continue;
+    const int ox = lx < 0 ? -lx : (lx >= bx ? lx - bx + 1 : 0), oy = ly < 0 ? -ly : (ly >= by ? ly - by + 1 : 0),
+              oz = lz < 0 ? -lz : (lz >= bz ? lz - bz + 1 : 0);
+    const int off = ox + oy + oz;
+    const bool black = (i + j + k) & 1;
+    if (off > (black ? 2 : 1)) continue;
+    if (black && off > 0) {
+      const int e = atomicAdd(&nhalo, 1);
+      hp[e] = t >> 1;
+      hg[e] = (int)(((i >> 1) - h0) + (int64_t)(j - j0) * H.px + (int64_t)(k - k0) * H.slab);
+      continue;
+    }
+    if (off > 0) ring[atomicAdd(&nring, 1)] = t;
+    const int f = (i > 0) | (i < L.nx - 1) << 1 | (j > 0) << 2 | (j < L.ny - 1) << 3 | (k > 0) << 4 | (k < L.nz - 1) << 5;
+    const float* ph = A.phi + L.at(i, j, k);
+    const bool n = ph[0] <= 0.0f;
+    auto alike = [&](int64_t o) { return n ? ph[o] <= 0.0f : ph[o] > 0.0f; };  // NaN: of no phase
+    const bool same = alike(0) && !(i == 0 && j == 0 && k == 0) && (!(f & 1) || alike(-1)) && (!(f & 2) || alike(1)) &&
+                      (!(f & 4) || alike(-L.px)) && (!(f & 8) || alike(L.px)) && (!(f & 16) || alike(-L.slab)) &&
+                      (!(f & 32) || alike(L.slab));
+    if (same) {
+      kind[t] = (unsigned char)(f | (n ? 64 : 128));
+      continue;
+    }
+    const int e = atomicAdd(&nmixed, 1);
+    if (e >= A.cap) {
+      kind[t] = kNotListed;
+      continue;
+    }
+    list[e] = t | (black ? 1 << 30 : 0) | min(i, 2) << 28;
+    if (black) me[(lz * by + ly) * bh + (lx >> 1)] = (unsigned short)e;
+    const int64_t g = L.at(i, j, k);
+    ma[e] = A.ax[g];
+    ma[A.cap + e] = A.ax[g + 1];
+    ma[2 * A.cap + e] = A.ay[g];
+    ma[3 * A.cap + e] = A.ay[g + L.px];
+    ma[4 * A.cap + e] = A.az[g];
+    ma[5 * A.cap + e] = A.az[g + L.slab];
+  }
+  // this thread's slots: index of the cell in the pair's first column, which
+  // of the two is black, whether that one exists and its column
+  int base[K];
+  unsigned second = 0u, have = 0u, col0 = 0u, col1 = 0u;
+  float r[K], q[K];
+#pragma unroll
+  for (int m = 0; m < K; ++m) {
+    const int t = tid + m * kT;
+    base[m] = -1;
+    r[m] = q[m] = 0.0f;
+    if (t < slots) {
+      const int h = t % bh, row = t / bh, ly = row % by, lz = row / by;
+      base[m] = (lz + 2) * sz + (ly + 2) * sy + 2 * h + 2;
+      const int o = (j0 + ly + k0 + lz + 1) & 1, i = i0 + 2 * h + o;
+      second |= (unsigned)o << m;
+      if (i < L.nx) have |= 1u << m;
+      if (i == 0) col0 |= 1u << m;
+      if (i == 1) col1 |= 1u << m;
+      go[t] = (int)(h + (int64_t)ly * H.px + (int64_t)lz * H.slab);
+      const int64_t g = hbase + go[t];
+      r[m] = A.r[g];
+      dv[t] = A.dinv[g];
+      xs[t] = x[g];
+      PB[base[m] >> 1] = A.p[g];
+    }
+  }
+  __syncthreads();
+  const int halos = nhalo, rings = nring, listed = min(nmixed, A.cap);
+  for (int e = tid; e < halos; e += kT) PB[hp[e]] = A.p[hbase + hg[e]];
+  // the first cell of the box, which carries the deflation term, where this brick needs its tau
+  const int origin = i0 == 0 && j0 <= 1 && k0 <= 1 ? (2 - k0) * sz + (2 - j0) * sy + 2 : -1;
+  const float e0 = (float)*A.extra0;
+  __syncthreads();
+
+  auto uniform = [&](int f) -> Six {
+    const float a = A.a[f >> 6];
+    if ((f & 63) == 63) return {a, a, a, a, a, a};
+    return {f & 1 ? a : 0.0f, f & 2 ? a : 0.0f, f & 4 ? a : 0.0f, f & 8 ? a : 0.0f, f & 16 ? a : 0.0f, f & 32 ? a : 0.0f};
+  };
+  auto entry = [&](int e) -> Six {
+    return {ma[e], ma[A.cap + e], ma[2 * A.cap + e], ma[3 * A.cap + e], ma[4 * A.cap + e], ma[5 * A.cap + e]};
+  };
+  auto fetched = [&](int t) -> Six {
+    const int64_t g = L.at(i0 + t % sy - 2, j0 + t % sz / sy - 2, k0 + t / sz - 2);
+    return {A.ax[g], A.ax[g + 1], A.ay[g], A.ay[g + L.px], A.az[g], A.az[g + L.slab]};
+  };
+  auto tau = [&](int t) {  // of a red cell that is not listed
+    const int f = kind[t];
+    if (f == kNotListed)
+      PR[t >> 1] = brick_tau(PB, t >> 1, t & 1, hy, hz, i0 + t % sy - 2 == 0, fetched(t), t == origin ? e0 : 0.0f);
+    else if (f)
+      PR[t >> 1] = brick_tau(PB, t >> 1, t & 1, hy, hz, !(f & 1), uniform(f), 0.0f);
+  };
+  double rz = in.rz, rr = in.rr, rz_prev = in.rz_prev, best = in.best_rr, alpha = in.alpha, beta = in.beta;
+  int iter = in.iter, stall = in.stall, status = PCG_RUNNING;
+  unsigned turn = 0;
+  while (status == PCG_RUNNING) {
+#pragma unroll
+    for (int m = 0; m < K; ++m)
+      if (base[m] >= 0) tau(base[m] + 1 - (int)(second >> m & 1u));
+    for (int e = tid; e < rings; e += kT) tau(ring[e]);
+    for (int e = tid; e < listed; e += kT)
+      if (!(list[e] >> 30)) {
+        const int t = list[e] & 0xfffffff;
+        PR[t >> 1] = brick_tau(PB, t >> 1, t & 1, hy, hz, list[e] >> 28 == 0, entry(e), t == origin ? e0 : 0.0f);
+      }
+    __syncthreads();
+    for (int e = tid; e < listed; e += kT)
+      if (list[e] >> 30) {
+        const int t = list[e] & 0xfffffff;
+        mq[e] = brick_schur(PB, PR, t >> 1, t & 1, hy, hz, list[e] >> 28 & 3, entry(e));
+      }
+    __syncthreads();
+    double pq = 0.0, none = 0.0;
+#pragma unroll
+    for (int m = 0; m < K; ++m)
+      if (have >> m & 1u) {
+        const int o = (int)(second >> m & 1u), t = base[m] + o, f = kind[t];
+        const int column = col0 >> m & 1u ? 0 : (col1 >> m & 1u ? 1 : 2);
+        if (f == 0)
+          q[m] = mq[me[tid + m * kT]];
+        else
+          q[m] = brick_schur(PB, PR, t >> 1, o, hy, hz, column, f == kNotListed ? fetched(t) : uniform(f));
+        pq += (double)PB[t >> 1] * (double)q[m];
+      }
+    if (!exchange(A.sums, A.count, nb, ++turn, false, pq, none)) {
+      status = PCG_TIMEOUT;
+      break;
+    }
+    alpha = rz / pq;
+    if (!(pq > 0.0) || !isfinite(alpha)) {
+      status = PCG_STAGNATED;
+      break;
+    }
+    const float al = (float)alpha;
+    double rz1 = 0.0, rr1 = 0.0;
+#pragma unroll
+    for (int m = 0; m < K; ++m)
+      if (have >> m & 1u) {
+        const int t = tid + m * kT;
+        r[m] -= al * q[m];
+        const float z = r[m] * __uint_as_float((unsigned)dv[t] << 16);
+        __stcg(A.z + hbase + go[t], z);
+        q[m] = z;
+        rz1 += (double)r[m] * (double)z;
+        rr1 += (double)r[m] * (double)r[m];
+      }
+    if (!exchange(A.sums, A.count, nb, ++turn, true, rz1, rr1)) {
+      status = PCG_TIMEOUT;
+      break;
+    }
+    // the decisions of k_cg_update, the same in every block
+    rz_prev = rz;
+    rz = rz1;
+    rr = rr1;
+    if (rr < 0.99 * best) {
+      best = rr;
+      stall = 0;
+    } else {
+      ++stall;
+    }
+    if (!isfinite(rz) || !isfinite(rr)) {
+      status = PCG_NONFINITE;  // x is not moved along that step
+      break;
+    }
+    if (in.criterion == 2 ? rr < in.tol * in.tol : (in.criterion == 1 ? rz < in.tol * in.tol : sqrt(rr) <= in.tol * sqrt(in.bb))) {
+      status = PCG_CONVERGED;
+    } else {
+      beta = rz / rz_prev;
+      ++iter;
+      if (iter >= in.max_iter) status = PCG_MAXITER;
+      else if (in.stall_limit > 0 && stall >= in.stall_limit) status = PCG_STAGNATED;
+      else if (in.reliable_delta > 0.0 && rr < in.reliable_delta * in.reliable_delta * in.max_rr)
+        status = PCG_RELIABLE_UPDATE;
+    }
+    const float be = (float)beta;
+#pragma unroll
+    for (int m = 0; m < K; ++m)
+      if (have >> m & 1u) {
+        const float pv = PB[base[m] >> 1];
+        xs[tid + m * kT] += alpha * (double)pv;
+        if (status == PCG_RUNNING) PB[base[m] >> 1] = pv * be + q[m];
+      }
+    if (status == PCG_RUNNING) {
+      constexpr int kFetch = 6;  // neighbours' z in flight
+      for (int f0 = tid; f0 < halos; f0 += kFetch * kT) {
+        int at[kFetch];
+        float z[kFetch];
+#pragma unroll
+        for (int m = 0; m < kFetch; ++m) {
+          const int e = f0 + m * kT;
+          at[m] = e < halos ? hp[e] : -1;
+          z[m] = at[m] >= 0 ? __ldcg(A.z + hbase + hg[e]) : 0.0f;
+        }
+#pragma unroll
+        for (int m = 0; m < kFetch; ++m)
+          if (at[m] >= 0) PB[at[m]] = PB[at[m]] * be + z[m];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int m = 0; m < K; ++m)
+    if (have >> m & 1u) {
+      const int t = tid + m * kT;
+      const int64_t g = hbase + go[t];
+      A.r[g] = r[m];
+      A.p[g] = PB[base[m] >> 1];
+      x[g] = xs[t];
+    }
+  if (blockIdx.x == 0 && tid == 0) {
+    PcgState* st = A.st;
+    st->rz = rz;
+    st->rr = rr;
+    st->rz_prev = rz_prev;
+    st->best_rr = best;
+    st->stall = stall;
+    st->alpha = alpha;
+    st->beta = beta;
+    st->iter = iter;
+    st->x_pending = 0;
+    st->status = status;
+    st->done = status == PCG_RELIABLE_UPDATE ? 2 : 1;
+  }
+}
+
+size_t rb_brick_bytes(int bh, int by, int bz) {
+  const int bx = 2 * bh;
+  const size_t slots = (size_t)bh * by * bz, padded = (size_t)(bx + 4) * (by + 4) * (bz + 4);
+  return slots * 8 + padded * 4 + (2 * (size_t)rb_halo(bx, by, bz) + rb_ring(bx, by, bz)) * 4 + slots * 8 +
+         (padded + 7) / 8 * 8;
+}
+constexpr size_t kRbEntryBytes = 6 * 4 + 4 + 4;
+
+const void* rb_kernel_of(int per_thread) {
+  switch (per_thread) {
+    case 2: return (const void*)k_rb_brick<2>;
+    case 4: return (const void*)k_rb_brick<4>;
+    case 6: return (const void*)k_rb_brick<6>;
+    case 8: return (const void*)k_rb_brick<8>;
+    default: return (const void*)k_rb_brick<12>;
   }
 }
 
@@ -525,6 +889,75 @@ cudaError_t brick_solve(const BrickPlan& P, const Op7<double>& A, const double* 
   if (e != cudaSuccess) return e;
   void* args[] = {&B};
   return cudaLaunchCooperativeKernel(kernel_of(P), dim3(P.gx * P.gy * P.gz), dim3(kT), args, P.smem, s);
+}
+
+// The same for the red-black iteration: bricks of whole pairs of columns.
+BrickPlan rb_brick_plan(const Lay& L, const Lay& H, int sms) {
+  BrickPlan best;
+  double least = 1e300;
+  sms = std::min(sms, kMaxBlocks);
+  for (int gz = 1; gz <= std::min(sms, L.nz); ++gz)
+    for (int gy = 1; gy <= std::min(sms / gz, L.ny); ++gy)
+      for (int gx = 1; gx <= std::min(sms / gz / gy, H.nx); ++gx) {
+        const int bh = (H.nx + gx - 1) / gx, by = (L.ny + gy - 1) / gy, bz = (L.nz + gz - 1) / gz;
+        const double cost = 2.0 * bh * by * bz + 3.0 * by * bz * (gx > 1) +
+                            2.0 * ((double)bh * bz * (gy > 1) + (double)bh * by * (gz > 1));
+        const int64_t slots = (int64_t)bh * by * bz;
+        if (cost >= least || slots > 12 * kT || rb_brick_bytes(bh, by, bz) > kSmem) continue;
+        BrickPlan P;
+        for (int k : {12, 8, 6, 4, 2})
+          if (slots <= (int64_t)k * kT) P.per_thread = k;
+        P.gx = gx;
+        P.gy = gy;
+        P.gz = gz;
+        P.smem = rb_brick_bytes(bh, by, bz);
+        P.cap = (int)std::min<int64_t>(3 * slots, (int64_t)((kSmem - P.smem) / kRbEntryBytes) / 4 * 4);
+        P.smem += P.cap * kRbEntryBytes;
+        best = P;
+        least = cost;
+      }
+  if (best.gx == 0) return best;
+  int most = 0, dev = 0, coop = 0;
+  const void* k = rb_kernel_of(best.per_thread);
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, k, kT, best.smem) != cudaSuccess ||
+      cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      !coop || most < 1) {
+    cudaGetLastError();
+    return BrickPlan{};
+  }
+  return best;
+}
+
+cudaError_t rb_brick_iterate(const BrickPlan& P, const RbOp& A, const float* phi, float* rh, float* ph, float* zh,
+                             const unsigned short* dinv, void* slots, PcgState* st, double dx, double rho_neg,
+                             double rho_pos, cudaStream_t s) {
+  RbBrickArgs B{};
+  B.L = A.L;
+  B.H = A.Lh;
+  B.gx = P.gx;
+  B.gy = P.gy;
+  B.gz = P.gz;
+  B.ax = A.ax;
+  B.ay = A.ay;
+  B.az = A.az;
+  B.phi = phi;
+  B.extra0 = A.extra0;
+  B.r = rh;
+  B.p = ph;
+  B.z = zh;
+  B.dinv = dinv;
+  B.sums = (double*)slots;
+  B.count = (unsigned*)(B.sums + 4 * kMaxBlocks);
+  B.st = st;
+  const double inv2 = 1.0 / (dx * dx);
+  B.a[1] = (float)((1.0 / rho_neg) * inv2);
+  B.a[2] = (float)((1.0 / rho_pos) * inv2);
+  B.cap = P.cap;
+  cudaError_t e = cudaMemsetAsync(B.count, 0, sizeof(unsigned), s);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&B};
+  return cudaLaunchCooperativeKernel(rb_kernel_of(P.per_thread), dim3(P.gx * P.gy * P.gz), dim3(kT), args, P.smem, s);
 }
 
 }  // namespace fsb

@@ -104,7 +104,7 @@ struct fs_ctx {
   MgState *mgst = nullptr, *mgst_host = nullptr;  // device, pinned
   cudaGraphExec_t mg_graph = nullptr;
   int mg_launches[3] = {0, 0, 0};  // kernels of its start, of one iteration, of its end
-  // resident FP64 pressure solve of small boxes (fs_brick.cu)
+  // resident pressure solve of small boxes (fs_brick.cu): FP64 Jacobi-PCG, or FP32 red-black
   BrickPlan brick;
   void* brick_slots = nullptr;
   PipeGeom pipe{};  // the oil/water pipe's geometry (pipe.on = 0: the box)
@@ -1000,6 +1000,8 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     }
   }
   const bool rb = c->red_black;
+  // one resident kernel between two reliable updates where the box fits the SMs
+  const bool resident = rb && c->fp32 && c->brick.gx > 0;
   build_pressure_operator<S, float>(phi, c->Lc, dx, P.rho_neg, P.rho_pos, (float*)c->pax, (float*)c->pay,
                                     (float*)c->paz, (float*)c->pdiag, c->scalars + 12, deflate(c), s,
                                     (c->lean || rb) ? c->pdinv : nullptr, pipe_of(c));
@@ -1092,7 +1094,18 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     double best = rel;
     for (;;) {
       ++passes;  // each pass runs at least one iteration or ends the solve; this bounds the host loop too
-      if (rb) {
+      if (resident) {
+        CK(rb_brick_iterate(c->brick, R, (const float*)phi, c->rb_r, c->rb_p, c->rb_q, c->rb_dinv, c->brick_slots,
+                            c->st, dx, P.rho_neg, P.rho_pos, s));
+        CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        c->launches += 1;
+        c->pcg_launched_iterations += c->st_host->iter - iters;
+        if (c->st_host->status == PCG_TIMEOUT) {
+          set_error("a block of the resident pressure solve did not answer (iteration %d)", c->st_host->iter);
+          return FS_TIMEOUT;
+        }
+      } else if (rb) {
         CKS(drive_pcg(c, 4,
                       [&] { rb_iteration(R, Ah, c->rb_r, c->rb_p, c->rb_q, c->rb_tau, c->st, c->partials, s); },
                       P.max_iteration, true, 5));
@@ -1896,10 +1909,10 @@ fs_status fs_create(const fs_grid_desc* grid, const fs_params* params, fs_ctx** 
   cg_prepare<float, double>();
   cg_prepare<float, float>();
   if (c->fp32) c->Lh = make_half_lay(c->Lc);
-  if (!c->fp32 && !prm.pipe) {
+  if (!prm.pipe) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) == cudaSuccess)
-      c->brick = brick_plan(c->Lc, sms);
+      c->brick = c->fp32 ? rb_brick_plan(c->Lc, c->Lh, sms) : brick_plan(c->Lc, sms);
   }
   if (c->fp32 && !prm.pipe && mg_prepare() != cudaSuccess) {
     set_error("shared memory of the multigrid cycle: %s", cudaGetErrorString(cudaGetLastError()));

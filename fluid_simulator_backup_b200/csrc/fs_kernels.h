@@ -242,7 +242,7 @@ template <class V, class R = V>
 void pcg_resume(const Op7<V>& A, const R* r, V* p, PcgState* st, double* partials, int restart, cudaStream_t s);
 int pcg_blocks(const Lay& L);
 
-// ---- resident FP64 pressure solve (fs_brick.cu)
+// ---- resident pressure solves of small boxes (fs_brick.cu): FP64 Jacobi-PCG
 struct BrickPlan {
   int gx = 0, gy = 0, gz = 0;  // bricks along each axis; gx = 0: the grid does not fit
   int per_thread = 0;
@@ -258,6 +258,14 @@ size_t brick_slots_bytes();
 cudaError_t brick_solve(const BrickPlan& P, const Op7<double>& A, const double* phi, const double* b, double* x,
                         double* zx, void* slots, PcgState* st, double dx, double rho_neg, double rho_pos,
                         cudaStream_t s);
+
+// The red-black iteration (rb_iteration and its vector updates) from the state
+// that pcg_resume leaves to the next pause or end, in one cooperative launch.
+// zh: a packed vector for the exchanged z.
+BrickPlan rb_brick_plan(const Lay& L, const Lay& H, int sms);
+cudaError_t rb_brick_iterate(const BrickPlan& P, const RbOp& A, const float* phi, float* rh, float* ph, float* zh,
+                             const unsigned short* dinv, void* slots, PcgState* st, double dx, double rho_neg,
+                             double rho_pos, cudaStream_t s);
 
 // ---- multigrid-preconditioned pressure solve (fs_multigrid.cu)
 constexpr int kMgMaxLevels = 14;
