@@ -25,90 +25,105 @@ namespace fsb {
 namespace {
 
 constexpr double kPi = 3.14159265358979323846;
+constexpr int kWenoThreads = 128;  // blocks (32, 2, 2) of the WENO kernels
 
-// ---- WENO5 one side with its gradient w.r.t. the five differences
-__device__ __forceinline__ double weno_side_grad(const double r[5], double eps, double g[5]) {
-  const double c1312 = 13.0 / 12.0;
-  const double t1 = (r[0] - 2.0 * r[1]) + r[2], q1 = (r[0] - 4.0 * r[1]) + 3.0 * r[2];
-  const double t2 = (r[1] - 2.0 * r[2]) + r[3], q2 = r[1] - r[3];
-  const double t3 = (r[2] - 2.0 * r[3]) + r[4], q3 = (3.0 * r[2] - 4.0 * r[3]) + r[4];
-  const double s1 = (c1312 * t1) * t1 + (0.25 * q1) * q1;
-  const double s2 = (c1312 * t2) * t2 + (0.25 * q2) * q2;
-  const double s3 = (c1312 * t3) * t3 + (0.25 * q3) * q3;
-  const double e1 = eps + s1, e2 = eps + s2, e3 = eps + s3;
-  const double qq1 = e1 * e1, qq2 = e2 * e2, qq3 = e3 * e3;
+// ---- WENO5 one side.  The terms that the derivative and its gradient share.
+// These kernels are bound by the latency and number of FP64 instructions (two
+// warps' worth per SM and cycle), so divisions by 3 are products with 1/3, the
+// gradient's three divisions by eps + IS_k are one reciprocal, samples are read
+// again (from L1) for the gradient instead of held over it, and the registers
+// are bounded to keep 20 warps per SM.  Measured at 96^3, FP32 states: a
+// Sussman step's adjoint 195 -> 66 us (230 registers, 8 warps per SM before), a
+// MAC component's 174 -> 60 us.
+struct WenoSide {
+  double t1, q1, t2, q2, t3, q3, e1, e2, e3, w1, w2, w3, u1, u2, u3;
+};
+__device__ __forceinline__ WenoSide weno_terms(const double r[5], double eps) {
+  const double c1312 = 13.0 / 12.0, third = 1.0 / 3.0;
+  WenoSide W;
+  W.t1 = (r[0] - 2.0 * r[1]) + r[2], W.q1 = (r[0] - 4.0 * r[1]) + 3.0 * r[2];
+  W.t2 = (r[1] - 2.0 * r[2]) + r[3], W.q2 = r[1] - r[3];
+  W.t3 = (r[2] - 2.0 * r[3]) + r[4], W.q3 = (3.0 * r[2] - 4.0 * r[3]) + r[4];
+  W.e1 = eps + ((c1312 * W.t1) * W.t1 + (0.25 * W.q1) * W.q1);
+  W.e2 = eps + ((c1312 * W.t2) * W.t2 + (0.25 * W.q2) * W.q2);
+  W.e3 = eps + ((c1312 * W.t3) * W.t3 + (0.25 * W.q3) * W.q3);
+  const double qq1 = W.e1 * W.e1, qq2 = W.e2 * W.e2, qq3 = W.e3 * W.e3;
   const double b1 = 0.1 * (qq2 * qq3), b2 = 0.6 * (qq1 * qq3), b3 = 0.3 * (qq1 * qq2);
   const double inv = 1.0 / ((b1 + b2) + b3);
-  const double w1 = b1 * inv, w2 = b2 * inv, w3 = b3 * inv;
-  const double u1 = (r[0] / 3.0 - r[1] * (7.0 / 6.0)) + r[2] * (11.0 / 6.0);
-  const double u2 = (r[1] * (-1.0 / 6.0) + r[2] * (5.0 / 6.0)) + r[3] / 3.0;
-  const double u3 = (r[2] / 3.0 + r[3] * (5.0 / 6.0)) - r[4] / 6.0;
-  const double D = (w1 * u1 + w2 * u2) + w3 * u3;
+  W.w1 = b1 * inv, W.w2 = b2 * inv, W.w3 = b3 * inv;
+  W.u1 = (r[0] * third - r[1] * (7.0 / 6.0)) + r[2] * (11.0 / 6.0);
+  W.u2 = (r[1] * (-1.0 / 6.0) + r[2] * (5.0 / 6.0)) + r[3] * third;
+  W.u3 = (r[2] * third + r[3] * (5.0 / 6.0)) - r[4] * (1.0 / 6.0);
+  return W;
+}
+__device__ __forceinline__ double weno_value(const WenoSide& W) { return (W.w1 * W.u1 + W.w2 * W.u2) + W.w3 * W.u3; }
+__device__ __forceinline__ double weno_side(const double r[5], double eps) { return weno_value(weno_terms(r, eps)); }
+
+// with its gradient w.r.t. the five differences
+__device__ __forceinline__ double weno_side_grad(const double r[5], double eps, double g[5]) {
+  const WenoSide W = weno_terms(r, eps);
+  const double D = weno_value(W), third = 1.0 / 3.0;
   // direct part: sum_k w_k du_k/dr
-  g[0] = w1 / 3.0;
-  g[1] = -w1 * (7.0 / 6.0) - w2 / 6.0;
-  g[2] = w1 * (11.0 / 6.0) + w2 * (5.0 / 6.0) + w3 / 3.0;
-  g[3] = w2 / 3.0 + w3 * (5.0 / 6.0);
-  g[4] = -w3 / 6.0;
+  g[0] = W.w1 * third;
+  g[1] = -W.w1 * (7.0 / 6.0) - W.w2 * (1.0 / 6.0);
+  g[2] = W.w1 * (11.0 / 6.0) + W.w2 * (5.0 / 6.0) + W.w3 * third;
+  g[3] = W.w2 * third + W.w3 * (5.0 / 6.0);
+  g[4] = -W.w3 * (1.0 / 6.0);
   // weights part: -2 w_k (u_k - D)/(eps + IS_k) * dIS_k/dr
-  const double k1 = -2.0 * w1 * (u1 - D) / e1, k2 = -2.0 * w2 * (u2 - D) / e2, k3 = -2.0 * w3 * (u3 - D) / e3;
+  const double e12 = W.e1 * W.e2, inv = -2.0 / (e12 * W.e3);
+  const double k1 = W.w1 * (W.u1 - D) * (inv * (W.e2 * W.e3)), k2 = W.w2 * (W.u2 - D) * (inv * (W.e1 * W.e3)),
+               k3 = W.w3 * (W.u3 - D) * (inv * e12);
   // dIS1/dr = 13/6 t1 (1,-2,1) + 1/2 q1 (1,-4,3)
-  const double a1 = (13.0 / 6.0) * t1, h1 = 0.5 * q1;
+  const double a1 = (13.0 / 6.0) * W.t1, h1 = 0.5 * W.q1;
   g[0] += k1 * (a1 + h1);
   g[1] += k1 * (-2.0 * a1 - 4.0 * h1);
   g[2] += k1 * (a1 + 3.0 * h1);
   // dIS2/dr = 13/6 t2 (0,1,-2,1) + 1/2 q2 (0,1,0,-1)
-  const double a2 = (13.0 / 6.0) * t2, h2 = 0.5 * q2;
+  const double a2 = (13.0 / 6.0) * W.t2, h2 = 0.5 * W.q2;
   g[1] += k2 * (a2 + h2);
   g[2] += k2 * (-2.0 * a2);
   g[3] += k2 * (a2 - h2);
   // dIS3/dr = 13/6 t3 (0,0,1,-2,1) + 1/2 q3 (0,0,3,-4,1)
-  const double a3 = (13.0 / 6.0) * t3, h3 = 0.5 * q3;
+  const double a3 = (13.0 / 6.0) * W.t3, h3 = 0.5 * W.q3;
   g[2] += k3 * (a3 + 3.0 * h3);
   g[3] += k3 * (-2.0 * a3 - 4.0 * h3);
   g[4] += k3 * (a3 + h3);
   return D;
 }
 
-// Bars of the seven samples f[-3..3] (fb[0..6]) of D- (side 0) or D+ (side 1)
-// scaled by m.  d_k = inv_h (f[k-3] - f[k-4]), k = 1..6.
-__device__ __forceinline__ void weno_pair_bar(const double f[7], double inv_h, double eps, int side, double m,
-                                              double fb[7]) {
-  double d[7];
-  for (int k = 1; k <= 6; ++k) d[k] = inv_h * (f[k] - f[k - 1]);  // samples stored at s + 3
-  double r[5], g[5], db[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (side == 0) {
-    r[0] = d[1]; r[1] = d[2]; r[2] = d[3]; r[3] = d[4]; r[4] = d[5];
-    weno_side_grad(r, eps, g);
-    for (int q = 0; q < 5; ++q) db[q + 1] = m * g[q];
-  } else {
-    r[0] = d[6]; r[1] = d[5]; r[2] = d[4]; r[3] = d[3]; r[4] = d[2];
-    weno_side_grad(r, eps, g);
-    for (int q = 0; q < 5; ++q) db[6 - q] = m * g[q];
-  }
-  for (int s = 0; s < 7; ++s) fb[s] = 0.0;
-  for (int k = 1; k <= 6; ++k) {
-    // d_k = inv_h (f[k] - f[k-1]) in 0-based sample storage
-    fb[k] += inv_h * db[k];
-    fb[k - 1] -= inv_h * db[k];
-  }
-}
-
+// D- (side 0) or D+ (side 1) along one axis and its gradient.  D+ is D- of the
+// mirrored stencil: seen along the step st' = +-st, both read the six samples
+// f[c + m st'], m = -3 .. 2, with differences r_q = h' (f(q - 2) - f(q - 3)),
+// h' = +-1/h.
+struct Upwind {
+  int64_t c, st;
+  double h, g[5];
+};
 template <class T>
-__device__ __forceinline__ void load7(const T* f, int64_t c, int64_t st, double out[7]) {
+__device__ __forceinline__ double upwind_grad(const T* __restrict__ f, int64_t c, int64_t st, int side, double inv_h,
+                                              double eps, Upwind& U) {
+  U.c = c;
+  U.st = side ? -st : st;
+  U.h = side ? -inv_h : inv_h;
+  double r[5], lo = f[c - 3 * U.st];
 #pragma unroll
-  for (int s = 0; s < 7; ++s) out[s] = f[c + (s - 3) * st];
+  for (int q = 0; q < 5; ++q) {
+    const double hi = f[c + (q - 2) * U.st];
+    r[q] = U.h * (hi - lo);
+    lo = hi;
+  }
+  return weno_side_grad(r, eps, U.g);
 }
-
-// scatter stencil bars; with `lo`/`n` given, samples whose coordinate along
-// the axis falls outside [0, n) are dropped (zero-ghost fields)
-__device__ __forceinline__ void scatter7(double* fb_arr, int64_t c, int64_t st, const double fb[7], int e, int n,
-                                         bool drop_ghosts) {
+// adds m dD/df to the samples' bars.  e: the cell's place along the axis; with
+// drop_ghosts, samples outside [0, n) get nothing (zero-ghost fields).
+__device__ __forceinline__ void upwind_scatter(const Upwind& U, double m, double* bar, int e, int n, bool drop_ghosts) {
+  const int dir = U.st > 0 ? 1 : -1;
+  const double mh = m * U.h;
 #pragma unroll
-  for (int s = 0; s < 7; ++s) {
-    if (fb[s] == 0.0) continue;
-    if (drop_ghosts && (e + s - 3 < 0 || e + s - 3 >= n)) continue;
-    atomicAdd(&fb_arr[c + (s - 3) * st], fb[s]);
+  for (int s = -3; s <= 2; ++s) {
+    const double b = (s > -3 ? mh * U.g[s + 2] : 0.0) - (s < 2 ? mh * U.g[s + 3] : 0.0);
+    if (b == 0.0 || (drop_ghosts && (unsigned)(e + s * dir) >= (unsigned)n)) continue;
+    atomicAdd(bar + U.c + s * U.st, b);
   }
 }
 
@@ -129,7 +144,7 @@ __device__ __forceinline__ double heaviside_d(double phi, double e) {
 // (the RK base term is handled by the caller).  fe_bar = c1 * out_bar.
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void k_adj_weno_levelset(const T* __restrict__ src, const T* __restrict__ u,
+__global__ void __launch_bounds__(kWenoThreads, 5) k_adj_weno_levelset(const T* __restrict__ src, const T* __restrict__ u,
                                     const T* __restrict__ v, const T* __restrict__ w,
                                     const double* __restrict__ out_bar, double* src_bar, double* u_bar,
                                     double* v_bar, double* w_bar, Lay L, Lay Lu, Lay Lv, Lay Lw, double inv_h,
@@ -146,23 +161,15 @@ __global__ void k_adj_weno_levelset(const T* __restrict__ src, const T* __restri
   const int64_t st[3] = {1, L.px, L.slab};
   double* vb[3] = {u_bar, v_bar, w_bar};
   const Lay* lv[3] = {&Lu, &Lv, &Lw};
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    double f[7], sb[7];
-    load7(src, c, st[a], f);
-    const int side = vel[a] > 0.0 ? 0 : 1;
-    // D of the selected side, for the velocity bar
-    double d[7];
-    for (int q = 1; q <= 6; ++q) d[q] = inv_h * (f[q] - f[q - 1]);
-    double r[5], g[5];
-    if (side == 0) { r[0] = d[1]; r[1] = d[2]; r[2] = d[3]; r[3] = d[4]; r[4] = d[5]; }
-    else { r[0] = d[6]; r[1] = d[5]; r[2] = d[4]; r[3] = d[3]; r[4] = d[2]; }
-    const double D = weno_side_grad(r, eps, g);
+    Upwind U;
+    const double D = upwind_grad(src, c, st[a], vel[a] > 0.0 ? 0 : 1, inv_h, eps, U);
     const double velb = -dt * D * fb;
     const int ia = a == 0, ja = a == 1, ka = a == 2;
     atomicAdd(&vb[a][lv[a]->at(i + ia, j + ja, k + ka)], 0.5 * velb);
     atomicAdd(&vb[a][lv[a]->at(i, j, k)], 0.5 * velb);
-    weno_pair_bar(f, inv_h, eps, side, -dt * vel[a] * fb, sb);
-    scatter7(src_bar, c, st[a], sb, 0, 0, false);
+    upwind_scatter(U, -dt * vel[a] * fb, src_bar, 0, 0, false);
   }
 }
 
@@ -228,7 +235,7 @@ __global__ void k_adj_extrap(double* bar, Lay L) {
 // MAC component WENO5 self-advection: out = comp - dt (uvel D_x + ...)
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void k_adj_weno_mac(const T* __restrict__ comp, const T* __restrict__ u,
+__global__ void __launch_bounds__(kWenoThreads, 5) k_adj_weno_mac(const T* __restrict__ comp, const T* __restrict__ u,
                                const T* __restrict__ v, const T* __restrict__ w,
                                const double* __restrict__ out_bar, double* comp_bar, double* u_bar, double* v_bar,
                                double* w_bar, Lay Lc, Lay Lu, Lay Lv, Lay Lw, int axis, double inv_h, double eps,
@@ -245,6 +252,7 @@ __global__ void k_adj_weno_mac(const T* __restrict__ comp, const T* __restrict__
   const int e[3] = {i, j, k};
   const int n[3] = {Lc.nx, Lc.ny, Lc.nz};
   const int64_t st[3] = {1, Lc.px, Lc.slab};
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
     // velocity component d at this face of component `axis`
     int fi[4], fj[4], fk[4], nf;
@@ -271,23 +279,15 @@ __global__ void k_adj_weno_mac(const T* __restrict__ comp, const T* __restrict__
              comps[d][Ld.at(fi[3], fj[3], fk[3])]) *
             0.25;
     }
-    double f[7], sb[7];
-    load7(comp, c, st[d], f);
-    const int side = vel > 0.0 ? 0 : 1;
-    double dd[7];
-    for (int q = 1; q <= 6; ++q) dd[q] = inv_h * (f[q] - f[q - 1]);
-    double r[5], g[5];
-    if (side == 0) { r[0] = dd[1]; r[1] = dd[2]; r[2] = dd[3]; r[3] = dd[4]; r[4] = dd[5]; }
-    else { r[0] = dd[6]; r[1] = dd[5]; r[2] = dd[4]; r[3] = dd[3]; r[4] = dd[2]; }
-    const double D = weno_side_grad(r, eps, g);
+    Upwind U;
+    const double D = upwind_grad(comp, c, st[d], vel > 0.0 ? 0 : 1, inv_h, eps, U);
     const double velb = -dt * D * ob * (nf == 1 ? 1.0 : 0.25);
     for (int q = 0; q < nf; ++q) {
       // faces outside the face grid of component d are zero ghosts
       if (fi[q] < 0 || fj[q] < 0 || fk[q] < 0 || fi[q] >= Ld.nx || fj[q] >= Ld.ny || fk[q] >= Ld.nz) continue;
       atomicAdd(&bars[d][Ld.at(fi[q], fj[q], fk[q])], velb);
     }
-    weno_pair_bar(f, inv_h, eps, side, -dt * vel * ob, sb);
-    scatter7(comp_bar, c, st[d], sb, e[d], n[d], true);
+    upwind_scatter(U, -dt * vel * ob, comp_bar, e[d], n[d], true);
   }
 }
 
@@ -309,7 +309,7 @@ __device__ __forceinline__ double godunov_sel(double s, double dm, double dp, in
 }
 
 template <class T>
-__global__ void k_adj_sussman(const T* __restrict__ src, const T* __restrict__ sgn,
+__global__ void __launch_bounds__(kWenoThreads, 5) k_adj_sussman(const T* __restrict__ src, const T* __restrict__ sgn,
                               const double* __restrict__ out_bar, double* src_bar, double* sgn_bar, Lay L,
                               double inv_h, double eps, double dtau, double c1, int typo) {
   FS_IJK(L);
@@ -317,15 +317,20 @@ __global__ void k_adj_sussman(const T* __restrict__ src, const T* __restrict__ s
   const double rb = c1 * out_bar[c];
   if (rb == 0.0) return;
   const int64_t st[3] = {1, L.px, L.slab};
-  double f[3][7], dm[3], dp[3];
+  double dm[3], dp[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    load7(src, c, st[a], f[a]);
-    double d[7], r[5], g[5];
-    for (int q = 1; q <= 6; ++q) d[q] = inv_h * (f[a][q] - f[a][q - 1]);
-    r[0] = d[1]; r[1] = d[2]; r[2] = d[3]; r[3] = d[4]; r[4] = d[5];
-    dm[a] = weno_side_grad(r, eps, g);
-    r[0] = d[6]; r[1] = d[5]; r[2] = d[4]; r[3] = d[3]; r[4] = d[2];
-    dp[a] = weno_side_grad(r, eps, g);
+    double d[6], r[5], lo = src[c - 3 * st[a]];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const double hi = src[c + (q - 2) * st[a]];
+      d[q] = inv_h * (hi - lo);
+      lo = hi;
+    }
+    dm[a] = weno_side(d, eps);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) r[q] = d[5 - q];
+    dp[a] = weno_side(r, eps);
   }
   const double s = sgn[c];
   int code[3];
@@ -352,11 +357,12 @@ __global__ void k_adj_sussman(const T* __restrict__ src, const T* __restrict__ s
     const double inv = 1.0 / sqrt(G);
     for (int a = 0; a < 3; ++a) gb[a] = mb * gsel[a] * inv;
   }
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
     if (code[a] == 2 || gb[a] == 0.0) continue;
-    double sb[7];
-    weno_pair_bar(f[a], inv_h, eps, code[a], gb[a], sb);
-    scatter7(src_bar, c, st[a], sb, 0, 0, false);
+    Upwind U;
+    upwind_grad(src, c, st[a], code[a], inv_h, eps, U);
+    upwind_scatter(U, gb[a], src_bar, 0, 0, false);
   }
 }
 
@@ -565,34 +571,70 @@ struct PhiXD {  // the forward kernel's one-layer extrapolated phi, with its tra
 };
 }  // namespace
 
-template <class T>
-__global__ void k_adj_visc(const T* __restrict__ phi, const T* __restrict__ ug, const T* __restrict__ vg,
-                           const T* __restrict__ wg, const T* __restrict__ x, const double* __restrict__ lam,
-                           double* u_bar, double* v_bar, double* w_bar, double* phi_bar, double* rho_bar, Lay Lc,
-                           Lay Lu, Lay Lv, Lay Lw, Lay Lf, int axis, double inv_h, double dt, double rn, double rp,
-                           double mn, double mp) {
+// One face of the component along `axis` per thread.  Ten samples of phi decide
+// all its coefficients: the two cells of the face and their neighbours along
+// the two tangential axes.  They are read once, their bars summed in
+// registers and scattered once; where all ten lie on one side of the
+// interface band the coefficients are constant and phi gets nothing.  (Bound by
+// the latency of the faces at the interface, whose warps are the last to finish: at
+// 96^3, per component, 329 us where every term read and scattered its own
+// samples through local arrays, 106 us so.)
+template <class T, int AXIS>
+__global__ void __launch_bounds__(128, 4) k_adj_visc(const T* __restrict__ phi, const T* __restrict__ ug,
+                                                     const T* __restrict__ vg, const T* __restrict__ wg,
+                                                     const T* __restrict__ x, const double* __restrict__ lam,
+                                                     double* u_bar, double* v_bar, double* w_bar, double* phi_bar,
+                                                     double* rho_bar, Lay Lc, Lay Lu, Lay Lv, Lay Lw, Lay Lf,
+                                                     double inv_h, double dt, double rn, double rp, double mn,
+                                                     double mp) {
   double rbn = 0.0, rbp = 0.0;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
-  const int e_ax = axis == 0 ? i : (axis == 1 ? j : k);
-  const int n_ax = axis == 0 ? Lf.nx : (axis == 1 ? Lf.ny : Lf.nz);
-  if (i < Lf.nx && j < Lf.ny && k < Lf.nz && !(e_ax == 0 || e_ax == n_ax - 1)) {
+  constexpr int T1 = AXIS == 0 ? 1 : 0, T2 = AXIS == 2 ? 1 : 2;  // the tangential axes
+  const int at[3] = {i, j, k}, nf[3] = {Lf.nx, Lf.ny, Lf.nz};
+  if (i < Lf.nx && j < Lf.ny && k < Lf.nz && at[AXIS] > 0 && at[AXIS] < nf[AXIS] - 1) {
     const int64_t f = Lf.at(i, j, k);
     const PhiXD<T> P{phi, Lc};
     const double e = 1.5 / inv_h, inv2 = inv_h * inv_h;
-    const int ea[3] = {axis == 0, axis == 1, axis == 2};
-    const int li = i - ea[0], lj = j - ea[1], lk = k - ea[2];
+    const int li = i - (AXIS == 0), lj = j - (AXIS == 1), lk = k - (AXIS == 2);
     const double lamf = lam[f], xf = x[f];
     const T* comp[3] = {ug, vg, wg};
     double* cbar[3] = {u_bar, v_bar, w_bar};
-    const Lay lay[3] = {Lu, Lv, Lw};
+    const Lay* lay[3] = {&Lu, &Lv, &Lw};
+    const int64_t cst[3] = {1, Lc.px, Lc.slab}, fst[3] = {1, Lf.px, Lf.slab};
+    // samples: lo, hi, then per tangential axis lo-, hi-, lo+, hi+
+    const int nc[3] = {Lc.nx, Lc.ny, Lc.nz};
+    const bool inside = at[T1] > 0 && at[T1] < nc[T1] - 1 && at[T2] > 0 && at[T2] < nc[T2] - 1;
+    const int64_t hi = Lc.at(i, j, k), lo = Lc.at(li, lj, lk);
+    double v[10], vb[10];
+    v[0] = phi[lo];
+    v[1] = phi[hi];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int d = t ? T2 : T1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = q & 2 ? 1 : -1;
+        v[2 + 4 * t + q] = inside ? (double)phi[(q & 1 ? hi : lo) + o * cst[d]]
+                                  : P.at((q & 1 ? i : li) + (d == 0) * o, (q & 1 ? j : lj) + (d == 1) * o,
+                                         (q & 1 ? k : lk) + (d == 2) * o);
+      }
+    }
+    bool above = true, below = true;  // false for NaN
+#pragma unroll
+    for (int q = 0; q < 10; ++q) {
+      above = above && v[q] > e;
+      below = below && v[q] < -e;
+      vb[q] = 0.0;
+    }
+    const bool uniform = above || below;
     // rho_f and its dependence
-    const double mrho = 0.5 * (P.at(li, lj, lk) + P.at(i, j, k));
-    const double H = heaviside(mrho, e), dH = heaviside_d(mrho, e);
+    const double mrho = 0.5 * (v[0] + v[1]);
+    const double H = above ? 1.0 : (below ? 0.0 : heaviside(mrho, e));
     const double rho_f = rn + (rp - rn) * H;
-    // u_bar[a] += rho_f lambda
-    atomicAdd(&cbar[axis][f], rho_f * lamf);
+    // u_bar[a] += rho_f lambda (the other faces' threads add to the other components only)
+    cbar[AXIS][f] += rho_f * lamf;
     // The rho_f bar is lambda (u_f - x_f), the viscous change of the face
     // velocity.  It is formed as (K x - E)/rho_f (K the viscous part of the
     // matrix, E the explicit transpose terms: rho_f (u - x) = K x - E for the
@@ -601,95 +643,91 @@ __global__ void k_adj_visc(const T* __restrict__ phi, const T* __restrict__ ug, 
     // a few digits when the viscous change is small.
     double Kx = 0.0, Ex = 0.0;
     // arms
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const int di = d == 0, dj = d == 1, dk = d == 2;
-      const double kk = d == axis ? 2.0 : 1.0;
-      const double K = kk * dt * inv2;
-      // the samples each mu averages, and the average
-      int lo_i[4], lo_j[4], lo_k[4], hi_i[4], hi_j[4], hi_k[4], ns;
-      if (d == axis) {
-        ns = 1;
-        lo_i[0] = li; lo_j[0] = lj; lo_k[0] = lk;
-        hi_i[0] = i; hi_j[0] = j; hi_k[0] = k;
-      } else {
-        ns = 4;
-        lo_i[0] = li - di; lo_j[0] = lj - dj; lo_k[0] = lk - dk;
-        lo_i[1] = li; lo_j[1] = lj; lo_k[1] = lk;
-        lo_i[2] = i - di; lo_j[2] = j - dj; lo_k[2] = k - dk;
-        lo_i[3] = i; lo_j[3] = j; lo_k[3] = k;
-        hi_i[0] = li; hi_j[0] = lj; hi_k[0] = lk;
-        hi_i[1] = li + di; hi_j[1] = lj + dj; hi_k[1] = lk + dk;
-        hi_i[2] = i; hi_j[2] = j; hi_k[2] = k;
-        hi_i[3] = i + di; hi_j[3] = j + dj; hi_k[3] = k + dk;
+      const int s0 = d == T1 ? 2 : 6;  // the samples of a tangential axis
+      const double K = (d == AXIS ? 2.0 : 1.0) * dt * inv2;
+      // mu_low[d] and mu_high[d] at the average of the samples around them
+      double mlo = v[0], mhi = v[1];
+      if (d != AXIS) {
+        mlo = 0.25 * (((v[s0] + v[0]) + v[s0 + 1]) + v[1]);
+        mhi = 0.25 * (((v[0] + v[s0 + 2]) + v[1]) + v[s0 + 3]);
       }
-      const double wgt = ns == 1 ? 1.0 : 0.25;
-      double mlo, mhi;
-      if (ns == 1) {
-        mlo = P.at(lo_i[0], lo_j[0], lo_k[0]);
-        mhi = P.at(hi_i[0], hi_j[0], hi_k[0]);
-      } else {
-        mlo = 0.25 * (((P.at(lo_i[0], lo_j[0], lo_k[0]) + P.at(lo_i[1], lo_j[1], lo_k[1])) + P.at(lo_i[2], lo_j[2], lo_k[2])) +
-                      P.at(lo_i[3], lo_j[3], lo_k[3]));
-        mhi = 0.25 * (((P.at(hi_i[0], hi_j[0], hi_k[0]) + P.at(hi_i[1], hi_j[1], hi_k[1])) + P.at(hi_i[2], hi_j[2], hi_k[2])) +
-                      P.at(hi_i[3], hi_j[3], hi_k[3]));
-      }
-      const double dmu_lo = (mp - mn) * heaviside_d(mlo, e), dmu_hi = (mp - mn) * heaviside_d(mhi, e);
-      const double mu_lo_d = mn + (mp - mn) * heaviside(mlo, e), mu_hi_d = mn + (mp - mn) * heaviside(mhi, e);
-      double glo = 0.0, ghi = 0.0;  // bars of mu_low[d], mu_high[d]
+      const double mu_lo = mn + (mp - mn) * (uniform ? H : heaviside(mlo, e));
+      const double mu_hi = mn + (mp - mn) * (uniform ? H : heaviside(mhi, e));
+      double glo = 0.0, ghi = 0.0;  // their bars
       // matrix, low arm: neighbour f - e_d (zero if it is a wall face or beyond)
       {
-        const int ni = i - di, nj = j - dj, nk = k - dk;
-        const int en = d == 0 ? ni : (d == 1 ? nj : nk);
-        const bool nb_wall = (d == axis && (en == 0)) || en < 0;
-        const double xn = nb_wall ? 0.0 : x[Lf.at(ni, nj, nk)];
-        const double ln = nb_wall ? 0.0 : lam[Lf.at(ni, nj, nk)];
+        const bool in = at[d] > (d == AXIS ? 1 : 0);
+        const double xn = in ? (double)x[f - fst[d]] : 0.0, ln = in ? lam[f - fst[d]] : 0.0;
         glo -= K * (lamf - ln) * (xf - xn);
-        Kx += K * mu_lo_d * (xf - xn);
+        Kx += K * mu_lo * (xf - xn);
       }
       // matrix, high arm: only when the neighbour row does not own it (wall or beyond)
       {
-        const int ni = i + di, nj = j + dj, nk = k + dk;
-        const int en = d == 0 ? ni : (d == 1 ? nj : nk);
-        const int nn = d == 0 ? Lf.nx : (d == 1 ? Lf.ny : Lf.nz);
-        const bool nb_wall = (d == axis && en == nn - 1) || en >= nn;
-        if (nb_wall) ghi -= K * lamf * xf;
-        const double xn = nb_wall ? 0.0 : x[Lf.at(ni, nj, nk)];
-        Kx += K * mu_hi_d * (xf - xn);
+        const bool in = at[d] + 1 < nf[d] - (d == AXIS ? 1 : 0);
+        if (!in) ghi -= K * lamf * xf;
+        const double xn = in ? (double)x[f + fst[d]] : 0.0;
+        Kx += K * mu_hi * (xf - xn);
       }
-      // right-hand side: explicit transpose terms for tangential d
-      if (d != axis) {
-        const T* vt = comp[d];
-        const Lay& Lt = lay[d];
-        const int ti = di, tj = dj, tk = dk;
-        const int64_t ia = Lt.at(i + ti, j + tj, k + tk), ib = Lt.at(i + ti - ea[0], j + tj - ea[1], k + tk - ea[2]);
-        const int64_t ja = Lt.at(i, j, k), jb = Lt.at(i - ea[0], j - ea[1], k - ea[2]);
-        const double hi_d = vt[ia] - vt[ib], lo_d = vt[ja] - vt[jb];
+      // right-hand side: explicit transpose terms for tangential d, and their
+      // transpose to that component (all four faces exist: it has one face
+      // more along d, and both cells of this face lie in the box)
+      if (d != AXIS) {
+        const Lay& Lt = *lay[d];
+        const int64_t tst[3] = {1, Lt.px, Lt.slab};
+        const int64_t ja = Lt.at(i, j, k), jb = ja - tst[AXIS], ia = ja + tst[d], ib = jb + tst[d];
+        const double hi_d = comp[d][ia] - comp[d][ib], lo_d = comp[d][ja] - comp[d][jb];
         ghi += lamf * dt * inv2 * hi_d;
         glo -= lamf * dt * inv2 * lo_d;
-        Ex += dt * inv2 * (mu_hi_d * hi_d - mu_lo_d * lo_d);
-        // transpose to the tangential component (its ghosts are zero constants)
-        // mu values of the forward
-        const double ch = lamf * dt * inv2 * mu_hi_d, cl = lamf * dt * inv2 * mu_lo_d;
-        auto inside = [&](int a, int b, int q) { return a >= 0 && b >= 0 && q >= 0 && a < Lt.nx && b < Lt.ny && q < Lt.nz; };
-        if (inside(i + ti, j + tj, k + tk)) atomicAdd(&cbar[d][ia], ch);
-        if (inside(i + ti - ea[0], j + tj - ea[1], k + tk - ea[2])) atomicAdd(&cbar[d][ib], -ch);
-        if (inside(i, j, k)) atomicAdd(&cbar[d][ja], -cl);
-        if (inside(i - ea[0], j - ea[1], k - ea[2])) atomicAdd(&cbar[d][jb], cl);
+        Ex += dt * inv2 * (mu_hi * hi_d - mu_lo * lo_d);
+        const double ch = lamf * dt * inv2 * mu_hi, cl = lamf * dt * inv2 * mu_lo;
+        atomicAdd(&cbar[d][ia], ch);
+        atomicAdd(&cbar[d][ib], -ch);
+        atomicAdd(&cbar[d][ja], -cl);
+        atomicAdd(&cbar[d][jb], cl);
       }
       // phi bars through the Heaviside of the averaged samples
-      const double plo = glo * dmu_lo * wgt, phi_hi = ghi * dmu_hi * wgt;
-      for (int q = 0; q < ns; ++q) {
-        P.scatter(phi_bar, lo_i[q], lo_j[q], lo_k[q], plo);
-        P.scatter(phi_bar, hi_i[q], hi_j[q], hi_k[q], phi_hi);
+      if (!uniform) {
+        const double dlo = glo * ((mp - mn) * heaviside_d(mlo, e)), dhi = ghi * ((mp - mn) * heaviside_d(mhi, e));
+        if (d == AXIS) {
+          vb[0] += dlo;
+          vb[1] += dhi;
+        } else {
+          vb[0] += 0.25 * (dlo + dhi);
+          vb[1] += 0.25 * (dlo + dhi);
+          vb[s0] += 0.25 * dlo;
+          vb[s0 + 1] += 0.25 * dlo;
+          vb[s0 + 2] += 0.25 * dhi;
+          vb[s0 + 3] += 0.25 * dhi;
+        }
       }
     }
     // rho_f bar: lambda (u_f - x_f) = lambda (K x - E)_f / rho_f
     const double rfb = lamf * (Kx - Ex) / rho_f;
-    rbn += rfb * (1.0 - H);
-    rbp += rfb * H;
-    const double pb_rho = rfb * (rp - rn) * dH * 0.5;
-    P.scatter(phi_bar, li, lj, lk, pb_rho);
-    P.scatter(phi_bar, i, j, k, pb_rho);
+    rbn = rfb * (1.0 - H);
+    rbp = rfb * H;
+    if (!uniform) {
+      const double pb_rho = rfb * (rp - rn) * heaviside_d(mrho, e) * 0.5;
+      vb[0] += pb_rho;
+      vb[1] += pb_rho;
+      if (vb[0] != 0.0) atomicAdd(&phi_bar[lo], vb[0]);
+      if (vb[1] != 0.0) atomicAdd(&phi_bar[hi], vb[1]);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int d = t ? T2 : T1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int o = q & 2 ? 1 : -1;
+          const double b = vb[2 + 4 * t + q];
+          if (!inside)
+            P.scatter(phi_bar, (q & 1 ? i : li) + (d == 0) * o, (q & 1 ? j : lj) + (d == 1) * o,
+                      (q & 1 ? k : lk) + (d == 2) * o, b);
+          else if (b != 0.0)
+            atomicAdd(&phi_bar[(q & 1 ? hi : lo) + o * cst[d]], b);
+        }
+      }
+    }
   }
   rbn = block_sum(rbn);
   __syncthreads();
@@ -723,7 +761,7 @@ template <class T>
 void adj_weno_levelset(const T* src, const T* u, const T* v, const T* w, const double* out_bar, double* src_bar,
                        double* u_bar, double* v_bar, double* w_bar, const Lay& L, const Lay& Lu, const Lay& Lv,
                        const Lay& Lw, double dx, double eps, double dt, double c1, cudaStream_t s) {
-  Launch3 g = launch3(L.nx, L.ny, L.nz, 32, 4, 2);
+  Launch3 g = launch3(L.nx, L.ny, L.nz, 32, 2, 2);
   k_adj_weno_levelset<T><<<g.grid, g.block, 0, s>>>(src, u, v, w, out_bar, src_bar, u_bar, v_bar, w_bar, L, Lu, Lv,
                                                     Lw, 1.0 / dx, eps, dt, c1);
 }
@@ -738,7 +776,7 @@ template <class T>
 void adj_weno_mac(const T* comp, const T* u, const T* v, const T* w, const double* out_bar, double* comp_bar,
                   double* u_bar, double* v_bar, double* w_bar, const Lay& Lc, const Lay& Lu, const Lay& Lv,
                   const Lay& Lw, int axis, double dx, double eps, double dt, cudaStream_t s) {
-  Launch3 g = launch3(Lc.nx, Lc.ny, Lc.nz, 32, 4, 2);
+  Launch3 g = launch3(Lc.nx, Lc.ny, Lc.nz, 32, 2, 2);
   k_adj_weno_mac<T><<<g.grid, g.block, 0, s>>>(comp, u, v, w, out_bar, comp_bar, u_bar, v_bar, w_bar, Lc, Lu, Lv, Lw,
                                                axis, 1.0 / dx, eps, dt);
 }
@@ -746,7 +784,7 @@ void adj_weno_mac(const T* comp, const T* u, const T* v, const T* w, const doubl
 template <class T>
 void adj_sussman(const T* src, const T* sgn, const double* out_bar, double* src_bar, double* sgn_bar, const Lay& L,
                  double dx, double eps, double dtau, double c1, int typo, cudaStream_t s) {
-  Launch3 g = launch3(L.nx, L.ny, L.nz, 32, 4, 2);
+  Launch3 g = launch3(L.nx, L.ny, L.nz, 32, 2, 2);
   k_adj_sussman<T><<<g.grid, g.block, 0, s>>>(src, sgn, out_bar, src_bar, sgn_bar, L, 1.0 / dx, eps, dtau, c1, typo);
 }
 
@@ -790,9 +828,10 @@ void adj_visc(const T* phi, const T* ug, const T* vg, const T* wg, const T* x, c
               const Lay& Lv, const Lay& Lw, int axis, double dx, double dt, double rn, double rp, double mn,
               double mp, cudaStream_t s) {
   const Lay& Lf = axis == 0 ? Lu : (axis == 1 ? Lv : Lw);
-  Launch3 g = launch3(Lf.nx, Lf.ny, Lf.nz);
-  k_adj_visc<T><<<g.grid, g.block, 0, s>>>(phi, ug, vg, wg, x, lam, u_bar, v_bar, w_bar, phi_bar, rho_bar, Lc, Lu, Lv,
-                                           Lw, Lf, axis, 1.0 / dx, dt, rn, rp, mn, mp);
+  Launch3 g = launch3(Lf.nx, Lf.ny, Lf.nz, 32, 2, 2);
+  auto* kernel = axis == 0 ? k_adj_visc<T, 0> : (axis == 1 ? k_adj_visc<T, 1> : k_adj_visc<T, 2>);
+  kernel<<<g.grid, g.block, 0, s>>>(phi, ug, vg, wg, x, lam, u_bar, v_bar, w_bar, phi_bar, rho_bar, Lc, Lu, Lv, Lw, Lf,
+                                    1.0 / dx, dt, rn, rp, mn, mp);
 }
 
 void adj_zero_walls(double* f, const Lay& L, int axis, cudaStream_t s) {
