@@ -954,6 +954,13 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
   if (c->debug)
     std::fprintf(stderr, "[fs] multigrid solve: %d iterations, %d true residuals, status %d, rel %.3e\n", m.iter,
                  m.outer, m.status, *rel_out);
+  if (m.status == PCG_NONFINITE && !(m.bb > 0)) {
+    // a right-hand side of NaN: nothing to solve, as in mixed_solve below; the
+    // report's divergence says it
+    *rel_out = 0.0;
+    *st_out = PCG_CONVERGED;
+    return FS_OK;
+  }
   if (m.status == PCG_NONFINITE) {
     set_error("non-finite defect residual");
     return FS_NONFINITE;

@@ -96,3 +96,14 @@ def test_unreachable_tolerance_and_cap():
         assert rep["status"] == fs.FS_NOT_CONVERGED and rep["iterations"] == 1
         s.set_params(max_iteration=1000)
         assert s.project(1e-3)["rel_residual"] <= 1e-8
+
+
+def test_right_hand_side_without_a_value():
+    """A velocity of NaN leaves nothing to solve: reported by the divergence, as
+    by the red-black solve, not refused."""
+    n = (20, 22, 21)
+    fields = [a.copy() for a in state(n, "sphere", 5)]
+    fields[1][3, 4, 5] = np.nan
+    for precond in (fs.FS_PRECOND_RED_BLACK, fs.FS_PRECOND_DEFAULT):
+        rep, _, _ = project(n, precond, fields, 1e-8)
+        assert rep["status"] == fs.FS_OK and rep["iterations"] == 0 and np.isnan(rep["div_l2"])
