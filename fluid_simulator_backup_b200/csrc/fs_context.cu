@@ -206,7 +206,7 @@ fs_status dalloc(fs_ctx* c, void** out, size_t bytes) {
 fs_status mg_alloc(fs_ctx* c) {
   Multigrid& M = c->mg;
   int ext[kMgMaxLevels][3];
-  M.levels = mg_plan(c->grid.nx, c->grid.ny, c->grid.nz, ext, &M.top);
+  M.levels = mg_plan(c->grid.nx, c->grid.ny, c->grid.nz, ext, &M.top, &M.blocks);
   for (int l = 0; l < M.levels; ++l) {
     MgLevel& m = M.level[l];
     m.L = make_lay(ext[l][0], ext[l][1], ext[l][2]);

@@ -278,9 +278,9 @@ struct MgLevel {
   float* b[2] = {};                    // and right-hand side (level 0: the residual r)
   float a[2] = {};                     // the uniform couplings of the two phases
 };
-// levels 0 .. top-1 run as grid kernels, top .. levels-1 in one thread block
+// levels 0 .. top-1 run as grid kernels, top .. levels-1 in one cluster of thread blocks
 struct Multigrid {
-  int levels = 0, top = 0;
+  int levels = 0, top = 0, blocks = 1;
   MgLevel level[kMgMaxLevels];
 };
 // Device state of one solve.  The host sets the first group.
@@ -296,9 +296,10 @@ struct MgState {
   double tol2, bb, rr, rr_true, rr0, best, max_rr;  // squared norms
   double rz, alpha, beta, anchor, shift;
   int iter, done, status, pause, restart, outer, stall;
+  int checked, flat;     // iteration of the last true residual; successive ones without progress
   unsigned int ticket, batches;
 };
-int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top);
+int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top, int* cluster);
 cudaError_t mg_prepare();
 int mg_max_blocks(const Lay& L);
 // Each returns the number of kernels launched.  mg_build: the operator of

@@ -20,8 +20,8 @@
 // x = b/d, and is done by the kernel that writes b), the reverse after, so
 // the cycle is symmetric and CG may use it.  Three half sweeps a side need
 // 14, 10 and 7 iterations on the three scenes where two need 23, 17, 12 and
-// four 12, 8, 5: the least traffic in total.  Levels of at most kMgCoarse
-// cells a side run in one thread block in shared memory (four half sweeps a
+// four 12, 8, 5: the least traffic in total.  The levels that fit the
+// shared memory of a cluster of blocks run in one kernel (four half sweeps a
 // side there).
 //
 // Bytes.  The couplings (12 bytes per cell) are most of what a sweep would
@@ -35,7 +35,7 @@
 // alpha q, r.r (k_mg_update); the true residual b - A x in FP64 in place of
 // r whenever the recursive one meets the tolerance or has dropped by
 // reliable_delta (k_mg_defect, which alone decides convergence); the cycle
-// z = M r; r.z (k_mg_dot); p = z + beta p (k_mg_direction).  All decisions
+// z = M r, whose last two sweeps sum r.z; p = z + beta p (k_mg_direction).  All decisions
 // are taken on the device: a solve is one graph launch and one host wait.
 // Vectors are FP32 with FP64 sums, the iterate and the true residual FP64,
 // as in the red-black solve.
@@ -50,9 +50,14 @@
 // the cell layout.
 #include <cuda_bf16.h>
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <atomic>
 
 #include "fs_kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace fsb {
 
@@ -375,7 +380,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_restrict(Lev v, Lev e, int colo
     const int64_t s = e.H.at(I >> 1, J, K);
     *reinterpret_cast<float2*>(e.b[g] + s) = make_float2(r.v[0], r.v[2]);
     *reinterpret_cast<float2*>(e.b[1 - g] + s) = make_float2(r.v[1], r.v[3]);
-    // (the one-block levels start from zero themselves and have no classes)
+    // (the cluster's levels start from zero themselves and have no classes)
     if (e.cls[0]) {
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
@@ -387,205 +392,324 @@ __global__ void __launch_bounds__(kThreads) k_mg_restrict(Lev v, Lev e, int colo
 }
 
 // ---------------------------------------------------------------------------
-// The small levels in one block: a whole V-cycle in shared memory.  Every
-// level's arrays are padded by one cell (x and the couplings 0 there): x, b,
-// 1/d and the three couplings.  A half sweep is bound by shared-memory reads
-// (14 per cell), so the slots' positions are found once per level, the
-// diagonal is inverted once, and levels of at most 32 cells a colour run in
-// the first warp alone, without block barriers.  Measured at 256^3 (16^3 and
-// below in the block): 42 us with positions, sums and a division in every
-// sweep and a barrier after each, 36 us so.
+// The small levels in one cluster of thread blocks: a whole V-cycle in the
+// shared memory of up to 16 SMs.  A level of more than kSplitSlots slots is
+// split into slabs along z, one per block, whose x has a halo plane on each
+// side: a block that relaxes a cell of its first or last plane writes the
+// value into the neighbour's halo too, and the cluster's barrier after each
+// half sweep makes it visible.  The levels below run in the first block, those
+// of at most 32 cells a colour in its first warp, without block barriers.
+// The arrays of a level (x, b, 1/d and the three couplings) share one zero
+// cell between rows and one zero row between planes, which stand for the walls.
+//
+// What bounds it: latency (a barrier and a chain of shared reads per half sweep,
+// about 0.3 us in one block, 1 us with the cluster's barrier) and the fetch of
+// its instructions, which every launch repeats: with the sweeps unrolled it takes
+// 37 us at 40^3, with loops 30 us; slabs of more than two slots a thread (38 x
+// 53 x 33) are slower than the six grid kernels of a level.  Measured, a whole
+// projection to 1e-6 with the levels above 16^3 as grid kernels and one block for
+// the rest -> so: 40^3 1.21 -> 1.00 ms, 64^3 1.55 -> 1.26, 96^3 2.09 -> 1.94.
 // ---------------------------------------------------------------------------
 constexpr int kCoarseThreads = 1024;
 constexpr int kCoarseSweeps = 4;
-constexpr int kCoarseItems = 4;      // slots of one colour per thread: up to 4096
+constexpr int kCoarseItems = 2;      // slots of one colour per thread: up to 2048 per slab, 1024 unsplit
 constexpr int kWarpCells = 32;       // of one colour: levels of one warp
-constexpr int kCoarseArrays = 6;
+constexpr int kSplitSlots = 512;     // larger levels are split
 
 struct CoarseLev {
-  int nx, ny, nz, sy, sz, n;  // extents; strides and size of the padded arrays
-  int off;                    // of x in shared memory; b, 1/d, ax, ay, az follow
-  const float *ax, *ay, *az;
+  int nx, ny, nz, sy, sz;  // extents; strides of the arrays
+  int split;               // over the cluster's blocks, else in the first one
+  int off;                 // of x in shared memory (planes + 2 planes of it)
+  int b, d, ax, ay, az;    // of the others from x, indexed as x is (no halo planes; az: the upper one)
+  const float *gx, *gy, *gz;
   Lay L;
 };
 struct CoarseArgs {
-  int levels;
+  int levels, floats;
   CoarseLev l[kMgMaxLevels];
   float* x[2];
   float* b[2];
   Lay H;  // packed layout of the top level
 };
 
-__device__ __forceinline__ int coarse_slots(const CoarseLev& v) { return ((v.nx + 1) >> 1) * v.ny * v.nz; }
+__host__ __device__ __forceinline__ int coarse_slots(int nx, int ny, int nz) { return ((nx + 1) >> 1) * ny * nz; }
 
-__device__ __forceinline__ void coarse_relax(const CoarseLev& v, float* x, int c) {
-  const float *b = x + v.n, *di = b + v.n, *ax = di + v.n, *ay = ax + v.n, *az = ay + v.n;
-  const float num = b[c] + (((ax[c] * x[c - 1] + ax[c + 1] * x[c + 1]) + (ay[c] * x[c - v.sy] + ay[c + v.sy] * x[c + v.sy])) +
-                            (az[c] * x[c - v.sz] + az[c + v.sz] * x[c + v.sz]));
-  x[c] = num * di[c];
+// the planes k0 .. k0 + n - 1 of a level that a block owns
+struct Slab {
+  int k0, n;
+};
+__device__ __forceinline__ Slab slab_of(const CoarseLev& v, int rank, int blocks) {
+  if (!v.split) return {0, rank == 0 ? v.nz : 0};
+  const int k0 = v.nz * rank / blocks;
+  return {k0, v.nz * (rank + 1) / blocks - k0};
+}
+__device__ __forceinline__ int owner_of(const CoarseLev& v, int k, int blocks) {
+  return v.split ? ((k + 1) * blocks - 1) / v.nz : 0;
+}
+
+__device__ __forceinline__ float coarse_relax(const CoarseLev& v, const float* x, int c) {
+  const float *ax = x + v.ax, *ay = x + v.ay, *az = x + v.az;
+  const float num = x[v.b + c] +
+                    (((ax[c] * x[c - 1] + ax[c + 1] * x[c + 1]) + (ay[c] * x[c - v.sy] + ay[c + v.sy] * x[c + v.sy])) +
+                     (az[c] * x[c - v.sz] + az[c + v.sz] * x[c + v.sz]));
+  return num * x[v.d + c];
 }
 __device__ __forceinline__ float coarse_residual(const CoarseLev& v, const float* x, int c) {
-  const float *b = x + v.n, *ax = b + 2 * v.n, *ay = ax + v.n, *az = ay + v.n;
+  const float *ax = x + v.ax, *ay = x + v.ay, *az = x + v.az;
   const float xc = x[c];
-  float s = b[c] + (ax[c] * (x[c - 1] - xc) + ax[c + 1] * (x[c + 1] - xc));
+  float s = x[v.b + c] + (ax[c] * (x[c - 1] - xc) + ax[c + 1] * (x[c + 1] - xc));
   s += ay[c] * (x[c - v.sy] - xc) + ay[c + v.sy] * (x[c + v.sy] - xc);
   s += az[c] * (x[c - v.sz] - xc) + az[c + v.sz] * (x[c + v.sz] - xc);
   return s;
 }
 
-// The slots a thread owns on a level: the padded index of the cell at i = 2h
-// in the low bits, and whether the slot's cells exist (a half slot at the end
-// of an odd row has one cell only, marked).
+// The slots a thread owns on a level: the index of the cell at i = 2h, and
+// whether the slot's cells exist (a half slot at the end of an odd row has one
+// cell only, marked).  below, above: where the neighbours' halo planes hold
+// this slab's first and last plane (nullptr: none).
+template <int N>
 struct CoarseItems {
-  int c[kCoarseItems];     // index of cell 2h, -1: none
-  unsigned par, half;      // bit m: (j + k) & 1; cell 2h + 1 does not exist
-  __device__ __forceinline__ void init(const CoarseLev& v, int tid, int threads) {
-    const int hx = (v.nx + 1) >> 1, count = hx * v.ny * v.nz;
+  int c[N];             // -1: none
+  unsigned par, half;   // bit m: (j + k) & 1; cell 2h + 1 does not exist
+  float *below, *above;
+  int last;             // first index of the last plane
+  __device__ __forceinline__ void init(const CoarseLev& v, const Slab& z, int tid, int threads) {
+    const int hx = (v.nx + 1) >> 1, count = hx * v.ny * z.n;
     par = half = 0u;
+    below = above = nullptr;
+    last = z.n * v.sz;
 #pragma unroll
-    for (int m = 0; m < kCoarseItems; ++m) {
+    for (int m = 0; m < N; ++m) {
       const int t = tid + m * threads;
       c[m] = -1;
       if (t < count) {
         const int h = t % hx, row = t / hx, j = row % v.ny, k = row / v.ny;
-        c[m] = (k + 1) * v.sz + (j + 1) * v.sy + 2 * h + 1;
-        par |= (unsigned)((j + k) & 1) << m;
+        c[m] = (k + 1) * v.sz + j * v.sy + 2 * h;
+        par |= (unsigned)((j + z.k0 + k) & 1) << m;
         half |= (unsigned)(2 * h + 1 >= v.nx) << m;
       }
     }
   }
+  __device__ __forceinline__ void neighbours(const CoarseLev& v, const Slab& z, float* x, int blocks,
+                                             const cg::cluster_group& cl) {
+    if (!v.split || z.n == 0) return;
+    if (z.k0 > 0) {
+      const int r = owner_of(v, z.k0 - 1, blocks);
+      below = cl.map_shared_rank(x, r) + slab_of(v, r, blocks).n * v.sz;
+    }
+    if (z.k0 + z.n < v.nz) above = cl.map_shared_rank(x, owner_of(v, z.k0 + z.n, blocks)) - z.n * v.sz;
+  }
+  __device__ __forceinline__ void store(const CoarseLev& v, float* x, int at, float value) const {
+    x[at] = value;
+    if (below && at < 2 * v.sz) below[at] = value;
+    if (above && at >= last) above[at] = value;
+  }
   __device__ __forceinline__ void sweep(const CoarseLev& v, float* x, int color) const {
 #pragma unroll
-    for (int m = 0; m < kCoarseItems; ++m) {
+    for (int m = 0; m < N; ++m) {
       if (c[m] < 0) continue;
       const int o = ((par >> m) ^ color) & 1;
       if (o && ((half >> m) & 1)) continue;
-      coarse_relax(v, x, c[m] + o);
+      store(v, x, c[m] + o, coarse_relax(v, x, c[m] + o));
     }
   }
 };
 
-// restrict from level v into w, by threads tid of `threads`
-__device__ __forceinline__ void coarse_restrict(const CoarseLev& v, const CoarseLev& w, float* sm, int tid, int threads) {
+// The residual of this block's planes of level v, summed into level w's b in
+// the blocks that own it: each fine plane adds its two cells per coarse cell
+// (two planes at most add to one, so the sum does not depend on their order).
+// Black was swept last, its residual is zero: only the red cells count.
+__device__ __forceinline__ void coarse_restrict(const CoarseLev& v, const CoarseLev& w, const Slab& z, float* sm,
+                                                int blocks, const cg::cluster_group& cl, int tid, int threads) {
   const float* x = sm + v.off;
-  float* wb = sm + w.off + w.n;
-  const int count = w.nx * w.ny * w.nz;
-  // the residual is zero in the colour swept last (black): only the four red cells count
+  const int plane = w.nx * w.ny, count = plane * z.n;
   for (int t = tid; t < count; t += threads) {
-    const int I = t % w.nx, row = t / w.nx, J = row % w.ny, K = row / w.ny;
+    const int lk = t / plane, k = z.k0 + lk, K = k >> 1, rest = t - lk * plane, J = rest / w.nx, I = rest - J * w.nx;
     float r = 0.0f;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int j = 2 * J + (m & 1), k = 2 * K + (m >> 1), i = 2 * I + ((j + k) & 1);
-      if (i < v.nx && j < v.ny && k < v.nz) r += coarse_residual(v, x, (k + 1) * v.sz + (j + 1) * v.sy + i + 1);
+    for (int m = 0; m < 2; ++m) {
+      const int j = 2 * J + m, i = 2 * I + ((j + k) & 1);
+      if (i < v.nx && j < v.ny) r += coarse_residual(v, x, (lk + 1) * v.sz + j * v.sy + i);
     }
-    wb[(K + 1) * w.sz + (J + 1) * w.sy + I + 1] = r;
+    const int own = owner_of(w, K, blocks);
+    float* wb = sm + w.off + w.b + (K - slab_of(w, own, blocks).k0 + 1) * w.sz + J * w.sy + I;
+    atomicAdd(own == (int)cl.block_rank() ? wb : cl.map_shared_rank(wb, own), r);
   }
 }
-__device__ __forceinline__ void coarse_prolong(const CoarseLev& v, const CoarseLev& w, float* sm, int tid, int threads) {
+template <int N>
+__device__ __forceinline__ void coarse_prolong(const CoarseLev& v, const CoarseLev& w, const Slab& z,
+                                               const CoarseItems<N>& it, float* sm, int blocks,
+                                               const cg::cluster_group& cl) {
   float* x = sm + v.off;
-  const float* wx = sm + w.off;
-  const int count = v.nx * v.ny * v.nz;
-  for (int t = tid; t < count; t += threads) {
-    const int i = t % v.nx, row = t / v.nx, j = row % v.ny, k = row / v.ny;
-    x[(k + 1) * v.sz + (j + 1) * v.sy + i + 1] += wx[((k >> 1) + 1) * w.sz + ((j >> 1) + 1) * w.sy + (i >> 1) + 1];
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    if (it.c[m] < 0) continue;
+    const int lk = it.c[m] / v.sz - 1, rest = it.c[m] - (lk + 1) * v.sz, j = rest / v.sy, i = rest - j * v.sy;
+    const int K = (z.k0 + lk) >> 1, own = owner_of(w, K, blocks);
+    const float* wx = sm + w.off + (K - slab_of(w, own, blocks).k0 + 1) * w.sz + (j >> 1) * w.sy + (i >> 1);
+    const float e = own == (int)cl.block_rank() ? *wx : *cl.map_shared_rank(wx, own);
+    it.store(v, x, it.c[m], x[it.c[m]] + e);
+    if (!((it.half >> m) & 1)) it.store(v, x, it.c[m] + 1, x[it.c[m] + 1] + e);
   }
 }
 
-__global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(CoarseArgs A, const MgState* st) {
-  if (stopped(st)) return;
+__global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(const __grid_constant__ CoarseArgs A, const MgState* st) {
+  if (stopped(st)) return;  // the same in every block
   extern __shared__ __align__(16) float sm[];
-  const int tid = threadIdx.x;
-  {
-    const CoarseLev& last = A.l[A.levels - 1];
-    const int total4 = (last.off + kCoarseArrays * last.n + 3) >> 2;
-    for (int t = tid; t < total4; t += kCoarseThreads)
-      reinterpret_cast<float4*>(sm)[t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  }
+  const cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, rank = (int)cl.block_rank(), blocks = (int)cl.num_blocks();
+  for (int t = tid; t < A.floats >> 2; t += kCoarseThreads)
+    reinterpret_cast<float4*>(sm)[t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   __syncthreads();
-  for (int q = 0; q < A.levels; ++q) {
-    const CoarseLev& v = A.l[q];
-    float* x = sm + v.off;
-    const int count = v.nx * v.ny * v.nz;
-    for (int t = tid; t < count; t += kCoarseThreads) {
-      const int i = t % v.nx, row = t / v.nx, j = row % v.ny, k = row / v.ny;
-      const int c = (k + 1) * v.sz + (j + 1) * v.sy + i + 1;
-      const int64_t g = v.L.at(i, j, k);
+  // the operators of this block's planes (and the low faces of the plane above a
+  // slab), all levels in one range of indices, so that their reads overlap
+  {
+    int q = 0, base = 0, plane = A.l[0].nx * A.l[0].ny;
+    Slab z = slab_of(A.l[0], rank, blocks);
+    auto count = [&]() { return z.n ? plane * (z.n + (z.k0 + z.n < A.l[q].nz ? 1 : 0)) : 0; };
+#pragma unroll 1
+    for (int t = tid;; t += kCoarseThreads) {
+      while (t - base >= count()) {
+        base += count();
+        if (++q == A.levels) break;
+        plane = A.l[q].nx * A.l[q].ny;
+        z = slab_of(A.l[q], rank, blocks);
+      }
+      if (q == A.levels) break;
+      const CoarseLev& v = A.l[q];
+      float* x = sm + v.off;
+      const int k = (t - base) / plane, rest = (t - base) - k * plane, j = rest / v.nx, i = rest - j * v.nx;
+      const int c = (k + 1) * v.sz + j * v.sy + i;
+      const int64_t g = v.L.at(i, j, z.k0 + k);
+      const float zm = v.gz[g];
+      if (k == z.n) {
+        x[v.az + c] = zm;
+        continue;
+      }
       // the low faces, then 1/d (the high walls' couplings are ghosts, 0)
-      const float xm = v.ax[g], ym = v.ay[g], zm = v.az[g];
-      const float d = ((xm + v.ax[g + 1]) + (ym + v.ay[g + v.L.px])) + (zm + v.az[g + v.L.slab]);
-      x[2 * v.n + c] = d > 0.0f ? 1.0f / d : 0.0f;
-      x[3 * v.n + c] = xm;
-      x[4 * v.n + c] = ym;
-      x[5 * v.n + c] = zm;
-      if (q == 0) x[v.n + c] = A.b[(i + j + k) & 1][A.H.at(i >> 1, j, k)];
+      const float xm = v.gx[g], ym = v.gy[g];
+      const float d = ((xm + v.gx[g + 1]) + (ym + v.gy[g + v.L.px])) + (zm + v.gz[g + v.L.slab]);
+      const float rhs = q == 0 ? A.b[(i + j + z.k0 + k) & 1][A.H.at(i >> 1, j, z.k0 + k)] : 0.0f;
+      x[v.d + c] = d > 0.0f ? 1.0f / d : 0.0f;
+      x[v.ax + c] = xm;
+      x[v.ay + c] = ym;
+      x[v.az + c] = zm;
+      if (q == 0) x[v.b + c] = rhs;
     }
   }
-  __syncthreads();
-  // levels 0 .. big-1 by the block, the rest by one warp
-  int big = 0;
-  while (big < A.levels && coarse_slots(A.l[big]) > kWarpCells) ++big;
-  for (int q = 0; q < big; ++q) {
-    const CoarseLev& v = A.l[q];
-    CoarseItems it;
-    it.init(v, tid, kCoarseThreads);
+  if (blocks > 1) cl.sync();
+  else __syncthreads();
+  int first = 0;  // the first level that is not split
+#pragma unroll 1
+  for (; first < A.levels && A.l[first].split; ++first) {
+    const CoarseLev& v = A.l[first];
+    const Slab z = slab_of(v, rank, blocks);
+    CoarseItems<kCoarseItems> it;
+    it.init(v, z, tid, kCoarseThreads);
+    it.neighbours(v, z, sm + v.off, blocks, cl);
+#pragma unroll 1
     for (int m = 0; m < kCoarseSweeps; ++m) {
       it.sweep(v, sm + v.off, m & 1);
-      __syncthreads();
+      cl.sync();
     }
-    if (q + 1 < A.levels) {
-      coarse_restrict(v, A.l[q + 1], sm, tid, kCoarseThreads);
-      __syncthreads();
-    }
+    coarse_restrict(v, A.l[first + 1], z, sm, blocks, cl, tid, kCoarseThreads);
+    cl.sync();
   }
-  if (tid < 32) {
-    for (int q = big; q < A.levels; ++q) {
+  if (rank == 0) {
+    // by the block, the last ones by one warp
+    int big = first;
+    while (big < A.levels && coarse_slots(A.l[big].nx, A.l[big].ny, A.l[big].nz) > kWarpCells) ++big;
+#pragma unroll 1
+    for (int q = first; q < big; ++q) {
       const CoarseLev& v = A.l[q];
-      CoarseItems it;
-      it.init(v, tid, 32);
-      // the coarsest level (at most 2 cells a side) is swept to a solve
-      const int sweeps = q == A.levels - 1 ? 2 * kCoarseSweeps : kCoarseSweeps;
-      for (int m = 0; m < sweeps; ++m) {
+      const Slab z{0, v.nz};
+      CoarseItems<1> it;
+      it.init(v, z, tid, kCoarseThreads);
+#pragma unroll 1
+      for (int m = 0; m < kCoarseSweeps; ++m) {
         it.sweep(v, sm + v.off, m & 1);
-        __syncwarp();
+        __syncthreads();
       }
-      if (q + 1 < A.levels) coarse_restrict(v, A.l[q + 1], sm, tid, 32);
-      __syncwarp();
-    }
-    for (int q = A.levels - 1; q >= big; --q) {
-      const CoarseLev& v = A.l[q];
-      CoarseItems it;
-      it.init(v, tid, 32);
-      if (q + 1 < A.levels) coarse_prolong(v, A.l[q + 1], sm, tid, 32);
-      __syncwarp();
-      const int sweeps = q == A.levels - 1 ? 2 * kCoarseSweeps : kCoarseSweeps;
-      for (int m = sweeps - 1; m >= 0; --m) {
-        it.sweep(v, sm + v.off, m & 1);
-        __syncwarp();
+      if (q + 1 < A.levels) {
+        coarse_restrict(v, A.l[q + 1], z, sm, 1, cl, tid, kCoarseThreads);
+        __syncthreads();
       }
     }
+    if (tid < 32) {
+#pragma unroll 1
+      for (int q = big; q < A.levels; ++q) {
+        const CoarseLev& v = A.l[q];
+        const Slab z{0, v.nz};
+        CoarseItems<1> it;
+        it.init(v, z, tid, 32);
+        // the coarsest level (at most 2 cells a side) is swept to a solve
+        const int sweeps = q == A.levels - 1 ? 2 * kCoarseSweeps : kCoarseSweeps;
+#pragma unroll 1
+        for (int m = 0; m < sweeps; ++m) {
+          it.sweep(v, sm + v.off, m & 1);
+          __syncwarp();
+        }
+        if (q + 1 < A.levels) coarse_restrict(v, A.l[q + 1], z, sm, 1, cl, tid, 32);
+        __syncwarp();
+      }
+#pragma unroll 1
+      for (int q = A.levels - 1; q >= big; --q) {
+        const CoarseLev& v = A.l[q];
+        const Slab z{0, v.nz};
+        CoarseItems<1> it;
+        it.init(v, z, tid, 32);
+        if (q + 1 < A.levels) coarse_prolong(v, A.l[q + 1], z, it, sm, 1, cl);
+        __syncwarp();
+        const int sweeps = q == A.levels - 1 ? 2 * kCoarseSweeps : kCoarseSweeps;
+#pragma unroll 1
+        for (int m = sweeps - 1; m >= 0; --m) {
+          it.sweep(v, sm + v.off, m & 1);
+          __syncwarp();
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = big - 1; q >= first; --q) {
+      const CoarseLev& v = A.l[q];
+      const Slab z{0, v.nz};
+      CoarseItems<1> it;
+      it.init(v, z, tid, kCoarseThreads);
+      if (q + 1 < A.levels) {
+        coarse_prolong(v, A.l[q + 1], z, it, sm, 1, cl);
+        __syncthreads();
+      }
+#pragma unroll 1
+      for (int m = kCoarseSweeps - 1; m >= 0; --m) {
+        it.sweep(v, sm + v.off, m & 1);
+        __syncthreads();
+      }
+    }
   }
-  __syncthreads();
-  for (int q = big - 1; q >= 0; --q) {
+  if (first > 0) cl.sync();
+#pragma unroll 1
+  for (int q = first - 1; q >= 0; --q) {
     const CoarseLev& v = A.l[q];
-    CoarseItems it;
-    it.init(v, tid, kCoarseThreads);
-    if (q + 1 < A.levels) {
-      coarse_prolong(v, A.l[q + 1], sm, tid, kCoarseThreads);
-      __syncthreads();
-    }
+    const Slab z = slab_of(v, rank, blocks);
+    CoarseItems<kCoarseItems> it;
+    it.init(v, z, tid, kCoarseThreads);
+    it.neighbours(v, z, sm + v.off, blocks, cl);
+    coarse_prolong(v, A.l[q + 1], z, it, sm, blocks, cl);
+    cl.sync();
+#pragma unroll 1
     for (int m = kCoarseSweeps - 1; m >= 0; --m) {
       it.sweep(v, sm + v.off, m & 1);
-      __syncthreads();
+      cl.sync();  // (the last one: no block leaves while another writes into it)
     }
   }
   {
     const CoarseLev& v = A.l[0];
+    const Slab z = slab_of(v, rank, blocks);
     const float* x = sm + v.off;
-    const int count = v.nx * v.ny * v.nz;
-    for (int t = tid; t < count; t += kCoarseThreads) {
-      const int i = t % v.nx, row = t / v.nx, j = row % v.ny, k = row / v.ny;
-      A.x[(i + j + k) & 1][A.H.at(i >> 1, j, k)] = x[(k + 1) * v.sz + (j + 1) * v.sy + i + 1];
+    const int plane = v.nx * v.ny;
+    for (int t = tid; t < plane * z.n; t += kCoarseThreads) {
+      const int k = t / plane, rest = t - k * plane, j = rest / v.nx, i = rest - j * v.nx;
+      A.x[(i + j + z.k0 + k) & 1][A.H.at(i >> 1, j, z.k0 + k)] = x[(k + 1) * v.sz + j * v.sy + i];
     }
   }
 }
@@ -746,7 +870,9 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv(Lev v, const float* __rest
 // x += alpha p (FP64), r -= alpha q, r.r and the first red half sweep of the
 // next cycle.  The last block asks for the true residual (pause) when the
 // recursive one meets the tolerance, has dropped by reliable_delta since the
-// last true one, or the iteration cap is reached.
+// last true one, has not for kCheckEvery iterations (at the floor of the
+// arithmetic, where x only drifts), or the iteration cap is reached.
+constexpr int kCheckEvery = 8;
 __global__ void __launch_bounds__(kThreads) k_mg_update(Lev v, const float* __restrict__ p,
                                                         const float* __restrict__ q, MgState* st, double* partials,
                                                         int w, int chunk) {
@@ -806,7 +932,8 @@ __global__ void __launch_bounds__(kThreads) k_mg_update(Lev v, const float* __re
     if (!isfinite(tot)) {
       st->status = PCG_STAGNATED;  // the FP32 recursion broke down; x may hold the bad step
       st->done = 1;
-    } else if (tot <= st->tol2 || tot < st->delta * st->delta * st->max_rr || st->iter >= st->max_iter) {
+    } else if (tot <= st->tol2 || tot < st->delta * st->delta * st->max_rr || st->iter >= st->max_iter ||
+               st->iter - st->checked >= kCheckEvery) {
       st->pause = 1;
     }
   }
@@ -913,6 +1040,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_mg_defect(Lev v, MgState* st, d
       st->restart = tot > 100.0 * st->rr;
     }
     st->pause = 0;
+    st->checked = st->iter;
     st->rr_true = tot;
     st->max_rr = tot;
     if (!isfinite(tot) || !isfinite(st->bb)) {
@@ -927,7 +1055,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_mg_defect(Lev v, MgState* st, d
     } else if (!INIT) {
       if (tot < 0.25 * st->best) st->stall = 0;
       else st->stall += 1;
-      if (tot > 1.0e4 * st->best || st->stall >= 24) {
+      if (tot < 0.9 * st->best) st->flat = 0;
+      else st->flat += 1;
+      if (tot > 1.0e4 * st->best || st->stall >= 24 || st->flat >= 4) {
         st->status = PCG_STAGNATED;  // diverged, or no further progress
         st->done = 1;
       }
@@ -1039,17 +1169,36 @@ __global__ void __launch_bounds__(kThreads) k_mg_shift(Lay L, const MgState* st,
   }
 }
 
-// shared floats of one level, rounded up to a float4
-size_t coarse_floats(int nx, int ny, int nz) {
-  return ((size_t)kCoarseArrays * (nx + 2) * (ny + 2) * (nz + 2) + 3) / 4 * 4;
+constexpr size_t kCoarseBytes = 224 * 1024;  // of the 227 KB a block may have
+// blocks of a cluster that k_mg_coarse may have (mg_prepare)
+std::atomic<int> cluster_blocks{1};
+
+cudaLaunchConfig_t coarse_launch(int blocks, size_t bytes, cudaLaunchAttribute* at, cudaStream_t s) {
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = blocks;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(blocks);
+  c.blockDim = dim3(kCoarseThreads);
+  c.dynamicSmemBytes = bytes;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return c;
 }
-constexpr size_t kCoarseBytes = 220 * 1024;  // of the 227 KB a block may have
+
+bool coarse_split(int nx, int ny, int nz, int blocks) { return blocks > 1 && coarse_slots(nx, ny, nz) > kSplitSlots; }
+// shared floats of one level in one block, rounded up to a float4
+size_t coarse_floats(int nx, int ny, int nz, int blocks) {
+  const size_t p = coarse_split(nx, ny, nz, blocks) ? (nz + blocks - 1) / blocks : nz;
+  return ((6 * p + 3) * (size_t)(nx + 1) * (ny + 1) + 3) / 4 * 4;
+}
 
 }  // namespace
 
 // The grids of the hierarchy: halved (rounding up) until at most 2 cells a
-// side; `top` is the first level from which on all fit one block.
-int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top) {
+// side; `top` is the first level from which on all fit a cluster of *cluster blocks.
+int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top, int* cluster) {
   int n = 0;
   for (;;) {
     ext[n][0] = nx;
@@ -1061,19 +1210,41 @@ int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top) {
     ny = (ny + 1) / 2;
     nz = (nz + 1) / 2;
   }
+  const int blocks = *cluster = cluster_blocks;
   size_t floats = 0;
   int t = n;
   while (t > 1) {
-    floats += coarse_floats(ext[t - 1][0], ext[t - 1][1], ext[t - 1][2]);
-    if (floats * sizeof(float) > kCoarseBytes) break;
+    const int *e = ext[t - 1], planes = coarse_split(e[0], e[1], e[2], blocks) ? (e[2] + blocks - 1) / blocks : e[2];
+    floats += coarse_floats(e[0], e[1], e[2], blocks);
+    if (floats * sizeof(float) > kCoarseBytes || coarse_slots(e[0], e[1], planes) > (planes < e[2] ? kCoarseItems : 1) * kCoarseThreads)
+      break;
     --t;
   }
   *top = t;
   return n;
 }
 
+// The largest cluster that the device runs: 16 blocks (of one GPC; more than the
+// portable 8), else 8, else one block.
 cudaError_t mg_prepare() {
-  return cudaFuncSetAttribute(k_mg_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseBytes);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_mg_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseBytes);
+  if (e != cudaSuccess) return e;
+  for (int blocks : {16, 8, 1}) {
+    if (blocks > 8 && cudaFuncSetAttribute(k_mg_coarse, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    cudaLaunchAttribute at{};
+    const cudaLaunchConfig_t cfg = coarse_launch(blocks, kCoarseBytes, &at, 0);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_mg_coarse, &cfg) == cudaSuccess && n > 0) {
+      cluster_blocks = blocks;
+      break;
+    }
+    cudaGetLastError();
+  }
+  return cudaSuccess;
 }
 
 int mg_max_blocks(const Lay& L) {
@@ -1123,29 +1294,40 @@ int cycle(const Multigrid& M, MgState* st, double* partials, cudaStream_t s) {
   CoarseArgs A{};
   size_t floats = 0;
   A.levels = M.levels - M.top;
+  const Lay& tl = M.level[M.top].L;
+  const int blocks = coarse_split(tl.nx, tl.ny, tl.nz, M.blocks) ? M.blocks : 1;
   for (int q = 0; q < A.levels; ++q) {
     const MgLevel& m = M.level[M.top + q];
     CoarseLev& w = A.l[q];
     w.nx = m.L.nx;
     w.ny = m.L.ny;
     w.nz = m.L.nz;
-    w.sy = w.nx + 2;
-    w.sz = w.sy * (w.ny + 2);
-    w.n = w.sz * (w.nz + 2);
+    w.sy = w.nx + 1;
+    w.sz = w.sy * (w.ny + 1);
+    w.split = coarse_split(w.nx, w.ny, w.nz, blocks);
+    const int p = w.split ? (w.nz + blocks - 1) / blocks : w.nz;
     w.off = (int)floats;
-    w.ax = m.ax;
-    w.ay = m.ay;
-    w.az = m.az;
+    w.b = (p + 1) * w.sz;
+    w.d = w.b + p * w.sz;
+    w.ax = w.d + p * w.sz;
+    w.ay = w.ax + p * w.sz;
+    w.az = w.ay + p * w.sz;
+    w.gx = m.ax;
+    w.gy = m.ay;
+    w.gz = m.az;
     w.L = m.L;
-    floats += coarse_floats(w.nx, w.ny, w.nz);
+    floats += coarse_floats(w.nx, w.ny, w.nz, blocks);
   }
+  A.floats = (int)floats;
   const MgLevel& t = M.level[M.top];
   for (int c = 0; c < 2; ++c) {
     A.x[c] = t.x[c];
     A.b[c] = t.b[c];
   }
   A.H = t.H;
-  k_mg_coarse<<<1, kCoarseThreads, floats * sizeof(float), s>>>(A, st);
+  cudaLaunchAttribute at{};
+  const cudaLaunchConfig_t cfg = coarse_launch(blocks, floats * sizeof(float), &at, s);
+  cudaLaunchKernelEx(&cfg, k_mg_coarse, A, (const MgState*)st);
   ++launches;
   for (int l = M.top - 1; l >= 0; --l) {
     const Lev v = lev_of(M.level[l]), e = lev_of(M.level[l + 1]);

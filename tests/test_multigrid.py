@@ -107,3 +107,16 @@ def test_right_hand_side_without_a_value():
     for precond in (fs.FS_PRECOND_RED_BLACK, fs.FS_PRECOND_DEFAULT):
         rep, _, _ = project(n, precond, fields, 1e-8)
         assert rep["status"] == fs.FS_OK and rep["iterations"] == 0 and np.isnan(rep["div_l2"])
+
+
+@pytest.mark.parametrize("n", [(30, 34, 18), (26, 24, 70), (66, 18, 40), (33, 65, 31), (64, 64, 64), (80, 20, 79)])
+def test_levels_split_over_a_cluster(n):
+    """Small levels in slabs over the blocks of a cluster: fewer planes than
+    blocks, uneven slabs, one and two slots a thread.  The same pressure as the
+    red-black solve, in the few iterations of an intact cycle (at most 40, as
+    above)."""
+    fields = state(n, "sphere", 7)
+    rep, p, _ = project(n, fs.FS_PRECOND_DEFAULT, fields, 1e-9)
+    assert rep["rel_residual"] <= 1e-9 and rep["iterations"] <= 40
+    p2 = project(n, fs.FS_PRECOND_RED_BLACK, fields, 1e-9)[1]
+    assert scaled(p, p2) < 2e-5
