@@ -40,9 +40,9 @@
 // Vectors are FP32 with FP64 sums, the iterate and the true residual FP64,
 // as in the red-black solve.
 //
-// Measured (B200, CUDA events around whole calls, before: red-black IC(0)):
-// a 256^3 rising-bubble timestep 646 -> 87 ms (its three solves 565 -> 30),
-// a projection of 150 x 210 x 131 cells 87.2 -> 6.5 ms, of 40^3 4.8 -> 1.3 ms.
+// Measured (B200, CUDA events around whole calls, before: red-black IC(0)): a
+// projection of 150 x 210 x 131 cells to 1e-6 85.6 -> 5.3 ms, of 40^3 4.7 -> 1.1
+// ms; the three solves of a 256^3 rising-bubble timestep 565 -> 22 ms.
 //
 // r and z are stored by colour in the packed half layout of fs_redblack.cu
 // (slot (h, j, k): red cell at i = 2h + ((j+k)&1), black at 2h + ((j+k+1)&1)),

@@ -503,46 +503,44 @@ __global__ void k_convert(D* __restrict__ dst, const S* __restrict__ src, Lay L)
   dst[c] = (D)src[c];
 }
 
-// packed (x fastest, no ghosts) FP64 <-> padded storage, rows walked by
-// consecutive threads with kRows rows in flight each: a plane's rows are read and
-// written whole whatever their length.  (One value per thread of a 32 x 4 x 2
-// block: 63 us at 256^3 between FP32 storage and FP64, 47 us so.)
-constexpr int kPackRows = 4;
+// packed (x fastest, no ghosts) FP64 <-> padded storage: a warp per row, each
+// thread with kPackLoads values in flight, so that a row is found with one 32-bit
+// division whatever its length.  Bound by HBM: 12 bytes per value between FP32
+// storage and FP64.  Measured at 256^3: a block of 256 threads on four rows 48
+// us, so 28 (pack) and 31 us (0.98 and 0.88 of what 12 bytes take at copy speed).
+constexpr int kPackLoads = 8;
 template <class T, bool PACK>
-__global__ void __launch_bounds__(256) k_transfer(double* __restrict__ packed, T* __restrict__ padded, Lay L) {
-  const int64_t rows = (int64_t)L.ny * L.nz;
-  // threads along a row: the row length rounded up to a power of two, at most the block
-  const int wide = blockDim.x, per = blockDim.y;
-  const int64_t r0 = ((int64_t)blockIdx.x * per + threadIdx.y) * kPackRows;
-  for (int i = threadIdx.x; i < L.nx; i += wide) {
-    T v[kPackRows];
-    double d[kPackRows];
+__global__ void __launch_bounds__(256) k_transfer(double* __restrict__ packed, T* __restrict__ padded, Lay L,
+                                                  unsigned rows) {
+  const unsigned r = blockIdx.x * 8u + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const int k = (int)(r / (unsigned)L.ny), j = (int)(r - (unsigned)k * (unsigned)L.ny);
+  double* __restrict__ a = packed + (int64_t)r * L.nx;
+  T* __restrict__ b = padded + L.at(0, j, k);
+  for (int i0 = threadIdx.x & 31; i0 < L.nx; i0 += 32 * kPackLoads) {
+    double d[kPackLoads];
+    T v[kPackLoads];
 #pragma unroll
-    for (int m = 0; m < kPackRows; ++m) {
-      const int64_t r = r0 + m;
-      if (r >= rows) continue;
-      const int k = (int)(r / L.ny), j = (int)(r - (int64_t)k * L.ny);
-      if (PACK) v[m] = padded[L.at(i, j, k)];
-      else d[m] = packed[r * L.nx + i];
+    for (int m = 0; m < kPackLoads; ++m) {
+      const int i = i0 + 32 * m;
+      if (i >= L.nx) continue;
+      if (PACK) v[m] = b[i];
+      else d[m] = a[i];
     }
 #pragma unroll
-    for (int m = 0; m < kPackRows; ++m) {
-      const int64_t r = r0 + m;
-      if (r >= rows) continue;
-      const int k = (int)(r / L.ny), j = (int)(r - (int64_t)k * L.ny);
-      if (PACK) packed[r * L.nx + i] = (double)v[m];
-      else padded[L.at(i, j, k)] = (T)d[m];
+    for (int m = 0; m < kPackLoads; ++m) {
+      const int i = i0 + 32 * m;
+      if (i >= L.nx) continue;
+      if (PACK) a[i] = (double)v[m];
+      else b[i] = (T)d[m];
     }
   }
 }
 
 template <class T, bool PACK>
 void transfer(double* packed, T* padded, const Lay& L, cudaStream_t s) {
-  int wide = 32;
-  while (wide < 256 && wide < L.nx) wide *= 2;
-  const dim3 block(wide, 256 / wide, 1);
-  const int64_t rows = (int64_t)L.ny * L.nz, per = (int64_t)block.y * kPackRows;
-  k_transfer<T, PACK><<<(unsigned)((rows + per - 1) / per), block, 0, s>>>(packed, padded, L);
+  const unsigned rows = (unsigned)L.ny * (unsigned)L.nz;
+  k_transfer<T, PACK><<<(rows + 7) / 8, 256, 0, s>>>(packed, padded, L, rows);
 }
 
 // ---------------------------------------------------------------------------
