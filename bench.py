@@ -43,6 +43,10 @@ BYTES_PER_UNKNOWN_PCG_FP64 = 120
 # cells): SpMV 16 (ax, ay, az 12; black p 2; black q 2) + residual update 7 +
 # direction update 15, at about half the iterations
 BYTES_PER_CELL_PCG_RB = 38
+# multigrid-preconditioned CG (per cell): spmv 9 (p, class read; q write) + update 35 (FP64 x and FP32 r read and
+# written, p, q, class read, first half sweep written) + FP64 true residual 23 (x, b, class read; r, z write; nearly
+# every iteration takes one) + five half sweeps of 6.5 + restriction 7 + direction 12 = 119, the coarser levels 7
+BYTES_PER_CELL_PCG_MG = 126
 # DRAM bytes (read + write) of one FP32 Jacobi PCG iteration at 256^3
 # measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of
 # k_cg_spmv, k_cg_update, k_cg_pupdate, one capture of the bench workload);
@@ -61,7 +65,7 @@ def scene(n):
 PRECONDITIONER = {"default": 0, "jacobi": 1, "bf16": 2, "red_black": 3, "red_black_jacobi": 4}
 PRECOND_CHOICE = "default"
 # what FS_PRECOND_DEFAULT selects in an FP32_REFINE context
-DEFAULT_FP32_PRECONDITIONER = "red_black"
+DEFAULT_FP32_PRECONDITIONER = "multigrid"
 
 
 def effective_preconditioner(fs):
@@ -594,6 +598,11 @@ def main():
     rb = main_prec == fs.FS_PRECISION_FP32_REFINE and effective_preconditioner(fs) in ("red_black", "red_black_jacobi")
     if main_prec == fs.FS_PRECISION_FP64:
         bpu, kernel = BYTES_PER_UNKNOWN_PCG_FP64, "FP64 Jacobi PCG iteration (spmv + update + direction, 3 kernels)"
+        traffic = None
+    elif effective_preconditioner(fs) == "multigrid":
+        bpu = BYTES_PER_CELL_PCG_MG
+        kernel = ("CG iteration preconditioned by one multigrid V-cycle (spmv, update, FP64 true residual, half sweeps "
+                  "per level, transfers, one cluster kernel for the small levels, direction)")
         traffic = None
     elif rb:
         bpu = BYTES_PER_CELL_PCG_RB
