@@ -14,6 +14,8 @@
 // (no penetration) and velocity ghosts beyond the walls are zero; both enter
 // the diagonal through their arm couplings and drop out of the right-hand
 // side.  Wall rows become identity rows with zero right-hand side.
+#include <algorithm>
+
 #include "fs_kernels.h"
 
 namespace fsb {
@@ -62,9 +64,12 @@ struct PhiX {  // phi with a one-layer linear extrapolation across the walls
 // those beyond a wall (the first and last lane of a row, the outer rows and
 // planes) go through the extrapolation.  The kernel is then bound by HBM and
 // L1 (phi and the velocities read, five arrays written: 36 bytes per face in
-// FP32).  Measured at 256^3, FP32, per component (x, y, z): with every sample
-// through the extrapolating accessor and seven Heavisides per face 1580, 3045,
-// 2883 us; in this form 378, 397, 441 us (128^3: 228, 383, 361 and 51, 55, 57).
+// FP32) and instruction issue: inside the box the samples are compared in the
+// storage type, so that only the faces near the interface convert them, and
+// dt / rho of a phase comes from the host.  Measured, FP32, per component (x, y,
+// z): with every sample through the extrapolating accessor and seven Heavisides
+// per face 1580, 3045, 2883 us at 256^3, in this form 292, 319, 273 us (128^3:
+// 228, 383, 361 and 53, 50, 52).
 // The component's axis is a template parameter so that every per-direction
 // array below is indexed by compile-time constants (registers, no stack).
 template <class T>
@@ -72,14 +77,26 @@ __device__ __noinline__ double phi_beyond_wall(const T* phi, const Lay& Lc, int 
   return PhiX<T>{phi, Lc}.at(i, j, k);
 }
 
+// phi > smear_limit(e) in the storage type only where phi > e
+template <class T> __device__ __forceinline__ T smear_limit(double e);
+template <> __device__ __forceinline__ double smear_limit<double>(double e) { return e; }
+template <> __device__ __forceinline__ float smear_limit<float>(double e) { return __double2float_ru(e); }
+
+template <class T, class V>
+struct ViscSystem {
+  const T *phi, *u, *v, *w;
+  Lay Lc, Lu, Lv, Lw, Lf;
+  double inv_h, dt, rn, rp, mn, mp, coef_n, coef_p;
+  V *ax, *ay, *az, *diag, *rhs;
+};
+
 template <class T, class V, int axis>
-__global__ void __launch_bounds__(256) k_visc_system(const T* __restrict__ phi, const T* __restrict__ u,
-                                                     const T* __restrict__ v, const T* __restrict__ w, Lay Lc, Lay Lu,
-                                                     Lay Lv, Lay Lw, Lay Lf, double inv_h, double dt, double rn,
-                                                     double rp, double mn, double mp, V* __restrict__ ax,
-                                                     V* __restrict__ ay, V* __restrict__ az, V* __restrict__ diag,
-                                                     V* __restrict__ rhs) {
-  FS_IJK(Lf);
+__device__ __forceinline__ void visc_face(const ViscSystem<T, V>& A, int i, int j, int k) {
+  const Lay &Lc = A.Lc, &Lu = A.Lu, &Lv = A.Lv, &Lw = A.Lw, &Lf = A.Lf;
+  const T *__restrict__ phi = A.phi, *__restrict__ u = A.u, *__restrict__ v = A.v, *__restrict__ w = A.w;
+  V *__restrict__ ax = A.ax, *__restrict__ ay = A.ay, *__restrict__ az = A.az, *__restrict__ diag = A.diag,
+    *__restrict__ rhs = A.rhs;
+  const double inv_h = A.inv_h, dt = A.dt, rn = A.rn, rp = A.rp, mn = A.mn, mp = A.mp;
   constexpr int e0 = axis == 0, e1 = axis == 1, e2 = axis == 2;
   const int64_t f = Lf.at(i, j, k);
   const int e_ax = axis == 0 ? i : (axis == 1 ? j : k);
@@ -105,34 +122,76 @@ __global__ void __launch_bounds__(256) k_visc_system(const T* __restrict__ phi, 
   };
   // the low and the high cell, and per tangential direction their two
   // neighbours (index: the direction; the axis' own entry is unused)
-  const double lo = at(-e0, -e1, -e2), hi = at(0, 0, 0);
-  double lm[3], lp[3], hm[3], hp[3];
-  bool above = lo > e && hi > e, below = lo < -e && hi < -e;  // (a NaN is neither)
+  double lo, hi, lm[3], lp[3], hm[3], hp[3];
+  int phase = 0;  // 1: all below -e, 2: all above e, 0: neither (or a NaN)
+  if (i > 0 && j > 0 && k > 0 && i < Lc.nx - 1 && j < Lc.ny - 1 && k < Lc.nz - 1) {
+    // inside the box: compared in the storage type, converted near the interface only
+    const int64_t back = e0 + e1 * sy + e2 * sz;
+    T s[10];
+    s[0] = phi[c - back];
+    s[1] = phi[c];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    if (d == axis) continue;
-    const int di = d == 0, dj = d == 1, dk = d == 2;
-    lm[d] = at(-e0 - di, -e1 - dj, -e2 - dk);
-    lp[d] = at(-e0 + di, -e1 + dj, -e2 + dk);
-    hm[d] = at(-di, -dj, -dk);
-    hp[d] = at(di, dj, dk);
-    above = above && lm[d] > e && lp[d] > e && hm[d] > e && hp[d] > e;
-    below = below && lm[d] < -e && lp[d] < -e && hm[d] < -e && hp[d] < -e;
+    for (int t = 0; t < 2; ++t) {
+      const int d = t ? (axis == 2 ? 1 : 2) : (axis == 0 ? 1 : 0);
+      const int64_t step = d == 0 ? 1 : (d == 1 ? (int64_t)sy : sz);
+      s[2 + 4 * t] = phi[c - back - step];
+      s[3 + 4 * t] = phi[c - back + step];
+      s[4 + 4 * t] = phi[c - step];
+      s[5 + 4 * t] = phi[c + step];
+    }
+    const T te = smear_limit<T>(e);
+    bool above = true, below = true;
+#pragma unroll
+    for (int q = 0; q < 10; ++q) {
+      above = above && s[q] > te;
+      below = below && s[q] < -te;
+    }
+    phase = above ? 2 : (below ? 1 : 0);
+    if (!phase) {
+      lo = (double)s[0];
+      hi = (double)s[1];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int d = t ? (axis == 2 ? 1 : 2) : (axis == 0 ? 1 : 0);
+        lm[d] = (double)s[2 + 4 * t];
+        lp[d] = (double)s[3 + 4 * t];
+        hm[d] = (double)s[4 + 4 * t];
+        hp[d] = (double)s[5 + 4 * t];
+      }
+    }
+  } else {
+    lo = at(-e0, -e1, -e2);
+    hi = at(0, 0, 0);
+    bool above = lo > e && hi > e, below = lo < -e && hi < -e;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      if (d == axis) continue;
+      const int di = d == 0, dj = d == 1, dk = d == 2;
+      lm[d] = at(-e0 - di, -e1 - dj, -e2 - dk);
+      lp[d] = at(-e0 + di, -e1 + dj, -e2 + dk);
+      hm[d] = at(-di, -dj, -dk);
+      hp[d] = at(di, dj, dk);
+      above = above && lm[d] > e && lp[d] > e && hm[d] > e && hp[d] > e;
+      below = below && lm[d] < -e && lp[d] < -e && hm[d] < -e && hp[d] < -e;
+    }
+    phase = above ? 2 : (below ? 1 : 0);
   }
   // coupling on the low arm along direction d (between this face and the
   // face one step back along d): normal arm -> the low cell, tangential arm
   // -> the edge shared by the four cells {low, high} x {d-1, d}
   double mu_low[3], mu_high[3], low[3], high[3], rho_f;
-  if (above || below) {
-    const double H = above ? 1.0 : 0.0;
-    const double mu = mn + (mp - mn) * H;
-    rho_f = rn + (rp - rn) * H;
+  double coef;  // dt / rho_f
+  if (phase) {
+    const double mu = phase == 2 ? mn + (mp - mn) : mn;
+    rho_f = phase == 2 ? rn + (rp - rn) : rn;
+    coef = phase == 2 ? A.coef_p : A.coef_n;
 #pragma unroll
     for (int d = 0; d < 3; ++d) mu_low[d] = mu_high[d] = mu;
   } else {
     auto mu_of = [&](double ph) { return mn + (mp - mn) * heaviside_visc(ph, e); };
     // density at the face from the face-averaged phi
     rho_f = rn + (rp - rn) * heaviside_visc(0.5 * (lo + hi), e);
+    coef = dt / rho_f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       if (d == axis) {
@@ -162,7 +221,6 @@ __global__ void __launch_bounds__(256) k_visc_system(const T* __restrict__ phi, 
   // direction t, d/dt( mu_edge * d(vel_t)/d(axis) ) with zero ghosts
   const T* own = axis == 0 ? u : (axis == 1 ? v : w);
   double ex = (double)own[f];
-  const double coef = dt / rho_f;
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
     if (t == axis) continue;
@@ -177,6 +235,14 @@ __global__ void __launch_bounds__(256) k_visc_system(const T* __restrict__ phi, 
     ex = ex + coef * (inv_h * (mu_high[t] * inv_h * (hi_a - hi_b) - mu_low[t] * inv_h * (lo_a - lo_b)));
   }
   rhs[f] = (V)(rho_f * ex);
+}
+
+template <class T, class V, int axis>
+__global__ void __launch_bounds__(256) k_visc_system(const __grid_constant__ ViscSystem<T, V> A, int chunk) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  if (i >= A.Lf.nx || j >= A.Lf.ny) return;
+  const int k0 = blockIdx.z * chunk, k1 = min(A.Lf.nz, k0 + chunk);
+  for (int k = k0; k < k1; ++k) visc_face<T, V, axis>(A, i, j, k);
 }
 
 // ---------------------------------------------------------------------------
@@ -343,16 +409,18 @@ void viscosity_system(const T* phi, const T* u, const T* v, const T* w, const La
                       const Lay& Lw, int axis, double dx, double dt, double rho_neg, double rho_pos, double mu_neg,
                       double mu_pos, V* ax, V* ay, V* az, V* diag, V* rhs, cudaStream_t s) {
   const Lay& Lf = axis == 0 ? Lu : (axis == 1 ? Lv : Lw);
-  Launch3 g = launch3(Lf.nx, Lf.ny, Lf.nz);
-  if (axis == 0)
-    k_visc_system<T, V, 0><<<g.grid, g.block, 0, s>>>(phi, u, v, w, Lc, Lu, Lv, Lw, Lf, 1.0 / dx, dt, rho_neg,
-                                                      rho_pos, mu_neg, mu_pos, ax, ay, az, diag, rhs);
-  else if (axis == 1)
-    k_visc_system<T, V, 1><<<g.grid, g.block, 0, s>>>(phi, u, v, w, Lc, Lu, Lv, Lw, Lf, 1.0 / dx, dt, rho_neg,
-                                                      rho_pos, mu_neg, mu_pos, ax, ay, az, diag, rhs);
-  else
-    k_visc_system<T, V, 2><<<g.grid, g.block, 0, s>>>(phi, u, v, w, Lc, Lu, Lv, Lw, Lf, 1.0 / dx, dt, rho_neg,
-                                                      rho_pos, mu_neg, mu_pos, ax, ay, az, diag, rhs);
+  const ViscSystem<T, V> A{phi,     u,       v,      w,      Lc,           Lu,
+                           Lv,      Lw,      Lf,     1.0 / dx, dt,         rho_neg,
+                           rho_pos, mu_neg,  mu_pos, dt / rho_neg, dt / (rho_neg + (rho_pos - rho_neg)),
+                           ax,      ay,      az,     diag,   rhs};
+  const unsigned bx = (Lf.nx + 31) / 32, by = (Lf.ny + 7) / 8;
+  // up to 8 planes a thread where that still leaves some 30 blocks per SM: at 256^3 405 us with one
+  // plane, 295 with 8 (block scheduling); at 128^3 52 us with one, 55 with 3
+  const int chunk = std::max(1, std::min(8, (int)((int64_t)bx * by * Lf.nz / (148 * 32))));
+  const dim3 grid(bx, by, (Lf.nz + chunk - 1) / chunk), block(32, 8, 1);
+  if (axis == 0) k_visc_system<T, V, 0><<<grid, block, 0, s>>>(A, chunk);
+  else if (axis == 1) k_visc_system<T, V, 1><<<grid, block, 0, s>>>(A, chunk);
+  else k_visc_system<T, V, 2><<<grid, block, 0, s>>>(A, chunk);
 }
 
 #define FS_VISC_INST(T, V)                                                                                          \
