@@ -41,7 +41,7 @@
 // as in the red-black solve.
 //
 // Measured (B200, CUDA events around whole calls, before: red-black IC(0)): a
-// projection of 150 x 210 x 131 cells to 1e-6 85.6 -> 5.3 ms, of 40^3 4.7 -> 1.1
+// projection of 150 x 210 x 131 cells to 1e-6 85.6 -> 5.0 ms, of 40^3 4.7 -> 1.0
 // ms; the three solves of a 256^3 rising-bubble timestep 565 -> 22 ms.
 //
 // r and z are stored by colour in the packed half layout of fs_redblack.cu
@@ -152,15 +152,30 @@ __device__ __forceinline__ float first_sweep(const Lev& v, int cl, float b, int 
   return d > 0.0f ? b / d : 0.0f;
 }
 
-struct F4 {
-  float v[4];
+// W consecutive slots or cells of a thread
+template <int W> struct FW {
+  float v[W];
 };
+using F4 = FW<4>;
 __device__ __forceinline__ F4 load4(const float* p) {
   const float4 q = *reinterpret_cast<const float4*>(p);
   return {{q.x, q.y, q.z, q.w}};
 }
 __device__ __forceinline__ void store4(float* p, const F4& a) {
   *reinterpret_cast<float4*>(p) = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
+}
+
+template <int W> __device__ __forceinline__ FW<W> loadw(const float* p) {
+  if constexpr (W == 4) return load4(p);
+  else return {{*p}};
+}
+template <int W> __device__ __forceinline__ void storew(float* p, const FW<W>& a) {
+  if constexpr (W == 4) store4(p, a);
+  else *p = a.v[0];
+}
+template <int W> __device__ __forceinline__ unsigned classes(const unsigned char* p) {  // a byte each
+  if constexpr (W == 4) return *reinterpret_cast<const unsigned*>(p);
+  else return *p;
 }
 
 // The coarse values over slots h .. h+3 (coarse cells I = h .. h+3, h a
@@ -176,8 +191,13 @@ __device__ __forceinline__ float coarse1(const Lev& e, int I, int J, int K) {
   return e.x[(I + J + K) & 1][e.H.at(I >> 1, J, K)];
 }
 
+template <int W> __device__ __forceinline__ FW<W> coarsew(const Lev& e, int h, int J, int K) {
+  if constexpr (W == 4) return coarse4(e, h, J, K);
+  else return {{coarse1(e, h, J, K)}};
+}
+
 // ---------------------------------------------------------------------------
-// Half sweep of one colour, four slots per thread.  The other colour's values
+// Half sweep of one colour, four slots per thread (W).  The other colour's values
 // in the thread's row are one vector (slot h holds the x neighbours of slots h
 // and h -+ 1) and, plane by plane, also its z neighbours: marching up, a plane
 // costs one new vector of them, the two y rows, b, one neighbouring slot and
@@ -187,6 +207,12 @@ __device__ __forceinline__ float coarse1(const Lev& e, int I, int J, int K) {
 // restriction 71 -> 48, the SpMV (likewise four cells) 77 -> 52, the update
 // 153 -> 112.
 //
+// W = 1 on grids where four would leave SMs idle (wide()): there the time is one
+// chain of loads, four times as long at the interface.  A half sweep with four and
+// with one: 48^3 5.4 -> 3.1 us, 75 x 105 x 66 8.8 -> 5.4, but on 96^3 (480 blocks with
+// four, against the rule's 444) 9.3 -> 12.9 with r.z; a restriction onto 40^3 and
+// smaller 7 -> 5.
+//
 // CORRECT: the first sweep after the coarse correction; the other colour's
 // values are read as x + e, which is all the correction has to do (the swept
 // colour's old values are not used, the other colour is swept next).  Values
@@ -194,7 +220,7 @@ __device__ __forceinline__ float coarse1(const Lev& e, int I, int J, int K) {
 // DOT: the last black (1) and red (2) sweep on the finest level also sum r.z;
 // the red one's last block adds both up and sets beta.
 // ---------------------------------------------------------------------------
-template <bool CORRECT, int DOT>
+template <int W, bool CORRECT, int DOT>
 __global__ void __launch_bounds__(kThreads) k_mg_sweep(Lev v, Lev e, int color, MgState* st, double* partials, int w,
                                                        int chunk) {
   if (stopped(st)) return;
@@ -202,7 +228,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_sweep(Lev v, Lev e, int color, 
   const Column q(w, H.ny, H.nz, chunk);
   double rz = 0.0;
   if (q.ok) {
-    const int h = 4 * q.i, j = q.j;
+    const int h = W * q.i, j = q.j;
     const float* __restrict__ xo = v.x[1 - color];
     const float* __restrict__ b = v.b[color];
     const unsigned char* __restrict__ cls = v.cls[color];
@@ -211,61 +237,61 @@ __global__ void __launch_bounds__(kThreads) k_mg_sweep(Lev v, Lev e, int color, 
     const int fyz0 = (j > 0) + (j < L.ny - 1);
     // other colour's row at plane k: x + e, zero in slots without a cell.
     // Slot m's cell of that colour is at i = 2 (h + m) + (1 - par).
-    auto correct = [&](F4& r, int par, int k) {
-      const F4 c = coarse4(e, h, j >> 1, k >> 1);
+    auto correct = [&](FW<W>& r, int par, int k) {
+      const FW<W> c = coarsew<W>(e, h, j >> 1, k >> 1);
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
+      for (int m = 0; m < W; ++m)
         if (2 * (h + m) + 1 - par < L.nx) r.v[m] += c.v[m];
     };
     const int p0 = (j + q.k0 + color) & 1;
-    F4 zm = load4(xo + s - H.slab), xc = load4(xo + s);
+    FW<W> zm = loadw<W>(xo + s - H.slab), xc = loadw<W>(xo + s);
     if (CORRECT) {
       if (q.k0 > 0) correct(zm, 1 - p0, q.k0 - 1);
       correct(xc, p0, q.k0);
     }
     for (int k = q.k0; k < q.k1; ++k, s += H.slab) {
       const int par = (j + k + color) & 1;
-      F4 zp = load4(xo + s + H.slab);
-      F4 ym = load4(xo + s - H.px), yp = load4(xo + s + H.px);
-      const F4 bv = load4(b + s);
-      const unsigned cl = *reinterpret_cast<const unsigned*>(cls + s);
-      float side = xo[par ? s + 4 : s - 1];
+      FW<W> zp = loadw<W>(xo + s + H.slab);
+      FW<W> ym = loadw<W>(xo + s - H.px), yp = loadw<W>(xo + s + H.px);
+      const FW<W> bv = loadw<W>(b + s);
+      const unsigned cl = classes<W>(cls + s);
+      float side = xo[par ? s + W : s - 1];
       if (CORRECT) {
         if (k < L.nz - 1) correct(zp, 1 - par, k + 1);
-        const F4 cm = coarse4(e, h, (j - 1) >> 1, k >> 1);
+        const FW<W> cm = coarsew<W>(e, h, (j - 1) >> 1, k >> 1);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) ym.v[m] += cm.v[m];  // (a ghost row's coarse row is a ghost too)
+        for (int m = 0; m < W; ++m) ym.v[m] += cm.v[m];  // (a ghost row's coarse row is a ghost too)
         if (j < L.ny - 1) {
-          const F4 cp = coarse4(e, h, (j + 1) >> 1, k >> 1);
+          const FW<W> cp = coarsew<W>(e, h, (j + 1) >> 1, k >> 1);
 #pragma unroll
-          for (int m = 0; m < 4; ++m) yp.v[m] += cp.v[m];
+          for (int m = 0; m < W; ++m) yp.v[m] += cp.v[m];
         }
         if (par) {
-          if (2 * (h + 4) < L.nx) side += coarse1(e, h + 4, j >> 1, k >> 1);
+          if (2 * (h + W) < L.nx) side += coarse1(e, h + W, j >> 1, k >> 1);
         } else if (h > 0) {
           side += coarse1(e, h - 1, j >> 1, k >> 1);
         }
       }
       const int fyz = fyz0 + (k > 0) + (k < L.nz - 1);
-      F4 out;
+      FW<W> out;
       const int c0 = cl & 255u;
-      if (c0 && cl == 0x01010101u * c0) {
+      if (c0 && cl == (W == 4 ? 0x01010101u : 1u) * c0) {
         const float ia = v.ia[c0];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
+        for (int m = 0; m < W; ++m) {
           const int i = 2 * (h + m) + par;
-          const float xs = par ? (m < 3 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
+          const float xs = par ? (m < W - 1 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
           // neighbours beyond a wall hold 0 and are not counted
           const float sum = fmaf(bv.v[m], ia, ((xc.v[m] + xs) + (ym.v[m] + yp.v[m])) + (zm.v[m] + zp.v[m]));
           out.v[m] = over_faces(sum, fyz + (i > 0) + (i < L.nx - 1));
         }
       } else {
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
+        for (int m = 0; m < W; ++m) {
           const int i = 2 * (h + m) + par;
           out.v[m] = 0.0f;
           if (i >= L.nx) continue;
-          const float xs = par ? (m < 3 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
+          const float xs = par ? (m < W - 1 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
           const int cm = (cl >> (8 * m)) & 255u;
           if (cm) {
             const float sum = fmaf(bv.v[m], v.ia[cm], ((xc.v[m] + xs) + (ym.v[m] + yp.v[m])) + (zm.v[m] + zp.v[m]));
@@ -280,10 +306,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_sweep(Lev v, Lev e, int color, 
           }
         }
       }
-      store4(x + s, out);
+      storew<W>(x + s, out);
       if (DOT) {
 #pragma unroll
-        for (int m = 0; m < 4; ++m) rz += (double)bv.v[m] * (double)out.v[m];
+        for (int m = 0; m < W; ++m) rz += (double)bv.v[m] * (double)out.v[m];
       }
       zm = xc;
       xc = zp;
@@ -324,25 +350,26 @@ __global__ void __launch_bounds__(kThreads) k_mg_sweep(Lev v, Lev e, int color, 
   }
 }
 
-// Residual of four slots of one row (colour `color`, the one not swept last),
+// Residual of W slots of one row (colour `color`, the one not swept last),
 // zero in slots without a cell.
-__device__ __forceinline__ F4 residual4(const Lev& v, int color, int h, int j, int k) {
-  F4 r = {{0.0f, 0.0f, 0.0f, 0.0f}};
+template <int W>
+__device__ __forceinline__ FW<W> residualw(const Lev& v, int color, int h, int j, int k) {
+  FW<W> r{};
   const Lay &L = v.L, &H = v.H;
   if (j >= L.ny || k >= L.nz) return r;
   const int par = (j + k + color) & 1;
   const int64_t s = H.at(h, j, k);
   const float* __restrict__ xo = v.x[1 - color];
-  const F4 xc = load4(xo + s), ym = load4(xo + s - H.px), yp = load4(xo + s + H.px), zm = load4(xo + s - H.slab),
-           zp = load4(xo + s + H.slab), own = load4(v.x[color] + s), b = load4(v.b[color] + s);
-  const unsigned cl = *reinterpret_cast<const unsigned*>(v.cls[color] + s);
-  const float side = xo[par ? s + 4 : s - 1];
+  const FW<W> xc = loadw<W>(xo + s), ym = loadw<W>(xo + s - H.px), yp = loadw<W>(xo + s + H.px), zm = loadw<W>(xo + s - H.slab),
+           zp = loadw<W>(xo + s + H.slab), own = loadw<W>(v.x[color] + s), b = loadw<W>(v.b[color] + s);
+  const unsigned cl = classes<W>(v.cls[color] + s);
+  const float side = xo[par ? s + W : s - 1];
   const int fyz = (j > 0) + (j < L.ny - 1) + (k > 0) + (k < L.nz - 1);
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
+  for (int m = 0; m < W; ++m) {
     const int i = 2 * (h + m) + par;
     if (i >= L.nx) continue;
-    const float xs = par ? (m < 3 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
+    const float xs = par ? (m < W - 1 ? xc.v[m + 1] : side) : (m > 0 ? xc.v[m - 1] : side);
     const float o = own.v[m];
     const int cm = (cl >> (8 * m)) & 255u;
     if (cm) {
@@ -363,30 +390,37 @@ __device__ __forceinline__ F4 residual4(const Lev& v, int color, int h, int j, i
 // Restriction: the residual of the colour that was not swept last (the other
 // one's is zero) summed over each aggregate into the coarse right-hand side,
 // and the coarse level's first red sweep.  The packed slots of coarse cell
-// (I, J, K) are (I, 2J..2J+1, 2K..2K+1): a thread takes four coarse cells.
+// (I, J, K) are (I, 2J..2J+1, 2K..2K+1): a thread takes W coarse cells.
+template <int W>
 __global__ void __launch_bounds__(kThreads) k_mg_restrict(Lev v, Lev e, int color, const MgState* st, int w,
                                                           int chunk) {
   if (stopped(st)) return;
   const Column q(w, e.L.ny, e.L.nz, chunk);
   if (!q.ok) return;
-  const int I = 4 * q.i, J = q.j;
+  const int I = W * q.i, J = q.j;
   for (int K = q.k0; K < q.k1; ++K) {
-    const F4 a = residual4(v, color, I, 2 * J, 2 * K), b = residual4(v, color, I, 2 * J + 1, 2 * K),
-             c = residual4(v, color, I, 2 * J, 2 * K + 1), d = residual4(v, color, I, 2 * J + 1, 2 * K + 1);
-    F4 r;
+    const FW<W> a = residualw<W>(v, color, I, 2 * J, 2 * K), b = residualw<W>(v, color, I, 2 * J + 1, 2 * K),
+             c = residualw<W>(v, color, I, 2 * J, 2 * K + 1), d = residualw<W>(v, color, I, 2 * J + 1, 2 * K + 1);
+    FW<W> r;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) r.v[m] = (a.v[m] + b.v[m]) + (c.v[m] + d.v[m]);
+    for (int m = 0; m < W; ++m) r.v[m] = (a.v[m] + b.v[m]) + (c.v[m] + d.v[m]);
     const int g = (J + K) & 1;  // the colour of the even coarse cells; cells past the box got 0
     const int64_t s = e.H.at(I >> 1, J, K);
-    *reinterpret_cast<float2*>(e.b[g] + s) = make_float2(r.v[0], r.v[2]);
-    *reinterpret_cast<float2*>(e.b[1 - g] + s) = make_float2(r.v[1], r.v[3]);
-    // (the cluster's levels start from zero themselves and have no classes)
-    if (e.cls[0]) {
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int Ir = I + 2 * m + g;  // red: even when g = 0, odd when g = 1
-        if (Ir < e.L.nx) e.x[0][s + m] = first_sweep(e, e.cls[0][s + m], g ? r.v[2 * m + 1] : r.v[2 * m], Ir, J, K);
+    if constexpr (W == 4) {
+      *reinterpret_cast<float2*>(e.b[g] + s) = make_float2(r.v[0], r.v[2]);
+      *reinterpret_cast<float2*>(e.b[1 - g] + s) = make_float2(r.v[1], r.v[3]);
+      // (the cluster's levels start from zero themselves and have no classes)
+      if (e.cls[0]) {
+  #pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const int Ir = I + 2 * m + g;  // red: even when g = 0, odd when g = 1
+          if (Ir < e.L.nx) e.x[0][s + m] = first_sweep(e, e.cls[0][s + m], g ? r.v[2 * m + 1] : r.v[2 * m], Ir, J, K);
+        }
       }
+    } else {
+      const int own = (I + g) & 1;
+      e.b[own][s] = r.v[0];
+      if (own == 0 && e.cls[0]) e.x[0][s] = first_sweep(e, e.cls[0][s], r.v[0], I, J, K);
     }
   }
 }
@@ -1279,16 +1313,31 @@ int mg_build(const Multigrid& M, const MgState* st, double dx, double rho_neg, d
 
 namespace {
 
+// slots of one colour per thread of a level's sweeps and restriction
+int wide(const MgLevel& m) {
+  const Columns g = columns(m.H.nx, m.H.ny, m.H.nz, 4);
+  return (int64_t)g.grid.x * g.grid.y < 3 * 148 ? 1 : 4;
+}
+template <bool CORRECT, int DOT>
+void sweep(const MgLevel& m, const MgLevel& coarse, int color, MgState* st, double* partials, cudaStream_t s) {
+  const int w = wide(m);
+  const Columns g = columns(m.H.nx, m.H.ny, m.H.nz, w);
+  auto* kernel = w == 4 ? k_mg_sweep<4, CORRECT, DOT> : k_mg_sweep<1, CORRECT, DOT>;
+  kernel<<<g.grid, kThreads, 0, s>>>(lev_of(m), lev_of(coarse), color, st, partials, g.w, g.chunk);
+}
+
 // z = M r: the V-cycle on the residual in level 0's b (x's first red sweep
 // done), and r.z with beta
 int cycle(const Multigrid& M, MgState* st, double* partials, cudaStream_t s) {
   int launches = 0;
   for (int l = 0; l < M.top; ++l) {
-    const Lev v = lev_of(M.level[l]), e = lev_of(M.level[l + 1]);
-    const Columns g = columns(v.H.nx, v.H.ny, v.H.nz, 4), ge = columns(e.L.nx, e.L.ny, e.L.nz, 4);
-    k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 1, st, partials, g.w, g.chunk);
-    k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
-    k_mg_restrict<<<ge.grid, kThreads, 0, s>>>(v, e, 1, st, ge.w, ge.chunk);
+    const MgLevel &m = M.level[l], &c = M.level[l + 1];
+    sweep<false, 0>(m, c, 1, st, partials, s);
+    sweep<false, 0>(m, c, 0, st, partials, s);
+    const int w = wide(c);
+    const Columns g = columns(c.L.nx, c.L.ny, c.L.nz, w);
+    auto* restriction = w == 4 ? k_mg_restrict<4> : k_mg_restrict<1>;
+    restriction<<<g.grid, kThreads, 0, s>>>(lev_of(m), lev_of(c), 1, st, g.w, g.chunk);
     launches += 3;
   }
   CoarseArgs A{};
@@ -1330,15 +1379,14 @@ int cycle(const Multigrid& M, MgState* st, double* partials, cudaStream_t s) {
   cudaLaunchKernelEx(&cfg, k_mg_coarse, A, (const MgState*)st);
   ++launches;
   for (int l = M.top - 1; l >= 0; --l) {
-    const Lev v = lev_of(M.level[l]), e = lev_of(M.level[l + 1]);
-    const Columns g = columns(v.H.nx, v.H.ny, v.H.nz, 4);
-    k_mg_sweep<true, 0><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+    const MgLevel &m = M.level[l], &c = M.level[l + 1];
+    sweep<true, 0>(m, c, 0, st, partials, s);
     if (l == 0) {
-      k_mg_sweep<false, 1><<<g.grid, kThreads, 0, s>>>(v, e, 1, st, partials, g.w, g.chunk);
-      k_mg_sweep<false, 2><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+      sweep<false, 1>(m, c, 1, st, partials, s);
+      sweep<false, 2>(m, c, 0, st, partials, s);
     } else {
-      k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 1, st, partials, g.w, g.chunk);
-      k_mg_sweep<false, 0><<<g.grid, kThreads, 0, s>>>(v, e, 0, st, partials, g.w, g.chunk);
+      sweep<false, 0>(m, c, 1, st, partials, s);
+      sweep<false, 0>(m, c, 0, st, partials, s);
     }
     launches += 3;
   }

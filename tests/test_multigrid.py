@@ -120,3 +120,14 @@ def test_levels_split_over_a_cluster(n):
     assert rep["rel_residual"] <= 1e-9 and rep["iterations"] <= 40
     p2 = project(n, fs.FS_PRECOND_RED_BLACK, fields, 1e-9)[1]
     assert scaled(p, p2) < 2e-5
+
+
+@pytest.mark.parametrize("n", [(88, 90, 86), (93, 91, 95), (97, 99, 98)])
+def test_slots_per_thread_on_either_side_of_the_rule(n):
+    """Finest grids whose half sweeps take one and four slots a thread (444
+    blocks of four lie between 92^3 and 96^3), with odd rows: the pressure of
+    the red-black solve, as above."""
+    fields = state(n, "sphere", 8)
+    rep, p, _ = project(n, fs.FS_PRECOND_DEFAULT, fields, 1e-9)
+    assert rep["rel_residual"] <= 1e-9 and rep["iterations"] <= 40
+    assert scaled(p, project(n, fs.FS_PRECOND_RED_BLACK, fields, 1e-9)[1]) < 2e-5
