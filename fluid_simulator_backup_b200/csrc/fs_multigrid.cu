@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_restrict(Lev v, Lev e, int colo
       *reinterpret_cast<float2*>(e.b[1 - g] + s) = make_float2(r.v[1], r.v[3]);
       // (the cluster's levels start from zero themselves and have no classes)
       if (e.cls[0]) {
-  #pragma unroll
+#pragma unroll
         for (int m = 0; m < 2; ++m) {
           const int Ir = I + 2 * m + g;  // red: even when g = 0, odd when g = 1
           if (Ir < e.L.nx) e.x[0][s + m] = first_sweep(e, e.cls[0][s + m], g ? r.v[2 * m + 1] : r.v[2 * m], Ir, J, K);
