@@ -118,6 +118,8 @@ __device__ __forceinline__ bool stop_test(const PcgState* st, double rz, double 
   }
 }
 
+// p = z + beta p.  A restart (beta = 0) does not read p: it holds whatever the
+// last solve that used the buffer left there, a NaN perhaps.
 template <class V, class RT>
 __global__ void __launch_bounds__(kRedThreads) k_pcg_pupdate(Op7<V> A, const RT* __restrict__ r, V* __restrict__ p,
                                                              PcgState* st) {
@@ -126,7 +128,8 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_pupdate(Op7<V> A, const RT*
   Cursor cur;
   for (cur.init(A.L); cur.valid(A.L); cur.next(A.L)) {
     const int64_t c = A.L.at(cur.i, cur.j, cur.k);
-    p[c] = (V)((RT)p[c] * beta + precond1<V, RT>(A, r[c], c));
+    const RT z = precond1<V, RT>(A, r[c], c);
+    p[c] = beta != RT(0) ? (V)((RT)p[c] * beta + z) : (V)z;
   }
 }
 
