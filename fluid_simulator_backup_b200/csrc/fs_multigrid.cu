@@ -1045,6 +1045,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_mg_defect(Lev v, MgState* st, d
         const float a1 = (float)r1;
         v.b[1 - par][s] = a1;
         if (par == 1) v.x[0][s] = first_sweep(v, cl.y, a1, i0 + 1, j, k);
+      } else {
+        // the slot past an odd row's end has no cell: the red-black solve, which
+        // shares these vectors, may have kept a value of its own in it
+        v.b[1 - par][s] = 0.0f;
+        if (par == 1) v.x[0][s] = 0.0f;
       }
       dn = xc;
       xc = up;

@@ -51,7 +51,7 @@ def same(a, b):
 
 
 @pytest.mark.parametrize("n,name", [((20, 22, 18), "u"), ((20, 22, 18), "phi"), ((21, 22, 20), "u"),
-                                    ((125, 126, 122), "u")])
+                                    ((21, 22, 20), "phi"), ((125, 126, 122), "u"), ((125, 126, 122), "phi")])
 def test_after_a_field_without_a_value(n, name):
     """A NaN velocity is a right-hand side of NaN (FS_OK, nothing solved), a NaN
     level set is an error (FS_NONFINITE, or FS_NOT_CONVERGED where only the FP32
@@ -101,3 +101,31 @@ def test_adjoint_after_a_field_without_a_value():
         after = adjoint(s)
     for k in bars:
         assert np.abs(after[k] - fresh[k]).max() <= 1e-4 * np.abs(fresh[k]).max(), k
+
+
+@pytest.mark.parametrize("n", [(21, 22, 20), (3, 4, 5), (93, 91, 95), (97, 99, 98)])
+def test_multigrid_after_red_black_with_odd_rows(n):
+    """An odd row's last packed slot holds a cell of one colour only; the
+    red-black solve's value there (large: velocities a thousand times the next
+    solve's, stopped after three iterations) must not enter the multigrid
+    solve's sums."""
+    fields = state(n, 4)
+    large = [fields[0]] + [1e3 * a for a in fields[1:4]] + [fields[4]]
+    with fs.Solver(n, 1.0 / n[0], **FP32) as s:
+        fresh = project(s, fields, fs.FS_PRECOND_DEFAULT)
+        project(s, large, fs.FS_PRECOND_RED_BLACK, max_iteration=3)
+        after = project(s, fields, fs.FS_PRECOND_DEFAULT, max_iteration=FP32["max_iteration"])
+    assert fresh[0] == fs.FS_OK and same(after, fresh), (after[:2], fresh[:2])
+
+
+def test_projection_after_step_adjoint_with_odd_rows():
+    n = (15, 14, 13)
+    fields = state(n, 5)
+    rng = np.random.default_rng(6)
+    with fs.Solver(n, 1.0 / n[0], **dict(FP32, reinit_iterations=2)) as s:
+        fresh = project(s, fields, fs.FS_PRECOND_DEFAULT)
+        upload(s, fields)
+        for k, a in zip(("adj_phi", "adj_u", "adj_v", "adj_w"), fields):
+            s.upload(k, 1e3 * rng.normal(size=a.shape))
+        s.step_adjoint(1e-4)
+        assert same(project(s, fields, fs.FS_PRECOND_DEFAULT), fresh)
