@@ -853,7 +853,7 @@ fs_status viscosity_t(fs_ctx* c, double dt, int* iters_out) {
 // cycle, a conditional while node whose body is one iteration, and the shift
 // of the result's constant.  The operands that change between calls are in
 // the device state, so one graph serves them all.  *st is PCG_STAGNATED when
-// the cycle gave up (x is then the best usable iterate).
+// the cycle gave up.  A solve that does not converge leaves its best iterate in x.
 template <class S>
 fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int* outer_out, double* rel_out,
                    int* st_out) {
@@ -965,13 +965,17 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
     set_error("non-finite defect residual");
     return FS_NONFINITE;
   }
-  if (m.status == PCG_MAXITER && m.rr_true > m.rr0) {
-    // the cap came before any progress: leave the better pressure
+  // the best pressure of the solve: x, where its last true residual is the smallest, else the kept one
+  const bool at_best = m.iter == m.checked && m.rr_true <= m.best;
+  if ((m.status == PCG_MAXITER || m.status == PCG_STAGNATED) && !at_best) {
     CK(cudaMemcpyAsync(x, c->p64bak, c->Lc.total * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    *rel_out = m.bb > 0 ? std::sqrt(m.rr0 / m.bb) : 0.0;
+    *rel_out = m.bb > 0 ? std::sqrt(m.best / m.bb) : 0.0;
+    if (m.status == PCG_MAXITER) {
+      mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, s);  // its constant (a stagnated solve goes on)
+      c->launches += 2;
+      CK(cudaGetLastError());
+    }
   }
-  if (m.status == PCG_STAGNATED && !(m.rr_true <= m.rr0))
-    CK(cudaMemcpyAsync(x, c->p64bak, c->Lc.total * sizeof(double), cudaMemcpyDeviceToDevice, s));
   return FS_OK;
 }
 

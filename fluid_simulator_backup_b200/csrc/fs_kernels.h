@@ -288,15 +288,16 @@ struct MgState {
   const void* phi;       // level set
   double* x;             // FP64 iterate, in and out
   const double* b;       // FP64 right-hand side
-  double* bak;           // receives the initial guess
+  double* bak;           // receives the iterate of the smallest true residual when x leaves it
   const double* bb_src;  // ||b||^2
   double tol;            // relative to ||b||
   double delta;          // reliable_delta
   int max_iter;
-  double tol2, bb, rr, rr_true, rr0, best, max_rr;  // squared norms
+  double tol2, bb, rr, rr_true, best, max_rr;  // squared norms
   double rz, alpha, beta, anchor, shift;
   int iter, done, status, pause, restart, outer, stall;
   int checked, flat;     // iteration of the last true residual; successive ones without progress
+  int save;              // x has the smallest true residual so far and bak does not hold it yet
   unsigned int ticket, batches;
 };
 int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top, int* cluster);
