@@ -848,6 +848,17 @@ fs_status viscosity_t(fs_ctx* c, double dt, int* iters_out) {
   return FS_OK;
 }
 
+// The constant of a pressure that came after mg_solve's own shift: the sum kept
+// before the cycles, restored in the x of the solve.
+fs_status mg_constant(fs_ctx* c) {
+  c->mgst_host->status = PCG_CONVERGED;  // (a stagnated state is not shifted)
+  CK(cudaMemcpyAsync(c->mgst, c->mgst_host, sizeof(MgState), cudaMemcpyHostToDevice, c->stream));
+  mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, c->stream);
+  c->launches += 2;
+  CK(cudaGetLastError());
+  return FS_OK;
+}
+
 // The multigrid-preconditioned solve of A(phi) x = b in the same precisions
 // as mixed_solve below, as ONE graph launch: the operator's set-up, the first
 // cycle, a conditional while node whose body is one iteration, and the shift
@@ -970,11 +981,7 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
   if ((m.status == PCG_MAXITER || m.status == PCG_STAGNATED) && !at_best) {
     CK(cudaMemcpyAsync(x, c->p64bak, c->Lc.total * sizeof(double), cudaMemcpyDeviceToDevice, s));
     *rel_out = m.bb > 0 ? std::sqrt(m.best / m.bb) : 0.0;
-    if (m.status == PCG_MAXITER) {
-      mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, s);  // its constant (a stagnated solve goes on)
-      c->launches += 2;
-      CK(cudaGetLastError());
-    }
+    if (m.status == PCG_MAXITER) CKS(mg_constant(c));  // (a stagnated solve goes on)
   }
   return FS_OK;
 }
@@ -997,17 +1004,22 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
   cudaStream_t s = c->stream;
   int iters = 0, outer = 0, st = 0;
   double rel = 0.0;
-  bool handed_over = false;  // from the multigrid solve
-  int mg_iters = 0, mg_outer = 0;
+  bool handed_over = false;  // from the multigrid solve, which has used up part of the cap
+  int mg_iters = 0, mg_outer = 0, cap = P.max_iteration;
   if constexpr (sizeof(S) == sizeof(float)) {
     if (c->multigrid && !transposed) {
       CKS(mg_solve<S>(c, phi, b, x, &mg_iters, &mg_outer, rel_out, st_out));
+      handed_over = *st_out == PCG_STAGNATED;
+      cap -= mg_iters;
+      if (handed_over && cap <= 0) {  // gave up at the cap: nothing is left to go on with
+        CKS(mg_constant(c));
+        *st_out = PCG_MAXITER;
+      }
       if (*st_out != PCG_STAGNATED) {
         *iters_out = mg_iters;
         *outer_out = mg_outer;
         return FS_OK;
       }
-      handed_over = true;
     }
   }
   const bool rb = c->red_black;
@@ -1091,7 +1103,7 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     PcgState init{};
     init.criterion = 2;  // absolute 2-norm of the recursive residual, in b's units
     init.tol = P.tolerance * std::sqrt(bb);
-    init.max_iter = P.max_iteration;
+    init.max_iter = cap;
     init.reliable_delta = c->reliable_delta;
     init.x = rb ? (void*)c->rb_x : (void*)x;
     init.bb = bb;  // ||b||^2 of the pressure system, for the recursive relative residual
@@ -1119,10 +1131,10 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
       } else if (rb) {
         CKS(drive_pcg(c, 4,
                       [&] { rb_iteration(R, Ah, c->rb_r, c->rb_p, c->rb_q, c->rb_tau, c->st, c->partials, s); },
-                      P.max_iteration, true, 5));
+                      cap, true, 5));
       } else {
         CKS(drive_pcg(c, 2, [&] { cg_iteration<float, double>(A, r32, p32, q32, c->st, c->partials, s); },
-                      P.max_iteration, true));
+                      cap, true));
       }
       const int status = c->st_host->status;
       iters = c->st_host->iter;
@@ -1155,7 +1167,7 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
         std::fprintf(stderr, "[fs] mixed solve%s: iteration %d, status %d, recursive %.3e, true %.3e, best %.3e%s\n",
                      rb ? " (red-black)" : "", iters, status, recursive, now, best, restart ? ", restart" : "");
       if (now <= P.tolerance) { st = PCG_CONVERGED; break; }
-      if (iters >= P.max_iteration || failures > 8 || passes > P.max_iteration + 8) {
+      if (iters >= cap || failures > 8 || passes > cap + 8) {
         // leave the best pressure found
         CK(cudaMemcpyAsync(x, c->p64bak, pbytes, cudaMemcpyDeviceToDevice, s));
         rel = best;
@@ -1172,14 +1184,7 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
     CK(cudaEventElapsedTime(&ms, c->evp0, c->evp1));
     c->pcg_ms += ms;
   }
-  if (handed_over) {
-    // the constant of the whole solve: the sum kept before the cycles
-    c->mgst_host->status = PCG_CONVERGED;
-    CK(cudaMemcpyAsync(c->mgst, c->mgst_host, sizeof(MgState), cudaMemcpyHostToDevice, s));
-    mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, s);
-    c->launches += 2;
-    CK(cudaGetLastError());
-  }
+  if (handed_over) CKS(mg_constant(c));
   *iters_out = mg_iters + iters;
   *outer_out = mg_outer + outer;
   *rel_out = rel;

@@ -53,8 +53,9 @@ def test_a_later_cap_is_never_worse(n, host_loop):
     residuals that smaller caps saw on the way (those the solve asks for by
     itself: the count of true residuals goes on by one from cap j to j + 1).
     After a hand-over the red-black solve evaluates the same residual in another
-    order, which at the floor is a matter of rounding: a factor of 3 there.
-    FP64 rounding of the residual of |p| <= 1e5 |b| dx^2 is below 1e-12 |b|."""
+    order, which at the floor (below 1e-13) is a matter of rounding: a factor of 3
+    there.  FP64 rounding of the residual of |p| <= 1e5 |b| dx^2 is below 1e-12
+    |b|.  Both solves together stay within the cap."""
     fields = state(n, 5)
     caps = range(1, 49)
     with solver(n, tolerance=1e-9, pressure_preconditioner=fs.FS_PRECOND_RED_BLACK) as s:
@@ -65,10 +66,9 @@ def test_a_later_cap_is_never_worse(n, host_loop):
     seen = np.inf
     for k in caps:
         rep, p = runs[k]
-        assert rep["status"] == fs.FS_NOT_CONVERGED
-        handed_over = rep["iterations"] != k
-        assert rel[k] <= seen * (3.0 if handed_over else 1.0 + 1e-9), (k, rel[k], seen)
-        if k + 1 in runs and not handed_over and runs[k + 1][0]["outer_iterations"] == rep["outer_iterations"] + 1:
+        assert rep["status"] == fs.FS_NOT_CONVERGED and rep["iterations"] <= k
+        assert rel[k] <= seen * (3.0 if seen < 1e-13 else 1.0 + 1e-9), (k, rel[k], seen)
+        if k + 1 in runs and runs[k + 1][0]["outer_iterations"] == rep["outer_iterations"] + 1:
             seen = min(seen, rel[k])
         if k >= 24:
             assert residual(n, fields, p) < 1e-12, k
