@@ -9,9 +9,12 @@
 // The couplings are not kept: away from the interface every face carries its
 // phase's 1/rho, and a byte per cell says which (and which faces lie on a
 // wall).  The cells next to the interface are a list of their own, worked off
-// by all threads before the rest (inline, each of a thread's 24 cells would wait
+// by all threads before the rest (inline, each of a thread's 12 cells would wait
 // for its couplings in turn: 41 us per iteration at 96^3), with their couplings
-// in shared memory as far as it reaches and in global memory beyond.
+// in shared memory as far as it reaches and in global memory beyond.  The list
+// is in the order of the cells, not in that of the warps' arrival: a listed cell
+// and one beyond the list's end round alike only as far as the compiler
+// contracts their expressions alike, and a solve has to repeat bit for bit.
 //
 // One iteration exchanges twice: p.q, then r.z with r.r.  The sums are also
 // the barrier, and every block adds them in the same order, so alpha, beta and
@@ -109,6 +112,32 @@ __device__ __forceinline__ bool exchange(double* all_sums, unsigned* count, int 
   return ok;
 }
 
+// Numbers the mixed ones of the places 0 .. n-1 in their order, by ballots over a
+// range of places per warp: put(t, e) for the e-th.  Called by all threads;
+// returns how many there are.
+template <class Mixed, class Put>
+__device__ __forceinline__ int number_mixed(int n, Mixed mixed, Put put) {
+  __shared__ int count[kT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int range = (n + kT - 1) / kT * 32, t0 = warp * range, t1 = min(n, t0 + range);
+  int own = 0;
+  for (int t = t0; t < t1; t += 32) own += __popc(__ballot_sync(0xffffffffu, t + lane < t1 && mixed(t + lane)));
+  if (lane == 0) count[warp] = own;
+  __syncthreads();
+  int e = 0, all = 0;
+  for (int w = 0; w < kT / 32; ++w) {
+    if (w < warp) e += count[w];
+    all += count[w];
+  }
+  for (int t = t0; t < t1; t += 32) {
+    const bool m = t + lane < t1 && mixed(t + lane);
+    const unsigned b = __ballot_sync(0xffffffffu, m);
+    if (m) put(t + lane, e + __popc(b & ((1u << lane) - 1u)));
+    e += __popc(b);
+  }
+  return all;
+}
+
 __device__ __forceinline__ bool brick_stop(const PcgState& s, double rz, double rr, double bb) {
   switch (s.criterion) {
     case 1: return rz < s.tol * s.tol;
@@ -154,8 +183,6 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
   unsigned short* mp = mt + A.cap;                    // its index in p
   unsigned short* me = mp + A.cap;                    // a mixed cell's entry (>= cap: not in the list)
   unsigned char* kind = (unsigned char*)(me + cells);
-  __shared__ int mixed;
-  if (tid == 0) mixed = 0;
   if (tid < 24) inv[tid] = tid % 8 && tid / 8 ? 1.0 / (A.a[tid / 8] * (double)(tid % 8)) : 0.0;
   __syncthreads();
   const PcgState par = *A.st;  // tol, criterion, max_iter
@@ -187,24 +214,24 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
                         (!(f & 16) || (ph[-L.slab] <= 0.0) == n) && (!(f & 32) || (ph[L.slab] <= 0.0) == n);
       const bool extra = base + o == A.c_extra;
       kind[t] = (unsigned char)(f | (same && !extra ? (n ? 64 : 128) : 0));
-      if (!same || extra) {
-        const int e = atomicAdd(&mixed, 1);
-        const int64_t g = base + o;
-        me[t] = (unsigned short)e;
-        if (e < A.cap) {
-          mt[e] = (unsigned short)t;
-          mp[e] = (unsigned short)pi[m];
-          mdi[e] = 1.0 / A.diag[g];
-          ma[e] = A.ax[g];
-          ma[A.cap + e] = A.ax[g + 1];
-          ma[2 * A.cap + e] = A.ay[g];
-          ma[3 * A.cap + e] = A.ay[g + L.px];
-          ma[4 * A.cap + e] = A.az[g];
-          ma[5 * A.cap + e] = A.az[g + L.slab];
-        }
-      }
     }
   }
+  __syncthreads();
+  const int listed = min(A.cap, number_mixed(cells, [&](int t) { return kind[t] < 64; }, [&](int t, int e) {
+    me[t] = (unsigned short)e;
+    if (e >= A.cap) return;
+    const int lx = t % bx, row = t / bx, ly = row % by, lz = row / by;
+    const int64_t g = base + go[t];
+    mt[e] = (unsigned short)t;
+    mp[e] = (unsigned short)((lz + 1) * sz + (ly + 1) * sy + lx + 1);
+    mdi[e] = 1.0 / A.diag[g];
+    ma[e] = A.ax[g];
+    ma[A.cap + e] = A.ax[g + 1];
+    ma[2 * A.cap + e] = A.ay[g];
+    ma[3 * A.cap + e] = A.ay[g + L.px];
+    ma[4 * A.cap + e] = A.az[g];
+    ma[5 * A.cap + e] = A.az[g + L.slab];
+  }));
   // the halo: index in p and offset in global memory of each cell inside the box
   const int fx = by * bz, fy = bx * bz, fz = bx * by;
   for (int h = tid; h < halo; h += kT) {
@@ -236,8 +263,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
   // A p of the mixed cells into mq, in flux form.  A wall's coupling is zero
   // and its halo entry of p stays finite.
   auto apply_mixed = [&]() {
-    const int n = min(mixed, A.cap);
-    for (int e = tid; e < n; e += kT) {
+    for (int e = tid; e < listed; e += kT) {
       const double* c = p + mp[e];
       const double v = c[0];
       double acc = ma[e] * (v - c[-1]) + ma[A.cap + e] * (v - c[1]);
@@ -281,7 +307,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
   auto precondition = [&](int m, double v) -> double {
     const int t = tid + m * kT, f = kind[t];
     if (f >> 6) return v * inv[(f >> 6) * 8 + __popc(f & 63)];
-    return me[t] < A.cap ? v * mdi[me[t]] : v / A.diag[base + go[t]];
+    return v * (me[t] < A.cap ? mdi[me[t]] : 1.0 / A.diag[base + go[t]]);
   };
 
   // r = b - A x, p = z (halo entries beyond a wall: 0)
@@ -543,11 +569,11 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
   unsigned short* me = (unsigned short*)(go + slots);  // a listed black cell's entry
   unsigned short* dv = me + slots;
   unsigned char* kind = (unsigned char*)(dv + slots);
-  __shared__ int nhalo, nring, nmixed;
+  __shared__ int nhalo, nring;
   const PcgState in = *A.st;
   if (in.done) return;  // the same in every block
   double* x = (double*)in.x;
-  if (tid == 0) nhalo = nring = nmixed = 0;
+  if (tid == 0) nhalo = nring = 0;
   for (int t = tid; t < padded; t += kT) kind[t] = 0;
   for (int t = tid; t < padded / 2; t += kT) PB[t] = PR[t] = 0.0f;
   __syncthreads();
@@ -579,15 +605,15 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
     const bool same = alike(0) && !(i == 0 && j == 0 && k == 0) && (!(f & 1) || alike(-1)) && (!(f & 2) || alike(1)) &&
                       (!(f & 4) || alike(-L.px)) && (!(f & 8) || alike(L.px)) && (!(f & 16) || alike(-L.slab)) &&
                       (!(f & 32) || alike(L.slab));
-    if (same) {
-      kind[t] = (unsigned char)(f | (n ? 64 : 128));
-      continue;
-    }
-    const int e = atomicAdd(&nmixed, 1);
-    if (e >= A.cap) {
-      kind[t] = kNotListed;
-      continue;
-    }
+    kind[t] = same ? (unsigned char)(f | (n ? 64 : 128)) : kNotListed;
+  }
+  __syncthreads();
+  const int mixed = number_mixed(padded, [&](int t) { return kind[t] == kNotListed; }, [&](int t, int e) {
+    if (e >= A.cap) return;
+    kind[t] = 0;
+    const int lz = t / sz - 2, ly = t % sz / sy - 2, lx = t % sy - 2;
+    const int i = i0 + lx, j = j0 + ly, k = k0 + lz;
+    const bool black = (i + j + k) & 1;
     list[e] = t | (black ? 1 << 30 : 0) | min(i, 2) << 28;
     if (black) me[(lz * by + ly) * bh + (lx >> 1)] = (unsigned short)e;
     const int64_t g = L.at(i, j, k);
@@ -597,7 +623,7 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
     ma[3 * A.cap + e] = A.ay[g + L.px];
     ma[4 * A.cap + e] = A.az[g];
     ma[5 * A.cap + e] = A.az[g + L.slab];
-  }
+  });
   // this thread's slots: index of the cell in the pair's first column, which
   // of the two is black, whether that one exists and its column
   int base[K];
@@ -625,7 +651,7 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
     }
   }
   __syncthreads();
-  const int halos = nhalo, rings = nring, listed = min(nmixed, A.cap);
+  const int halos = nhalo, rings = nring, listed = min(mixed, A.cap);
   for (int e = tid; e < halos; e += kT) PB[hp[e]] = A.p[hbase + hg[e]];
   // the first cell of the box, which carries the deflation term, where this brick needs its tau
   const int origin = i0 == 0 && j0 <= 1 && k0 <= 1 ? (2 - k0) * sz + (2 - j0) * sy + 2 : -1;
