@@ -20,8 +20,9 @@
 // the barrier, and every block adds them in the same order, so alpha, beta and
 // the decisions are the same everywhere.  The halo of p follows from p = z + beta p with the neighbours' z, which they
 // store before the second exchange; no third one is needed.  The blocks wait
-// on one another, so the launch is cooperative; every wait has a limit, after
-// which the solve ends with PCG_TIMEOUT.
+// on one another, so the launch is cooperative; every wait has a limit.  A block
+// whose wait ran out sets timed_out, whatever the others made of that exchange,
+// and leaves; the waits of those that go on then run out too.
 //
 // Measured (B200), per iteration, three kernels in a graph -> this one: 32^3
 // 17.8 -> 6.2 us, 64^3 22.9 -> 7.9, 96^3 46.9 -> 16.7, 112^3 62.8 -> 35.8.  The
@@ -37,7 +38,6 @@ namespace {
 
 constexpr int kT = 512;                    // threads of a block
 constexpr int kMaxBlocks = 256;            // one poller per block
-constexpr unsigned kSpin = 1u << 22;       // polls before a wait gives up (seconds)
 constexpr size_t kSmem = 227 * 1024 - 2048;  // dynamic shared memory of a block (static: the reductions)
 
 struct BrickArgs {
@@ -48,6 +48,7 @@ struct BrickArgs {
   double* sums;       // [2][2][kMaxBlocks]: turn, value, block
   unsigned* count;    // blocks that have stored their sums, over all turns
   int cap;            // mixed cells whose couplings fit in shared memory
+  unsigned polls;     // before a wait gives up
   PcgState* st;
   double a[3];           // uniform coupling of a phase (1: phi <= 0, 2: phi > 0)
   int64_t c_extra;       // cell that carries extra0, -1: none
@@ -60,9 +61,10 @@ struct BrickArgs {
 // read the sums and add them in the same order.  Measured with 144 blocks:
 // 1.8 us, against 4.5 us where every block polls the 144 sums themselves (the
 // polls queue in front of the stores they wait for).  `turn` counts the
-// exchanges of the solve from 1.  Returns false when a wait ran out.
-__device__ __forceinline__ bool exchange(double* all_sums, unsigned* count, int nb, unsigned turn, bool two, double& v0,
-                                         double& v1) {
+// exchanges of the solve from 1.  Returns false when this block's wait ran out
+// after `polls` polls; the others' may not have.
+__device__ __forceinline__ bool exchange(double* all_sums, unsigned* count, unsigned polls, int nb, unsigned turn,
+                                         bool two, double& v0, double& v1) {
   __shared__ double part[2][kT / 32];
   __shared__ int bad;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -87,7 +89,7 @@ __device__ __forceinline__ bool exchange(double* all_sums, unsigned* count, int 
       for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(count) : "memory");
         if ((int)(got - want) >= 0) break;
-        if (++n >= kSpin) {
+        if (++n >= polls) {
           bad = 1;
           break;
         }
@@ -339,8 +341,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
       rr += r[m] * r[m];
       bb += bv * bv;
     }
-  bool alive = exchange(A.sums, A.count, nb, ++turn, true, rz, rr);
-  alive = exchange(A.sums, A.count, nb, ++turn, false, bb, zero) && alive;
+  bool alive = exchange(A.sums, A.count, A.polls, nb, ++turn, true, rz, rr);
+  alive = exchange(A.sums, A.count, A.polls, nb, ++turn, false, bb, zero) && alive;
   int iter = 0, status = PCG_RUNNING;
   if (!alive) status = PCG_TIMEOUT;
   else if (!isfinite(rz) || !isfinite(rr)) status = PCG_NONFINITE;
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
         q[m] = apply(m);
         pq += p[pi[m]] * q[m];
       }
-    if (!exchange(A.sums, A.count, nb, ++turn, false, pq, zero)) {
+    if (!exchange(A.sums, A.count, A.polls, nb, ++turn, false, pq, zero)) {
       status = PCG_TIMEOUT;
       break;
     }
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
         rz1 += r[m] * z;
         rr1 += r[m] * r[m];
       }
-    if (!exchange(A.sums, A.count, nb, ++turn, true, rz1, rr1)) {
+    if (!exchange(A.sums, A.count, A.polls, nb, ++turn, true, rz1, rr1)) {
       status = PCG_TIMEOUT;
       break;
     }
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_brick(const __grid_constant__ Bri
     for (int m = 0; m < K; ++m)
       if (pi[m] >= 0) A.x[base + go[tid + m * kT]] = xs[tid + m * kT];
   }
+  if (tid == 0 && status == PCG_TIMEOUT) A.st->timed_out = 1;
   if (blockIdx.x == 0 && tid == 0) {
     A.st->rz = rz;
     A.st->rr = rr;
@@ -493,6 +496,7 @@ struct RbBrickArgs {
   const unsigned short* dinv;
   double* sums;
   unsigned* count;
+  unsigned polls;
   PcgState* st;
   float a[3];  // uniform coupling of a phase
   int cap;     // mixed cells listed in shared memory
@@ -709,7 +713,7 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
           q[m] = brick_schur(PB, PR, t >> 1, o, hy, hz, column, f == kNotListed ? fetched(t) : uniform(f));
         pq += (double)PB[t >> 1] * (double)q[m];
       }
-    if (!exchange(A.sums, A.count, nb, ++turn, false, pq, none)) {
+    if (!exchange(A.sums, A.count, A.polls, nb, ++turn, false, pq, none)) {
       status = PCG_TIMEOUT;
       break;
     }
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
         rz1 += (double)r[m] * (double)z;
         rr1 += (double)r[m] * (double)r[m];
       }
-    if (!exchange(A.sums, A.count, nb, ++turn, true, rz1, rr1)) {
+    if (!exchange(A.sums, A.count, A.polls, nb, ++turn, true, rz1, rr1)) {
       status = PCG_TIMEOUT;
       break;
     }
@@ -794,6 +798,7 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
       A.p[g] = PB[base[m] >> 1];
       x[g] = xs[t];
     }
+  if (tid == 0 && status == PCG_TIMEOUT) A.st->timed_out = 1;
   if (blockIdx.x == 0 && tid == 0) {
     PcgState* st = A.st;
     st->rz = rz;
@@ -905,6 +910,7 @@ cudaError_t brick_solve(const BrickPlan& P, const Op7<double>& A, const double* 
   B.zx = zx;
   B.sums = (double*)slots;
   B.count = (unsigned*)(B.sums + 4 * kMaxBlocks);
+  B.polls = P.polls;
   B.st = st;
   const double inv2 = 1.0 / (dx * dx);
   B.a[1] = (1.0 / rho_neg) * inv2;
@@ -975,6 +981,7 @@ cudaError_t rb_brick_iterate(const BrickPlan& P, const RbOp& A, const float* phi
   B.dinv = dinv;
   B.sums = (double*)slots;
   B.count = (unsigned*)(B.sums + 4 * kMaxBlocks);
+  B.polls = P.polls;
   B.st = st;
   const double inv2 = 1.0 / (dx * dx);
   B.a[1] = (float)((1.0 / rho_neg) * inv2);

@@ -588,7 +588,7 @@ fs_status run_pcg(fs_ctx* c, int key, const Op7<V>& A, const V* b, const V* x0, 
   if (c->debug)
     std::fprintf(stderr, "[fs] pcg key %d: %d iterations, status %d, rel %.3e\n", key, s.iter, s.status,
                  s.bb > 0 ? std::sqrt(s.rr / s.bb) : 0.0);
-  if (s.status == PCG_TIMEOUT) {
+  if (s.timed_out) {
     set_error("a block of the resident pressure solve did not answer (key %d, iteration %d)", key, s.iter);
     return FS_TIMEOUT;
   }
@@ -1124,7 +1124,7 @@ fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, i
         CK(cudaStreamSynchronize(s));
         c->launches += 1;
         c->pcg_launched_iterations += c->st_host->iter - iters;
-        if (c->st_host->status == PCG_TIMEOUT) {
+        if (c->st_host->timed_out) {
           set_error("a block of the resident pressure solve did not answer (iteration %d)", c->st_host->iter);
           return FS_TIMEOUT;
         }

@@ -135,13 +135,15 @@ struct PcgState {
   int x_pending;    // alpha is set and x += alpha p is still due (applied by the direction update)
   unsigned int ticket;
   unsigned int ticket2;  // completion count of the direction update
+  int timed_out;         // set by each block of a resident solve whose wait ran out
 };
 
 // STAGNATED: the iteration can make no further progress in its arithmetic
 // (p.Ap <= 0 or no improvement for stall_limit iterations); the iterate is
 // kept and the caller decides.  RELIABLE_UPDATE: paused (done = 2) for the
 // caller to replace the recursive residual by the true one.
-// TIMEOUT: a wait of the resident solve (fs_brick.cu) ran out.
+// TIMEOUT: a wait of the resident solve (fs_brick.cu) ran out; the status is the
+// first block's, timed_out every block's.
 enum { PCG_RUNNING = 0, PCG_CONVERGED = 1, PCG_MAXITER = 2, PCG_NONFINITE = 3, PCG_STAGNATED = 4,
        PCG_RELIABLE_UPDATE = 5, PCG_TIMEOUT = 6 };
 
@@ -249,6 +251,7 @@ struct BrickPlan {
   bool xg = false;             // the iterate stays in global memory
   size_t smem = 0;
   int cap = 0;                 // cells next to the interface listed in shared memory
+  unsigned polls = 1u << 22;   // of a wait before it gives up (seconds)
 };
 BrickPlan brick_plan(const Lay& L, int sms);
 size_t brick_slots_bytes();
