@@ -4,9 +4,9 @@
 //
 // What bounds it.  At 64^3 and 96^3 an iteration of three kernels (fs_krylov.cu)
 // takes 20 to 31 us, nearly all of it launches, grid-wide reductions and cold
-// starts: the vectors are a few MB.  Here one block per SM keeps a brick of the
-// box: r and q in registers, p (with a one-cell halo) and x in shared memory.
-// The couplings are not kept: away from the interface every face carries its
+// starts: the vectors are a few MB.  Here one block per SM (fewer in the smallest
+// boxes) keeps a brick of the box: r and q in registers, p (with a one-cell halo)
+// and x in shared memory.  The couplings are not kept: away from the interface every face carries its
 // phase's 1/rho, and a byte per cell says which (and which faces lie on a
 // wall).  The cells next to the interface are a list of their own, worked off
 // by all threads before the rest (inline, each of a thread's 12 cells would wait
@@ -39,6 +39,13 @@ namespace {
 constexpr int kT = 512;                    // threads of a block
 constexpr int kMaxBlocks = 256;            // one poller per block
 constexpr size_t kSmem = 227 * 1024 - 2048;  // dynamic shared memory of a block (static: the reductions)
+
+// At least this many cells per block: a box of 24^3 or less leaves most SMs to
+// the solves of other contexts.  One context does not notice (FP64 projection to
+// 1e-8, one block per SM -> so: 16^3 0.88 -> 0.79 ms, 24^3 1.19 -> 1.25, 32^3 1.53
+// -> 1.57; 1024 cells a block: 0.85, 1.37, 1.66), sixteen do (each: 16^3 0.65 ->
+// 0.12, 24^3 0.97 -> 0.23, 32^3 1.26 -> 0.65).
+constexpr int64_t kBlockCells = 512;
 
 struct BrickArgs {
   Lay L;
@@ -815,6 +822,12 @@ __global__ void __launch_bounds__(kT, 1) k_rb_brick(const __grid_constant__ RbBr
   }
 }
 
+// blocks that a box may have
+int blocks_for(const Lay& L, int sms) {
+  const int64_t cells = (int64_t)L.nx * L.ny * L.nz;
+  return (int)std::min<int64_t>(std::min(sms, kMaxBlocks), (cells + kBlockCells - 1) / kBlockCells);
+}
+
 size_t rb_brick_bytes(int bh, int by, int bz) {
   const int bx = 2 * bh;
   const size_t slots = (size_t)bh * by * bz, padded = (size_t)(bx + 4) * (by + 4) * (bz + 4);
@@ -835,13 +848,13 @@ const void* rb_kernel_of(int per_thread) {
 
 }  // namespace
 
-// The division of the box into at most `sms` bricks: the smallest largest
+// The division of the box into at most blocks_for() bricks: the smallest largest
 // brick, counting a halo cell as a third of a cell and one on an x face (a
 // strided access) as a whole one.
 BrickPlan brick_plan(const Lay& L, int sms) {
   BrickPlan best;
   double least = 1e300;
-  sms = std::min(sms, kMaxBlocks);
+  sms = blocks_for(L, sms);
   for (int gz = 1; gz <= std::min(sms, L.nz); ++gz)
     for (int gy = 1; gy <= std::min(sms / gz, L.ny); ++gy)
       for (int gx = 1; gx <= std::min(sms / gz / gy, L.nx); ++gx) {
@@ -927,7 +940,7 @@ cudaError_t brick_solve(const BrickPlan& P, const Op7<double>& A, const double* 
 BrickPlan rb_brick_plan(const Lay& L, const Lay& H, int sms) {
   BrickPlan best;
   double least = 1e300;
-  sms = std::min(sms, kMaxBlocks);
+  sms = blocks_for(L, sms);
   for (int gz = 1; gz <= std::min(sms, L.nz); ++gz)
     for (int gy = 1; gy <= std::min(sms / gz, L.ny); ++gy)
       for (int gx = 1; gx <= std::min(sms / gz / gy, H.nx); ++gx) {
