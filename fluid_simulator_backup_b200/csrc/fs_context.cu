@@ -860,11 +860,14 @@ fs_status mg_constant(fs_ctx* c) {
 }
 
 // The multigrid-preconditioned solve of A(phi) x = b in the same precisions
-// as mixed_solve below, as ONE graph launch: the operator's set-up, the first
-// cycle, a conditional while node whose body is one iteration, and the shift
-// of the result's constant.  The operands that change between calls are in
-// the device state, so one graph serves them all.  *st is PCG_STAGNATED when
-// the cycle gave up.  A solve that does not converge leaves its best iterate in x.
+// as mixed_solve below, as ONE graph launch: the operator's set-up and the guess's
+// residual, a conditional while node whose body is one iteration (none when the
+// guess meets the tolerance), and the shift of the result's constant.  (The set-up
+// in a conditional node of its own with the loop inside it would spare such a
+// guess 20 us, but costs every other solve 15 to 40.)  The operands that change
+// between calls are in the device state, so one graph serves them all.  *st is
+// PCG_STAGNATED when the cycle gave up.  A solve that does not converge leaves
+// its best iterate in x.
 template <class S>
 fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int* outer_out, double* rel_out,
                    int* st_out) {
@@ -887,7 +890,10 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
     int n = mg_build<S>(c->mg, c->mgst, dx, P.rho_neg, P.rho_pos, c->scalars + 12, s);
     rb_schur_dinv(R, c->rb_dinv, s);
     mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, false, s);
-    return n + 2 + mg_start<S>(c->mg, p, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, s);
+    return n + 2 + mg_start<S>(c->mg, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, s);
+  };
+  auto iteration = [&](bool loop, cudaGraphConditionalHandle h) {
+    return mg_iteration<S>(c->mg, p, q, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, loop, h, s);
   };
   auto finish = [&]() {
     mg_anchor(c->mg, c->rb_dinv, c->mgst, c->partials, true, s);
@@ -896,17 +902,18 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
   CK(cudaMemcpyAsync(c->mgst, c->mgst_host, sizeof(MgState), cudaMemcpyHostToDevice, s));
   CK(cudaEventRecord(c->evp0, s));
   if (c->prm.host_loop) {
-    int n = start();
-    CK(cudaMemcpyAsync(c->mgst_host, c->mgst, sizeof(MgState), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    int done = 0;
-    while (!c->mgst_host->done && done <= P.max_iteration) {
-      n += mg_iteration<S>(c->mg, p, q, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, false,
-                           cudaGraphConditionalHandle{}, s);
+    auto fetch = [&]() -> fs_status {
       CK(cudaGetLastError());
-      ++done;
       CK(cudaMemcpyAsync(c->mgst_host, c->mgst, sizeof(MgState), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
+      return FS_OK;
+    };
+    int n = start(), done = 0;
+    CKS(fetch());
+    while (!c->mgst_host->done && done <= P.max_iteration) {
+      n += iteration(false, cudaGraphConditionalHandle{});
+      ++done;
+      CKS(fetch());
     }
     n += finish();
     c->launches += n;
@@ -936,7 +943,7 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
       CK(cudaGraphAddNode(&loop, g, &last, 1, &cp));
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-      c->mg_launches[1] = mg_iteration<S>(c->mg, p, q, c->mgst, c->partials, dx, P.rho_neg, P.rho_pos, true, h, s);
+      c->mg_launches[1] = iteration(true, h);
       CK(cudaStreamEndCapture(s, &body));
       CK(cudaStreamBeginCaptureToGraph(s, g, &loop, nullptr, 1, cudaStreamCaptureModeThreadLocal));
       c->mg_launches[2] = finish();

@@ -307,14 +307,14 @@ int mg_plan(int nx, int ny, int nz, int ext[kMgMaxLevels][3], int* top, int* clu
 cudaError_t mg_prepare();
 int mg_max_blocks(const Lay& L);
 // Each returns the number of kernels launched.  mg_build: the operator of
-// every level from st->phi.  mg_start: true residual, first cycle and
-// direction.  mg_iteration: one CG iteration; with `loop` its last kernel
-// continues the graph's while node `handle`.
+// every level from st->phi.  mg_start: the true residual of the guess, which may end
+// the solve (st->done).  mg_iteration: cycle, direction and step of one CG iteration;
+// with `loop` its last kernel continues the graph's while node `handle`.
 template <class T>
 int mg_build(const Multigrid& M, const MgState* st, double dx, double rho_neg, double rho_pos, double* extra0,
              cudaStream_t s);
 template <class T>
-int mg_start(const Multigrid& M, float* p, MgState* st, double* partials, double dx, double rho_neg, double rho_pos,
+int mg_start(const Multigrid& M, MgState* st, double* partials, double dx, double rho_neg, double rho_pos,
              cudaStream_t s);
 template <class T>
 int mg_iteration(const Multigrid& M, float* p, float* q, MgState* st, double* partials, double dx, double rho_neg,

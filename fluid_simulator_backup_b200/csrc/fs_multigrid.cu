@@ -31,12 +31,14 @@
 // about 6.5 bytes per cell instead of 18, the SpMV 9 instead of 20, and the
 // FP64 residual 21 instead of 28 without a division.
 //
-// One iteration: q = A p and p.q (k_mg_spmv); x += alpha p in FP64, r -=
-// alpha q, r.r (k_mg_update); the true residual b - A x in FP64 in place of
-// r whenever the recursive one meets the tolerance or has dropped by
-// reliable_delta (k_mg_defect, which alone decides convergence); the cycle
-// z = M r, whose last two sweeps sum r.z; p = z + beta p (k_mg_direction).  All decisions
-// are taken on the device: a solve is one graph launch and one host wait.
+// One iteration: the cycle z = M r, whose last two sweeps sum r.z; p = z + beta
+// p (k_mg_direction); q = A p and p.q (k_mg_spmv); x += alpha p in FP64, r -=
+// alpha q, r.r (k_mg_update); the true residual b - A x in FP64 in place of r
+// whenever the recursive one meets the tolerance or has dropped by
+// reliable_delta (k_mg_defect, which alone decides convergence and comes last, so
+// that no cycle follows it, and none at all a guess that meets the tolerance).
+// All decisions are taken on the device: a solve is one graph launch and one host
+// wait.
 // Vectors are FP32 with FP64 sums, the iterate and the true residual FP64,
 // as in the red-black solve.
 //
@@ -1003,13 +1005,29 @@ __device__ __noinline__ double mixed_flux(const T* phi, const Lay& L, int64_t c,
   return flux;
 }
 
+// Whether the solve's loop goes on: bounded by the iteration cap whatever the
+// state says.  Called by one thread after each iteration.
+__device__ __forceinline__ void loop_next(MgState* st, cudaGraphConditionalHandle handle, bool stop) {
+  const unsigned int n = st->batches + 1u;
+  st->batches = n;
+  cudaGraphSetConditional(handle, !stop && n < (unsigned int)st->max_iter + 2u ? 1u : 0u);
+}
+
 // The true residual r = b - A x in FP64 (A from phi in FP64), its norm, the
 // first red half sweep, and the decisions that rest on it.  INIT: the start
-// of a solve (unconditional; also keeps the initial guess in st->bak).
+// of a solve (unconditional; also keeps the initial guess in st->bak).  Else the
+// last kernel of an iteration: with `loop` it also continues the graph's loop.
 template <class T, bool INIT>
 __global__ void __launch_bounds__(kThreads, 3) k_mg_defect(Lev v, MgState* st, double* partials, double rn, double rp,
-                                                           double inv2, int w, int chunk) {
-  if (!INIT && (stopped(st) || !state_read(&st->pause))) return;
+                                                           double inv2, int w, int chunk, int loop,
+                                                           cudaGraphConditionalHandle handle) {
+  if (!INIT) {
+    const bool stop = stopped(st);
+    if (stop || !state_read(&st->pause)) {
+      if (loop && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) loop_next(st, handle, stop);
+      return;
+    }
+  }
   const Lay &L = v.L, &H = v.H;
   const Column col(w, H.ny, H.nz, chunk);
   const T* __restrict__ phi = (const T*)st->phi;
@@ -1118,21 +1136,14 @@ __global__ void __launch_bounds__(kThreads, 3) k_mg_defect(Lev v, MgState* st, d
       st->best = tot;
       st->save = 1;
     }
+    if (!INIT && loop) loop_next(st, handle, st->done != 0);
   }
 }
 
-// p = z + beta p.  With a loop handle one thread also continues the graph's
-// loop while the solve runs (bounded by the iteration cap whatever the
-// state says).
-__global__ void __launch_bounds__(kThreads) k_mg_direction(Lev v, float* __restrict__ p, MgState* st, int w, int chunk,
-                                                           int loop, cudaGraphConditionalHandle handle) {
-  const bool stop = stopped(st);
-  if (loop && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-    const unsigned int n = st->batches + 1u;
-    st->batches = n;
-    cudaGraphSetConditional(handle, (!stop && n < (unsigned int)st->max_iter + 2u) ? 1u : 0u);
-  }
-  if (stop) return;
+// p = z + beta p
+__global__ void __launch_bounds__(kThreads) k_mg_direction(Lev v, float* __restrict__ p, const MgState* st, int w,
+                                                           int chunk) {
+  if (stopped(st)) return;
   const Lay &L = v.L, &H = v.H;
   const Column col(w, L.ny, L.nz, chunk);
   if (!col.ok) return;
@@ -1414,24 +1425,16 @@ int cycle(const Multigrid& M, MgState* st, double* partials, cudaStream_t s) {
   return launches;
 }
 
-int direction(const Multigrid& M, float* p, MgState* st, bool loop, cudaGraphConditionalHandle handle,
-              cudaStream_t s) {
-  const Lev v = lev_of(M.level[0]);
-  const Columns g = columns(v.L.nx, v.L.ny, v.L.nz, 4);
-  k_mg_direction<<<g.grid, kThreads, 0, s>>>(v, p, st, g.w, g.chunk, loop ? 1 : 0, handle);
-  return 1;
-}
-
 }  // namespace
 
 template <class T>
-int mg_start(const Multigrid& M, float* p, MgState* st, double* partials, double dx, double rho_neg, double rho_pos,
+int mg_start(const Multigrid& M, MgState* st, double* partials, double dx, double rho_neg, double rho_pos,
              cudaStream_t s) {
   const Lev v = lev_of(M.level[0]);
   const Columns g = columns(v.H.nx, v.H.ny, v.H.nz, 1);
-  k_mg_defect<T, true><<<g.grid, kThreads, 0, s>>>(v, st, partials, rho_neg, rho_pos, 1.0 / (dx * dx), g.w, g.chunk);
-  int n = 1 + cycle(M, st, partials, s);
-  return n + direction(M, p, st, false, cudaGraphConditionalHandle{}, s);
+  k_mg_defect<T, true><<<g.grid, kThreads, 0, s>>>(v, st, partials, rho_neg, rho_pos, 1.0 / (dx * dx), g.w, g.chunk, 0,
+                                                   cudaGraphConditionalHandle{});
+  return 1;
 }
 
 template <class T>
@@ -1439,12 +1442,13 @@ int mg_iteration(const Multigrid& M, float* p, float* q, MgState* st, double* pa
                  double rho_pos, bool loop, cudaGraphConditionalHandle handle, cudaStream_t s) {
   const Lev v = lev_of(M.level[0]);
   const Columns g = columns(v.L.nx, v.L.ny, v.L.nz, 4), gd = columns(v.H.nx, v.H.ny, v.H.nz, 1);
+  const int n = cycle(M, st, partials, s);
+  k_mg_direction<<<g.grid, kThreads, 0, s>>>(v, p, st, g.w, g.chunk);
   k_mg_spmv<<<g.grid, kThreads, 0, s>>>(v, p, q, st, partials, g.w, g.chunk);
   k_mg_update<<<g.grid, kThreads, 0, s>>>(v, p, q, st, partials, g.w, g.chunk);
   k_mg_defect<T, false><<<gd.grid, kThreads, 0, s>>>(v, st, partials, rho_neg, rho_pos, 1.0 / (dx * dx), gd.w,
-                                                     gd.chunk);
-  int n = 3 + cycle(M, st, partials, s);
-  return n + direction(M, p, st, loop, handle, s);
+                                                     gd.chunk, loop ? 1 : 0, handle);
+  return n + 4;
 }
 
 void mg_anchor(const Multigrid& M, const unsigned short* dinv, MgState* st, double* partials, bool after,
@@ -1463,7 +1467,7 @@ void mg_loop_start(cudaGraphConditionalHandle handle, const MgState* st, cudaStr
 }
 
 template int mg_build<float>(const Multigrid&, const MgState*, double, double, double, double*, cudaStream_t);
-template int mg_start<float>(const Multigrid&, float*, MgState*, double*, double, double, double, cudaStream_t);
+template int mg_start<float>(const Multigrid&, MgState*, double*, double, double, double, cudaStream_t);
 template int mg_iteration<float>(const Multigrid&, float*, float*, MgState*, double*, double, double, double, bool,
                                  cudaGraphConditionalHandle, cudaStream_t);
 
