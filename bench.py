@@ -548,6 +548,13 @@ def main():
             if dist is not None:
                 dist.destroy_process_group()
             return
+        from oracle import refsim
+        if not refsim.available():
+            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libfsref.so is not built (the "
+                              "reference's sources are not on the machine that built this tree)"}))
+            if dist is not None:
+                dist.destroy_process_group()
+            return
         # whole reference frames at 48^3 and 64^3 (about a minute on one host
         # thread), scaled to n^3; the steps printed are the frames run.  At
         # 32^3 the reference's PCG stalls above the matched tolerance after
