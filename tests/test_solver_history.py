@@ -129,3 +129,31 @@ def test_projection_after_step_adjoint_with_odd_rows():
             s.upload(k, 1e3 * rng.normal(size=a.shape))
         s.step_adjoint(1e-4)
         assert same(project(s, fields, fs.FS_PRECOND_DEFAULT), fresh)
+
+
+@pytest.mark.parametrize("precision", [fs.FS_PRECISION_FP64, fs.FS_PRECISION_FP32_REFINE])
+def test_resumed_step_repeats(precision, tmp_path):
+    """A step after a checkpoint, in the context that wrote it (after a step, a
+    step adjoint and a projection there) and in a fresh one that reads it: equal in
+    every bit, in a box whose resident FP64 solve has more mixed cells than its
+    list holds."""
+    n = (97, 95, 96)
+    fields = state(n, 7)
+    kw = dict(FP32, precision=precision, tolerance=1e-7, viscosity=1, reinit_iterations=2, max_iteration=20000)
+    path = str(tmp_path / "state")
+    out = []
+    with fs.Solver(n, 1.0 / n[0], **kw) as s:
+        upload(s, fields)
+        s.step(1e-4)
+        s.step_adjoint(1e-4)
+        s.write_state(path)
+        s.project(1e-4)
+        s.read_state(path)
+        s.step(1e-4)
+        out.append([s.download(k) for k in NAMES])
+    with fs.Solver(n, 1.0 / n[0], **kw) as s:
+        s.read_state(path)
+        s.step(1e-4)
+        out.append([s.download(k) for k in NAMES])
+    for k, a, b in zip(NAMES, *out):
+        assert np.array_equal(a, b), k
