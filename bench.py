@@ -44,8 +44,8 @@ BYTES_PER_UNKNOWN_PCG_FP64 = 120
 # direction update 15, at about half the iterations
 BYTES_PER_CELL_PCG_RB = 38
 # multigrid-preconditioned CG (per cell): spmv 9 (p, class read; q write) + update 35 (FP64 x and FP32 r read and
-# written, p, q, class read, first half sweep written) + FP64 true residual 23 (x, b, class read; r, z write; nearly
-# every iteration takes one) + five half sweeps of 6.5 + restriction 7 + direction 12 = 119, the coarser levels 7
+# written, p, q, class read, first half sweep written) + FP64 true residual 23 (x, b, class read; r, z write; more
+# than half of the iterations take one) + five half sweeps of 6.5 + restriction 7 + direction 12 = 119, the coarser levels 7
 BYTES_PER_CELL_PCG_MG = 126
 # DRAM bytes (read + write) of one FP32 Jacobi PCG iteration at 256^3
 # measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of

@@ -6,9 +6,9 @@
 // takes 20 to 31 us, nearly all of it launches, grid-wide reductions and cold
 // starts: the vectors are a few MB.  Here one block per SM (fewer in the smallest
 // boxes) keeps a brick of the box: r and q in registers, p (with a one-cell halo)
-// and x in shared memory.  The couplings are not kept: away from the interface every face carries its
-// phase's 1/rho, and a byte per cell says which (and which faces lie on a
-// wall).  The cells next to the interface are a list of their own, worked off
+// and x in shared memory.  The couplings are not kept: away from the interface
+// every face carries its phase's 1/rho, and a byte per cell says which (and which
+// faces lie on a wall).  The cells next to the interface are a list of their own, worked off
 // by all threads before the rest (inline, each of a thread's 12 cells would wait
 // for its couplings in turn: 41 us per iteration at 96^3), with their couplings
 // in shared memory as far as it reaches and in global memory beyond.  The list
@@ -18,16 +18,17 @@
 //
 // One iteration exchanges twice: p.q, then r.z with r.r.  The sums are also
 // the barrier, and every block adds them in the same order, so alpha, beta and
-// the decisions are the same everywhere.  The halo of p follows from p = z + beta p with the neighbours' z, which they
-// store before the second exchange; no third one is needed.  The blocks wait
+// the decisions are the same everywhere.  The halo of p follows from p = z + beta
+// p with the neighbours' z, which they store before the second exchange; no third
+// one is needed.  The blocks wait
 // on one another, so the launch is cooperative; every wait has a limit.  A block
 // whose wait ran out sets timed_out, whatever the others made of that exchange,
 // and leaves; the waits of those that go on then run out too.
 //
 // Measured (B200), per iteration, three kernels in a graph -> this one: 32^3
-// 17.8 -> 6.2 us, 64^3 22.9 -> 7.9, 96^3 46.9 -> 16.7, 112^3 62.8 -> 35.8.  The
-// two exchanges take 3.7 us of it; the rest is instruction issue and latency at
-// 16 warps per SM (the registers hold r and q).
+// 17.8 -> 5.8 us, 64^3 22.9 -> 7.7, 96^3 46.9 -> 14.6, 112^3 62.8 -> 29.9.  The
+// two exchanges take 3.7 us of it (144 blocks); the rest is instruction issue and
+// latency at 16 warps per SM (the registers hold r and q).
 #include <algorithm>
 
 #include "fs_kernels.h"
@@ -492,7 +493,7 @@ const void* kernel_of(const BrickPlan& P) {
 // expressions of fs_redblack.cu and fs_krylov.cu in the same order; only the
 // sums over the grid add in another one.  Measured, a whole projection to 1e-8 with five
 // kernels per iteration -> with this one: 32^3 (120 iterations) 4.0 -> 1.5 ms,
-// 64^3 (218) 7.2 -> 2.6, 96^3 (327) 14.2 -> 5.6, 120^3 (395) 25.3 -> 14.1.
+// 64^3 (218) 7.2 -> 2.6, 96^3 (327) 14.2 -> 5.6, 120^3 (396) 25.3 -> 14.3.
 // ---------------------------------------------------------------------------
 struct RbBrickArgs {
   Lay L, H;

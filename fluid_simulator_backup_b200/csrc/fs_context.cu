@@ -999,10 +999,11 @@ fs_status mg_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int*
 // symmetric operator.  *iters, *outer, *rel and *st report the Krylov
 // iterations, the defect corrections, the final relative FP64 residual and
 // the PCG status.
-// transposed: the adjoint's solve.  It keeps the red-black iteration: the
-// density bars amplify what a solve leaves over by about 1e7 (96^3 dam break:
-// 1.1e-4 relative at tolerance 1e-11, where the multigrid solve is 5e-7 off),
-// so another iteration's remainder would move them.
+// transposed: the adjoint's solve.  It keeps the red-black iteration, although
+// the multigrid solve at the same tolerance leaves the density bars nearer to
+// their converged values (tolerance 1e-11, 96^3 dam break: 1.1e-2 and 7e-6 off
+// with red-black, 4e-5 and 2e-6 with multigrid): another iteration moves the bars
+// by what this one leaves over, a change of results.
 template <class S>
 fs_status mixed_solve(fs_ctx* c, S* phi, double* b, double* x, int* iters_out, int* outer_out, double* rel_out,
                       int* st_out, bool transposed = false) {

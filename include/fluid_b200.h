@@ -112,7 +112,7 @@ typedef struct {
   int precision;                    /* fs_precision */
   int stop;                         /* fs_stop for the pressure solve */
   double tolerance;                 /* pressure tolerance (relative divergence in FP32_REFINE) */
-  int max_iteration;                /* PCG iteration cap per solve (inner cap in FP32_REFINE) */
+  int max_iteration;                /* PCG iteration cap per solve (FP32_REFINE: of all its Krylov iterations) */
   double inner_tolerance;           /* FP32_REFINE: residual reduction one FP32 Krylov sequence is trusted
                                        for before it restarts from the FP64 residual (default 1e-3) */
   int max_outer;                    /* FP32_REFINE: unused (kept for layout); the iteration cap applies */
@@ -134,9 +134,10 @@ typedef struct {
                                        1: FP32 and summed in FP64, 2: FP32 throughout (default) */
   int verbose;                      /* 1: solver progress on stderr */
   int host_loop;                    /* 0 (default): each Krylov solve is one CUDA graph launch (a conditional while
-                                       node repeating 16-iteration batches); 1: the same kernels launched from the
-                                       host, 16 iterations between polls of the solver state (for profilers that do
-                                       not descend into conditional graph nodes) */
+                                       node repeating batches of iterations: 16, viscosity 4, multigrid 1); 1: the
+                                       same kernels launched from the host, the solver state polled after each batch
+                                       (for profilers that do not descend into conditional graph nodes).  The
+                                       resident solves of small boxes are one kernel either way */
   /* Oil/water pipe mode, the reference's oil_water_simulation with a vertical
      pipe (PIPE_OPTIONS.is_vertical): 0 (default) the air/water box with walls;
      1 a pipe along y, periodic in y with the reference's node convention (cell
@@ -317,7 +318,9 @@ fs_status fs_read_state(fs_ctx* ctx, const char* path);
 fs_status fs_adjoint_reset(fs_ctx* ctx);
 fs_status fs_adjoint_density_bars(fs_ctx* ctx, double* rho_neg_bar, double* rho_pos_bar);
 /* Whole step: ADJ_* = bars of the step's output -> bars of its input.  The
- * primal fields end in the step's OUTPUT state (the forward ran once). */
+ * primal fields end in the step's OUTPUT state (the forward ran once, in an
+ * evaluation order of its own that the gradients belong to: fs_step's fields to
+ * rounding, 2e-16 of them in FP64 and 6e-8 in FP32, not to the last bit). */
 fs_status fs_step_adjoint(fs_ctx* ctx, double dt, fs_step_report* report);
 /* Operator adjoints; the primal fields are left as they were. */
 fs_status fs_advect_levelset_adjoint(fs_ctx* ctx, double dt);  /* phi -> phi (u, v, w bars added) */
